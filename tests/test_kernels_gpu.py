@@ -108,6 +108,21 @@ def test_gemm_simt_is_true_float32_and_row_independent(dev, status):
         assert torch.equal(ops.gemm_simt(a[r:r + 1].contiguous(), b, status)[0], full[r])
 
 
+@pytest.mark.parametrize("rows,n,k", [(4, 9, 260), (5, 17, 132), (8, 16, 128), (9, 15, 68), (16, 33, 64), (17, 33, 36), (65, 40, 44),
+                                      (200, 4100, 44), (200, 4100, 37), (130, 15001, 36), (129, 9472, 20)])
+def test_gemm_simt_tiles_agree(dev, status, rows, n, k):
+    """Every tile computes an output by the same chain, so a row's bits are those of the row alone; against
+    float64 the chain's error is at most k roundings of the sum of magnitudes."""
+    from vosti_b200 import ops
+    x = torch.randn(rows, k, device=dev)
+    w = torch.randn(n, k, device=dev)
+    y = ops.gemm_simt(x, w, status)
+    for r in (0, rows // 2, rows - 1):
+        assert torch.equal(ops.gemm_simt(x[r:r + 1].contiguous(), w, status)[0], y[r])
+    bound = k * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
+    assert bool(((y.double() - x.double() @ w.double().T).abs() <= bound).all()) and status.item() == 0
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("T", [19, 150])          # few tokens: a warp per head; many: blocks streaming over tokens
 @pytest.mark.parametrize("nq,nkv,d,use_norm,use_rope", [(6, 3, 48, True, True), (4, 4, 16, False, True),
