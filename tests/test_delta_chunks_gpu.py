@@ -1,0 +1,118 @@
+"""The delta rules' long portions in chunks (csrc/delta_chunks.cu) against the recurrences in float64 and against
+the token-by-token kernels: lengths around the chunk and the line between the two ways, ragged steps with short
+requests between long ones, grouped heads, widths of the value side, decays of every kind (none, total,
+mixed), start states, and containment of a token that is not finite."""
+import pytest
+import torch
+
+from gpu_util import Harness
+from vosti_b200 import ops
+from vosti_b200.engine.batch import StepEntry
+from vosti_b200.parts import StateSpec
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+DK = 128
+
+
+def decays(kind, T, heads, gen):
+    u = torch.rand(T, heads, DK, generator=gen, dtype=torch.float64)
+    if kind == "near one":
+        return 0.98 + 0.02 * u
+    if kind == "strong":
+        return u ** 8                                  # down to underflow within a chunk
+    if kind == "none and total":
+        return (u > 0.1).double()
+    return torch.where(u > 0.5, 1 - 1e-3 * u, u * 0.3)
+
+
+def inputs(rule, T, heads, x_heads, dv, kind, gen):
+    normal = lambda *s: torch.randn(*s, generator=gen, dtype=torch.float64)
+    unit = lambda t: t / t.norm(dim=-1, keepdim=True)
+    g, v = decays(kind, T, heads, gen), normal(T, heads, dv)
+    if rule == "gated":
+        k = unit(normal(T, x_heads, DK))
+        k[1::3] = unit(k[1::3] + 4 * k[0:1])           # keys that look alike: the triangular solve matters
+        return dict(q=unit(normal(T, x_heads, DK)), k=k, v=v, beta=torch.rand(T, heads, generator=gen, dtype=torch.float64), g=g)
+    k = normal(T, heads, DK)
+    k[1::3] = k[1::3] + 4 * k[0:1]
+    b = unit(k)
+    rate = torch.rand(T, heads, DK, generator=gen, dtype=torch.float64)
+    return dict(q=normal(T, heads, DK), k=k, v=v, b=b, a=rate * b, g=g)
+
+
+def recurrence(rule, ins, S, heads):
+    """Token by token in float64; S [heads, key, value]."""
+    ins = {n: (t.float().double() if t is not None else None) for n, t in ins.items()}
+    out = []
+    wide = lambda t: t.repeat_interleave(heads // t.shape[0], 0)
+    for t in range(ins["v"].shape[0]):
+        k, q, v, g = wide(ins["k"][t]), wide(ins["q"][t]), ins["v"][t], ins["g"][t]
+        if rule == "gated":
+            S = S * g[:, :, None]
+            u = ins["beta"][t][:, None] * (v - torch.einsum("hkv,hk->hv", S, k))
+            S = S + k[:, :, None] * u[:, None, :]
+        else:
+            d = torch.einsum("hkv,hk->hv", S, ins["b"][t])
+            S = S * g[:, :, None] - ins["a"][t][:, :, None] * d[:, None, :] + k[:, :, None] * v[:, None, :]
+        out.append(torch.einsum("hkv,hk->hv", S, q))
+    return torch.stack(out), S
+
+
+def scan(rule, ins, harness, ctx, heads, x_heads, dv):
+    flat = {n: t.reshape(t.shape[0], -1).float().contiguous().to(DEV) for n, t in ins.items()}
+    state = harness.cache.layer_caches[0].state
+    if rule == "gated":
+        return ops.delta_scan(flat["q"], flat["k"], flat["v"], flat["beta"], flat["g"], state, ctx, kv_heads=x_heads, heads=heads,
+                              dk=DK, dv=dv)
+    return ops.general_delta_scan(flat["q"], flat["k"], flat["v"], flat["g"], flat["b"], flat["a"], state, ctx, heads=heads, d=DK)
+
+
+@pytest.mark.parametrize("kind", ["near one", "strong", "none and total", "mixed"])
+@pytest.mark.parametrize("rule,heads,x_heads,dv,lengths", [
+    ("gated", 2, 1, 128, (49,)), ("gated", 4, 2, 48, (64, 1, 65)), ("gated", 1, 1, 160, (48, 130, 7)), ("gated", 6, 2, 16, (300, 95)),
+    ("general", 2, 2, 128, (49,)), ("general", 1, 1, 128, (96, 48, 1, 97)), ("general", 3, 3, 128, (257, 63))])
+def test_chunks(rule, heads, x_heads, dv, lengths, kind):
+    gen = torch.Generator().manual_seed(sum(lengths) + heads)
+    T = sum(lengths)
+    ins = inputs(rule, T, heads, x_heads, dv, kind, gen)
+    starts = torch.randn(len(lengths), heads, dv, DK, generator=gen)
+    got = {}
+    for way in ("chunks", "tokens"):
+        harness = Harness([None], [StateSpec((heads * DK * dv,), torch.float32)], torch.float32, max_requests=len(lengths))
+        ctx = harness.context([StepEntry(i, [0] * n) for i, n in enumerate(lengths)])
+        assert ctx.layout["delta"]["longs"] == sum(n > ops.DELTA_SHORT for n in lengths)
+        if way == "tokens":
+            ctx.layout = {k: v for k, v in ctx.layout.items() if k != "delta"}
+        state = harness.cache.layer_caches[0].state
+        for i, slot in enumerate(ctx.host_state_slots):
+            state[slot] = starts[i].reshape(-1).to(DEV)
+        out = scan(rule, ins, harness, ctx, heads, x_heads, dv)
+        got[way] = out.cpu().double(), state[ctx.host_state_slots].cpu().double()
+    at = 0
+    for i, n in enumerate(lengths):
+        part = {name: t[at:at + n] for name, t in ins.items()}
+        want, end = recurrence(rule, part, starts[i].double().transpose(1, 2), heads)
+        rel = lambda a, b: float((a - b).norm() / b.norm())
+        for which, exact in ((0, want.reshape(n, -1)), (1, end.transpose(1, 2).reshape(-1))):
+            error = {way: rel(got[way][which][at:at + n] if which == 0 else got[way][which][i], exact) for way in got}
+            # both ways are float32 evaluations of the same sums: of the same order of rounding
+            assert error["chunks"] <= 2 * error["tokens"] + 2.0 ** -22, (i, n, which, error)
+        at += n
+
+
+@pytest.mark.parametrize("rule", ["gated", "general"])
+def test_a_token_that_is_not_finite_reaches_no_earlier_one(rule):
+    gen = torch.Generator().manual_seed(3)
+    ins = inputs(rule, 80, 1, 1, 128, "mixed", gen)
+    outs = []
+    for value in (None, float("inf"), float("nan")):
+        case = {n: t.clone() for n, t in ins.items()}
+        if value is not None:
+            for name in case:
+                case[name][45] = value
+        harness = Harness([None], [StateSpec((DK * 128,), torch.float32)], torch.float32)
+        ctx = harness.context([StepEntry("r", [0] * 80)])
+        outs.append(scan(rule, case, harness, ctx, 1, 1, 128).cpu())
+    for out in outs[1:]:
+        assert torch.equal(out[:45], outs[0][:45]) and not torch.isfinite(out[45:]).any()

@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(SCAN_THREADS)
 delta_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
                   const float* __restrict__ beta, const float* __restrict__ decay, float* __restrict__ out,
                   float* state, int64_t state_stride, const int* __restrict__ cu_q, const int* __restrict__ state_slots,
-                  int num_slots, int kv_heads, int heads, int dk, int dv) {
+                  int num_slots, int kv_heads, int heads, int dk, int dv, int most) {
   extern __shared__ __align__(16) float smem[];
   constexpr int PER_WARP = 32 / KS;             // columns of a warp
   constexpr int PAD = KS * R;                   // staged channels per token
@@ -206,6 +206,7 @@ delta_scan_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
   const int slot = state_slots[b];
   if (slot < 0 || slot >= num_slots) return;
   const int start = cu_q[b], n = cu_q[b + 1] - start;
+  if (most > 0 && n > most) return;             // a long portion: csrc/delta_chunks.cu
   const int g = h / (heads / kv_heads);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int ks = lane / PER_WARP, local = warp * PER_WARP + lane % PER_WARP, col = col0 + local;
@@ -415,7 +416,7 @@ __global__ void __launch_bounds__(SCAN_THREADS)
 general_scan_kernel(const float* __restrict__ r, const float* __restrict__ k, const float* __restrict__ v,
                     const float* __restrict__ decay, const float* __restrict__ unit, const float* __restrict__ removal,
                     float* __restrict__ out, float* state, int64_t state_stride, const int* __restrict__ cu_q,
-                    const int* __restrict__ state_slots, int num_slots, int heads, int dk, int dv) {
+                    const int* __restrict__ state_slots, int num_slots, int heads, int dk, int dv, int most) {
   extern __shared__ __align__(16) float smem[];
   constexpr int PER_WARP = 32 / KS;
   constexpr int PAD = KS * R;
@@ -429,6 +430,7 @@ general_scan_kernel(const float* __restrict__ r, const float* __restrict__ k, co
   const int slot = state_slots[b];
   if (slot < 0 || slot >= num_slots) return;
   const int start = cu_q[b], n = cu_q[b + 1] - start;
+  if (most > 0 && n > most) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int ks = lane / PER_WARP, local = warp * PER_WARP + lane % PER_WARP, col = col0 + local;
   const bool live = col < dv;
@@ -594,9 +596,10 @@ static int scan_rows(int dk) {
   return dk <= 32 ? 8 : 16;
 }
 
+// `most` > 0: requests that bring more tokens than that are left alone (the chunked kernels take them).
 VOSTI_API int vosti_delta_scan(const float* q, const float* k, const float* v, const float* beta, const float* decay,
                                float* out, float* state, int64_t state_stride, const int* cu_q, const int* state_slots,
-                               int num_slots, int requests, int kv_heads, int heads, int dk, int dv, cudaStream_t stream) {
+                               int num_slots, int requests, int kv_heads, int heads, int dk, int dv, int most, cudaStream_t stream) {
   VOSTI_REQUIRE(kv_heads > 0 && heads > 0 && heads % kv_heads == 0 && dk > 0 && dv > 0, "delta_scan: bad head sizes");
   VOSTI_REQUIRE(dk <= 256, "delta_scan: %d key channels (at most 256 are taken)", dk);
   VOSTI_REQUIRE(heads <= 65535, "delta_scan: too many heads");
@@ -624,7 +627,7 @@ VOSTI_API int vosti_delta_scan(const float* q, const float* k, const float* v, c
       configured = true;                                                                                            \
     }                                                                                                               \
     vosti_launch(delta_scan_kernel<KS, R>, grid, dim3(threads), smem, stream, q, k, v, beta, decay, out, state,    \
-                 state_stride, cu_q, state_slots, num_slots, kv_heads, heads, dk, dv);                              \
+                 state_stride, cu_q, state_slots, num_slots, kv_heads, heads, dk, dv, most);                              \
   } while (0)
 #define VOSTI_SCAN_KS(R)                                                                                            \
   switch (ks) {                                                                                                     \
@@ -673,7 +676,7 @@ VOSTI_API int vosti_general_delta_prep(const void* proj, int proj_f32, int strid
 VOSTI_API int vosti_general_delta_scan(const float* r, const float* k, const float* v, const float* decay, const float* unit,
                                        const float* removal, float* out, float* state, int64_t state_stride, const int* cu_q,
                                        const int* state_slots, int num_slots, int requests, int heads, int dk, int dv,
-                                       cudaStream_t stream) {
+                                       int most, cudaStream_t stream) {
   VOSTI_REQUIRE(heads > 0 && dk > 0 && dv > 0, "general_delta_scan: bad head sizes");
   VOSTI_REQUIRE(dk <= 256, "general_delta_scan: %d key channels (at most 256 are taken)", dk);
   VOSTI_REQUIRE(heads <= 65535, "general_delta_scan: too many heads");
@@ -700,7 +703,7 @@ VOSTI_API int vosti_general_delta_scan(const float* r, const float* k, const flo
       configured = true;                                                                                            \
     }                                                                                                               \
     vosti_launch(general_scan_kernel<KS, R>, grid, dim3(threads), smem, stream, r, k, v, decay, unit, removal, out, \
-                 state, state_stride, cu_q, state_slots, num_slots, heads, dk, dv);                                 \
+                 state, state_stride, cu_q, state_slots, num_slots, heads, dk, dv, most);                                 \
   } while (0)
 #define VOSTI_SCAN_KS(R)                                                                                            \
   switch (ks) {                                                                                                     \

@@ -27,6 +27,7 @@ def library() -> ctypes.CDLL:
     if _LIB is None:
         lib = ctypes.CDLL(str(_build.library_path()))
         lib.vosti_last_error.restype = ctypes.c_char_p
+        lib.vosti_delta_chunk_floats.restype = ctypes.c_int64
         _LIB = lib
     return _LIB
 
@@ -1645,14 +1646,54 @@ def delta_prep(proj: torch.Tensor, rates: torch.Tensor, offsets: dict, *, kv_hea
     return q, k, v, beta, decay, gate
 
 
+DELTA_CHUNK = 32     # tokens of a chunk (csrc/delta_chunks.cu)
+# Requests that bring at most this many tokens are served token by token: 0.34 us a token and layer, against some 12 us
+# and 1.2 us a chunk for the chunked kernels (16 heads of 128, one request).
+DELTA_SHORT = 48
+
+
+def delta_step_layout(q_lens):
+    """How the delta rules divide a step (registered with the step layout as "delta"): the requests that bring more than
+    DELTA_SHORT tokens are cut into chunks, the longest first, the others go token by token; with one order of
+    arithmetic asked for (set_fixed_order) all of them do."""
+    requests, firsts, longs, starts = [], [], [], []
+    if not FIXED_ORDER and max(q_lens, default=0) > DELTA_SHORT:
+        for n, i in sorted(((n, i) for i, n in enumerate(q_lens) if n > DELTA_SHORT), key=lambda e: (-e[0], e[1])):
+            longs.append(i)
+            starts.append(len(requests))
+            requests.extend([i] * -(-n // DELTA_CHUNK))
+            firsts.extend(range(0, n, DELTA_CHUNK))
+    arrays = {"chunk_request": requests, "chunk_first": firsts, "long_requests": longs, "long_chunk0": starts} if longs else {}
+    return arrays, {"chunks": len(requests), "longs": len(longs), "shorts": len(q_lens) - len(longs)}
+
+
+def _delta_chunks(ctx, x, y, decay, b, k, v, beta, out, state, x_heads: int, heads: int, dk: int, dv: int) -> int:
+    """Run the step's long portions through the chunked kernels, where they take the head sizes. Returns the most tokens a
+    request may bring to be left to the token-by-token kernel (0: it takes every request, -1: there is none left)."""
+    layout = (getattr(ctx, "layout", None) or {}).get("delta")
+    lib = library()
+    if layout is None or layout["longs"] == 0 or not lib.vosti_delta_chunk_fits(heads, dk, dv):
+        return 0
+    arrays = ctx.extras
+    scratch = torch.empty(layout["chunks"] * lib.vosti_delta_chunk_floats(heads, dv, int(b is not None)), dtype=torch.float32, device=out.device)
+    _check(lib.vosti_delta_chunks(
+        _p(x), _p(y), _p(decay), _p(b), _p(k), _p(v), _p(beta), x_heads, heads, dk, dv, _p(out), _p(state), ctypes.c_int64(state.shape[1]),
+        _p(ctx.cu_q), _p(ctx.state_slots), state.shape[0], _p(arrays["delta.chunk_request"]), _p(arrays["delta.chunk_first"]),
+        layout["chunks"], _p(arrays["delta.long_requests"]), _p(arrays["delta.long_chunk0"]), layout["longs"], _p(scratch), _stream()),
+        "delta_chunks", kernels=2)
+    return DELTA_SHORT if layout["shorts"] else -1
+
+
 def delta_scan(q, k, v, beta, decay, state: torch.Tensor, ctx, *, kv_heads: int, heads: int, dk: int, dv: int) -> torch.Tensor:
     """The recurrence over every request's tokens of this step, from and to its state slot;
     returns the read-outs, float32 [tokens, heads * dv]."""
     _contig(q, k, v, beta, decay, state)
     out = torch.empty((q.shape[0], heads * dv), dtype=torch.float32, device=q.device)
-    _check(library().vosti_delta_scan(_p(q), _p(k), _p(v), _p(beta), _p(decay), _p(out), _p(state),
-                                      ctypes.c_int64(state.shape[1]), _p(ctx.cu_q), _p(ctx.state_slots), state.shape[0],
-                                      ctx.num_requests, kv_heads, heads, dk, dv, _stream()), "delta_scan")
+    most = _delta_chunks(ctx, k, q, decay, None, None, v, beta, out, state, kv_heads, heads, dk, dv)
+    if most >= 0:
+        _check(library().vosti_delta_scan(_p(q), _p(k), _p(v), _p(beta), _p(decay), _p(out), _p(state),
+                                          ctypes.c_int64(state.shape[1]), _p(ctx.cu_q), _p(ctx.state_slots), state.shape[0],
+                                          ctx.num_requests, kv_heads, heads, dk, dv, most, _stream()), "delta_scan")
     return out
 
 
@@ -1701,9 +1742,11 @@ def general_delta_scan(r, k, v, decay, unit, removal, state: torch.Tensor, ctx, 
     state slot; returns the read-outs, float32 [tokens, heads * d]."""
     _contig(r, k, v, decay, unit, removal, state)
     out = torch.empty((r.shape[0], heads * d), dtype=torch.float32, device=r.device)
-    _check(library().vosti_general_delta_scan(_p(r), _p(k), _p(v), _p(decay), _p(unit), _p(removal), _p(out), _p(state),
-                                              ctypes.c_int64(state.shape[1]), _p(ctx.cu_q), _p(ctx.state_slots),
-                                              state.shape[0], ctx.num_requests, heads, d, d, _stream()), "general_delta_scan")
+    most = _delta_chunks(ctx, removal, r, decay, unit, k, v, None, out, state, heads, heads, d, d)
+    if most >= 0:
+        _check(library().vosti_general_delta_scan(_p(r), _p(k), _p(v), _p(decay), _p(unit), _p(removal), _p(out), _p(state),
+                                                  ctypes.c_int64(state.shape[1]), _p(ctx.cu_q), _p(ctx.state_slots),
+                                                  state.shape[0], ctx.num_requests, heads, d, d, most, _stream()), "general_delta_scan")
     return out
 
 

@@ -34,7 +34,7 @@ import torch
 from .. import ops
 from ..config.schema import ConfigError, PartSpec
 from ..weights.loader import WeightSpec
-from .base import Mixer, PositionEncoding, StateSpec, register_part
+from .base import Mixer, PositionEncoding, StateSpec, register_part, register_step_layout
 from .linear import linear, prepare_weight
 
 
@@ -136,3 +136,5 @@ class GatedDeltaRule(Mixer):
 
 
 register_part("mixer", "gated_delta", GatedDeltaRule, replace=True)
+# both delta rules cut long portions into chunks, laid out with every step
+register_step_layout("delta", ops.delta_step_layout)
