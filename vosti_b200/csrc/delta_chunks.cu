@@ -20,7 +20,7 @@
 //   delta_chunk_prepare   one block per (chunk, head), all side by side: A, Q (B, R), then one thread per key
 //                         channel (W, O1) and per value column (U, O0)
 //   delta_chunk_run       one block per (request, head, 16 value columns): the chunks one after the other; per
-//                         chunk [W; O1] S0 and the state's update, both as 8 x 8 register tiles whose summands
+//                         chunk [W; O1] S0 and the state's update, both as 8 x 4 register tiles whose summands
 //                         are spread over 8 (4) lanes
 //
 // The token-by-token kernel waits for a shared-memory read, a chain of multiply-adds and two shuffle reductions
@@ -314,12 +314,12 @@ __device__ __forceinline__ void copy16(float* dst, const float* src, bool there 
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(there ? 16 : 0) : "memory");
 }
 
-constexpr int WO_PITCH = WO + 4, S_PITCH = COLS + 4;
+constexpr int WO_PITCH = WO + 4, S_PITCH = COLS + 4, RUN_THREADS = 256;
 template <bool PAIR> constexpr int STAGE_FLOATS = DK * WO_PITCH + (PAIR ? 2 : 1) * CHUNK * (DK + S_PITCH) + DK;
 template <bool PAIR> constexpr int RUN_STAGES = PAIR ? 2 : 3;
 
 template <bool PAIR>
-__global__ void __launch_bounds__(128) delta_chunk_run_kernel(ChunkArgs a) {
+__global__ void __launch_bounds__(RUN_THREADS) delta_chunk_run_kernel(ChunkArgs a) {
   extern __shared__ __align__(16) float chunk_shared[];
   constexpr int STAGES = RUN_STAGES<PAIR>, STAGE = STAGE_FLOATS<PAIR>, ROWS = (PAIR ? 2 : 1) * CHUNK;
   float* const S = chunk_shared + STAGES * STAGE;               // [DK][S_PITCH]
@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(128) delta_chunk_run_kernel(ChunkArgs a) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t row = (int64_t)a.heads * a.dv;
   float* const state = a.state + (int64_t)slot * a.state_stride + ((int64_t)h * a.dv + col0) * DK;
-  for (int i = tid; i < COLS * DK; i += 128) S[(i % DK) * S_PITCH + i / DK] = state[i];
+  for (int i = tid; i < COLS * DK; i += RUN_THREADS) S[(i % DK) * S_PITCH + i / DK] = state[i];
 
   auto load = [&](int chunk) {
     if (chunk < chunks) {
@@ -342,14 +342,15 @@ __global__ void __launch_bounds__(128) delta_chunk_run_kernel(ChunkArgs a) {
       float* const uv = ends + ROWS * DK;
       float* const gam = uv + ROWS * S_PITCH;
       const int64_t place = (place0 + chunk) * a.heads + h;
-      for (int i = tid; i < DK * (WO / 4); i += 128) {
+      for (int i = tid; i < DK * (WO / 4); i += RUN_THREADS) {
         const int r = i / (WO / 4), c = (i % (WO / 4)) * 4;
         copy16(wo + r * WO_PITCH + c, a.wo + (place * DK + r) * WO + c);
       }
-      for (int i = tid; i < ROWS * (DK / 4); i += 128) copy16(ends + i * 4, a.ends + place * ROWS * DK + i * 4);
-      const int r = tid / (COLS / 4), c = (tid % (COLS / 4)) * 4;           // 128 threads: 32 rows of 4 words
-      copy16(uv + r * S_PITCH + c, a.us + (place * CHUNK + r) * a.dv + col0 + c);
-      if (PAIR) {
+      for (int i = tid; i < ROWS * (DK / 4); i += RUN_THREADS) copy16(ends + i * 4, a.ends + place * ROWS * DK + i * 4);
+      const int r = (tid & 127) / (COLS / 4), c = (tid % (COLS / 4)) * 4;   // 32 rows of 4 words of U, and of v
+      if (tid < 128) {
+        copy16(uv + r * S_PITCH + c, a.us + (place * CHUNK + r) * a.dv + col0 + c);
+      } else if (PAIR) {
         const int t = chunk * CHUNK + r;
         copy16(uv + (CHUNK + r) * S_PITCH + c, a.v + (start + min(t, n - 1)) * row + (int64_t)h * a.dv + col0 + c, t < n);
       }
@@ -359,10 +360,10 @@ __global__ void __launch_bounds__(128) delta_chunk_run_kernel(ChunkArgs a) {
   };
 #pragma unroll
   for (int i = 0; i < STAGES - 1; ++i) load(i);
-  // [W; O1] S: lane = 8 summands' groups x 4 tiles of 8 rows x 8 columns
-  const int kg = lane & 7, tile = warp * 4 + (lane >> 3), rt = tile >> 1, ct = tile & 1;
-  // the update: lane = 4 groups of tokens x 8 tiles of 8 key channels (4 and 4) x 8 columns
-  const int tg = lane >> 3, kt = (warp >> 1) * 8 + (lane & 7), ct2 = warp & 1;
+  // [W; O1] S: lane = 8 summands' groups x 4 tiles of 8 rows x 4 columns
+  const int kg = lane & 7, rt = warp, ct = lane >> 3;
+  // the update: lane = 4 groups of tokens x 8 tiles of 8 key channels (4 and 4) x 4 columns
+  const int tg = lane >> 3, kt = (warp >> 2) * 8 + (lane & 7), ct2 = warp & 3;
 #pragma unroll 1
   for (int chunk = 0; chunk < chunks; ++chunk) {
     load(chunk + STAGES - 1);
@@ -372,27 +373,27 @@ __global__ void __launch_bounds__(128) delta_chunk_run_kernel(ChunkArgs a) {
     const float* const gam = uv + ROWS * S_PITCH;
     // this thread's outputs are row rt * 8 + kg: a u (the first 32 rows), or an o, whose first part is out there
     const int i = (rt & 3) * 8 + kg;
-    float* const out = a.out + (start + chunk * CHUNK + i) * row + (int64_t)h * a.dv + col0 + ct * 8;
+    float* const out = a.out + (start + chunk * CHUNK + i) * row + (int64_t)h * a.dv + col0 + ct * 4;
     const bool reads = rt >= 4, writes = reads && chunk * CHUNK + i < n;
-    float4 base0 = make_float4(0.f, 0.f, 0.f, 0.f), base1 = base0;
-    if (writes) { base0 = at4(out); base1 = at4(out + 4); }
+    float4 base = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (writes) base = at4(out);
     asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 1) : "memory");
     __syncthreads();
-    float acc[8][8];
+    float acc[8][4];
 #pragma unroll
     for (int r = 0; r < 8; ++r)
 #pragma unroll
-      for (int c = 0; c < 8; ++c) acc[r][c] = 0.f;
+      for (int c = 0; c < 4; ++c) acc[r][c] = 0.f;
 #pragma unroll 2
     for (int s = 0; s < DK / 8; ++s) {
       const int k = s * 8 + kg;
       const float4 a0 = at4(wo + k * WO_PITCH + rt * 8), a1 = at4(wo + k * WO_PITCH + rt * 8 + 4);
-      const float4 s0 = at4(S + k * S_PITCH + ct * 8), s1 = at4(S + k * S_PITCH + ct * 8 + 4);
-      const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w}, sv[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+      const float4 s0 = at4(S + k * S_PITCH + ct * 4);
+      const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w}, sv[4] = {s0.x, s0.y, s0.z, s0.w};
 #pragma unroll
       for (int r = 0; r < 8; ++r)
 #pragma unroll
-        for (int c = 0; c < 8; ++c) acc[r][c] = fmaf(av[r], sv[c], acc[r][c]);
+        for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(av[r], sv[c], acc[r][c]);
     }
     // the lanes' sums meet while the rows are dealt out: half of what a lane has left goes at every step
 #pragma unroll
@@ -401,37 +402,33 @@ __global__ void __launch_bounds__(128) delta_chunk_run_kernel(ChunkArgs a) {
 #pragma unroll
       for (int r = 0; r < half; ++r)
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
+        for (int c = 0; c < 4; ++c) {
           const float keep = upper ? acc[r + half][c] : acc[r][c], give = upper ? acc[r][c] : acc[r + half][c];
           acc[r][c] = keep + __shfl_xor_sync(0xffffffffu, give, half);
         }
     }
     if (reads) {
-      if (writes) {
-        put4(out, base0.x + acc[0][0], base0.y + acc[0][1], base0.z + acc[0][2], base0.w + acc[0][3]);
-        put4(out + 4, base1.x + acc[0][4], base1.y + acc[0][5], base1.z + acc[0][6], base1.w + acc[0][7]);
-      }
+      if (writes) put4(out, base.x + acc[0][0], base.y + acc[0][1], base.z + acc[0][2], base.w + acc[0][3]);
     } else {
-      float* const u = uv + i * S_PITCH + ct * 8;
-      const float4 u0 = at4(u), u1 = at4(u + 4);
+      float* const u = uv + i * S_PITCH + ct * 4;
+      const float4 u0 = at4(u);
       put4(u, u0.x + acc[0][0], u0.y + acc[0][1], u0.z + acc[0][2], u0.w + acc[0][3]);
-      put4(u + 4, u1.x + acc[0][4], u1.y + acc[0][5], u1.z + acc[0][6], u1.w + acc[0][7]);
     }
     __syncthreads();
 #pragma unroll
     for (int r = 0; r < 8; ++r)
 #pragma unroll
-      for (int c = 0; c < 8; ++c) acc[r][c] = 0.f;
+      for (int c = 0; c < 4; ++c) acc[r][c] = 0.f;
 #pragma unroll 2
     for (int s = 0; s < ROWS / 4; ++s) {
       const int j = s * 4 + tg;
       const float4 a0 = at4(ends + j * DK + kt * 4), a1 = at4(ends + j * DK + 64 + kt * 4);
-      const float4 s0 = at4(uv + j * S_PITCH + ct2 * 8), s1 = at4(uv + j * S_PITCH + ct2 * 8 + 4);
-      const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w}, sv[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+      const float4 s0 = at4(uv + j * S_PITCH + ct2 * 4);
+      const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w}, sv[4] = {s0.x, s0.y, s0.z, s0.w};
 #pragma unroll
       for (int r = 0; r < 8; ++r)
 #pragma unroll
-        for (int c = 0; c < 8; ++c) acc[r][c] = fmaf(av[r], sv[c], acc[r][c]);
+        for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(av[r], sv[c], acc[r][c]);
     }
 #pragma unroll
     for (int half = 4; half >= 2; half >>= 1) {
@@ -439,7 +436,7 @@ __global__ void __launch_bounds__(128) delta_chunk_run_kernel(ChunkArgs a) {
 #pragma unroll
       for (int r = 0; r < half; ++r)
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
+        for (int c = 0; c < 4; ++c) {
           const float keep = upper ? acc[r + half][c] : acc[r][c], give = upper ? acc[r][c] : acc[r + half][c];
           acc[r][c] = keep + __shfl_xor_sync(0xffffffffu, give, half * 4);
         }
@@ -448,15 +445,14 @@ __global__ void __launch_bounds__(128) delta_chunk_run_kernel(ChunkArgs a) {
     for (int r = 0; r < 2; ++r) {
       const int k = (tg >> 1) * 64 + kt * 4 + (tg & 1) * 2 + r;
       const float g = gam[k];
-      float* const s = S + k * S_PITCH + ct2 * 8;
-      const float4 s0 = at4(s), s1 = at4(s + 4);
+      float* const s = S + k * S_PITCH + ct2 * 4;
+      const float4 s0 = at4(s);
       put4(s, fmaf(g, s0.x, acc[r][0]), fmaf(g, s0.y, acc[r][1]), fmaf(g, s0.z, acc[r][2]), fmaf(g, s0.w, acc[r][3]));
-      put4(s + 4, fmaf(g, s1.x, acc[r][4]), fmaf(g, s1.y, acc[r][5]), fmaf(g, s1.z, acc[r][6]), fmaf(g, s1.w, acc[r][7]));
     }
     __syncthreads();
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
-  for (int i = tid; i < COLS * DK; i += 128) state[i] = S[(i % DK) * S_PITCH + i / DK];
+  for (int i = tid; i < COLS * DK; i += RUN_THREADS) state[i] = S[(i % DK) * S_PITCH + i / DK];
 }
 
 template <bool PAIR>
@@ -472,7 +468,7 @@ int launch_chunks(const ChunkArgs& a, int chunks, int longs, cudaStream_t stream
   vosti_launch(delta_chunk_prepare_kernel<PAIR>, dim3(chunks, a.heads), dim3(256), prepare_bytes, stream, a);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) { vosti_set_error("%s", cudaGetErrorString(e)); return (int)e; }
-  vosti_launch(delta_chunk_run_kernel<PAIR>, dim3(longs, a.heads, a.dv / COLS), dim3(128), run_bytes, stream, a);
+  vosti_launch(delta_chunk_run_kernel<PAIR>, dim3(longs, a.heads, a.dv / COLS), dim3(RUN_THREADS), run_bytes, stream, a);
   VOSTI_LAUNCH_CHECK();
 }
 
