@@ -116,3 +116,66 @@ def test_a_token_that_is_not_finite_reaches_no_earlier_one(rule):
         outs.append(scan(rule, case, harness, ctx, 1, 1, 128).cpu())
     for out in outs[1:]:
         assert torch.equal(out[:45], outs[0][:45]) and not torch.isfinite(out[45:]).any()
+
+
+def near(got, want):
+    """float32 sums of at most 128 terms and elementary functions against float64: some tens of roundings."""
+    return torch.allclose(got.double().cpu(), want, rtol=64 * 2.0 ** -24, atol=64 * 2.0 ** -24)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("taps,per_head,silu", [(1, False, False), (2, True, True), (4, False, True), (4, True, False)])
+@pytest.mark.parametrize("kv,heads,lengths", [(1, 2, (1, 2, 3)), (2, 4, (5, 1, 7, 1200))])
+def test_preparation_of_wide_heads(dtype, taps, per_head, silu, kv, heads, lengths):
+    """Heads of 128 (whole words, one or four tokens a warp), portions shorter than the taps and starts from a tail."""
+    gen = torch.Generator().manual_seed(taps + heads)
+    T, D = sum(lengths), DK
+    cq, cv = kv * D, heads * D
+    cc, cd = 2 * cq + cv, heads if per_head else heads * D
+    normal = lambda *s, std=1.0: (torch.randn(*s, generator=gen) * std).to(dtype)
+    proj, rates = normal(T, cc + heads), torch.randn(T, cd + cv, generator=gen)
+    conv_w, a_log, dt_bias = normal(cc, taps, std=0.5), normal(heads, std=0.5), normal(cd)
+    size = heads * D * D + (taps - 1) * cc
+    harness = Harness([None], [StateSpec((size,), torch.float32)], torch.float32, max_requests=len(lengths))
+    ctx = harness.context([StepEntry(i, [0] * n) for i, n in enumerate(lengths)])
+    state = harness.cache.layer_caches[0].state
+    tails = torch.randn(len(lengths), taps - 1, cc, generator=gen)
+    for i, slot in enumerate(ctx.host_state_slots):
+        state[slot, heads * D * D:] = tails[i].reshape(-1).to(DEV)
+    offsets = {"q": 0, "k": cq, "v": 2 * cq, "b": cc}
+    got = ops.delta_prep(proj.to(DEV), rates.to(DEV), offsets, kv_heads=kv, heads=heads, dk=D, dv=D, taps=taps, conv_w=conv_w.to(DEV),
+                         a_log=a_log.to(DEV), dt_bias=dt_bias.to(DEV), state=state, conv_offset=heads * D * D, ctx=ctx,
+                         decay_per_head=per_head, gate_silu=silu)
+    x, r = proj.double(), rates.double()
+    rows, at = [], 0
+    for i, n in enumerate(lengths):
+        full = torch.cat([tails[i].double(), x[at:at + n, :cc]])
+        y = sum(full[j:j + n] * conv_w.double()[:, j] for j in range(taps))
+        rows.append(y * torch.sigmoid(y))
+        assert torch.equal(state[ctx.host_state_slots[i], heads * D * D:].cpu().view(taps - 1, cc).double(), full[n:])
+        at += n
+    y = torch.cat(rows)
+    unit = lambda t: (t.view(T, kv, D) / torch.sqrt((t.view(T, kv, D) ** 2).sum(-1, keepdim=True) + 1e-6)).reshape(T, cq)
+    decay = torch.exp(-torch.exp(a_log.double())[:, None] * torch.nn.functional.softplus((r[:, :cd] + dt_bias.double()).view(T, heads, -1)))
+    z = r[:, cd:]
+    want = (unit(y[:, :cq]) * D ** -0.5, unit(y[:, cq:2 * cq]), y[:, 2 * cq:], torch.sigmoid(x[:, cc:]),
+            decay.expand(T, heads, D).reshape(T, cv), z * torch.sigmoid(z) if silu else torch.sigmoid(z))
+    for name, a, b in zip("q k v beta decay gate".split(), got, want):
+        assert near(a, b), (name, float((a.double().cpu() - b).abs().max()))
+    assert harness.status.item() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_general_preparation_of_wide_heads(dtype):
+    gen = torch.Generator().manual_seed(8)
+    T, heads, D = 37, 5, DK
+    W = heads * D
+    proj, inner = torch.randn(T, 5 * W + 12, generator=gen).to(dtype), torch.randn(T, W, generator=gen)
+    w0, bias = torch.randn(W, generator=gen).to(dtype), torch.randn(W, generator=gen).to(dtype)
+    offsets = {name: i * W for i, name in enumerate(("r", "k", "v", "g", "a"))}
+    got = ops.general_delta_prep(proj.to(DEV), inner.to(DEV), offsets, heads=heads, d=D, w0=w0.to(DEV), a_bias=bias.to(DEV))
+    r, k, v, g, a = (proj.double()[:, i * W:(i + 1) * W] for i in range(5))
+    unit = (k.view(T, heads, D) / torch.sqrt((k.view(T, heads, D) ** 2).sum(-1, keepdim=True) + 1e-6)).reshape(T, W)
+    decay = torch.exp(-torch.exp(torch.tensor(-0.5, dtype=torch.float64)) * torch.sigmoid(inner.double() + w0.double()))
+    for one, want in zip(got, (r, k, v, decay, unit, torch.sigmoid(a + bias.double()) * unit, torch.sigmoid(g))):
+        assert near(one, want)
