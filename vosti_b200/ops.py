@@ -1520,6 +1520,7 @@ LATENT_SEGMENT = 256           # keys per segment when few query rows share the 
 LATENT_SPLIT_MAX_ROWS = 2048   # (token, head) rows up to which the keys are cut into segments
 LATENT_MMA_SEGMENT = 128       # the same for the tensor-core kernel, whose CTA takes 16 or 32 rows
 LATENT_MMA_SPLIT_BELOW = 296   # CTAs (two per SM) below which it cuts the keys
+LATENT_TC_ROWS = 128           # (token, head) rows of the longest portion from which the tensor-memory kernel's tiles are filled
 
 
 def latent_attend(ctx, qk: torch.Tensor, c_cache: torch.Tensor, r_cache: torch.Tensor, group, *, scale: float,
@@ -1530,7 +1531,8 @@ def latent_attend(ctx, qk: torch.Tensor, c_cache: torch.Tensor, r_cache: torch.T
     logit without key or value to every softmax denominator. Returns the weighted latents, float32
     [tokens, heads, rank]. bfloat16 with a rank of
     128, 256 or 512 and a rotated part in multiples of 32 runs on the tensor cores
-    (csrc/attention_latent_mma.cu), everything else on the CUDA cores (csrc/attention_latent.cu)."""
+    (csrc/attention_latent_mma.cu; portions whose keys it would not cut, at rank 512 with a rotated part of 64 and pages of a
+    multiple of 16, in csrc/attention_latent_tc.cu), everything else on the CUDA cores (csrc/attention_latent.cu)."""
     _contig(qk, c_cache, r_cache, sink)
     flag = _same_dtype(qk, c_cache, r_cache)
     tokens, heads = qk.shape[0], qk.shape[1]
@@ -1549,6 +1551,12 @@ def latent_attend(ctx, qk: torch.Tensor, c_cache: torch.Tensor, r_cache: torch.T
             segments = key_segments(ctx.max_kv_len, window, LATENT_MMA_SEGMENT, min(ctx.max_q_len, -(-tile // heads) + 1))
         if segments > 1:
             scratch = _workspace(qk.device, tokens * heads * segments * (rank + 2))
+        elif rows >= LATENT_TC_ROWS and scale > 0 and lib.vosti_latent_attend_tc_fits(rank, rot, group.page_size):
+            _check(lib.vosti_latent_attend_tc(
+                _p(qk), _p(c_cache), _p(r_cache), _p(out), _p(ctx.positions), _p(ctx.cu_q), _p(group.block_table),
+                group.block_table.shape[1], group.page_size, num_pages, ctx.num_requests, ctx.max_q_len, tokens, heads, rank, rot,
+                ctypes.c_float(scale), window, _p(sink), _p(ctx.status), _stream()), "latent_attend_tc")
+            return out
         _check(lib.vosti_latent_attend_mma(
             _p(qk), _p(c_cache), _p(r_cache), _p(out), _p(ctx.positions), _p(ctx.cu_q), _p(group.block_table),
             group.block_table.shape[1], group.page_size, num_pages, ctx.num_requests, ctx.max_q_len, heads, rank, rot,
