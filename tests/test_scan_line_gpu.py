@@ -1,0 +1,49 @@
+"""The selective scan's one pass over long portions (csrc/selective_scan.cu) against float64: lengths around the tile,
+single tokens beside them, channels that do not fill a block, start states, both serving types."""
+import pytest
+import torch
+
+from gpu_util import Harness
+from vosti_b200 import ops
+from vosti_b200.engine.batch import StepEntry
+from vosti_b200.parts import StateSpec
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+N = 16
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("inner,lengths", [(2048, (65,)), (2049, (64, 1, 129)), (2068, (300, 63, 128, 2))])
+def test_against_float64(dtype, inner, lengths):
+    gen = torch.Generator().manual_seed(inner)
+    normal = lambda *s, std=1.0: torch.randn(*s, generator=gen) * std
+    T = sum(lengths)
+    x, xz = normal(T, inner).to(dtype), normal(T, 2 * inner).to(dtype)
+    dtp, bc = normal(T, inner), normal(T, 2 * N)
+    bias, a_log, skip = (torch.rand(inner, generator=gen) * 7 - 6).to(dtype), normal(inner, N, std=0.5).to(dtype), normal(inner).to(dtype)
+    starts = normal(len(lengths), inner, N)
+    harness = Harness([None], [StateSpec((inner * N + 4,), torch.float32)], torch.float32, max_requests=len(lengths))
+    ctx = harness.context([StepEntry(i, [0] * n) for i, n in enumerate(lengths)])
+    state = harness.cache.layer_caches[0].state
+    for i, slot in enumerate(ctx.host_state_slots):
+        state[slot, :inner * N] = starts[i].reshape(-1).to(DEV)
+    d = lambda t: t.to(DEV)
+    assert ops.library().vosti_scan_one_pass(inner, N)
+    got = ops.scan_run(d(x), d(dtp), d(bias), d(bc), d(a_log), d(skip), d(xz), state, ctx, inner=inner, states=N)
+    at, A = 0, -torch.exp(a_log.double())
+    for i, n in enumerate(lengths):
+        S, rows = starts[i].double(), []
+        for t in range(at, at + n):
+            dt = torch.nn.functional.softplus(dtp[t].double() + bias.double())
+            S = torch.exp(dt[:, None] * A) * S + (dt * x[t].double())[:, None] * bc[t, :N].double()
+            z = xz[t, inner:].double()
+            rows.append((S @ bc[t, N:].double() + skip.double() * x[t].double()) * z * torch.sigmoid(z))
+        want, end = torch.stack(rows), S
+        have, held = got[at:at + n].double().cpu(), state[ctx.host_state_slots[i], :inner * N].double().cpu().view(inner, N)
+        # float32 throughout: n roundings of a state at most, few in the mean; the result rounded once to its type
+        rel = lambda a, b: float((a - b).norm() / b.norm())
+        assert rel(held, end) <= n ** 0.5 * 2.0 ** -22, rel(held, end)
+        assert rel(have, want) <= n ** 0.5 * 2.0 ** -22 + (2.0 ** -8 if dtype == torch.bfloat16 else 0.0), rel(have, want)
+        at += n
+    assert harness.status.item() == 0

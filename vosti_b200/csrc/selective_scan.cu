@@ -213,6 +213,10 @@ scan_tail_kernel(const T* __restrict__ xz, int64_t xz_stride, float* state, int6
 }
 
 constexpr int SCAN_CHANNELS = 32;      // channels of a block
+// Channels from which a long portion runs in one pass (scan_line_kernel): a token then costs its 68 ns however few
+// channels there are, the chunks fill the GPU from few channels. 2,048 tokens in one pass and in chunks: 142 and 173 us at
+// 2,048 channels, 143 and 114 us at 1,024.
+constexpr int SCAN_LINE_FROM = 2048;
 
 // One block runs at most `chunk` tokens of one request for 32 channels; LANES lanes share a channel
 // and lane r keeps its states r, r + LANES, ... (PER of them at most) in registers. The block first
@@ -235,7 +239,7 @@ __global__ void __launch_bounds__(SCAN_CHANNELS * LANES)
 scan_run_kernel(const T* __restrict__ x, const float* __restrict__ dtp, const void* __restrict__ dt_bias,
                 const float* __restrict__ bc, const void* __restrict__ a_log, const void* __restrict__ d_skip, int w_f32,
                 const T* __restrict__ z, int64_t z_stride, float* state, int64_t state_stride, const int* __restrict__ cu_q,
-                const int* __restrict__ state_slots, int num_slots, int inner, int N, int chunk, float* ws, float* ws_dt,
+                const int* __restrict__ state_slots, int num_slots, int inner, int N, int chunk, int most, float* ws, float* ws_dt,
                 T* __restrict__ y, unsigned* status) {
   extern __shared__ float scan_shared[];
   float* sB = scan_shared;                                   // [chunk, 2 N]: B | C of each token
@@ -247,7 +251,7 @@ scan_run_kernel(const T* __restrict__ x, const float* __restrict__ dtp, const vo
   const int b = blockIdx.y, k = blockIdx.z;
   const int first = cu_q[b], count = cu_q[b + 1] - first, slot = state_slots[b];
   const int chunks = (count + chunk - 1) / chunk;
-  if (k >= (LOCAL ? chunks - 1 : chunks)) return;
+  if (count > most || k >= (LOCAL ? chunks - 1 : chunks)) return;
   if (slot < 0 || slot >= num_slots) {
     if (threadIdx.x == 0 && k == 0) raise_fault(status, VOSTI_FAULT_SLOT_RANGE);
     return;
@@ -324,6 +328,165 @@ scan_run_kernel(const T* __restrict__ x, const float* __restrict__ dtp, const vo
   for (int i = threadIdx.x; i < tokens * SCAN_CHANNELS; i += threads) {
     const int ch = c0 + i % SCAN_CHANNELS;
     if (ch < inner) y[(int64_t)(t0 + i / SCAN_CHANNELS) * inner + ch] = from_f32<T>(sg[i]);
+  }
+}
+
+// A long portion of 16 states a channel, tokens in order in one pass. The chain from token to token is one
+// multiply-add a state; everything else of a token (its exponentials above all) is off the chain, so 32 channels
+// a block and a token every 130 cycles (68 ns) need no chunks, whose first pass computes every exponential a second
+// time. Warps 0 to 3 run the recurrence, four lanes a channel with four neighbouring states each; warps 4 to 11
+// meanwhile finish the tile before (skip, gate, store) and bring the tile after (softplus, SiLU) into the
+// other buffer. 1,499 + 549 tokens of 4,096 channels: 147 us, against 324 us of the three chunk kernels; 2,048 tokens
+// 144 against 324, 1,024 tokens beside 30 single ones 89 against 226.
+constexpr int LINE_TOKENS = 64, LINE_STATES = 16, LINE_AHEAD = 4;          // (the dealing out of sums is written for four)
+constexpr int LINE_BRING = 256, LINE_THREADS = 128 + LINE_BRING;         // threads that bring, and all of a block
+constexpr int LINE_BUFFER = LINE_TOKENS * (2 * LINE_STATES + 4 * SCAN_CHANNELS);      // B | C, x, dt, gate, read-outs
+
+template <typename T>
+__global__ void __launch_bounds__(LINE_THREADS)
+scan_line_kernel(const T* __restrict__ x, const float* __restrict__ dtp, const void* __restrict__ dt_bias,
+                 const float* __restrict__ bc, const void* __restrict__ a_log, const void* __restrict__ d_skip, int w_f32,
+                 const T* __restrict__ z, int64_t z_stride, float* state, int64_t state_stride, const int* __restrict__ cu_q,
+                 const int* __restrict__ state_slots, int num_slots, int inner, T* __restrict__ y, unsigned* status) {
+  extern __shared__ __align__(16) float scan_shared[];
+  constexpr int N = LINE_STATES, TILE = LINE_TOKENS * SCAN_CHANNELS;
+  pdl_wait();
+  pdl_launch_dependents();
+  const int b = blockIdx.y;
+  const int first = cu_q[b], count = cu_q[b + 1] - first, slot = state_slots[b];
+  if (count <= LINE_TOKENS) return;                // scan_run_kernel's
+  if (slot < 0 || slot >= num_slots) {
+    if (threadIdx.x == 0) raise_fault(status, VOSTI_FAULT_SLOT_RANGE);
+    return;
+  }
+  const int tiles = (count + LINE_TOKENS - 1) / LINE_TOKENS;
+  const int c0 = blockIdx.x * SCAN_CHANNELS;
+  const bool runs = threadIdx.x < 128;
+  const int tid = runs ? threadIdx.x : threadIdx.x - 128;
+  auto buffer = [&](int tile) { return scan_shared + (tile & 1) * LINE_BUFFER; };
+
+  // the bringing side: a thread takes one channel and every eighth token
+  const int ch = c0 + (tid & 31);
+  const bool there = ch < inner;
+  const float bias = !runs && there && dt_bias != nullptr ? load_flex(dt_bias, w_f32, ch) : 0.f;
+  const float skip = !runs && there && d_skip != nullptr ? load_flex(d_skip, w_f32, ch) : 0.f;
+  constexpr int EVERY = LINE_BRING / 32, EACH = LINE_TOKENS / EVERY, SHARE = LINE_TOKENS * 2 * N / LINE_BRING;
+  // loads first, all of them in flight (places past the end read the last token's and are dropped when stored)
+  T xv[EACH], gv[EACH];
+  float dv[EACH], bv[SHARE];
+  auto fetch = [&](int tile) {
+    const int t0 = first + tile * LINE_TOKENS, tokens = min(LINE_TOKENS, count - tile * LINE_TOKENS);
+    const int cc = there ? ch : inner - 1;
+#pragma unroll
+    for (int i = 0; i < EACH; ++i) {
+      const int64_t t = t0 + min((tid >> 5) + EVERY * i, tokens - 1);
+      xv[i] = x[t * inner + cc];
+      dv[i] = dtp[t * inner + cc];
+      gv[i] = z[t * z_stride + cc];
+    }
+#pragma unroll
+    for (int i = 0; i < SHARE; ++i) bv[i] = bc[(int64_t)t0 * 2 * N + min(tid + i * LINE_BRING, tokens * 2 * N - 1)];
+  };
+  auto put = [&](int tile) {
+    float* const sB = buffer(tile);
+    float* const sx = sB + LINE_TOKENS * 2 * N;
+    const int tokens = min(LINE_TOKENS, count - tile * LINE_TOKENS);
+#pragma unroll
+    for (int i = 0; i < SHARE; ++i) sB[tid + i * LINE_BRING] = tid + i * LINE_BRING < tokens * 2 * N ? bv[i] : 0.f;
+#pragma unroll
+    for (int i = 0; i < EACH; ++i) {
+      const int t = (tid >> 5) + EVERY * i, at = t * SCAN_CHANNELS + (tid & 31);
+      sx[at] = t < tokens ? to_f32(xv[i]) : 0.f;
+      sx[TILE + at] = t < tokens ? softplus_f(dv[i] + bias) : 0.f;             // (a step size of 0 changes nothing)
+      sx[2 * TILE + at] = silu_f(to_f32(gv[i]));
+    }
+  };
+  auto finish = [&](int tile) {
+    const float* const sx = buffer(tile) + LINE_TOKENS * 2 * N;
+    const int t0 = first + tile * LINE_TOKENS, tokens = min(LINE_TOKENS, count - tile * LINE_TOKENS);
+    for (int t = tid >> 5; t < tokens; t += EVERY) {
+      const int at = t * SCAN_CHANNELS + (tid & 31);
+      if (there) y[(int64_t)(t0 + t) * inner + ch] = from_f32<T>((sx[3 * TILE + at] + skip * sx[at]) * sx[2 * TILE + at]);
+    }
+  };
+
+  // the running side
+  const int cl = tid >> 2, r = tid & 3, c = c0 + cl;
+  const bool live = c < inner;
+  float* const S = state + (int64_t)slot * state_stride + (int64_t)(live ? c : inner - 1) * N + r * 4;
+  float s[4] = {0.f, 0.f, 0.f, 0.f}, a[4] = {0.f, 0.f, 0.f, 0.f};
+  if (runs) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      s[j] = S[j];
+      a[j] = -expf(load_flex(a_log, w_f32, (int64_t)(live ? c : inner - 1) * N + r * 4 + j));
+    }
+  } else {
+    fetch(0);
+    put(0);
+  }
+  __syncthreads();
+  for (int tile = 0; tile < tiles; ++tile) {
+    if (runs) {
+      const float* const sB = buffer(tile);
+      float* const sx = buffer(tile) + LINE_TOKENS * 2 * N;
+      const int tokens = min(LINE_TOKENS, count - tile * LINE_TOKENS);
+      // A group's operands and exponentials are made before the chain of the group before it runs (its store would hold
+      // the loads back); four tokens' sums over the four lanes meet while they are dealt out, a lane stores one.
+      struct Group { float e[LINE_AHEAD][4], in[LINE_AHEAD][4]; float4 C[LINE_AHEAD]; };
+      auto make = [&](Group& g, int i0) {
+#pragma unroll
+        for (int u = 0; u < LINE_AHEAD; ++u) {
+          const int i = i0 + u;
+          const float xc = sx[i * SCAN_CHANNELS + cl], dt = sx[TILE + i * SCAN_CHANNELS + cl];
+          const float4 B = *reinterpret_cast<const float4*>(sB + i * 2 * N + r * 4);
+          g.C[u] = *reinterpret_cast<const float4*>(sB + i * 2 * N + N + r * 4);
+          const float dx = dt * xc;
+          g.in[u][0] = dx * B.x;
+          g.in[u][1] = dx * B.y;
+          g.in[u][2] = dx * B.z;
+          g.in[u][3] = dx * B.w;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) g.e[u][j] = expf(dt * a[j]);
+        }
+      };
+      auto chain = [&](const Group& g, int i0) {
+        float part[LINE_AHEAD];
+#pragma unroll
+        for (int u = 0; u < LINE_AHEAD; ++u) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) s[j] = fmaf(g.e[u][j], s[j], g.in[u][j]);
+          part[u] = fmaf(s[3], g.C[u].w, fmaf(s[2], g.C[u].z, fmaf(s[1], g.C[u].y, s[0] * g.C[u].x)));
+        }
+        const bool upper = r & 2, odd = r & 1;
+        const float two0 = (upper ? part[2] : part[0]) + __shfl_xor_sync(0xffffffffu, upper ? part[0] : part[2], 2);
+        const float two1 = (upper ? part[3] : part[1]) + __shfl_xor_sync(0xffffffffu, upper ? part[1] : part[3], 2);
+        sx[3 * TILE + (i0 + r) * SCAN_CHANNELS + cl] = (odd ? two1 : two0) + __shfl_xor_sync(0xffffffffu, odd ? two0 : two1, 1);
+      };
+      Group even, odd;
+      make(even, 0);
+#pragma unroll 1
+      for (int i0 = 0; i0 < tokens; i0 += 2 * LINE_AHEAD) {
+        make(odd, i0 + LINE_AHEAD);
+        chain(even, i0);
+        if (i0 + 2 * LINE_AHEAD < LINE_TOKENS) make(even, i0 + 2 * LINE_AHEAD);
+        chain(odd, i0 + LINE_AHEAD);
+      }
+    } else {
+      // the same buffer: a thread puts into the places that it finished, and B | C were last read a barrier ago
+      if (tile + 1 < tiles) fetch(tile + 1);
+      if (tile > 0) finish(tile - 1);
+      if (tile + 1 < tiles) put(tile + 1);
+    }
+    __syncthreads();
+  }
+  if (runs) {
+    if (live) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) S[j] = s[j];
+    }
+  } else {
+    finish(tiles - 1);
   }
 }
 
@@ -418,32 +581,35 @@ VOSTI_API int vosti_scan_conv(const void* xz, int64_t xz_stride, const void* con
 // Tokens a block of scan_run takes (a portion longer than this is run as chunks side by side):
 // the chunk's inputs fit the shared memory every block may have without asking.
 VOSTI_API int vosti_scan_chunk(int N) { return N <= 32 ? 64 : 32; }
+// Whether long portions run in one pass, without chunks and their workspace.
+VOSTI_API int vosti_scan_one_pass(int inner, int N) { return N == LINE_STATES && inner >= SCAN_LINE_FROM; }
 
 // x [tokens, inner] (after the convolution), dtp float32 [tokens, inner], bc float32 [tokens, 2 N] = B | C,
 // z [tokens, z_stride] (its first `inner` columns), y [tokens, inner]; a_log [inner, N], dt_bias and
 // d_skip [inner] share a type. The state S [inner, N] is the start of the slot. When the longest
 // portion exceeds vosti_scan_chunk(N) tokens, ws [tokens / chunk + requests, inner, N] and ws_dt
-// [tokens / chunk + requests, inner] (float32) are needed and three kernels run instead of one.
+// [tokens / chunk + requests, inner] (float32) are needed and three kernels run instead of one, unless
+// vosti_scan_one_pass(inner, N); `shortest` says whether requests of at most a chunk are among them.
 VOSTI_API int vosti_scan_run(const void* x, const float* dtp, const void* dt_bias, const float* bc, const void* a_log,
                              const void* d_skip, int w_f32, const void* z, int64_t z_stride, float* state,
                              int64_t state_stride, const int* cu_q, const int* state_slots, int num_slots, int requests,
-                             int longest, int inner, int N, float* ws, float* ws_dt, void* y, int is_f32, unsigned* status,
+                             int longest, int shortest, int inner, int N, float* ws, float* ws_dt, void* y, int is_f32, unsigned* status,
                              cudaStream_t stream) {
   VOSTI_REQUIRE(requests >= 0 && inner > 0 && N > 0 && N <= 128 && longest >= 0, "scan_run: bad sizes inner=%d states=%d (at most 128)",
                 inner, N);
   VOSTI_REQUIRE(requests <= 65535, "scan_run: too many requests for one launch");
   if (requests == 0 || longest == 0) return VOSTI_OK;
   const int chunk = vosti_scan_chunk(N);
-  const int chunks = (longest + chunk - 1) / chunk;
+  int chunks = (longest + chunk - 1) / chunk, most = longest;
   VOSTI_REQUIRE(chunks <= 65535, "scan_run: a portion of %d tokens is too long for one launch", longest);
-  VOSTI_REQUIRE(chunks == 1 || (ws != nullptr && ws_dt != nullptr), "scan_run: a portion of several chunks needs its workspace");
+  VOSTI_REQUIRE(chunks == 1 || vosti_scan_one_pass(inner, N) || (ws != nullptr && ws_dt != nullptr), "scan_run: a portion of several chunks needs its workspace");
   const int groups = (inner + SCAN_CHANNELS - 1) / SCAN_CHANNELS;
   const size_t shared = (size_t)chunk * (2 * N + 3 * SCAN_CHANNELS) * sizeof(float);
   const int lanes = N <= 4 ? 1 : N <= 8 ? 2 : N <= 32 ? 4 : 8;       // 4 to 8 states a lane at the usual sizes
   const int per = (N + lanes - 1) / lanes <= 4 ? 4 : (N + lanes - 1) / lanes <= 8 ? 8 : 16;
 #define VOSTI_SCAN(TT, L, P, LOCAL, GRID)                                                                                       \
   vosti_launch(scan_run_kernel<TT, L, P, LOCAL>, GRID, dim3(SCAN_CHANNELS * L), shared, stream, (const TT*)x, dtp, dt_bias, bc, a_log, \
-               d_skip, w_f32, (const TT*)z, z_stride, state, state_stride, cu_q, state_slots, num_slots, inner, N, chunk, ws, \
+               d_skip, w_f32, (const TT*)z, z_stride, state, state_stride, cu_q, state_slots, num_slots, inner, N, chunk, most, ws, \
                ws_dt, (TT*)y, status)
 #define VOSTI_SCAN_SHAPE(TT, LOCAL, GRID)                                                         \
   do {                                                                                            \
@@ -454,6 +620,26 @@ VOSTI_API int vosti_scan_run(const void* x, const float* dtp, const void* dt_bia
     else if (per <= 8) VOSTI_SCAN(TT, 8, 8, LOCAL, GRID);                                         \
     else VOSTI_SCAN(TT, 8, 16, LOCAL, GRID);                                                      \
   } while (0)
+  if (chunks > 1 && vosti_scan_one_pass(inner, N)) {
+    static bool configured = false;
+    if (!configured) {
+      cudaFuncSetAttribute(scan_line_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * LINE_BUFFER * (int)sizeof(float));
+      cudaFuncSetAttribute(scan_line_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * LINE_BUFFER * (int)sizeof(float));
+      configured = true;
+    }
+    const dim3 grid(groups, requests);
+    if (is_f32)
+      vosti_launch(scan_line_kernel<float>, grid, dim3(LINE_THREADS), 2 * LINE_BUFFER * sizeof(float), stream, (const float*)x, dtp, dt_bias, bc, a_log,
+                   d_skip, w_f32, (const float*)z, z_stride, state, state_stride, cu_q, state_slots, num_slots, inner, (float*)y, status);
+    else
+      vosti_launch(scan_line_kernel<bf16>, grid, dim3(LINE_THREADS), 2 * LINE_BUFFER * sizeof(float), stream, (const bf16*)x, dtp, dt_bias, bc, a_log,
+                   d_skip, w_f32, (const bf16*)z, z_stride, state, state_stride, cu_q, state_slots, num_slots, inner, (bf16*)y, status);
+    if (shortest > LINE_TOKENS) VOSTI_LAUNCH_CHECK();
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) { vosti_set_error("%s", cudaGetErrorString(e)); return (int)e; }
+    chunks = 1;                                    // the short requests are left
+    most = LINE_TOKENS;
+  }
   if (chunks > 1) {
     const dim3 grid(groups, requests, chunks - 1);
     if (is_f32) VOSTI_SCAN_SHAPE(float, true, grid); else VOSTI_SCAN_SHAPE(bf16, true, grid);
