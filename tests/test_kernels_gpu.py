@@ -326,6 +326,31 @@ def test_gemm_tc(dev, status, tokens, features, k):
     assert status.item() == 0
 
 
+@pytest.mark.parametrize("tokens,features,k", [(129, 128, 1024), (300, 8, 4096), (2048, 128, 4096), (2048, 32, 2056), (5000, 96, 1536),
+                                               (257, 120, 12288)])
+def test_gemm_tc_of_one_feature_tile_over_many_tokens_splits(dev, status, tokens, features, k):
+    """Products of at most 128 features over many tokens take K splits; unsplit in one order of arithmetic."""
+    from vosti_b200 import ops
+    x = torch.randn(tokens, k, device=dev).bfloat16()
+    w = (torch.randn(features, k, device=dev) / math.sqrt(k)).bfloat16()
+    assert ops.library().vosti_gemm_tc_splits(tokens, features, k) > 1
+    want = x.double() @ w.double().T
+    y = ops.gemm_tc(x, w, status, out_dtype=torch.float32)
+    assert torch.allclose(y.double(), want, atol=2e-4, rtol=2e-4)
+    assert torch.equal(y, ops.gemm_tc(x, ops.PackedWeight(w), status, out_dtype=torch.float32))
+    assert torch.equal(ops.gemm_tc(x, w, status, allow_partial=True), y.bfloat16())
+    if features % 32 == 0:
+        g, u = (want.view(tokens, -1, 2, 16)[:, :, i].reshape(tokens, -1) for i in range(2))
+        assert torch.allclose(ops.gemm_tc(x, w, status, swiglu=True).double(), g * torch.sigmoid(g) * u, atol=2e-2, rtol=2e-2)
+    ops.set_fixed_order(True)
+    try:
+        assert ops.library().vosti_gemm_tc_splits(tokens, features, k) == 1
+        assert torch.allclose(ops.gemm_tc(x, w, status, out_dtype=torch.float32).double(), want, atol=2e-4, rtol=2e-4)
+    finally:
+        ops.set_fixed_order(False)
+    assert status.item() == 0
+
+
 def test_gemm_tc_refuses_what_it_cannot_do(dev, status):
     from vosti_b200 import ops
     assert not ops.gemm_tc_supported(64, 48) and not ops.gemm_tc_supported(64, 100)

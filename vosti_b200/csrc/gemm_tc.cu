@@ -611,7 +611,7 @@ VOSTI_API int vosti_gemm_tc_grouped(const void* x, const void* w, void* y, const
   const int splits = vosti_gemm_tc_grouped_splits(tokens, rows, experts, features, k);
   VOSTI_REQUIRE(splits == 1 || (workspace != nullptr && workspace_elems >= (int64_t)splits * rows * features),
                 "gemm_tc_grouped: workspace too small for %d splits", splits);
-  const int bn = token_tile(tokens);
+  const int bn = token_tile(tokens) < 128 ? token_tile(tokens) : 128;
   const int x_rows = (tokens + 7) / 8 * 8 < bn ? (tokens + 7) / 8 * 8 : bn;
   VOSTI_REQUIRE(weight_map(w, w_rows, BK, BM, &mw) && make_map(&mx, x, rows, k, x_rows), "gemm_tc_grouped: cuTensorMapEncodeTiled failed");
   void* dst = splits > 1 ? (void*)workspace : y;
@@ -648,8 +648,21 @@ VOSTI_API int vosti_gemm_tc_grouped(const void* x, const void* w, void* y, const
 VOSTI_API int vosti_gemm_tc_splits(int tokens, int features, int k) {
   const int k_blocks = (k + BK - 1) / BK;
   const int tiles = ((features + BM - 1) / BM) * ((tokens + token_tile(tokens) - 1) / token_tile(tokens));
-  if (tokens > 128 || g_vosti_fixed_order) return 1;
+  if (g_vosti_fixed_order) return 1;
   int splits;
+  if (tokens > 128) {
+    // Many tokens on pairs of SMs: unsplit, but for products of a single feature tile, of which the pairs make one CTA per
+    // 128 tokens (2,048 tokens: 16 of 148 SMs, 27 us at K = 4,096, against 13 us split and summed). Split, the
+    // tokens go in tiles of 128 through the single-CTA kernel; a split has at least 4 k-blocks and the partial sums
+    // stay within 32 MB of scratch.
+    const int token_tiles = (tokens + 127) / 128;
+    if (features > BM || k_blocks < 16 || token_tiles > 148 / 2) return 1;
+    splits = 148 / token_tiles;
+    if (splits > k_blocks / 4) splits = k_blocks / 4;
+    if (splits > 16) splits = 16;
+    while (splits > 1 && (int64_t)splits * tokens * features > (int64_t)1 << 23) --splits;
+    return splits;
+  }
   if (token_tile(tokens) <= 64) {
     // two CTAs of this tile size fit an SM: fill both slots of every SM, never a second round
     splits = (2 * 148) / tiles;
@@ -691,7 +704,7 @@ VOSTI_API int vosti_gemm_tc(const void* x, const void* w, void* y, int tokens, i
     const char* env = getenv("VOSTI_GEMM_PAIR");
     return env == nullptr || env[0] != '0';
   }();
-  if (tokens > 128 && use_pairs) {
+  if (tokens > 128 && splits == 1 && use_pairs) {
     // many tokens, two SMs per tile (cta_group::2)
     using namespace pair_kernel;
     VOSTI_REQUIRE(weight_map(w, w_rows, w_cols, BM, &mw_storage) && make_map(&mx, x, tokens, k, BM),
@@ -715,7 +728,7 @@ VOSTI_API int vosti_gemm_tc(const void* x, const void* w, void* y, int tokens, i
                           features, k_blocks, ld_out, epilogue, w_tiles, PlainEpilogue{}, status);
     VOSTI_LAUNCH_CHECK();
   }
-  if (tokens > 128) {
+  if (tokens > 128 && splits == 1) {
     // many tokens: persistent kernel with tokens on the M side
     VOSTI_REQUIRE(weight_map(w, w_rows, w_cols, WIDE_BN, &mw_storage) && make_map(&mx, x, tokens, k, BM),
                   "gemm_tc: cuTensorMapEncodeTiled failed");
@@ -737,7 +750,7 @@ VOSTI_API int vosti_gemm_tc(const void* x, const void* w, void* y, int tokens, i
                  features, k_blocks, ld_out, epilogue, w_tiles, status);
     VOSTI_LAUNCH_CHECK();
   }
-  const int bn = token_tile(tokens);
+  const int bn = token_tile(tokens) < 128 ? token_tile(tokens) : 128;
   const int x_rows = (tokens + 7) / 8 * 8 < bn ? (tokens + 7) / 8 * 8 : bn;   // the token box: no more rows than needed
   VOSTI_REQUIRE(weight_map(w, w_rows, w_cols, BM, &mw_storage) && make_map(&mx, x, tokens, k, x_rows),
                 "gemm_tc: cuTensorMapEncodeTiled failed");
@@ -752,8 +765,7 @@ VOSTI_API int vosti_gemm_tc(const void* x, const void* w, void* y, int tokens, i
   switch (bn) {
     case 32: rc = lone ? launch<32, 5, 2>(VOSTI_GEMM_ARGS) : launch<32, 5>(VOSTI_GEMM_ARGS); break;
     case 64: rc = lone ? launch<64, 4, 2>(VOSTI_GEMM_ARGS) : launch<64, 4>(VOSTI_GEMM_ARGS); break;
-    case 128: rc = lone ? launch<128, 3, 2>(VOSTI_GEMM_ARGS) : launch<128, 6>(VOSTI_GEMM_ARGS); break;
-    default: rc = launch<256, 4>(VOSTI_GEMM_ARGS); break;
+    default: rc = lone ? launch<128, 3, 2>(VOSTI_GEMM_ARGS) : launch<128, 6>(VOSTI_GEMM_ARGS); break;
   }
 #undef VOSTI_GEMM_ARGS
   if (rc != 0) return rc;

@@ -519,7 +519,7 @@ def gemm_tc(x: torch.Tensor, w, status: torch.Tensor, *, out_dtype: Optional[tor
     splits = lib.vosti_gemm_tc_splits(tokens, features, k)
     elems = splits * tokens * features if splits > 1 else 0
     ws = _workspace(x.device, elems, scratch) if elems else None
-    defer = bool(allow_partial and splits > 1 and epilogue in (EPI_BF16, EPI_F32))
+    defer = bool(allow_partial and splits > 1 and tokens <= 128 and epilogue in (EPI_BF16, EPI_F32))
     out = None if defer else torch.empty((tokens, width), dtype=out_dtype, device=x.device)
     if splits > 1:
         _SPLIT_GENERATION[scratch] = _SPLIT_GENERATION.get(scratch, 0) + 1
