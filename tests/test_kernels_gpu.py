@@ -246,6 +246,28 @@ def test_attention_simt(dev, status, dtype, nq, nkv, d, page, window):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("nq,nkv,d,page,window", [(6, 2, 48, 16, 0), (4, 1, 16, 8, 0), (8, 8, 128, 16, 0), (32, 1, 64, 4, 0),
+                                                   (6, 2, 80, 4, 13), (2, 1, 256, 64, 0), (32, 8, 128, 16, 40)])
+def test_attention_simt_of_portions_gives_the_bits_of_single_tokens(dev, status, dtype, nq, nkv, d, page, window):
+    """Portions share their tiles of keys in a block (requests that meet in a block among them); a row's bits are
+    those of its token alone, which takes a warp of its own."""
+    from vosti_b200 import ops
+    lens_k, lens_q = [40, 33, 1, 130, 95], [40, 3, 1, 77, 31]
+    case = paged_case(dev, dtype, lens_q, lens_k, nq, nkv, d, page)
+    scale = 0.37 * d ** -0.5
+    q, kc, vc = case["q"].to(dev, dtype), dev_cache(case, "k_cache", dev, dtype), dev_cache(case, "v_cache", dev, dtype)
+    positions, request_of, table = case["positions"].to(dev), case["request_of"].to(dev), case["table"].to(dev)
+    common = dict(block_table=table, page_size=page, nq=nq, nkv=nkv, head_dim=d, scale=scale, window=window, status=status)
+    out = ops.attention_simt(q, kc, vc, positions=positions, request_of=request_of, **common)
+    assert torch.isfinite(out).all(), "a masked or unused (NaN) cache entry was read"
+    assert torch.allclose(out.float().cpu(), reference_attention(case, scale, window), **tol(dtype)) and status.item() == 0
+    for t in (0, 39, 40, 42, 43, 44, 120, 121, 151):
+        one = ops.attention_simt(q[t:t + 1].contiguous(), kc, vc, positions=positions[t:t + 1].contiguous(),
+                                 request_of=request_of[t:t + 1].contiguous(), **common)
+        assert torch.equal(one[0], out[t]), t
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 def test_attention_finds_one_far_key(dev, status, dtype):
     """One key among hundreds is made to stand out (query and key scaled); the output must be
     that key's value. Placed at a page's first and last slot and at the window's edge."""

@@ -296,7 +296,7 @@ def attention_simt(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor
     num_pages = k_cache.numel() // (page_size * nkv * head_dim)
     _check(library().vosti_attention_simt(
         _p(q), _p(k_cache), _p(v_cache), _p(out), _p(positions), _p(request_of), _p(block_table),
-        block_table.shape[1], page_size, num_pages, tokens, nq, nkv, head_dim, ctypes.c_float(scale),
+        block_table.shape[1], page_size, num_pages, tokens, block_table.shape[0], nq, nkv, head_dim, ctypes.c_float(scale),
         window, flag, _p(status), _stream()), "attention")
     return out
 
