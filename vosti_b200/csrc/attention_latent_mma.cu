@@ -19,7 +19,7 @@
 // window a CTA's segments are counted from the one that holds its rows' first key. A sink (one logit per
 // head) joins a row's denominator once, at the end or at the merge.
 // Sizes: rank 128, 256 or 512; rot a multiple of 32; bfloat16 only. Everything else takes the
-// CUDA-core kernel.
+// CUDA-core kernel; portions whose keys are not cut, at rank 512, take csrc/attention_latent_tc.cu.
 #include "common.cuh"
 #include "latent.cuh"
 #include "mma_util.cuh"

@@ -23,6 +23,11 @@
 //                         chunk [W; O1] S0 and the state's update, both as 8 x 4 register tiles whose summands
 //                         are spread over 8 (4) lanes
 //
+// 2,048 tokens of one request, 16 heads of 128: 82 us and 194 us (the token-by-token kernel: 698 us); the
+// generalized rule over 1,031 + 700 + 317 tokens: 140 us and 278 us (628 us). The first is bound by shared-memory
+// latency at two blocks an SM (issue slots 43 % busy), the second by the shared-memory pipe of the 128 SMs that
+// have a block: 16-byte operand reads, the shuffles that deal the sums out, the copies of the next chunks.
+//
 // The token-by-token kernel waits for a shared-memory read, a chain of multiply-adds and two shuffle reductions
 // between any two tokens; here the chain between chunks is two small products over 32 tokens.
 #include <type_traits>

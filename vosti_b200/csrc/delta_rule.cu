@@ -21,6 +21,7 @@
 //                  are independent; a column's dk entries are spread over KS lanes of a warp,
 //                  R contiguous ones to a lane, and the two sums over them are shuffles.
 //   delta_out      one warp per (token, head): the output stage
+// Portions of more than a few tokens run in chunks instead of delta_scan / general_scan (csrc/delta_chunks.cu).
 //
 // Two forms of the gated rule share these kernels: the decay is one number per (head, key channel)
 // from a low-rank pair, or one number per head from a plain projection (`decay_per_head`: the rates

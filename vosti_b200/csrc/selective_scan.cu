@@ -18,6 +18,7 @@
 //               channel and split its states; tokens in order. A portion of several chunks takes three
 //               launches (each chunk from zero, the chunks' start states, each chunk from its start).
 //               Everything after the projections is float32.
+//   scan_line   the recurrence of a long portion in one pass, for 16 states a channel and wide mixers.
 #include "common.cuh"
 
 namespace {
