@@ -653,15 +653,13 @@ VOSTI_API int vosti_gemm_tc_splits(int tokens, int features, int k) {
   if (tokens > 128) {
     // Many tokens on pairs of SMs: unsplit, but for products of a single feature tile, of which the pairs make one CTA per
     // 128 tokens (2,048 tokens: 16 of 148 SMs, 27 us at K = 4,096, against 13 us split and summed). Split, the
-    // tokens go in tiles of 128 through the single-CTA kernel; a split has at least 4 k-blocks and the partial sums
-    // stay within 32 MB of scratch.
+    // tokens go in tiles of 128 through the single-CTA kernel; a split has at least 4 k-blocks. 148 tiles of
+    // 128 x 128 partial sums at most: 10 MB, within the least that a scratch buffer is made with, so it never moves.
     const int token_tiles = (tokens + 127) / 128;
     if (features > BM || k_blocks < 16 || token_tiles > 148 / 2) return 1;
     splits = 148 / token_tiles;
     if (splits > k_blocks / 4) splits = k_blocks / 4;
-    if (splits > 16) splits = 16;
-    while (splits > 1 && (int64_t)splits * tokens * features > (int64_t)1 << 23) --splits;
-    return splits;
+    return splits < 16 ? splits : 16;
   }
   if (token_tile(tokens) <= 64) {
     // two CTAs of this tile size fit an SM: fill both slots of every SM, never a second round

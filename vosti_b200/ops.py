@@ -1614,6 +1614,7 @@ def scan_run(x: torch.Tensor, dtp: torch.Tensor, dt_bias: Optional[torch.Tensor]
     ws = ws_dt = None
     one_pass = ctx.max_q_len > chunk and bool(library().vosti_scan_one_pass(inner, states))
     several = ctx.max_q_len > chunk and not one_pass
+    shortest = min(ctx.host_q_lens) if one_pass else 0        # (never in a decode step, which may be recorded)
     if several:                  # chunks of a long portion run side by side: start states and step-size sums per chunk
         places = x.shape[0] // chunk + ctx.num_requests
         ws = torch.empty((places, inner, states), dtype=torch.float32, device=x.device)
@@ -1621,8 +1622,8 @@ def scan_run(x: torch.Tensor, dtp: torch.Tensor, dt_bias: Optional[torch.Tensor]
     _check(library().vosti_scan_run(
         _p(x), _p(dtp), _p(dt_bias), _p(bc), _p(a_log), _p(d_skip), _is_f32(a_log), _p(z), ctypes.c_int64(xz.shape[1]),
         _p(state), ctypes.c_int64(state.shape[1]), _p(ctx.cu_q), _p(ctx.state_slots), state.shape[0], ctx.num_requests,
-        ctx.max_q_len, min(ctx.host_q_lens, default=0), inner, states, _p(ws), _p(ws_dt), _p(y), _is_f32(x), _p(ctx.status), _stream()), "scan_run",
-        kernels=3 if several else 2 if one_pass and min(ctx.host_q_lens) <= chunk else 1)
+        ctx.max_q_len, shortest, inner, states, _p(ws), _p(ws_dt), _p(y), _is_f32(x), _p(ctx.status), _stream()), "scan_run",
+        kernels=3 if several else 2 if one_pass and shortest <= chunk else 1)
     return y
 
 
@@ -1672,7 +1673,8 @@ def delta_step_layout(q_lens):
             starts.append(len(requests))
             requests.extend([i] * -(-n // DELTA_CHUNK))
             firsts.extend(range(0, n, DELTA_CHUNK))
-    arrays = {"chunk_request": requests, "chunk_first": firsts, "long_requests": longs, "long_chunk0": starts} if longs else {}
+    # one array: per chunk its request, then its first token, then the long requests, then their first chunks
+    arrays = {"plan": requests + firsts + longs + starts} if longs else {}
     return arrays, {"chunks": len(requests), "longs": len(longs), "shorts": len(q_lens) - len(longs)}
 
 
@@ -1683,12 +1685,13 @@ def _delta_chunks(ctx, x, y, decay, b, k, v, beta, out, state, x_heads: int, hea
     lib = library()
     if layout is None or layout["longs"] == 0 or not lib.vosti_delta_chunk_fits(heads, dk, dv):
         return 0
-    arrays = ctx.extras
-    scratch = torch.empty(layout["chunks"] * lib.vosti_delta_chunk_floats(heads, dv, int(b is not None)), dtype=torch.float32, device=out.device)
+    plan, chunks, longs = ctx.extras["delta.plan"], layout["chunks"], layout["longs"]
+    at = lambda i: ctypes.c_void_p(plan.data_ptr() + 4 * i)
+    scratch = torch.empty(chunks * lib.vosti_delta_chunk_floats(heads, dv, int(b is not None)), dtype=torch.float32, device=out.device)
     _check(lib.vosti_delta_chunks(
         _p(x), _p(y), _p(decay), _p(b), _p(k), _p(v), _p(beta), x_heads, heads, dk, dv, _p(out), _p(state), ctypes.c_int64(state.shape[1]),
-        _p(ctx.cu_q), _p(ctx.state_slots), state.shape[0], _p(arrays["delta.chunk_request"]), _p(arrays["delta.chunk_first"]),
-        layout["chunks"], _p(arrays["delta.long_requests"]), _p(arrays["delta.long_chunk0"]), layout["longs"], _p(scratch), _stream()),
+        _p(ctx.cu_q), _p(ctx.state_slots), state.shape[0], at(0), at(chunks), chunks, at(2 * chunks),
+        at(2 * chunks + longs), longs, _p(scratch), _stream()),
         "delta_chunks", kernels=2)
     return DELTA_SHORT if layout["shorts"] else -1
 
