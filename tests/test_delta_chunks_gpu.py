@@ -72,7 +72,8 @@ def scan(rule, ins, harness, ctx, heads, x_heads, dv):
 @pytest.mark.parametrize("rule,heads,x_heads,dv,lengths", [
     ("gated", 2, 1, 128, (49,)), ("gated", 4, 2, 48, (64, 1, 65)), ("gated", 1, 1, 160, (48, 130, 7)), ("gated", 6, 2, 16, (300, 95)),
     ("general", 2, 2, 128, (49,)), ("general", 1, 1, 128, (96, 48, 1, 97)), ("general", 3, 3, 128, (257, 63))])
-def test_chunks(rule, heads, x_heads, dv, lengths, kind):
+def test_chunks(monkeypatch, rule, heads, x_heads, dv, lengths, kind):
+    monkeypatch.setattr(ops, "delta_takes_chunks", lambda *a: True)         # also where token by token is faster
     gen = torch.Generator().manual_seed(sum(lengths) + heads)
     T = sum(lengths)
     ins = inputs(rule, T, heads, x_heads, dv, kind, gen)
@@ -102,7 +103,8 @@ def test_chunks(rule, heads, x_heads, dv, lengths, kind):
 
 
 @pytest.mark.parametrize("rule", ["gated", "general"])
-def test_a_token_that_is_not_finite_reaches_no_earlier_one(rule):
+def test_a_token_that_is_not_finite_reaches_no_earlier_one(monkeypatch, rule):
+    monkeypatch.setattr(ops, "delta_takes_chunks", lambda *a: True)
     gen = torch.Generator().manual_seed(3)
     ins = inputs(rule, 80, 1, 1, 128, "mixed", gen)
     outs = []

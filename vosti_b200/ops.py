@@ -1657,15 +1657,25 @@ def delta_prep(proj: torch.Tensor, rates: torch.Tensor, offsets: dict, *, kv_hea
 
 
 DELTA_CHUNK = 32     # tokens of a chunk (csrc/delta_chunks.cu)
-# Requests that bring at most this many tokens are served token by token: 0.34 us a token and layer, against some 12 us
-# and 1.2 us a chunk for the chunked kernels (16 heads of 128, one request).
-DELTA_SHORT = 48
+DELTA_SHORT = 48     # requests that bring at most this many tokens are always served token by token
+
+
+def delta_takes_chunks(longest: int, tokens: int, chunks: int, width: float, pair: bool) -> bool:
+    """Whether the chunked kernels are the faster way for a step's long portions: `longest` and `tokens` of them, cut into
+    `chunks`; `width` is heads * dv over the 16 * 128 measured, `pair` the generalized rule. Token by token a
+    step takes its longest portion's chain plus a share of the GPU a token; chunks take about 4 us (5.2) each when all of a
+    chunk's heads fill the GPU, 3 us when they do not, and two launches. Measured at 16 heads of 128, us, tokens
+    and chunks: gated, one request of 64: 24 and 29, 96: 35 and 32, 256: 89 and 47; four of 128: 81 and 77; sixteen
+    of 256: 462 and 533. Generalized, one of 96: 37 and 45, 128: 48 and 49; four of 96: 99 and 85; sixteen of 256: 801 and 687."""
+    one_by_one = (0.18 * longest + 0.184 * width * tokens) if pair else (0.25 * longest + 0.097 * width * tokens)
+    each, fixed = (5.2, 33.0) if pair else (4.0, 23.0)
+    return fixed + max(0.75 * each * -(-longest // DELTA_CHUNK), each * width * chunks) < 0.95 * one_by_one
 
 
 def delta_step_layout(q_lens):
-    """How the delta rules divide a step (registered with the step layout as "delta"): the requests that bring more than
-    DELTA_SHORT tokens are cut into chunks, the longest first, the others go token by token; with one order of
-    arithmetic asked for (set_fixed_order) all of them do."""
+    """How the delta rules may divide a step (registered with the step layout as "delta"): the requests that bring more than
+    DELTA_SHORT tokens are cut into chunks, the longest first (a layer takes them if `delta_takes_chunks`), the others
+    go token by token; with one order of arithmetic asked for (set_fixed_order) all of them do."""
     requests, firsts, longs, starts = [], [], [], []
     if not FIXED_ORDER and max(q_lens, default=0) > DELTA_SHORT:
         for n, i in sorted(((n, i) for i, n in enumerate(q_lens) if n > DELTA_SHORT), key=lambda e: (-e[0], e[1])):
@@ -1675,7 +1685,9 @@ def delta_step_layout(q_lens):
             firsts.extend(range(0, n, DELTA_CHUNK))
     # one array: per chunk its request, then its first token, then the long requests, then their first chunks
     arrays = {"plan": requests + firsts + longs + starts} if longs else {}
-    return arrays, {"chunks": len(requests), "longs": len(longs), "shorts": len(q_lens) - len(longs)}
+    lengths = [q_lens[i] for i in longs]
+    return arrays, {"chunks": len(requests), "longs": len(longs), "shorts": len(q_lens) - len(longs),
+                    "longest": max(lengths, default=0), "tokens": sum(lengths)}
 
 
 def _delta_chunks(ctx, x, y, decay, b, k, v, beta, out, state, x_heads: int, heads: int, dk: int, dv: int) -> int:
@@ -1684,6 +1696,8 @@ def _delta_chunks(ctx, x, y, decay, b, k, v, beta, out, state, x_heads: int, hea
     layout = (getattr(ctx, "layout", None) or {}).get("delta")
     lib = library()
     if layout is None or layout["longs"] == 0 or not lib.vosti_delta_chunk_fits(heads, dk, dv):
+        return 0
+    if not delta_takes_chunks(layout["longest"], layout["tokens"], layout["chunks"], heads * dv / 2048, b is not None):
         return 0
     plan, chunks, longs = ctx.extras["delta.plan"], layout["chunks"], layout["longs"]
     at = lambda i: ctypes.c_void_p(plan.data_ptr() + 4 * i)
