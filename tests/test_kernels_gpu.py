@@ -373,6 +373,28 @@ def test_gemm_tc_of_one_feature_tile_over_many_tokens_splits(dev, status, tokens
     assert status.item() == 0
 
 
+def test_split_products_over_many_tokens_leave_the_shared_scratch_alone(dev, status):
+    """A partial sum that is still to be added stays valid, and its values stay, while a split product over more
+    than 128 tokens runs; such a product under way on one stream keeps its values while another stream runs one."""
+    from vosti_b200 import ops
+    few, many = torch.randn(8, 4096, device=dev).bfloat16(), [torch.randn(2048, 4096, device=dev).bfloat16() for _ in range(2)]
+    wide, narrow = (torch.randn(n, 4096, device=dev).bfloat16() / 64 for n in (4096, 128))
+    want_few, want = ops.gemm_tc(few, wide, status), [ops.gemm_tc(x, narrow, status) for x in many]
+    partial = ops.gemm_tc(few, wide, status, allow_partial=True)
+    assert isinstance(partial, ops.PartialSum) and ops.library().vosti_gemm_tc_splits(2048, 128, 4096) > 1
+    ops.gemm_tc(many[0], narrow, status)
+    assert torch.equal(ops.materialize(partial), want_few)
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    got = [[], []]
+    for _ in range(50):
+        for i, stream in enumerate(streams):
+            with torch.cuda.stream(stream):
+                got[i].append(ops.gemm_tc(many[i], narrow, status))
+    torch.cuda.synchronize()
+    assert all(torch.equal(y, want[i]) for i in range(2) for y in got[i]) and status.item() == 0
+
+
 def test_gemm_tc_refuses_what_it_cannot_do(dev, status):
     from vosti_b200 import ops
     assert not ops.gemm_tc_supported(64, 48) and not ops.gemm_tc_supported(64, 100)

@@ -653,8 +653,8 @@ VOSTI_API int vosti_gemm_tc_splits(int tokens, int features, int k) {
   if (tokens > 128) {
     // Many tokens on pairs of SMs: unsplit, but for products of a single feature tile, of which the pairs make one CTA per
     // 128 tokens (2,048 tokens: 16 of 148 SMs, 27 us at K = 4,096, against 13 us split and summed). Split, the
-    // tokens go in tiles of 128 through the single-CTA kernel; a split has at least 4 k-blocks. 148 tiles of
-    // 128 x 128 partial sums at most: 10 MB, within the least that a scratch buffer is made with, so it never moves.
+    // tokens go in tiles of 128 through the single-CTA kernel; a split has at least 4 k-blocks. The partial sums are
+    // 148 tiles of 128 x 128 at most (10 MB).
     const int token_tiles = (tokens + 127) / 128;
     if (features > BM || k_blocks < 16 || token_tiles > 148 / 2) return 1;
     splits = 148 / token_tiles;

@@ -495,8 +495,8 @@ def gemm_tc(x: torch.Tensor, w, status: torch.Tensor, *, out_dtype: Optional[tor
     """y = x @ w.T on the tensor cores (bfloat16 operands, float32 accumulation); w is a
     [features, k] tensor or a `PackedWeight`. With `swiglu` the rows of w are blocks of 16 gate
     rows followed by their 16 up rows and y = act(gate) * up has half as many columns, act being
-    `activation`: "silu", "relu" or "relu2" (the square of relu). `scratch` names the buffer of the K splits:
-    two results that stay unsummed at the same time need buffers of their own."""
+    `activation`: "silu", "relu" or "relu2" (the square of relu). `scratch` names the buffer of the K splits of up
+    to 128 tokens: two results that stay unsummed at the same time need buffers of their own."""
     packed = isinstance(w, PackedWeight)
     w_data = w.data if packed else w
     _contig(x, w_data)
@@ -518,10 +518,15 @@ def gemm_tc(x: torch.Tensor, w, status: torch.Tensor, *, out_dtype: Optional[tor
     lib = library()
     splits = lib.vosti_gemm_tc_splits(tokens, features, k)
     elems = splits * tokens * features if splits > 1 else 0
-    ws = _workspace(x.device, elems, scratch) if elems else None
-    defer = bool(allow_partial and splits > 1 and tokens <= 128 and epilogue in (EPI_BF16, EPI_F32))
+    # more than 128 tokens: sums of the call's own, so that products on several streams and a partial sum that is
+    # still to be added don't meet in the shared buffer (one torch.empty of at most 10 MB a call)
+    own = tokens > 128
+    ws = None
+    if elems:
+        ws = torch.empty(elems, dtype=torch.float32, device=x.device) if own else _workspace(x.device, elems, scratch)
+    defer = bool(allow_partial and splits > 1 and not own and epilogue in (EPI_BF16, EPI_F32))
     out = None if defer else torch.empty((tokens, width), dtype=out_dtype, device=x.device)
-    if splits > 1:
+    if splits > 1 and not own:
         _SPLIT_GENERATION[scratch] = _SPLIT_GENERATION.get(scratch, 0) + 1
     _check(lib.vosti_gemm_tc(_p(x), _p(w_data), _p(out), tokens, features, k, epilogue, _p(ws),
                              ctypes.c_int64(ws.numel() if ws is not None else 0), int(defer), int(packed), _p(status),
