@@ -88,6 +88,16 @@ def test_no_product_is_split_when_one_order_of_arithmetic_is_asked_for(lib):
     assert lib.vosti_gemm_tc_splits(8, 4096, 12288) > 1
 
 
+def test_narrow_products_over_many_tokens_split_where_that_is_faster(lib):
+    """The sizes on both sides of the line at which splitting was measured faster and slower than one pass."""
+    for tokens, features, k in [(129, 8, 1024), (2400, 128, 1024), (3200, 64, 1280), (3840, 128, 1536), (5000, 64, 2048),
+                                (6300, 128, 2560), (9400, 128, 4096), (9400, 8, 12288)]:
+        assert lib.vosti_gemm_tc_splits(tokens, features, k) > 1, (tokens, features, k)
+    for tokens, features, k in [(4800, 8, 1024), (4096, 64, 1024), (4800, 32, 1280), (6300, 32, 1536), (8192, 128, 2048),
+                                (9400, 128, 2560), (9473, 8, 12288), (2048, 129, 4096), (2048, 128, 960)]:
+        assert lib.vosti_gemm_tc_splits(tokens, features, k) == 1, (tokens, features, k)
+
+
 def test_weight_bytes_of_a_decode_step_in_closed_form():
     """What bench.py counts as the weights a decode step must read: every tensor the model
     expects except the embedding table (read by rows), two bytes each. For the 8B sizes that is

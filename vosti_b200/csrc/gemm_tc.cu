@@ -655,8 +655,12 @@ VOSTI_API int vosti_gemm_tc_splits(int tokens, int features, int k) {
     // 128 tokens (2,048 tokens: 16 of 148 SMs, 27 us at K = 4,096, against 13 us split and summed). Split, the
     // tokens go in tiles of 128 through the single-CTA kernel; a split has at least 4 k-blocks. The partial sums are
     // 148 tiles of 128 x 128 at most (10 MB).
+    // The sums grow with the tokens and what a split saves with K, so the line is token tiles against k-blocks. Measured,
+    // unsplit and split, us, 64 features: K = 1,024, 2,400 tokens 9.3 and 9.1, 4,800 9.5 and 11.0; K = 2,048, 5,000
+    // tokens 14.1 and 12.5, 8,192 14.2 and 14.4; 128 features: K = 1,536, 3,200 tokens 12.9 and 11.8, 6,400 13.3 and
+    // 15.1; K = 2,048, 9,400 tokens 16.1 and 18.4; K = 4,096, 9,400 26.4 and 24.7. (At the line itself the two are within 4 %.)
     const int token_tiles = (tokens + 127) / 128;
-    if (features > BM || k_blocks < 16 || token_tiles > 148 / 2) return 1;
+    if (features > BM || k_blocks < 16 || token_tiles > 148 / 2 || token_tiles > k_blocks * 5 / 3) return 1;
     splits = 148 / token_tiles;
     if (splits > k_blocks / 4) splits = k_blocks / 4;
     return splits < 16 ? splits : 16;
