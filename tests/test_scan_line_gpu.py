@@ -47,3 +47,21 @@ def test_against_float64(dtype, inner, lengths):
         assert rel(have, want) <= n ** 0.5 * 2.0 ** -22 + (2.0 ** -8 if dtype == torch.bfloat16 else 0.0), rel(have, want)
         at += n
     assert harness.status.item() == 0
+
+
+def test_channels_that_forget_at_once_keep_finite_states():
+    """A rate beyond float32's range (exp of A_log overflows) means that a state holds its last token alone; the
+    places of a tile past the portion's last token must not touch it (70 tokens: two whole groups of four are empty)."""
+    gen = torch.Generator().manual_seed(5)
+    normal = lambda *s: torch.randn(*s, generator=gen)
+    T, inner = 70, 2048
+    x, xz, dtp, bc, a_log = normal(T, inner), normal(T, 2 * inner), normal(T, inner), normal(T, 2 * N), normal(inner, N)
+    a_log[::3, ::2] = 100.0
+    harness = Harness([None], [StateSpec((inner * N,), torch.float32)], torch.float32)
+    ctx = harness.context([StepEntry("r", [0] * T)])
+    state, d = harness.cache.layer_caches[0].state, lambda t: t.to(DEV)
+    y = ops.scan_run(d(x), d(dtp), None, d(bc), d(a_log), None, d(xz), state, ctx, inner=inner, states=N)
+    end = state[ctx.host_state_slots[0]].view(inner, N).double().cpu()
+    last = (torch.nn.functional.softplus(dtp[-1].double()) * x[-1].double())[:, None] * bc[-1, :N].double()
+    assert torch.isfinite(y).all() and torch.isfinite(end).all()
+    assert torch.allclose(end[::3, ::2], last[::3, ::2], rtol=2.0 ** -20, atol=1e-30)

@@ -19,6 +19,8 @@
 //               launches (each chunk from zero, the chunks' start states, each chunk from its start).
 //               Everything after the projections is float32.
 //   scan_line   the recurrence of a long portion in one pass, for 16 states a channel and wide mixers.
+#include <cfloat>
+
 #include "common.cuh"
 
 namespace {
@@ -420,7 +422,9 @@ scan_line_kernel(const T* __restrict__ x, const float* __restrict__ dtp, const v
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       s[j] = S[j];
-      a[j] = -expf(load_flex(a_log, w_f32, (int64_t)(live ? c : inner - 1) * N + r * 4 + j));
+      // (finite also where the rate is not: a tile's places past the last token have a step size of 0 and must change nothing)
+      const float rate = expf(load_flex(a_log, w_f32, (int64_t)(live ? c : inner - 1) * N + r * 4 + j));
+      a[j] = rate == INFINITY ? -FLT_MAX : -rate;
     }
   } else {
     fetch(0);
