@@ -1,5 +1,7 @@
 """The selective scan's one pass over long portions (csrc/selective_scan.cu) against float64: lengths around the tile,
 single tokens beside them, channels that do not fill a block, start states, both serving types."""
+from dataclasses import replace
+
 import pytest
 import torch
 
@@ -65,3 +67,21 @@ def test_channels_that_forget_at_once_keep_finite_states():
     last = (torch.nn.functional.softplus(dtp[-1].double()) * x[-1].double())[:, None] * bc[-1, :N].double()
     assert torch.isfinite(y).all() and torch.isfinite(end).all()
     assert torch.allclose(end[::3, ::2], last[::3, ::2], rtol=2.0 ** -20, atol=1e-30)
+
+
+def test_a_step_without_host_lengths_gives_the_same_bits():
+    """A context made by hand may leave out the host's copies of the lengths; the longest portion is all that is needed."""
+    gen = torch.Generator().manual_seed(6)
+    d = lambda *s: torch.randn(*s, generator=gen).to(DEV)
+    lengths, inner = (100, 3, 70), 2048
+    T = sum(lengths)
+    x, xz, dtp, bc, a_log = d(T, inner), d(T, 2 * inner), d(T, inner), d(T, 2 * N), d(inner, N)
+    got = []
+    for known in (True, False):
+        harness = Harness([None], [StateSpec((inner * N,), torch.float32)], torch.float32, max_requests=len(lengths))
+        ctx = harness.context([StepEntry(i, [0] * n) for i, n in enumerate(lengths)])
+        state = harness.cache.layer_caches[0].state
+        if not known:
+            ctx = replace(ctx, host_q_lens=[], host_kv_lens=[])
+        got.append((ops.scan_run(x, dtp, None, bc, a_log, None, xz, state, ctx, inner=inner, states=N), state.clone()))
+    assert all(torch.equal(a, b) for a, b in zip(*got))

@@ -1619,7 +1619,7 @@ def scan_run(x: torch.Tensor, dtp: torch.Tensor, dt_bias: Optional[torch.Tensor]
     ws = ws_dt = None
     one_pass = ctx.max_q_len > chunk and bool(library().vosti_scan_one_pass(inner, states))
     several = ctx.max_q_len > chunk and not one_pass
-    shortest = min(ctx.host_q_lens) if one_pass else 0        # (never in a decode step, which may be recorded)
+    shortest = min(ctx.host_q_lens, default=0) if one_pass else 0     # (not known: there may be short requests)
     if several:                  # chunks of a long portion run side by side: start states and step-size sums per chunk
         places = x.shape[0] // chunk + ctx.num_requests
         ws = torch.empty((places, inner, states), dtype=torch.float32, device=x.device)
