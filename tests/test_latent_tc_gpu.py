@@ -61,3 +61,29 @@ def test_against_float64(monkeypatch, heads, lengths, past, page, window, with_s
         # the weights carry 16 bits (two bfloat16 terms), the scores are float32 sums of 576 products
         assert torch.allclose(got[at:at + n], want, atol=2e-4, rtol=2e-4), float((got[at:at + n] - want).abs().max())
         at += n
+
+
+def test_the_cut_does_not_show_in_fixed_order():
+    """With one order of arithmetic asked for, no kernel is chosen by how many tokens a portion has: a prompt in one
+    portion (640 rows) and in portions of five tokens (80 rows) gives the same bits."""
+    heads, T, page = 16, 40, 16
+    gen = torch.Generator(device=DEV).manual_seed(9)
+    normal = lambda *s: torch.randn(*s, generator=gen, device=DEV)
+    qk, rows = (normal(T, heads, RANK + ROT) * 0.3).bfloat16(), (normal(T, RANK).bfloat16(), normal(T, ROT).bfloat16())
+    got = []
+    ops.set_fixed_order(True)
+    try:
+        for cut in (T, 5):
+            harness = Harness([PagedCacheSpec(entries=2, heads=1, width=RANK, widths=(RANK, ROT))], [None], torch.bfloat16,
+                              num_pages=8, page_size=page)
+            layer, parts = harness.cache.layer_caches[0], []
+            for first in range(0, T, cut):
+                ctx = harness.context([StepEntry("r", [0] * cut)])
+                at = torch.arange(first, first + cut, device=DEV)
+                for pool, row in zip(layer.tensors, rows):
+                    pool[ctx.groups[0].block_table[0, at // page].long(), 0, at % page] = row[first:first + cut]
+                parts.append(ops.latent_attend(ctx, qk[first:first + cut].contiguous(), layer.k, layer.v, ctx.groups[0], scale=0.07))
+            got.append(torch.cat(parts))
+    finally:
+        ops.set_fixed_order(False)
+    assert torch.equal(*got)

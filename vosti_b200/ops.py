@@ -1537,7 +1537,7 @@ def latent_attend(ctx, qk: torch.Tensor, c_cache: torch.Tensor, r_cache: torch.T
     [tokens, heads, rank]. bfloat16 with a rank of
     128, 256 or 512 and a rotated part in multiples of 32 runs on the tensor cores
     (csrc/attention_latent_mma.cu; portions whose keys it would not cut, at rank 512 with a rotated part of 64 and pages of a
-    multiple of 16, in csrc/attention_latent_tc.cu), everything else on the CUDA cores (csrc/attention_latent.cu)."""
+    multiple of 16, in csrc/attention_latent_tc.cu unless one order of arithmetic is asked for), everything else on the CUDA cores (csrc/attention_latent.cu)."""
     _contig(qk, c_cache, r_cache, sink)
     flag = _same_dtype(qk, c_cache, r_cache)
     tokens, heads = qk.shape[0], qk.shape[1]
@@ -1556,7 +1556,7 @@ def latent_attend(ctx, qk: torch.Tensor, c_cache: torch.Tensor, r_cache: torch.T
             segments = key_segments(ctx.max_kv_len, window, LATENT_MMA_SEGMENT, min(ctx.max_q_len, -(-tile // heads) + 1))
         if segments > 1:
             scratch = _workspace(qk.device, tokens * heads * segments * (rank + 2))
-        elif rows >= LATENT_TC_ROWS and scale > 0 and lib.vosti_latent_attend_tc_fits(rank, rot, group.page_size):
+        elif rows >= LATENT_TC_ROWS and scale > 0 and not FIXED_ORDER and lib.vosti_latent_attend_tc_fits(rank, rot, group.page_size):
             _check(lib.vosti_latent_attend_tc(
                 _p(qk), _p(c_cache), _p(r_cache), _p(out), _p(ctx.positions), _p(ctx.cu_q), _p(group.block_table),
                 group.block_table.shape[1], group.page_size, num_pages, ctx.num_requests, ctx.max_q_len, tokens, heads, rank, rot,
