@@ -98,6 +98,27 @@ def test_narrow_products_over_many_tokens_split_where_that_is_faster(lib):
         assert lib.vosti_gemm_tc_splits(tokens, features, k) == 1, (tokens, features, k)
 
 
+def test_latent_portions_take_the_kernel_that_was_measured_faster():
+    """Steps (heads, tokens and keys of the requests) on both sides of the line between tiles of 32 and of 128 rows."""
+    from vosti_b200 import ops
+
+    def takes(heads, q, past, window=0):
+        kv = [a + b for a, b in zip(q, past)]
+        tiles = -(-max(q) * heads // 32) * len(q)
+        return ops.latent_takes_tiles(q, kv, heads, window, tiles < ops.LATENT_MMA_SPLIT_BELOW)
+
+    singles = lambda n, count, keys: ([n] + [1] * count, [0] + [keys] * count)
+    for heads, (q, past) in [(16, ([1024], [0])), (16, ([600, 600], [0, 100])), (8, ([2048], [0])), (16, singles(300, 20, 2000)),
+                             (16, singles(640, 60, 500)), (64, ([8] * 16, [100] * 16)), (64, ([128], [0])), (64, singles(8, 300, 1000)),
+                             (64, singles(16, 150, 600)), (128, ([64], [0])), (128, singles(8, 300, 100))]:
+        assert takes(heads, q, past), (heads, q, past)
+    for heads, (q, past) in [(16, ([8], [0])), (16, ([64], [0])), (8, ([64], [0])), (64, ([64], [0])), (128, ([8], [0])),
+                             (16, singles(8, 300, 100)), (16, singles(8, 300, 1000)), (16, singles(16, 150, 600)),
+                             (8, singles(16, 150, 600)), (64, singles(8, 300, 100)), (16, ([9] * 40, [100] * 40))]:
+        assert not takes(heads, q, past), (heads, q, past)
+    assert takes(16, [700], [0], window=128) and not takes(16, *singles(8, 300, 5000), window=100)
+
+
 def test_weight_bytes_of_a_decode_step_in_closed_form():
     """What bench.py counts as the weights a decode step must read: every tensor the model
     expects except the embedding table (read by rows), two bytes each. For the 8B sizes that is

@@ -1525,7 +1525,38 @@ LATENT_SEGMENT = 256           # keys per segment when few query rows share the 
 LATENT_SPLIT_MAX_ROWS = 2048   # (token, head) rows up to which the keys are cut into segments
 LATENT_MMA_SEGMENT = 128       # the same for the tensor-core kernel, whose CTA takes 16 or 32 rows
 LATENT_MMA_SPLIT_BELOW = 296   # CTAs (two per SM) below which it cuts the keys
-LATENT_TC_ROWS = 128           # (token, head) rows of the longest portion from which the tensor-memory kernel's tiles are filled
+LATENT_TC_ROWS = 128           # (token, head) rows of the longest portion that fill a tile of the tensor-memory kernel: fewer never take it
+
+
+def latent_takes_tiles(q_lens, kv_lens, heads: int, window: int, few: bool) -> bool:
+    """Whether tiles of 128 rows in tensor memory (csrc/attention_latent_tc.cu) are the faster way for a step's uncut keys, against
+    tiles of 32 rows (csrc/attention_latent_mma.cu): `q_lens` and `kv_lens` of its requests, `few` if the 32-row tiles are
+    fewer than LATENT_MMA_SPLIT_BELOW. A CTA takes about 5 us + 71 ns a key (two CTAs a tile of 128) or 1 us + 100 ns; a step takes
+    its longest CTA and, beyond one CTA an SM, an SM's share of them all. A request of one token fills neither tile, so
+    many of them beside a portion are better off in the small ones. Measured at 16 heads, us, tiles of 32 and of 128 rows:
+    one prompt of 64 tokens 9.9 and 11.5, of 1,024 216 and 71; a portion of 8 beside 300 single tokens at 100 keys 41 and 72,
+    at 1,000 271 and 375; 300 beside 20 at 2,000 199 and 152; at 64 heads 8 beside 300 at 1,000 457 and 385."""
+    def cost(rows, each, key, start):
+        ctas = total = longest = 0.0
+        for n, kv in zip(q_lens, kv_lens):
+            tiles = each * -(-n * heads // rows)
+            if window > 0:
+                kv = min(kv, n + window)
+            keys = max(kv - n / 2, 1.0)
+            ctas += tiles
+            total += tiles * (key * (keys if window <= 0 else min(keys, window + rows / heads)) + start)
+            longest = max(longest, key * kv)
+        return longest + (start if few else 0.0) + (total / 148 if ctas > 148 else 0.0)
+    return cost(128, 2, 0.071, 5.0) < 0.9 * cost(32, 1, 0.1, 1.0)
+
+
+def _latent_takes_tiles(ctx, heads: int, window: int, few: bool) -> bool:
+    if len(ctx.host_q_lens) != ctx.num_requests or len(ctx.host_kv_lens) != ctx.num_requests:
+        return False
+    made = ctx.layout.setdefault("latent", {})               # once a step, not once a layer
+    if (heads, window) not in made:
+        made[heads, window] = latent_takes_tiles(ctx.host_q_lens, ctx.host_kv_lens, heads, window, few)
+    return made[heads, window]
 
 
 def latent_attend(ctx, qk: torch.Tensor, c_cache: torch.Tensor, r_cache: torch.Tensor, group, *, scale: float,
@@ -1537,7 +1568,7 @@ def latent_attend(ctx, qk: torch.Tensor, c_cache: torch.Tensor, r_cache: torch.T
     [tokens, heads, rank]. bfloat16 with a rank of
     128, 256 or 512 and a rotated part in multiples of 32 runs on the tensor cores
     (csrc/attention_latent_mma.cu; portions whose keys it would not cut, at rank 512 with a rotated part of 64 and pages of a
-    multiple of 16, in csrc/attention_latent_tc.cu unless one order of arithmetic is asked for), everything else on the CUDA cores (csrc/attention_latent.cu)."""
+    multiple of 16, in csrc/attention_latent_tc.cu where `latent_takes_tiles`, unless one order of arithmetic is asked for), everything else on the CUDA cores (csrc/attention_latent.cu)."""
     _contig(qk, c_cache, r_cache, sink)
     flag = _same_dtype(qk, c_cache, r_cache)
     tokens, heads = qk.shape[0], qk.shape[1]
@@ -1556,7 +1587,8 @@ def latent_attend(ctx, qk: torch.Tensor, c_cache: torch.Tensor, r_cache: torch.T
             segments = key_segments(ctx.max_kv_len, window, LATENT_MMA_SEGMENT, min(ctx.max_q_len, -(-tile // heads) + 1))
         if segments > 1:
             scratch = _workspace(qk.device, tokens * heads * segments * (rank + 2))
-        elif rows >= LATENT_TC_ROWS and scale > 0 and not FIXED_ORDER and lib.vosti_latent_attend_tc_fits(rank, rot, group.page_size):
+        elif (rows >= LATENT_TC_ROWS and scale > 0 and not FIXED_ORDER and lib.vosti_latent_attend_tc_fits(rank, rot, group.page_size)
+              and _latent_takes_tiles(ctx, heads, window, ctas < LATENT_MMA_SPLIT_BELOW)):
             _check(lib.vosti_latent_attend_tc(
                 _p(qk), _p(c_cache), _p(r_cache), _p(out), _p(ctx.positions), _p(ctx.cu_q), _p(group.block_table),
                 group.block_table.shape[1], group.page_size, num_pages, ctx.num_requests, ctx.max_q_len, tokens, heads, rank, rot,
