@@ -268,6 +268,57 @@ def test_attention_simt_of_portions_gives_the_bits_of_single_tokens(dev, status,
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("nq,nkv,d,window", [(4, 4, 64, 0), (8, 2, 128, 0), (6, 2, 48, 13), (32, 1, 64, 0), (12, 1, 16, 0)])
+def test_attention_simt_gives_the_same_bits_every_way(monkeypatch, dev, status, dtype, nq, nkv, d, window):
+    """Warps, blocks that share their keys, and blocks beside warps: windows of one, two and more requests, ragged ends."""
+    from vosti_b200 import ops
+    lens_q, lens_k = [40, 3, 1, 1, 1, 50, 2, 1, 70], [40, 33, 90, 1, 65, 130, 2, 64, 95]
+    case = paged_case(dev, dtype, lens_q, lens_k, nq, nkv, d, 16)
+    args = [case["q"].to(dev, dtype), dev_cache(case, "k_cache", dev, dtype), dev_cache(case, "v_cache", dev, dtype)]
+    common = dict(positions=case["positions"].to(dev), request_of=case["request_of"].to(dev), block_table=case["table"].to(dev), page_size=16,
+                  nq=nq, nkv=nkv, head_dim=d, scale=0.37 * d ** -0.5, window=window, status=status, q_lens=lens_q, kv_lens=lens_k)
+    got = []
+    for way in range(3):
+        monkeypatch.setattr(ops, "simt_way", lambda *a: way)
+        got.append(ops.attention_simt(*args, **common))
+    assert torch.equal(got[1], got[0]) and torch.equal(got[2], got[0]) and status.item() == 0
+    assert torch.allclose(got[0].float().cpu(), reference_attention(case, 0.37 * d ** -0.5, window), **tol(dtype))
+
+
+@pytest.mark.parametrize("nq,nkv,known", [(16, 16, True), (16, 16, False), (8, 2, True)])
+def test_attention_simt_of_a_portion_beside_single_tokens_costs_no_more_than_the_two(dev, status, nq, nkv, known):
+    """Requests that meet in a block of rows are not served one after the other: a portion of 128 tokens beside 32 single
+    ones at long contexts takes no more than 1.5 times a step of the portion and a step of the single ones (as warps; by
+    blocks alone it was more than twice and up to 9 times that)."""
+    from vosti_b200 import ops
+    d, page, keys = 64, 16, 1500
+
+    def step(lens_q, lens_k):
+        pages = [-(-n // page) for n in lens_k]
+        table, at = torch.zeros(len(lens_q), max(pages), dtype=torch.int32), 0
+        for i, n in enumerate(pages):
+            table[i, :n] = torch.arange(at, at + n)
+            at += n
+        kc, vc = torch.randn(at, nkv, page, d, device=dev), torch.randn(at, nkv, page, d, device=dev)
+        positions = torch.cat([torch.arange(k - n, k) for n, k in zip(lens_q, lens_k)]).int().to(dev)
+        request_of = torch.cat([torch.full((n,), i) for i, n in enumerate(lens_q)]).int().to(dev)
+        q, table = torch.randn(sum(lens_q), nq * d, device=dev), table.to(dev)
+        run = lambda: ops.attention_simt(q, kc, vc, positions=positions, request_of=request_of, block_table=table, page_size=page,
+                                         nq=nq, nkv=nkv, head_dim=d, scale=d ** -0.5, window=0, status=status,
+                                         **(dict(q_lens=lens_q, kv_lens=lens_k) if known else {}))
+        run()
+        times = []
+        for _ in range(5):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record(), run(), b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b))
+        return sorted(times)[2]
+    both, portion, singles = step([128] + [1] * 32, [128] + [keys] * 32), step([128], [128]), step([1] * 32, [keys] * 32)
+    assert both <= 1.5 * (portion + singles), (both, portion, singles)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 def test_attention_finds_one_far_key(dev, status, dtype):
     """One key among hundreds is made to stand out (query and key scaled); the output must be
     that key's value. Placed at a page's first and last slot and at the window's edge."""

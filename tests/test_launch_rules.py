@@ -119,6 +119,24 @@ def test_latent_portions_take_the_kernel_that_was_measured_faster():
     assert takes(16, [700], [0], window=128) and not takes(16, *singles(8, 300, 5000), window=100)
 
 
+def test_cuda_core_attention_takes_the_way_that_was_measured_faster():
+    """Steps (query and kv heads, tokens and keys of the requests) where warps (0), blocks of rows (1) and both (2) were."""
+    from vosti_b200.ops import simt_way
+    some = ([64, 1, 5, 1, 40, 1, 2, 1], [500, 2000, 1500, 900, 40, 2500, 1200, 700])
+    beside = lambda n, kv, count, keys: ([n] + [1] * count, [kv] + [keys] * count)
+    for way, nq, nkv, (q, kv) in [
+            (1, 32, 8, ([384], [384])), (1, 32, 8, ([4], [3000])), (1, 16, 16, ([16], [16])), (1, 32, 8, ([8] * 4, [2000] * 4)),
+            (1, 16, 16, ([8] * 64, [1000] * 64)), (1, 32, 8, ([4] * 64, [1000] * 64)), (1, 16, 16, some), (1, 64, 2, beside(128, 128, 32, 3000)),
+            (2, 16, 16, beside(300, 900, 60, 1500)), (2, 32, 8, beside(300, 900, 60, 1500)),
+            (0, 16, 16, beside(128, 128, 32, 3000)), (0, 32, 8, beside(64, 64, 12, 2000)), (0, 16, 16, ([5] * 8, [3000] * 8)),
+            (0, 16, 16, ([4] * 16, [1000] * 16)), (0, 16, 16, ([4] * 64, [1000] * 64)), (0, 16, 16, ([8] * 4, [2000] * 4)),
+            (0, 16, 16, ([32] + [3] * 9, [400] + [2000] * 9)), (0, 32, 8, ([32] + [3] * 9, [400] + [2000] * 9)),
+            (0, 32, 8, ([5] * 8, [3000] * 8)), (0, 32, 8, ([1] * 12, [2000] * 12)), (0, 32, 1, ([4], [4])), (0, 16, 16, ([8], [8])),
+            (0, 66, 2, ([384], [384]))]:
+        assert simt_way(q, kv, nq, nkv) == way, (nq, nkv, q, kv, simt_way(q, kv, nq, nkv))
+    assert simt_way([128] + [0] + [9], [128, 50, 9], 32, 8, window=40) == 1
+
+
 def test_weight_bytes_of_a_decode_step_in_closed_form():
     """What bench.py counts as the weights a decode step must read: every tensor the model
     expects except the embedding table (read by rows), two bytes each. For the 8B sizes that is

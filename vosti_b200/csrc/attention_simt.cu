@@ -49,17 +49,27 @@ __device__ __forceinline__ float dot_row<bf16>(const float* __restrict__ q, cons
   return s;
 }
 
+// Whether the window of `per` tokens around token t (windows start at multiples of `per`) holds tokens of more than two
+// requests; all lanes of a warp ask together (per <= 32).
+__device__ __forceinline__ bool crowded(const int* __restrict__ request_of, int t, int per, int tokens) {
+  const int lane = threadIdx.x & 31, at = t / per * per + lane;
+  const bool starts = lane > 0 && lane < per && at < tokens && request_of[at] != request_of[at - 1];
+  return __popc(__ballot_sync(0xffffffffu, starts)) > 1;
+}
+
+// `window_tokens` > 0: only the tokens of crowded windows of that many (attention_simt_rows_kernel takes the others)
 template <typename T>
 __global__ void __launch_bounds__(WARPS * 32)
 attention_simt_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, const T* __restrict__ v_cache,
                       T* __restrict__ out, const int* __restrict__ positions, const int* __restrict__ request_of,
                       const int* __restrict__ block_table, int max_pages, int page_size, int num_pages,
-                      int tokens, int nq, int nkv, int d, float scale_log2, int window, unsigned* status) {
+                      int tokens, int nq, int nkv, int d, float scale_log2, int window, int window_tokens, unsigned* status) {
   extern __shared__ float q_smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t wid = (int64_t)blockIdx.x * WARPS + warp;
   if (wid >= (int64_t)tokens * nq) return;
   const int t = (int)(wid / nq), h = (int)(wid % nq);
+  if (window_tokens > 0 && !crowded(request_of, t, window_tokens, tokens)) return;
   const int g = h * nkv / nq;
   float* qs = q_smem + warp * d;
   const T* qrow = q + ((int64_t)t * nq + h) * d;
@@ -137,7 +147,10 @@ __device__ __forceinline__ float4 load_four(const bf16* p) {
 // key over the head size in order, the online softmax by tiles of 32 keys, the keys in order. The kernel above read every
 // key and value row once per query row, each lane along a row of its own: 384 tokens of 32 heads of 128
 // over 8, float32: 500 us, against 146 us here.
-// Tokens of several requests in a block are taken request by request.
+// Tokens of several requests in a block are taken request by request, so with `skip_crowded` a block of more than two
+// requests leaves its tokens to the kernel above: a request of few tokens costs a block as long as a full one (190 ns a
+// key; a warp of the kernel above 380 ns, but side by side). 128 tokens beside 32 single ones at 3,000 keys, 16
+// heads of 128, took 21.4 ms served by blocks alone, and 2.3 ms by warps alone.
 constexpr int ROWS = 32, ROW_WARPS = 8, PER_WARP = ROWS / ROW_WARPS;
 
 template <typename T, int COLS>                    // COLS: 32-column groups of a head, rounded up
@@ -145,7 +158,7 @@ __global__ void __launch_bounds__(ROW_WARPS * 32)
 attention_simt_rows_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, const T* __restrict__ v_cache,
                            T* __restrict__ out, const int* __restrict__ positions, const int* __restrict__ request_of,
                            const int* __restrict__ block_table, int max_pages, int page_size, int num_pages,
-                           int tokens, int nq, int nkv, int d, float scale_log2, int window, unsigned* status) {
+                           int tokens, int nq, int nkv, int d, float scale_log2, int window, int skip_crowded, unsigned* status) {
   extern __shared__ __align__(16) float rows_smem[];
   const int pitch = d + 4;                         // an odd number of 16-byte words (d is a multiple of 16): lanes in different banks
   float* const ks = rows_smem;                     // [32][pitch]
@@ -155,6 +168,7 @@ attention_simt_rows_kernel(const T* __restrict__ q, const T* __restrict__ k_cach
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int group = nq / nkv, per_block = ROWS / group;        // tokens of a block
   const int g = blockIdx.y, t_begin = blockIdx.x * per_block, t_end = min(tokens, t_begin + per_block);
+  if (skip_crowded && crowded(request_of, t_begin, per_block, tokens)) return;
   for (int i = threadIdx.x; i < (t_end - t_begin) * group * d; i += ROW_WARPS * 32) {
     const int row = i / d, t = t_begin + row / group;
     qs[i] = to_f32(q[((int64_t)t * nq + g * group + row % group) * d + i % d]);
@@ -270,10 +284,11 @@ attention_simt_rows_kernel(const T* __restrict__ q, const T* __restrict__ k_cach
 }  // namespace
 
 // q, out: [tokens, nq, d]; caches: [num_pages, nkv, page_size, d];
-// block_table: [requests, max_pages]; positions, request_of: int32[tokens].
+// block_table: [requests, max_pages]; positions, request_of: int32[tokens]. `way` (the bits are the same): 0 a warp per
+// (token, head), 1 blocks of rows that share their keys, 2 blocks where at most two requests meet in one, warps elsewhere.
 VOSTI_API int vosti_attention_simt(const void* q, const void* k_cache, const void* v_cache, void* out,
                                    const int* positions, const int* request_of, const int* block_table,
-                                   int max_pages, int page_size, int num_pages, int tokens, int requests, int nq, int nkv,
+                                   int max_pages, int page_size, int num_pages, int tokens, int way, int nq, int nkv,
                                    int d, float scale, int window, int is_f32, unsigned* status,
                                    cudaStream_t stream) {
   VOSTI_REQUIRE(tokens >= 0 && nq > 0 && nkv > 0 && nq % nkv == 0, "attention: bad head counts nq=%d nkv=%d", nq, nkv);
@@ -281,10 +296,11 @@ VOSTI_API int vosti_attention_simt(const void* q, const void* k_cache, const voi
   VOSTI_REQUIRE(page_size > 0 && max_pages > 0 && num_pages > 0, "attention: bad cache geometry");
   VOSTI_REQUIRE(window >= 0, "attention: window must be >= 0 (0 = all keys)");
   if (tokens == 0) return VOSTI_OK;
-  // Portions (four tokens a request or more in the mean) share their keys; with fewer a block would take its requests one
-  // after the other. The rows' kernel wants up to 32 heads a kv head and values, too, in whole words.
+  // The rows' kernel wants up to 32 heads a kv head and values, too, in whole words.
+  VOSTI_REQUIRE(way >= 0 && way <= 2, "attention: unknown way %d", way);
   const int group = nq / nkv;
-  if (tokens >= 4 * (int64_t)requests && group <= ROWS && nkv <= 65535 && reinterpret_cast<uintptr_t>(k_cache) % 16 == 0 &&
+  int window_tokens = 0;
+  if (way > 0 && group <= ROWS && nkv <= 65535 && reinterpret_cast<uintptr_t>(k_cache) % 16 == 0 &&
       reinterpret_cast<uintptr_t>(v_cache) % 16 == 0 && (int64_t)num_pages * nkv * page_size < ((int64_t)1 << 31)) {
     const size_t rows_bytes = ((size_t)32 * (d + 4) + 32 * d + ROWS * d) * sizeof(float);
     constexpr int most = (32 * (MAX_D + 4) + 32 * MAX_D + ROWS * MAX_D) * (int)sizeof(float);
@@ -298,12 +314,15 @@ VOSTI_API int vosti_attention_simt(const void* q, const void* k_cache, const voi
     }                                                                                                                    \
     attention_simt_rows_kernel<T, COLS><<<grid, ROW_WARPS * 32, rows_bytes, stream>>>((const T*)q, (const T*)k_cache,     \
         (const T*)v_cache, (T*)out, positions, request_of, block_table, max_pages, page_size, num_pages, tokens, nq, nkv, \
-        d, scale * LOG2E, window, status);                                                                               \
+        d, scale * LOG2E, window, (int)(way == 2), status);                                                              \
   } while (0)
     if (is_f32) { if (d <= 64) VOSTI_ROWS(float, 2); else if (d <= 128) VOSTI_ROWS(float, 4); else VOSTI_ROWS(float, 8); }
     else { if (d <= 64) VOSTI_ROWS(bf16, 2); else if (d <= 128) VOSTI_ROWS(bf16, 4); else VOSTI_ROWS(bf16, 8); }
 #undef VOSTI_ROWS
-    VOSTI_LAUNCH_CHECK();
+    if (way == 1) VOSTI_LAUNCH_CHECK();
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) { vosti_set_error("%s", cudaGetErrorString(e)); return (int)e; }
+    window_tokens = ROWS / group;
   }
   const int64_t warps = (int64_t)tokens * nq;
   const int64_t blocks = (warps + WARPS - 1) / WARPS;
@@ -312,10 +331,10 @@ VOSTI_API int vosti_attention_simt(const void* q, const void* k_cache, const voi
   if (is_f32)
     attention_simt_kernel<float><<<(unsigned)blocks, WARPS * 32, smem, stream>>>((const float*)q, (const float*)k_cache,
         (const float*)v_cache, (float*)out, positions, request_of, block_table, max_pages, page_size, num_pages,
-        tokens, nq, nkv, d, scale * LOG2E, window, status);
+        tokens, nq, nkv, d, scale * LOG2E, window, window_tokens, status);
   else
     attention_simt_kernel<bf16><<<(unsigned)blocks, WARPS * 32, smem, stream>>>((const bf16*)q, (const bf16*)k_cache,
         (const bf16*)v_cache, (bf16*)out, positions, request_of, block_table, max_pages, page_size, num_pages,
-        tokens, nq, nkv, d, scale * LOG2E, window, status);
+        tokens, nq, nkv, d, scale * LOG2E, window, window_tokens, status);
   VOSTI_LAUNCH_CHECK();
 }

@@ -286,18 +286,65 @@ def qkv_post(qkv: torch.Tensor, k_cache: Optional[torch.Tensor], v_cache: Option
     return q_out
 
 
+SIMT_ROWS = 32       # (token, head) rows of a block that shares its tiles of keys (csrc/attention_simt.cu)
+
+
+def simt_way(q_lens, kv_lens, nq: int, nkv: int, window: int = 0) -> int:
+    """How the CUDA-core attention runs a step of requests with `q_lens` tokens and `kv_lens` keys (the bits are the same): 0 a warp
+    per (token, head), 1 blocks that share their tiles of keys, 2 blocks where tokens of at most two requests meet in one
+    and warps, afterwards, elsewhere. A block takes its requests one after the other, about 0.19 us a key; a warp takes
+    0.38 us a key at least, all of them side by side until they fill the GPU (0.21 ns a token, head and key); blocks cost
+    2.7 us to start with (heads of 128). Measured at 16 heads, us, warps, blocks and both: a portion of 128 beside 32 single
+    tokens at 3,000 keys 2,263, 21,412 and 2,301; 300 at 900 keys beside 60 at 1,500 1,832, 13,078 and 1,527; 64 requests of 8
+    at 1,000 1,678, 1,233 and 1,687; 8 of 5 at 3,000 2,161, 4,862 and 3,671; one of 4 at 3,000 1,127 and 571."""
+    tokens, group = sum(q_lens), nq // nkv
+    if tokens < 4 * len(q_lens) or group > SIMT_ROWS:        # (fewer than four tokens a request in the mean: not measured)
+        return 0
+    per = SIMT_ROWS // group
+    seen = (lambda kv: min(kv, window + per)) if window > 0 else (lambda kv: kv)
+    edges, at = {}, 0                    # by block: (tokens, keys) of the requests that begin or end in it
+    longest = inner = inner_total = warp_total = 0
+    for n, kv in zip(q_lens, kv_lens):
+        if n == 0:
+            continue
+        first, last, mean = at // per, (at + n - 1) // per, seen(max(kv - n // 2, 1))
+        for block in {first, last}:
+            edges.setdefault(block, []).append((min(at + n, (block + 1) * per) - max(at, block * per), seen(kv)))
+        if last - first > 1:             # blocks of this request alone
+            inner, inner_total = max(inner, seen(kv)), inner_total + (last - first - 1) * mean
+        longest, warp_total, at = max(longest, seen(kv)), warp_total + n * mean, at + n
+
+    def blocks(kept):
+        chain = max([inner] + [sum(keys for _, keys in entry) for entry in kept])
+        total = inner_total + sum(keys for entry in kept for _, keys in entry)
+        return 2.7 + 0.19 * max(chain, total * nkv / 148) if chain else 0.0
+    warps = max(0.38 * longest, 0.00021 * nq * warp_total)
+    few = [entry for entry in edges.values() if len(entry) <= 2]
+    many = [pair for entry in edges.values() if len(entry) > 2 for pair in entry]
+    one = blocks(edges.values())
+    two = blocks(few) + 3.0 + max(0.38 * max((keys for _, keys in many), default=0), 0.00021 * nq * sum(n * keys for n, keys in many))
+    if one < 0.95 * warps and (one <= two or not many):
+        return 1
+    return 2 if many and two < 0.9 * warps else 0
+
+
 def attention_simt(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, *, positions: torch.Tensor,
                    request_of: torch.Tensor, block_table: torch.Tensor, page_size: int, nq: int, nkv: int,
-                   head_dim: int, scale: float, window: int, status: torch.Tensor) -> torch.Tensor:
+                   head_dim: int, scale: float, window: int, status: torch.Tensor,
+                   q_lens: Optional[Sequence[int]] = None, kv_lens: Optional[Sequence[int]] = None) -> torch.Tensor:
+    """`q_lens` and `kv_lens`: the requests' tokens and keys where the host knows them; the launch is chosen by them."""
     _contig(q, k_cache, v_cache, positions, request_of, block_table)
     flag = _same_dtype(q, k_cache, v_cache)
     tokens = q.shape[0]
     out = torch.empty_like(q)
     num_pages = k_cache.numel() // (page_size * nkv * head_dim)
+    way = int(block_table.shape[0] == 1 and tokens >= 4)
+    if q_lens and kv_lens and sum(q_lens) == tokens and nkv > 0:
+        way = simt_way(q_lens, kv_lens, nq, nkv, window)
     _check(library().vosti_attention_simt(
         _p(q), _p(k_cache), _p(v_cache), _p(out), _p(positions), _p(request_of), _p(block_table),
-        block_table.shape[1], page_size, num_pages, tokens, block_table.shape[0], nq, nkv, head_dim, ctypes.c_float(scale),
-        window, flag, _p(status), _stream()), "attention")
+        block_table.shape[1], page_size, num_pages, tokens, way, nq, nkv, head_dim, ctypes.c_float(scale),
+        window, flag, _p(status), _stream()), "attention", kernels=2 if way == 2 else 1)
     return out
 
 
@@ -740,7 +787,8 @@ def attention(ctx, q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor
     if q.dtype != torch.bfloat16 or nq // nkv > 16:
         return attention_simt(q, k_cache, v_cache, positions=ctx.positions, request_of=ctx.request_of,
                               block_table=group.block_table, page_size=group.page_size, nq=nq, nkv=nkv,
-                              head_dim=head_dim, scale=scale, window=window, status=ctx.status)
+                              head_dim=head_dim, scale=scale, window=window, status=ctx.status,
+                              q_lens=ctx.host_q_lens, kv_lens=ctx.host_kv_lens)
     _contig(q, k_cache, v_cache)
     out = torch.empty_like(q)
     common = dict(block_table=group.block_table, page_size=group.page_size, nq=nq, nkv=nkv, head_dim=head_dim,
