@@ -123,6 +123,43 @@ def test_gemm_simt_tiles_agree(dev, status, rows, n, k):
     assert bool(((y.double() - x.double() @ w.double().T).abs() <= bound).all()) and status.item() == 0
 
 
+@pytest.mark.parametrize("xdt,wdt,ydt", [(torch.bfloat16, torch.bfloat16, torch.bfloat16), (torch.bfloat16, torch.float32, torch.bfloat16),
+                                         (torch.float32, torch.bfloat16, torch.float32), (torch.float32, torch.float32, torch.float32)])
+@pytest.mark.parametrize("rows,n,k", [(200, 4100, 44), (130, 15001, 36), (300, 4100, 37), (65, 9000, 333), (33, 100, 7)])
+def test_gemm_simt_tiles_agree_for_other_types_and_gathered_rows(dev, status, xdt, wdt, ydt, rows, n, k):
+    """The tiles for many rows (whole words and single elements) give the bits of a row alone, rows picked among them."""
+    from vosti_b200 import ops
+    x, w = torch.randn(rows + 50, k, device=dev).to(xdt), torch.randn(n, k, device=dev).to(wdt)
+    index = torch.randint(0, rows + 50, (rows,), device=dev, dtype=torch.int32)
+    y = ops.gemm_simt(x, w, status, out_dtype=ydt, row_index=index)
+    picked = x[index.long()].contiguous()
+    assert torch.equal(ops.gemm_simt(picked, w, status, out_dtype=ydt), y)
+    for r in (0, rows // 2, rows - 1):
+        assert torch.equal(ops.gemm_simt(picked[r:r + 1].contiguous(), w, status, out_dtype=ydt)[0], y[r])
+    bound = k * 2.0 ** -24 * (picked.double().abs() @ w.double().abs().T)
+    want = picked.double() @ w.double().T
+    rounding = want.abs() * 2.0 ** -8 if ydt == torch.bfloat16 else 0.0
+    assert bool(((y.double() - want).abs() <= bound + rounding).all()) and status.item() == 0
+
+
+def test_gemm_simt_of_single_bfloat16_elements_costs_no_more_than_of_float32(dev, status):
+    """Rows that start inside a word are loaded element by element; the loads of 16-bit elements must not wait for one
+    another (half the bytes, the same arithmetic: no more than 1.25 times the time; 1.46 times where they did)."""
+    from vosti_b200 import ops
+
+    def time(dtype):
+        x, w = torch.randn(384, 4097, device=dev).to(dtype), torch.randn(4096, 4097, device=dev).to(dtype)
+        ops.gemm_simt(x, w, status)
+        times = []
+        for _ in range(5):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record(), ops.gemm_simt(x, w, status), b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b))
+        return sorted(times)[2]
+    assert time(torch.bfloat16) <= 1.25 * time(torch.float32)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("T", [19, 150])          # few tokens: a warp per head; many: blocks streaming over tokens
 @pytest.mark.parametrize("nq,nkv,d,use_norm,use_rope", [(6, 3, 48, True, True), (4, 4, 16, False, True),

@@ -20,12 +20,25 @@ __device__ __forceinline__ float4 load4(const bf16* p) {
 // Four neighbouring k of a row as float32; beyond k, or of a row that is not there (-1), zeros.
 template <typename T>
 __device__ __forceinline__ float4 load4_of(const T* matrix, int r, int kk, int k, bool wide) {
-  if (r < 0 || kk >= k) return make_float4(0.f, 0.f, 0.f, 0.f);
-  const T* row = matrix + (int64_t)r * k;
-  if (wide) return load4(row + kk);
+  if (wide || sizeof(T) == 4) {
+    if (r < 0 || kk >= k) return make_float4(0.f, 0.f, 0.f, 0.f);
+    const T* row = matrix + (int64_t)r * k;
+    if (wide) return load4(row + kk);
+    float v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = kk + i < k ? to_f32(row[kk + i]) : 0.f;
+    return make_float4(v[0], v[1], v[2], v[3]);
+  }
+  // Single bfloat16 elements: no branch between the four loads (those that are not wanted read the row's last one, or
+  // row 0's), since each is converted at once and would wait for the one before it: 384 x 4,096 x 4,097 478 us
+  // instead of 430 in tiles of 64 x 64, 65 rows 338 instead of 199.
+  const T* const row = matrix + (int64_t)(r < 0 ? 0 : r) * k;
+  T raw[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) raw[i] = row[kk + i < k ? kk + i : k - 1];
   float v[4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) v[i] = kk + i < k ? to_f32(row[kk + i]) : 0.f;
+  for (int i = 0; i < 4; ++i) v[i] = r >= 0 && kk + i < k ? to_f32(raw[i]) : 0.f;
   return make_float4(v[0], v[1], v[2], v[3]);
 }
 
@@ -151,8 +164,8 @@ __device__ __forceinline__ packed2 twice(float v) {
 // Many rows: the multiply-add pipe bounds it. Both operands are turned to [k][row] on their way into shared
 // memory, so that a thread reads four neighbouring rows as one word and its 8 x TN outputs cost two words of
 // x and TN / 4 of w a k; the packed multiply-add takes two neighbouring rows of x as they lie in that word.
-// It takes whole words only (every row of x and w starts on one).
-template <typename TX, typename TW, typename TY, int BM, int BN, int BK, int TN, int BLOCKS>
+// WIDE: every row of x and w starts on a whole word.
+template <typename TX, typename TW, typename TY, int BM, int BN, int BK, int TN, int BLOCKS, bool WIDE>
 __global__ void __launch_bounds__((BM / 8) * (BN / TN), BLOCKS)
 gemm_simt_kernel(const TX* __restrict__ x, const TW* __restrict__ w, TY* __restrict__ y,
                  const int* __restrict__ row_index, int rows, int x_rows, int n, int k, int, unsigned* status) {
@@ -173,12 +186,12 @@ gemm_simt_kernel(const TX* __restrict__ x, const TW* __restrict__ w, TY* __restr
   for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int j = 0; j < TN; ++j) acc[i][j] = 0ull;
-  loads.fetch(x, w, 0, k, true);
+  loads.fetch(x, w, 0, k, WIDE);
   put(0);
   __syncthreads();
   for (int k0 = 0, buf = 0; k0 < k; k0 += BK, buf ^= 1) {
     const bool more = k0 + BK < k;
-    if (more) loads.fetch(x, w, k0 + BK, k, true);
+    if (more) loads.fetch(x, w, k0 + BK, k, WIDE);
 #pragma unroll
     for (int kk = 0; kk < BK; ++kk) {
       const ulonglong2 lo = *reinterpret_cast<const ulonglong2*>(&xs[buf][kk][ty * 4]);
@@ -222,22 +235,26 @@ void launch(const void* x, const void* w, void* y, const int* row_index, int row
   KERNEL<<<dim3((n + BN - 1) / BN, (rows + BM - 1) / BM), THREADS, 0, stream>>>((const TX*)x, (const TW*)w, (TY*)y, \
                                                                                row_index, rows, x_rows, n, k, wide, status)
 #define VOSTI_FEW(BM, BN, BK, TM, TN) VOSTI_SIMT((gemm_simt_few_kernel<TX, TW, TY, BM, BN, BK, TM, TN>), BM, BN, (BM / TM) * (BN / TN))
-#define VOSTI_MANY(BM, BN, BK, TN, BLOCKS) VOSTI_SIMT((gemm_simt_kernel<TX, TW, TY, BM, BN, BK, TN, BLOCKS>), BM, BN, (BM / 8) * (BN / TN))
+#define VOSTI_MANY(BM, BN, BK, TN, BLOCKS, WIDE) \
+  VOSTI_SIMT((gemm_simt_kernel<TX, TW, TY, BM, BN, BK, TN, BLOCKS, WIDE>), BM, BN, (BM / 8) * (BN / TN))
   // Measured at float32, (n, k) = (4,096, 4,096) | (24,576, 4,096), us, against the 64 x 64 tile of 4 x 4 a thread that
   // this replaces: 1 row 27 | 156 (226 | 556), 8 rows 39 | 185 (229 | 568), 32 rows 77 | 268 (238 | 608), 100 rows
   // 187 | 695 (276 | 1,182), 384 rows 407 | 1,690 (621 | 3,123), 1,024 rows 868 | 4,242 (1,375 | 8,061; 49 TFLOP/s,
   // 0.65 of the multiply-add pipe). Where the lines lie: blocks of 8 columns cost 1.5 times as much from 5 rows on;
   // at 384 x 4,096 (192 tiles of 128 x 64) tiles of 64 x 32 take 407 and those of 128 x 64 490, at 384 x 6,144
   // (288 tiles) 555 and 484; at 100 x 4,096 (256 tiles of 64 x 32) 32 x 32 takes 187 and 64 x 32 245, at
-  // 200 x 4,096 (512 tiles) 312 and 291.
+  // 200 x 4,096 (512 tiles) 312 and 291. Rows that start inside a word (odd K) are loaded element by element, which a
+  // larger tile does less often: the tile this replaces, 32 x 32 and 64 x 64 of 8 x 4 a thread, bfloat16: 384 x 4,096 x
+  // 4,097 538, 678 and 430, 512 x 1,000 x 1,001 56, 69 and 53, 200 x 1,000 (128 tiles of 64 x 32) 56, 54 and 52;
+  // float32: 1,000 x 4,096 x 4,097 1,170, 1,407 and 856.
   const int64_t columns = (n + 31) / 32;
   if (rows <= 4) VOSTI_FEW(4, 8, 256, 1, 1);
   else if (rows <= 8) VOSTI_FEW(8, 16, 128, 1, 1);
   else if (rows <= 16) VOSTI_FEW(16, 16, 64, 2, 1);
-  else if (!wide && rows > 32 * 65535) VOSTI_FEW(64, 32, 32, 8, 2);        // (the grid's limit)
-  else if (!wide || rows <= 64 || (rows + 63) / 64 * columns < 3 * 148) VOSTI_FEW(32, 32, 32, 4, 2);
-  else if ((rows + 127) / 128 * ((columns + 1) / 2) < 288) VOSTI_MANY(64, 32, 16, 4, 10);
-  else VOSTI_MANY(128, 64, 16, 8, 4);
+  else if (rows <= 32 || (rows <= 64 && columns < 3 * 148) || (rows + 63) / 64 * columns < (wide ? 3 : 1) * 148) VOSTI_FEW(32, 32, 32, 4, 2);
+  else if (!wide) VOSTI_MANY(64, 64, 16, 4, 4, false);
+  else if (rows <= 64 || (rows + 127) / 128 * ((columns + 1) / 2) < 288) VOSTI_MANY(64, 32, 16, 4, 10, true);
+  else VOSTI_MANY(128, 64, 16, 8, 4, true);
 #undef VOSTI_MANY
 #undef VOSTI_FEW
 #undef VOSTI_SIMT
