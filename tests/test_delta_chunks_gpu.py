@@ -120,6 +120,44 @@ def test_a_token_that_is_not_finite_reaches_no_earlier_one(monkeypatch, rule):
         assert torch.equal(out[:45], outs[0][:45]) and not torch.isfinite(out[45:]).any()
 
 
+@pytest.mark.parametrize("rule", ["gated", "general"])
+def test_rounds_of_chunks_give_the_same_bits(monkeypatch, rule):
+    """Chunks that don't fit the scratch together run in rounds that may end anywhere in a request."""
+    monkeypatch.setattr(ops, "delta_takes_chunks", lambda *a: True)
+    gen = torch.Generator().manual_seed(4)
+    lengths, heads, dv = (150, 7, 64, 49, 260), 2, 128
+    ins = inputs(rule, sum(lengths), heads, heads, dv, "mixed", gen)
+    starts = torch.randn(len(lengths), heads * dv * DK, generator=gen)
+    got = []
+    for chunks in (100, 1, 4, 7):
+        monkeypatch.setattr(ops, "DELTA_SCRATCH", chunks * ops.library().vosti_delta_chunk_floats(heads, dv, int(rule == "general")))
+        harness = Harness([None], [StateSpec((heads * DK * dv,), torch.float32)], torch.float32, max_requests=len(lengths))
+        ctx = harness.context([StepEntry(i, [0] * n) for i, n in enumerate(lengths)])
+        state = harness.cache.layer_caches[0].state
+        for i, slot in enumerate(ctx.host_state_slots):
+            state[slot] = starts[i].to(DEV)
+        out = scan(rule, ins, harness, ctx, heads, heads, dv)
+        got.append((out, state[ctx.host_state_slots].clone()))
+    assert all(torch.equal(a, b) for other in got[1:] for a, b in zip(got[0], other))
+
+
+def test_scratch_is_bounded(monkeypatch):
+    """12,000 tokens of 16 heads would take 396 MB of chunks at once; a layer never takes more than 256."""
+    monkeypatch.setattr(ops, "delta_takes_chunks", lambda *a: True)
+    T, heads, kv = 12000, 16, 4
+    harness = Harness([None], [StateSpec((heads * DK * 128,), torch.float32)], torch.float32)
+    ctx = harness.context([StepEntry("r", [0] * T)])
+    r = lambda *s: torch.rand(*s, device=DEV)
+    q, k, v, beta, g = r(T, kv * DK) / 20, r(T, kv * DK) / 20, r(T, heads * 128), r(T, heads), r(T, heads * DK)
+    torch.cuda.synchronize()
+    held = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    out = ops.delta_scan(q, k, v, beta, g, harness.cache.layer_caches[0].state, ctx, kv_heads=kv, heads=heads, dk=DK, dv=128)
+    peak = torch.cuda.max_memory_allocated() - held
+    # (the allocator hands out large blocks in whole 2 MB: up to that much more for each of the two)
+    assert peak <= out.numel() * 4 + (256 << 20) + (4 << 20) and torch.isfinite(out).all()
+
+
 def near(got, want):
     """float32 sums of at most 128 terms and elementary functions against float64: some tens of roundings."""
     return torch.allclose(got.double().cpu(), want, rtol=64 * 2.0 ** -24, atol=64 * 2.0 ** -24)

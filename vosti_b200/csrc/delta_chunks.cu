@@ -49,6 +49,7 @@ struct ChunkArgs {
   int num_slots;
   const int *chunk_request, *chunk_first;        // per chunk: its request and its first token in the portion
   const int *long_requests, *long_chunk0;        // per long request: its number and its first chunk
+  int from, count;                               // this launch's chunks; the scratch holds them, from 0 on
   float *wo, *ends, *us, *gammas;                // [chunk, head, DK, WO], [.., (2) CHUNK, DK], [.., CHUNK, dv], [.., DK]
 };
 
@@ -108,7 +109,7 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_prepare_kernel(ChunkArgs a
   float* const sbeta = extra + (PAIR ? 0 : 2 * HALF * PITCH);
   pdl_wait();
   pdl_launch_dependents();
-  const int chunk = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int chunk = a.from + blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int request = a.chunk_request[chunk], first = a.chunk_first[chunk];
   const int64_t t0 = a.cu_q[request] + first;
   const int count = min(CHUNK, a.cu_q[request + 1] - a.cu_q[request] - first);
@@ -252,7 +253,7 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_prepare_kernel(ChunkArgs a
 
   const float* const MA = mats;
   const float* const MQ = mats + CHUNK * CHUNK;
-  const int64_t place = (int64_t)chunk * a.heads + h;
+  const int64_t place = (int64_t)blockIdx.x * a.heads + h;
   if (tid < DK) {
     const int c = tid;
     float w[CHUNK], gamma = 1.f, first_half = 1.f;
@@ -334,19 +335,21 @@ __global__ void __launch_bounds__(RUN_THREADS) delta_chunk_run_kernel(ChunkArgs 
   const int slot = a.state_slots[request];
   if (slot < 0 || slot >= a.num_slots) return;
   const int start = a.cu_q[request], n = a.cu_q[request + 1] - start, chunks = (n + CHUNK - 1) / CHUNK;
-  const int64_t place0 = (int64_t)a.long_chunk0[blockIdx.x];
+  const int place0 = a.long_chunk0[blockIdx.x] - a.from;         // of the request's first chunk in the scratch
+  const int begin = max(0, -place0), end = min(chunks, a.count - place0);
+  if (begin >= end) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t row = (int64_t)a.heads * a.dv;
   float* const state = a.state + (int64_t)slot * a.state_stride + ((int64_t)h * a.dv + col0) * DK;
   for (int i = tid; i < COLS * DK; i += RUN_THREADS) S[(i % DK) * S_PITCH + i / DK] = state[i];
 
   auto load = [&](int chunk) {
-    if (chunk < chunks) {
+    if (chunk < end) {
       float* const wo = chunk_shared + chunk % STAGES * STAGE;
       float* const ends = wo + DK * WO_PITCH;
       float* const uv = ends + ROWS * DK;
       float* const gam = uv + ROWS * S_PITCH;
-      const int64_t place = (place0 + chunk) * a.heads + h;
+      const int64_t place = (int64_t)(place0 + chunk) * a.heads + h;
       for (int i = tid; i < DK * (WO / 4); i += RUN_THREADS) {
         const int r = i / (WO / 4), c = (i % (WO / 4)) * 4;
         copy16(wo + r * WO_PITCH + c, a.wo + (place * DK + r) * WO + c);
@@ -364,13 +367,13 @@ __global__ void __launch_bounds__(RUN_THREADS) delta_chunk_run_kernel(ChunkArgs 
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
 #pragma unroll
-  for (int i = 0; i < STAGES - 1; ++i) load(i);
+  for (int i = 0; i < STAGES - 1; ++i) load(begin + i);
   // [W; O1] S: lane = 8 summands' groups x 4 tiles of 8 rows x 4 columns
   const int kg = lane & 7, rt = warp, ct = lane >> 3;
   // the update: lane = 4 groups of tokens x 8 tiles of 8 key channels (4 and 4) x 4 columns
   const int tg = lane >> 3, kt = (warp >> 2) * 8 + (lane & 7), ct2 = warp & 3;
 #pragma unroll 1
-  for (int chunk = 0; chunk < chunks; ++chunk) {
+  for (int chunk = begin; chunk < end; ++chunk) {
     load(chunk + STAGES - 1);
     const float* const wo = chunk_shared + chunk % STAGES * STAGE;
     const float* const ends = wo + DK * WO_PITCH;
@@ -461,7 +464,7 @@ __global__ void __launch_bounds__(RUN_THREADS) delta_chunk_run_kernel(ChunkArgs 
 }
 
 template <bool PAIR>
-int launch_chunks(const ChunkArgs& a, int chunks, int longs, cudaStream_t stream) {
+int launch_chunks(ChunkArgs a, int chunks, int fit, int longs, cudaStream_t stream) {
   constexpr int prepare_bytes = prepare_floats<PAIR>() * (int)sizeof(float);
   constexpr int run_bytes = (RUN_STAGES<PAIR> * STAGE_FLOATS<PAIR> + DK * S_PITCH) * (int)sizeof(float);
   static bool configured = false;
@@ -470,11 +473,16 @@ int launch_chunks(const ChunkArgs& a, int chunks, int longs, cudaStream_t stream
     cudaFuncSetAttribute(delta_chunk_run_kernel<PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, run_bytes);
     configured = true;
   }
-  vosti_launch(delta_chunk_prepare_kernel<PAIR>, dim3(chunks, a.heads), dim3(256), prepare_bytes, stream, a);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) { vosti_set_error("%s", cudaGetErrorString(e)); return (int)e; }
-  vosti_launch(delta_chunk_run_kernel<PAIR>, dim3(longs, a.heads, a.dv / COLS), dim3(RUN_THREADS), run_bytes, stream, a);
-  VOSTI_LAUNCH_CHECK();
+  for (a.from = 0; a.from < chunks; a.from += fit) {            // (a request's state waits in its slot between two rounds)
+    a.count = chunks - a.from < fit ? chunks - a.from : fit;
+    vosti_launch(delta_chunk_prepare_kernel<PAIR>, dim3(a.count, a.heads), dim3(256), prepare_bytes, stream, a);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) { vosti_set_error("%s", cudaGetErrorString(e)); return (int)e; }
+    vosti_launch(delta_chunk_run_kernel<PAIR>, dim3(longs, a.heads, a.dv / COLS), dim3(RUN_THREADS), run_bytes, stream, a);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) { vosti_set_error("%s", cudaGetErrorString(e)); return (int)e; }
+  }
+  return VOSTI_OK;
 }
 
 }  // namespace
@@ -489,27 +497,30 @@ VOSTI_API int64_t vosti_delta_chunk_floats(int heads, int dv, int pair) {
 
 // The recurrence over the requests `long_requests`. Gated rule: x = k and y = q [tokens, x_heads, 128], beta
 // [tokens, heads], b and k null. Generalized rule: x = removal, b = unit, k, y = r (x_heads = heads), beta null.
+// `scratch` has room for `fit` chunks: with fewer than there are, they run in rounds of so many (two launches each).
 VOSTI_API int vosti_delta_chunks(const float* x, const float* y, const float* decay, const float* b, const float* k, const float* v,
                                  const float* beta, int x_heads, int heads, int dk, int dv, float* out, float* state,
                                  int64_t state_stride, const int* cu_q, const int* state_slots, int num_slots,
                                  const int* chunk_request, const int* chunk_first, int chunks, const int* long_requests,
-                                 const int* long_chunk0, int longs, float* scratch, cudaStream_t stream) {
+                                 const int* long_chunk0, int longs, float* scratch, int fit, cudaStream_t stream) {
   VOSTI_REQUIRE(vosti_delta_chunk_fits(heads, dk, dv) && x_heads > 0 && heads % x_heads == 0, "delta_chunks: head sizes it does not take");
   VOSTI_REQUIRE((b == nullptr) == (k == nullptr) && (b == nullptr) == (beta != nullptr), "delta_chunks: one rule or the other");
   VOSTI_REQUIRE(state_stride % 4 == 0 && ((reinterpret_cast<uintptr_t>(state) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) |
                 reinterpret_cast<uintptr_t>(decay) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
                 reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(scratch)) & 15) == 0, "delta_chunks: operands start on 16-byte boundaries");
   if (chunks == 0 || longs == 0) return VOSTI_OK;
+  VOSTI_REQUIRE(scratch != nullptr && fit > 0, "delta_chunks: no scratch");
+  if (fit > chunks) fit = chunks;
   ChunkArgs a = {};
   a.x = x; a.y = y; a.g = decay; a.b = b; a.k = k; a.v = v; a.beta = beta;
   a.x_heads = x_heads; a.heads = heads; a.dv = dv;
   a.out = out; a.state = state; a.state_stride = state_stride;
   a.cu_q = cu_q; a.state_slots = state_slots; a.num_slots = num_slots;
   a.chunk_request = chunk_request; a.chunk_first = chunk_first; a.long_requests = long_requests; a.long_chunk0 = long_chunk0;
-  const int64_t places = (int64_t)chunks * heads;
+  const int64_t places = (int64_t)fit * heads;
   a.wo = scratch;
   a.ends = a.wo + places * DK * WO;
   a.us = a.ends + places * (b != nullptr ? 2 : 1) * CHUNK * DK;
   a.gammas = a.us + places * CHUNK * dv;
-  return b != nullptr ? launch_chunks<true>(a, chunks, longs, stream) : launch_chunks<false>(a, chunks, longs, stream);
+  return b != nullptr ? launch_chunks<true>(a, chunks, fit, longs, stream) : launch_chunks<false>(a, chunks, fit, longs, stream);
 }

@@ -1743,6 +1743,7 @@ def delta_prep(proj: torch.Tensor, rates: torch.Tensor, offsets: dict, *, kv_hea
 
 DELTA_CHUNK = 32     # tokens of a chunk (csrc/delta_chunks.cu)
 DELTA_SHORT = 48     # requests that bring at most this many tokens are always served token by token
+DELTA_SCRATCH = 1 << 26      # floats (256 MB) of scratch at most: about 8,000 tokens of 16 heads of 128; more chunks run in rounds
 
 
 def delta_takes_chunks(longest: int, tokens: int, chunks: int, width: float, pair: bool) -> bool:
@@ -1786,12 +1787,14 @@ def _delta_chunks(ctx, x, y, decay, b, k, v, beta, out, state, x_heads: int, hea
         return 0
     plan, chunks, longs = ctx.extras["delta.plan"], layout["chunks"], layout["longs"]
     at = lambda i: ctypes.c_void_p(plan.data_ptr() + 4 * i)
-    scratch = torch.empty(chunks * lib.vosti_delta_chunk_floats(heads, dv, int(b is not None)), dtype=torch.float32, device=out.device)
+    each = lib.vosti_delta_chunk_floats(heads, dv, int(b is not None))
+    fit = max(1, min(chunks, DELTA_SCRATCH // each))
+    scratch = torch.empty(fit * each, dtype=torch.float32, device=out.device)
     _check(lib.vosti_delta_chunks(
         _p(x), _p(y), _p(decay), _p(b), _p(k), _p(v), _p(beta), x_heads, heads, dk, dv, _p(out), _p(state), ctypes.c_int64(state.shape[1]),
         _p(ctx.cu_q), _p(ctx.state_slots), state.shape[0], at(0), at(chunks), chunks, at(2 * chunks),
-        at(2 * chunks + longs), longs, _p(scratch), _stream()),
-        "delta_chunks", kernels=2)
+        at(2 * chunks + longs), longs, _p(scratch), fit, _stream()),
+        "delta_chunks", kernels=2 * -(-chunks // fit))
     return DELTA_SHORT if layout["shorts"] else -1
 
 
