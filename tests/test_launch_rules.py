@@ -137,6 +137,33 @@ def test_cuda_core_attention_takes_the_way_that_was_measured_faster():
     assert simt_way([128] + [0] + [9], [128, 50, 9], 32, 8, window=40) == 1
 
 
+def test_delta_rules_take_the_form_that_was_measured_faster():
+    """Steps (heads, values a head, tokens of the requests) on both sides of the line between chunks and token by token, for
+    both rules; chunks are taken nowhere that they were measured slower."""
+    from vosti_b200.ops import delta_step_layout, delta_takes_chunks
+    takes = lambda pair, heads, dv, q: delta_takes_chunks(delta_step_layout(q)[1], heads, dv, pair)
+    gated = {True: [(16, 128, [96]), (16, 128, [256]), (16, 128, [2048]), (16, 128, [128] * 2), (16, 128, [256] * 4), (16, 128, [1031, 700, 317]),
+                    (16, 128, [300] + [1] * 30), (4, 128, [96]), (4, 128, [128]), (4, 128, [256] * 8), (2, 128, [128] * 2), (8, 128, [128] * 4),
+                    (32, 128, [256]), (32, 128, [700]), (16, 64, [128] * 2), (8, 256, [128]), (64, 128, [256])],
+             False: [(16, 128, [49]), (16, 128, [64]), (16, 128, [64] * 4), (16, 128, [256] * 8), (16, 128, [256] * 16), (16, 128, [64] * 16),
+                     (8, 256, [96]), (8, 256, [96] * 4), (32, 128, [96] * 4), (16, 64, [256] * 8), (64, 128, [128] * 4), (64, 128, [64] + [1] * 30),
+                     (4, 128, [49])]}
+    general = {True: [(16, 128, [256]), (16, 128, [2048]), (16, 128, [128] * 2), (16, 128, [96] * 4), (16, 128, [128] * 4), (16, 128, [256] * 16),
+                      (16, 128, [1031, 700, 317]), (4, 128, [128]), (4, 128, [256]), (8, 128, [128] * 4), (32, 128, [128]), (32, 128, [256] * 8),
+                      (4, 128, [300] + [1] * 30), (64, 128, [128])],
+               False: [(16, 128, [49]), (16, 128, [96]), (4, 128, [64]), (4, 128, [96] * 4), (16, 128, [64] * 16), (32, 128, [64] * 16),
+                       (32, 128, [128] * 16), (64, 128, [96] * 8), (64, 128, [64] * 4), (4, 128, [64] + [1] * 30), (4, 128, [100] + [48] * 8)]}
+    for pair, table in ((False, gated), (True, general)):
+        for want, steps in table.items():
+            for step in steps:
+                assert takes(pair, *step) == want, (pair, step)
+    arrays, values = delta_step_layout([20, 70, 100, 1])
+    assert values == {"chunks": 7, "longs": 2, "shorts": 2, "longest": 100, "tokens": 170, "short_longest": 20, "short_tokens": 21}
+    assert arrays["plan"] == [2] * 4 + [1] * 3 + [0, 32, 64, 96, 0, 32, 64] + [2, 1] + [0, 4]
+    assert delta_step_layout([1, 48, 3]) == ({}, {"chunks": 0, "longs": 0, "shorts": 3, "longest": 0, "tokens": 0, "short_longest": 48,
+                                                  "short_tokens": 52})
+
+
 def test_weight_bytes_of_a_decode_step_in_closed_form():
     """What bench.py counts as the weights a decode step must read: every tensor the model
     expects except the embedding table (read by rows), two bytes each. For the 8B sizes that is

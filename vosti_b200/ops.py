@@ -1746,16 +1746,31 @@ DELTA_SHORT = 48     # requests that bring at most this many tokens are always s
 DELTA_SCRATCH = 1 << 26      # floats (256 MB) of scratch at most: about 8,000 tokens of 16 heads of 128; more chunks run in rounds
 
 
-def delta_takes_chunks(longest: int, tokens: int, chunks: int, width: float, pair: bool) -> bool:
-    """Whether the chunked kernels are the faster way for a step's long portions: `longest` and `tokens` of them, cut into
-    `chunks`; `width` is heads * dv over the 16 * 128 measured, `pair` the generalized rule. Token by token a
-    step takes its longest portion's chain plus a share of the GPU a token; chunks take about 4 us (5.2) each when all of a
-    chunk's heads fill the GPU, 3 us when they do not, and two launches. Measured at 16 heads of 128, us, tokens
-    and chunks: gated, one request of 64: 24 and 29, 96: 35 and 32, 256: 89 and 47; four of 128: 81 and 77; sixteen
-    of 256: 462 and 533. Generalized, one of 96: 37 and 45, 128: 48 and 49; four of 96: 99 and 85; sixteen of 256: 801 and 687."""
-    one_by_one = (0.18 * longest + 0.184 * width * tokens) if pair else (0.25 * longest + 0.097 * width * tokens)
-    each, fixed = (5.2, 33.0) if pair else (4.0, 23.0)
-    return fixed + max(0.75 * each * -(-longest // DELTA_CHUNK), each * width * chunks) < 0.95 * one_by_one
+def delta_takes_chunks(layout: dict, heads: int, dv: int, pair: bool) -> bool:
+    """Whether the chunked kernels are the faster way for a step laid out by `delta_step_layout` (`pair`: the generalized rule).
+    Both sides in us, fitted to sweeps of 2 to 64 heads of 128 (values of 64, 128 and 256), 1 to 16 long requests of 49 to
+    2,048 tokens and shorter ones beside them. Token by token a step takes its longest portion's chain or, with
+    more blocks than the GPU holds, a share of the GPU a token. Chunks take two launches, the longest portion's chunks
+    in turn or a share of the GPU a chunk, the preparation of all of them, and one more launch for the short requests.
+    Where both are close, token by token stays. Measured, tokens and chunks, 16 heads: gated, one request of 64: 24 and
+    29, 96: 35 and 33, 256: 89 and 47; two of 128 58 and 49; sixteen of 256 461 and 533. Generalized, one of 96: 37 and 45, 128: 49 and 49;
+    two of 128 95 and 65; four of 96 99 and 85; sixteen of 64 208 and 229. 4 heads, one of 128: gated 44 and 27, generalized 45 and 37.
+    (What single tokens cost a chain beside them is put too low: a portion of 64 beside 30 stays with 59 us, chunks take 41.)"""
+    launch, chain, long, share, each = (1.4, 0.34, 0.258, 0.174, 1.04) if pair else (1.2, 0.335, 0.254, 0.089, 1.16)
+    width = heads * dv / 2048
+    rounds = layout["longs"] * width                     # blocks of the chunks' run, in 128
+
+    def one_by_one(longest, tokens, requests):
+        return launch + max(chain * longest, long * longest + width * (share * tokens + each * requests)) if requests else 0.0
+    launch2, turn, part, prepare, full, third, start = (22.3, 3.27, 3.78, 20.1, 3.2, 5.8, 1.96) if pair else (14.9, 2.79, 3.09, 12.2, 3.2, 0.0, 1.52)
+    chunks, longs, shorts = layout["chunks"], layout["longs"], layout["shorts"]
+    cost = launch2 + max(turn * -(-layout["longest"] // DELTA_CHUNK), part * width * chunks + start * rounds) + prepare * heads * chunks / 296
+    cost += 5.0 * ((dv - 1) // 128)                      # (the preparation takes 128 value columns at a time)
+    cost += full * min(1.0, max(0.0, (128 * rounds + heads * chunks - 96) / 64))          # (beyond that the two launches don't overlap)
+    if shorts:
+        cost += third + one_by_one(layout["short_longest"], layout["short_tokens"], shorts)
+    tokens = one_by_one(layout["longest"], layout["tokens"] + layout["short_tokens"], longs + shorts)
+    return cost < (0.88 if rounds > 24 else 0.95 if pair else 0.97) * tokens
 
 
 def delta_step_layout(q_lens):
@@ -1772,8 +1787,9 @@ def delta_step_layout(q_lens):
     # one array: per chunk its request, then its first token, then the long requests, then their first chunks
     arrays = {"plan": requests + firsts + longs + starts} if longs else {}
     lengths = [q_lens[i] for i in longs]
-    return arrays, {"chunks": len(requests), "longs": len(longs), "shorts": len(q_lens) - len(longs),
-                    "longest": max(lengths, default=0), "tokens": sum(lengths)}
+    short = [n for n in q_lens if n <= DELTA_SHORT] if longs else q_lens
+    return arrays, {"chunks": len(requests), "longs": len(longs), "shorts": len(short), "longest": max(lengths, default=0),
+                    "tokens": sum(lengths), "short_longest": max(short, default=0), "short_tokens": sum(short)}
 
 
 def _delta_chunks(ctx, x, y, decay, b, k, v, beta, out, state, x_heads: int, heads: int, dk: int, dv: int) -> int:
@@ -1783,7 +1799,7 @@ def _delta_chunks(ctx, x, y, decay, b, k, v, beta, out, state, x_heads: int, hea
     lib = library()
     if layout is None or layout["longs"] == 0 or not lib.vosti_delta_chunk_fits(heads, dk, dv):
         return 0
-    if not delta_takes_chunks(layout["longest"], layout["tokens"], layout["chunks"], heads * dv / 2048, b is not None):
+    if not delta_takes_chunks(layout, heads, dv, b is not None):
         return 0
     plan, chunks, longs = ctx.extras["delta.plan"], layout["chunks"], layout["longs"]
     at = lambda i: ctypes.c_void_p(plan.data_ptr() + 4 * i)
