@@ -120,6 +120,31 @@ def test_a_token_that_is_not_finite_reaches_no_earlier_one(monkeypatch, rule):
         assert torch.equal(out[:45], outs[0][:45]) and not torch.isfinite(out[45:]).any()
 
 
+@pytest.mark.parametrize("rule,lengths,chunks", [("gated", (49, 3), False), ("gated", (300, 1), True), ("general", (64,), False),
+                                                 ("general", (700, 20), True), ("gated", (1000,), True)])
+def test_the_rule_itself_chooses(monkeypatch, rule, lengths, chunks):
+    """Steps with long portions that the rule leaves token by token, and others: which kernels run, and what comes out."""
+    gen = torch.Generator().manual_seed(len(lengths))
+    heads, dv = 2, 128
+    ins = inputs(rule, sum(lengths), heads, heads, dv, "mixed", gen)
+    calls = []
+    monkeypatch.setattr(ops, "_check", lambda code, what, kernels=1, check=ops._check: (calls.append(what), check(code, what, kernels))[1])
+    got = []
+    for laid_out in (True, False):
+        harness = Harness([None], [StateSpec((heads * DK * dv,), torch.float32)], torch.float32, max_requests=len(lengths))
+        ctx = harness.context([StepEntry(i, [0] * n) for i, n in enumerate(lengths)])
+        assert ctx.layout["delta"]["longs"] > 0
+        if not laid_out:
+            ctx.layout = {}
+        del calls[:]
+        out = scan(rule, ins, harness, ctx, heads, heads, dv)
+        got.append((out, harness.cache.layer_caches[0].state[ctx.host_state_slots].clone()))
+        assert ("delta_chunks" in calls) == (chunks and laid_out), calls
+        assert len(calls) == (2 if chunks and laid_out and min(lengths) <= ops.DELTA_SHORT else 1)
+    for a, b in zip(*got):           # (two float32 evaluations of sums whose terms cancel by a few hundred times at most)
+        assert torch.allclose(a, b, rtol=1e-4, atol=1e-4) if chunks else torch.equal(a, b)
+
+
 @pytest.mark.parametrize("rule", ["gated", "general"])
 def test_rounds_of_chunks_give_the_same_bits(monkeypatch, rule):
     """Chunks that don't fit the scratch together run in rounds that may end anywhere in a request."""

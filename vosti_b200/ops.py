@@ -1777,19 +1777,19 @@ def delta_step_layout(q_lens):
     """How the delta rules may divide a step (registered with the step layout as "delta"): the requests that bring more than
     DELTA_SHORT tokens are cut into chunks, the longest first (a layer takes them if `delta_takes_chunks`), the others
     go token by token; with one order of arithmetic asked for (set_fixed_order) all of them do."""
+    if FIXED_ORDER or max(q_lens, default=0) <= DELTA_SHORT:          # (every decode step, whatever the model)
+        return {}, {"chunks": 0, "longs": 0, "shorts": len(q_lens)}
     requests, firsts, longs, starts = [], [], [], []
-    if not FIXED_ORDER and max(q_lens, default=0) > DELTA_SHORT:
-        for n, i in sorted(((n, i) for i, n in enumerate(q_lens) if n > DELTA_SHORT), key=lambda e: (-e[0], e[1])):
-            longs.append(i)
-            starts.append(len(requests))
-            requests.extend([i] * -(-n // DELTA_CHUNK))
-            firsts.extend(range(0, n, DELTA_CHUNK))
+    for n, i in sorted(((n, i) for i, n in enumerate(q_lens) if n > DELTA_SHORT), key=lambda e: (-e[0], e[1])):
+        longs.append(i)
+        starts.append(len(requests))
+        requests.extend([i] * -(-n // DELTA_CHUNK))
+        firsts.extend(range(0, n, DELTA_CHUNK))
+    lengths, short = [q_lens[i] for i in longs], [n for n in q_lens if n <= DELTA_SHORT]
     # one array: per chunk its request, then its first token, then the long requests, then their first chunks
-    arrays = {"plan": requests + firsts + longs + starts} if longs else {}
-    lengths = [q_lens[i] for i in longs]
-    short = [n for n in q_lens if n <= DELTA_SHORT] if longs else q_lens
-    return arrays, {"chunks": len(requests), "longs": len(longs), "shorts": len(short), "longest": max(lengths, default=0),
-                    "tokens": sum(lengths), "short_longest": max(short, default=0), "short_tokens": sum(short)}
+    return {"plan": requests + firsts + longs + starts}, {
+        "chunks": len(requests), "longs": len(longs), "shorts": len(short), "longest": lengths[0], "tokens": sum(lengths),
+        "short_longest": max(short, default=0), "short_tokens": sum(short)}
 
 
 def _delta_chunks(ctx, x, y, decay, b, k, v, beta, out, state, x_heads: int, heads: int, dk: int, dv: int) -> int:
