@@ -133,13 +133,6 @@ attention_simt_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, co
   }
 }
 
-__device__ __forceinline__ float4 load_four(const float* p) { return *reinterpret_cast<const float4*>(p); }
-__device__ __forceinline__ float4 load_four(const bf16* p) {
-  const uint2 raw = *reinterpret_cast<const uint2*>(p);
-  const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
-  const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
-  return make_float4(lo.x, lo.y, hi.x, hi.y);
-}
 
 // The same for portions: a block takes up to ROWS (token, head) rows that read one kv head, TOKENS neighbouring tokens of
 // the heads that share it, and stages every tile of 32 keys and values in shared memory once for all of them; a

@@ -156,13 +156,6 @@ __global__ void __launch_bounds__(256) delta_prep_kernel(PrepArgs a) {
 // for 2,048 tokens of 16 heads (4 key heads), against the 16 us its 105 MB take.
 constexpr int WIDE_TAPS = 4;
 
-__device__ __forceinline__ float4 load_four(const float* p) { return *reinterpret_cast<const float4*>(p); }
-__device__ __forceinline__ float4 load_four(const bf16* p) {
-  const uint2 raw = *reinterpret_cast<const uint2*>(p);
-  const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
-  const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
-  return make_float4(lo.x, lo.y, hi.x, hi.y);
-}
 __device__ __forceinline__ void store_four(float* p, const float (&v)[4]) { *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]); }
 __device__ __forceinline__ void spread(float4 v, float (&to)[4]) { to[0] = v.x; to[1] = v.y; to[2] = v.z; to[3] = v.w; }
 

@@ -10,20 +10,13 @@
 
 namespace {
 
-__device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
-__device__ __forceinline__ float4 load4(const bf16* p) {
-  const uint2 raw = *reinterpret_cast<const uint2*>(p);
-  const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
-  const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
-  return make_float4(lo.x, lo.y, hi.x, hi.y);
-}
 // Four neighbouring k of a row as float32; beyond k, or of a row that is not there (-1), zeros.
 template <typename T>
 __device__ __forceinline__ float4 load4_of(const T* matrix, int r, int kk, int k, bool wide) {
   if (wide || sizeof(T) == 4) {
     if (r < 0 || kk >= k) return make_float4(0.f, 0.f, 0.f, 0.f);
     const T* row = matrix + (int64_t)r * k;
-    if (wide) return load4(row + kk);
+    if (wide) return load_four(row + kk);
     float v[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) v[i] = kk + i < k ? to_f32(row[kk + i]) : 0.f;

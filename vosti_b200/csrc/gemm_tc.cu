@@ -611,7 +611,7 @@ VOSTI_API int vosti_gemm_tc_grouped(const void* x, const void* w, void* y, const
   const int splits = vosti_gemm_tc_grouped_splits(tokens, rows, experts, features, k);
   VOSTI_REQUIRE(splits == 1 || (workspace != nullptr && workspace_elems >= (int64_t)splits * rows * features),
                 "gemm_tc_grouped: workspace too small for %d splits", splits);
-  const int bn = token_tile(tokens) < 128 ? token_tile(tokens) : 128;
+  const int bn = token_tile(tokens);
   const int x_rows = (tokens + 7) / 8 * 8 < bn ? (tokens + 7) / 8 * 8 : bn;
   VOSTI_REQUIRE(weight_map(w, w_rows, BK, BM, &mw) && make_map(&mx, x, rows, k, x_rows), "gemm_tc_grouped: cuTensorMapEncodeTiled failed");
   void* dst = splits > 1 ? (void*)workspace : y;

@@ -113,13 +113,6 @@ scan_conv_kernel(const T* __restrict__ xz, int64_t xz_stride, const void* __rest
 // that of the kernel above, operation by operation.
 constexpr int CONV_AHEAD = 4;
 
-__device__ __forceinline__ float4 conv_load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
-__device__ __forceinline__ float4 conv_load4(const bf16* p) {
-  const uint2 raw = *reinterpret_cast<const uint2*>(p);
-  const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
-  const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
-  return make_float4(lo.x, lo.y, hi.x, hi.y);
-}
 __device__ __forceinline__ void conv_store4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
 __device__ __forceinline__ void conv_store4(bf16* p, float4 v) {
   const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
@@ -153,7 +146,7 @@ scan_conv4_kernel(const T* __restrict__ xz, int64_t xz_stride, const void* __res
     float4 x[CONV_AHEAD];
 #pragma unroll
     for (int a = 0; a < CONV_AHEAD; ++a)
-      if (t0 + a < t_end) x[a] = conv_load4(xz + (int64_t)(t0 + a) * xz_stride + c);
+      if (t0 + a < t_end) x[a] = load_four(xz + (int64_t)(t0 + a) * xz_stride + c);
 #pragma unroll
     for (int a = 0; a < CONV_AHEAD; ++a) {
       const int t = t0 + a;
@@ -168,8 +161,8 @@ scan_conv4_kernel(const T* __restrict__ xz, int64_t xz_stride, const void* __res
 #pragma unroll
         for (int k = 1; k < TAPS; ++k) {               // the input k tokens back: of this portion, or from the tail
           const int back = t - first;
-          const float4 v = k <= back ? conv_load4(xz + (int64_t)(t - k) * xz_stride + c)
-                                     : conv_load4(tail + (int64_t)(TAPS - 1 - (k - back)) * inner + c);
+          const float4 v = k <= back ? load_four(xz + (int64_t)(t - k) * xz_stride + c)
+                                     : load_four(tail + (int64_t)(TAPS - 1 - (k - back)) * inner + c);
           win[TAPS - 1 - k][0] = v.x; win[TAPS - 1 - k][1] = v.y; win[TAPS - 1 - k][2] = v.z; win[TAPS - 1 - k][3] = v.w;
         }
       } else {
