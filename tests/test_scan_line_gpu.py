@@ -85,3 +85,25 @@ def test_a_step_without_host_lengths_gives_the_same_bits():
             ctx = replace(ctx, host_q_lens=[], host_kv_lens=[])
         got.append((ops.scan_run(x, dtp, None, bc, a_log, None, xz, state, ctx, inner=inner, states=N), state.clone()))
     assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
+@pytest.mark.parametrize("with_bias,with_skip", [(False, False), (True, False), (False, True)])
+def test_without_step_bias_or_skip(with_bias, with_skip):
+    """One pass over 130 tokens against float64, the optional vectors left out."""
+    gen = torch.Generator().manual_seed(7)
+    normal = lambda *s: torch.randn(*s, generator=gen)
+    T, inner = 130, 2048
+    x, xz, dtp, bc, a_log = normal(T, inner), normal(T, 2 * inner), normal(T, inner) - 2, normal(T, 2 * N), normal(inner, N) * 0.5
+    bias, skip = (normal(inner) if with_bias else None), (normal(inner) if with_skip else None)
+    harness = Harness([None], [StateSpec((inner * N,), torch.float32)], torch.float32)
+    ctx = harness.context([StepEntry("r", [0] * T)])
+    state, d = harness.cache.layer_caches[0].state, lambda t: None if t is None else t.to(DEV)
+    y = ops.scan_run(d(x), d(dtp), d(bias), d(bc), d(a_log), d(skip), d(xz), state, ctx, inner=inner, states=N).double().cpu()
+    S, A, rows = torch.zeros(inner, N, dtype=torch.float64), -torch.exp(a_log.double()), []
+    for t in range(T):
+        dt = torch.nn.functional.softplus(dtp[t].double() + (bias.double() if with_bias else 0.0))
+        S = torch.exp(dt[:, None] * A) * S + (dt * x[t].double())[:, None] * bc[t, :N].double()
+        z = xz[t, inner:].double()
+        rows.append((S @ bc[t, N:].double() + (skip.double() * x[t].double() if with_skip else 0.0)) * z * torch.sigmoid(z))
+    want = torch.stack(rows)
+    assert float((y - want).norm() / want.norm()) <= T ** 0.5 * 2.0 ** -22
