@@ -1799,7 +1799,10 @@ def _delta_chunks(ctx, x, y, decay, b, k, v, beta, out, state, x_heads: int, hea
     lib = library()
     if layout is None or layout["longs"] == 0 or not lib.vosti_delta_chunk_fits(heads, dk, dv):
         return 0
-    if not delta_takes_chunks(layout, heads, dv, b is not None):
+    takes, key = layout.setdefault("takes", {}), (heads, dv, b is not None)      # once a step, not once a layer
+    if key not in takes:
+        takes[key] = delta_takes_chunks(layout, heads, dv, b is not None)
+    if not takes[key]:
         return 0
     plan, chunks, longs = ctx.extras["delta.plan"], layout["chunks"], layout["longs"]
     at = lambda i: ctypes.c_void_p(plan.data_ptr() + 4 * i)
