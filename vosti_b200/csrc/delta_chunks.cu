@@ -23,6 +23,9 @@
 //                         chunk [W; O1] S0 and the state's update, both as 8 x 4 register tiles whose summands
 //                         are spread over 8 (4) lanes
 //
+// The scratch takes 516 floats a token and head (644 in the generalized rule); its caller bounds it and the chunks run in
+// rounds. Which steps come here and which go token by token: delta_takes_chunks in ops.py, with both sides' times.
+//
 // 2,048 tokens of one request, 16 heads of 128: 82 us and 194 us (the token-by-token kernel: 698 us); the
 // generalized rule over 1,031 + 700 + 317 tokens: 140 us and 278 us (628 us). The first is bound by shared-memory
 // latency at two blocks an SM (issue slots 43 % busy), the second by the shared-memory pipe of the 128 SMs that
@@ -334,22 +337,24 @@ __global__ void __launch_bounds__(RUN_THREADS) delta_chunk_run_kernel(ChunkArgs 
   const int request = a.long_requests[blockIdx.x], h = blockIdx.y, col0 = blockIdx.z * COLS;
   const int slot = a.state_slots[request];
   if (slot < 0 || slot >= a.num_slots) return;
-  const int start = a.cu_q[request], n = a.cu_q[request + 1] - start, chunks = (n + CHUNK - 1) / CHUNK;
-  const int place0 = a.long_chunk0[blockIdx.x] - a.from;         // of the request's first chunk in the scratch
-  const int begin = max(0, -place0), end = min(chunks, a.count - place0);
-  if (begin >= end) return;
+  // the request's chunks in this launch: from chunk `begin` on, or from its first one
+  const int chunk0 = a.long_chunk0[blockIdx.x] - a.from, begin = max(0, -chunk0);
+  const int start = a.cu_q[request] + begin * CHUNK, n = min(a.cu_q[request + 1] - start, (a.count - chunk0 - begin) * CHUNK);
+  if (n <= 0) return;
+  const int chunks = (n + CHUNK - 1) / CHUNK;
+  const int64_t place0 = (int64_t)chunk0 + begin;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t row = (int64_t)a.heads * a.dv;
   float* const state = a.state + (int64_t)slot * a.state_stride + ((int64_t)h * a.dv + col0) * DK;
   for (int i = tid; i < COLS * DK; i += RUN_THREADS) S[(i % DK) * S_PITCH + i / DK] = state[i];
 
   auto load = [&](int chunk) {
-    if (chunk < end) {
+    if (chunk < chunks) {
       float* const wo = chunk_shared + chunk % STAGES * STAGE;
       float* const ends = wo + DK * WO_PITCH;
       float* const uv = ends + ROWS * DK;
       float* const gam = uv + ROWS * S_PITCH;
-      const int64_t place = (int64_t)(place0 + chunk) * a.heads + h;
+      const int64_t place = (place0 + chunk) * a.heads + h;
       for (int i = tid; i < DK * (WO / 4); i += RUN_THREADS) {
         const int r = i / (WO / 4), c = (i % (WO / 4)) * 4;
         copy16(wo + r * WO_PITCH + c, a.wo + (place * DK + r) * WO + c);
@@ -367,13 +372,13 @@ __global__ void __launch_bounds__(RUN_THREADS) delta_chunk_run_kernel(ChunkArgs 
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
 #pragma unroll
-  for (int i = 0; i < STAGES - 1; ++i) load(begin + i);
+  for (int i = 0; i < STAGES - 1; ++i) load(i);
   // [W; O1] S: lane = 8 summands' groups x 4 tiles of 8 rows x 4 columns
   const int kg = lane & 7, rt = warp, ct = lane >> 3;
   // the update: lane = 4 groups of tokens x 8 tiles of 8 key channels (4 and 4) x 4 columns
   const int tg = lane >> 3, kt = (warp >> 2) * 8 + (lane & 7), ct2 = warp & 3;
 #pragma unroll 1
-  for (int chunk = begin; chunk < end; ++chunk) {
+  for (int chunk = 0; chunk < chunks; ++chunk) {
     load(chunk + STAGES - 1);
     const float* const wo = chunk_shared + chunk % STAGES * STAGE;
     const float* const ends = wo + DK * WO_PITCH;
