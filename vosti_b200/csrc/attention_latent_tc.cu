@@ -4,8 +4,8 @@
 //
 //   grid = (row tiles x 2 column halves, requests), the tiles with most keys first. A CTA takes 128 consecutive
 //   (token, head) rows of a request and 256 of the 512 columns of the result: the product of all 512 would fill
-//   tensor memory and leave no room for scores, so both halves make the scores (576 of 1,600 multiply-adds a key
-//   and row, the weights counting twice). Its query rows (144 KB) stay in shared memory, which leaves two stages of 32
+//   tensor memory and leave no room for scores, so both halves make the scores (1,152 of the 2,176 multiply-adds issued
+//   a key and row; the others are 512 for each of a weight's two terms). Its query rows (144 KB) stay in shared memory, which leaves two stages of 32
 //   keys. Roles:
 //     * 4 softmax warps, one thread per row: scores from tensor memory, online softmax (base 2, float32, the
 //       reference maximum raised lazily), and the weights back to tensor memory as TWO bfloat16 numbers, p = hi + lo,
@@ -13,9 +13,11 @@
 //     * 2 loader warps, 16 keys each: nine boxes of 64 elements (eight of the latent, one rotated) straight from the page;
 //     * 2 issuing threads: S = Q K^T (M 128, N 32, K 576) and O += P V (M 128, N 256, hi and lo over the same keys; V
 //       is the latents' own rows, read MN-major).
-//   16 heads over 2,048 tokens: 280 us, 390 TFLOP/s as issued, against 735 us of the mma.sync kernel. What bounds it is the
-//   scores' shared-memory traffic: with N = 32 every MMA reads 4 KB of queries for 1 KB of keys.
+//   16 heads over 2,048 tokens: 257 us (73 GFLOP, 146 as issued: 570 TFLOP/s), against 721 us of the mma.sync kernel. What
+//   bounds it is the scores' shared-memory traffic: with N = 32 every MMA reads 4 KB of queries for 1 KB of keys.
 //   Two score buffers, two weight buffers: the scores of a tile are made while the one before passes the softmax.
+//   A key whose latents are not finite reaches the rows of its own 128-row tile that do not see it (a weight of 0 meets it in
+//   the product), earlier tokens of its own request, as in the other tensor-core kernels of portions.
 #include "common.cuh"
 #include "latent.cuh"
 #include "mma_util.cuh"

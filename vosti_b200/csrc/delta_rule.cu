@@ -151,9 +151,10 @@ __global__ void __launch_bounds__(256) delta_prep_kernel(PrepArgs a) {
 
 // The same for heads of 128 channels and up to four taps (WIDE_TAPS): a lane owns four neighbouring channels of its
 // unit and a warp takes TOKENS_EACH tokens one after the other, so that the taps' weights, the decay's constants
-// and the last inputs stay in registers and every access is a whole word; a v head's warp also makes its head's
-// beta, decay and gate. The kernel above bounded itself by its scalar loads (each input read once per tap): 87 us
-// for 2,048 tokens of 16 heads (4 key heads), against the 16 us its 105 MB take.
+// and the last inputs stay in registers and a token's inputs and results are whole words; a v head's warp also makes
+// its head's beta, decay and gate. The kernel above is bound by its scalar loads (each input read once per tap): 87 us
+// for 2,048 tokens of 16 heads (4 key heads); this one takes 61, against the 16 that the 105 MB take. What is left of that is
+// the weights: 16 single elements a lane and four constants, more loads than the data of four tokens need.
 constexpr int WIDE_TAPS = 4;
 
 __device__ __forceinline__ void store_four(float* p, const float (&v)[4]) { *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]); }

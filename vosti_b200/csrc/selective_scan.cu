@@ -211,7 +211,8 @@ scan_tail_kernel(const T* __restrict__ xz, int64_t xz_stride, float* state, int6
 constexpr int SCAN_CHANNELS = 32;      // channels of a block
 // Channels from which a long portion runs in one pass (scan_line_kernel): a token then costs its 68 ns however few
 // channels there are, the chunks fill the GPU from few channels. 2,048 tokens in one pass and in chunks: 142 and 173 us at
-// 2,048 channels, 143 and 114 us at 1,024.
+// 2,048 channels, 143 and 114 us at 1,024. At 2,048 channels it is also the faster way for short portions and many (us, chunks
+// and one pass): one of 65 tokens 47 and 9, sixteen of 65 105 and 58, sixty-four of 65 345 and 237, sixteen of 200 243 and 119.
 constexpr int SCAN_LINE_FROM = 2048;
 
 // One block runs at most `chunk` tokens of one request for 32 channels; LANES lanes share a channel
