@@ -1601,7 +1601,7 @@ def latent_takes_tiles(q_lens, kv_lens, heads: int, window: int, few: bool) -> b
 def _latent_takes_tiles(ctx, heads: int, window: int, few: bool) -> bool:
     if len(ctx.host_q_lens) != ctx.num_requests or len(ctx.host_kv_lens) != ctx.num_requests:
         return False
-    made = ctx.layout.setdefault("latent", {})               # once a step, not once a layer
+    made = ctx.layout.setdefault("latent_attend.tiles", {})  # once a step, not once a layer
     if (heads, window) not in made:
         made[heads, window] = latent_takes_tiles(ctx.host_q_lens, ctx.host_kv_lens, heads, window, few)
     return made[heads, window]
