@@ -1,0 +1,70 @@
+"""The float32 product on the tensor cores (csrc/gemm_f32.cu): against float64, bits of a row alone and among others in every
+tile width, rows picked, rows that start inside a word, operands that are not finite."""
+import pytest
+import torch
+
+from vosti_b200 import ops
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.fixture
+def status():
+    return torch.zeros(1, dtype=torch.int32, device=DEV)
+
+
+def draw(seed, rows, n, k):
+    gen = torch.Generator(device=DEV).manual_seed(seed)
+    return torch.randn(rows, k, generator=gen, device=DEV), torch.randn(n, k, generator=gen, device=DEV)
+
+
+def bound(x, w):
+    """Per output, over the sum of magnitudes: a rounding of the running sum per 64 k and K segment, at most four truncations (two
+    roundings' worth each) of a 64-k sum, 5 K / 16 truncations of sums 2^-8 as large, and the terms left out."""
+    k = x.shape[1]
+    steps = -(-k // 64) + 8 + 2 * 4 + 2 * (5 * k / 16) * 2.0 ** -8 + 4
+    return steps * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
+
+
+# rows around the widths of the token tiles, n and k around 128 and 64, one to eight K segments
+@pytest.mark.parametrize("rows,n,k", [(1, 16, 128), (32, 127, 130), (33, 129, 191), (64, 300, 256), (65, 64, 2048), (128, 4100, 513),
+                                      (129, 128, 4096), (193, 640, 1027), (257, 257, 640), (385, 25000, 132), (600, 384, 1000)])
+def test_against_float64_and_rows_alone(status, rows, n, k):
+    x, w = draw(rows + n + k, rows, n, k)
+    y = ops.gemm_f32(x, w, status)
+    want = x.double() @ w.double().T
+    assert bool(((y.double() - want).abs() <= bound(x, w)).all()) and status.item() == 0
+    chain = ops.gemm_simt(x, w, status)
+    assert (y.double() - want).norm() <= (chain.double() - want).norm()
+    for a, b in [(0, 1), (rows // 2, rows // 2 + 1), (0, min(rows, 40)), (max(rows - 70, 0), rows), (0, min(rows, 150)), (0, min(rows, 200))]:
+        assert torch.equal(ops.gemm_f32(x[a:b].contiguous(), w, status), y[a:b])
+    index = torch.randint(0, rows, (rows // 2 + 3,), device=DEV, dtype=torch.int32)
+    assert torch.equal(ops.gemm_f32(x, w, status, row_index=index), y[index.long()]) and status.item() == 0
+    # the same numbers on places that are not whole words
+    xs, ws = torch.empty(rows * k + 1, device=DEV), torch.empty(n * k + 3, device=DEV)
+    xs[1:], ws[3:] = x.view(-1), w.view(-1)
+    assert torch.equal(ops.gemm_f32(xs[1:].view(rows, k), ws[3:].view(n, k), status), y)
+
+
+def test_positive_sums_and_small_and_large_operands(status):
+    x, w = draw(5, 70, 200, 4096)
+    for a, b in ((x.abs(), w.abs()), (x * 1e-30, w * 1e3), (x * 1e-25, w * 1e-12), (x * 1e20, w * 1e15)):
+        want = a.double() @ b.double().T
+        rel = lambda y: ((y.double() - want).norm() / want.norm()).item()
+        assert rel(ops.gemm_f32(a, b, status)) <= rel(ops.gemm_simt(a, b, status))
+
+
+def test_operands_that_are_not_finite(status):
+    x, w = draw(6, 40, 200, 512)
+    x[3, 7], x[5, 9], x[6, :], w[10, 3], x[7, 11], w[:, 11] = float("inf"), float("nan"), -3.4028234e38, float("-inf"), 3.4028e38, 0.25
+    y, chain = ops.gemm_f32(x, w, status), ops.gemm_simt(x, w, status)
+    assert torch.equal(torch.isnan(y), torch.isnan(chain)) and torch.equal(torch.isinf(y), torch.isinf(chain))
+    finite = torch.isfinite(chain)
+    assert torch.allclose(y[finite], chain[finite], rtol=1e-4, atol=1e-4)
+
+
+def test_a_row_index_out_of_range_is_reported(status):
+    x, w = draw(7, 5, 64, 128)
+    y = ops.gemm_f32(x, w, status, row_index=torch.tensor([0, 5, -1, 4], dtype=torch.int32, device=DEV))
+    assert status.item() != 0 and not y[1:3].any() and torch.equal(y[[0, 3]], ops.gemm_f32(x, w, status)[[0, 4]])

@@ -1,8 +1,9 @@
 """Matrix product y = x @ w.T for the parts, choosing the kernel by operand types.
 
-bfloat16 x bfloat16 goes to the tensor-core kernel when it takes the sizes; every
-other combination (the float32 path, a 32-bit weight under bfloat16 serving, sizes
-the tensor-core kernel refuses) goes to the CUDA-core kernel with float32 arithmetic.
+bfloat16 x bfloat16 goes to the tensor-core kernel when it takes the sizes, float32 x float32 to the
+tensor-core kernel that splits every operand into three bfloat16 terms (float32 results, no reduced precision);
+every other combination (a 32-bit weight under bfloat16 serving, sizes those kernels refuse) goes to the
+CUDA-core kernel with float32 arithmetic.
 The choice depends on types and on (N, K) only, never on the number of rows.
 """
 from __future__ import annotations
@@ -21,6 +22,11 @@ PACK_WEIGHTS = os.environ.get("VOSTI_PACK_WEIGHTS", "1") != "0"
 def uses_tensor_cores(x_dtype: torch.dtype, w) -> bool:
     return (x_dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and w.is_cuda
             and ops.gemm_tc_supported(w.shape[0], w.shape[1]))
+
+
+def uses_split_float32(x_dtype: torch.dtype, w) -> bool:
+    return (x_dtype == torch.float32 and w.dtype == torch.float32 and w.is_cuda
+            and ops.gemm_f32_supported(w.shape[0], w.shape[1]))
 
 
 def prepare_weight(w: torch.Tensor, serving_dtype: torch.dtype):
@@ -53,4 +59,6 @@ def linear(ctx, x: torch.Tensor, w: torch.Tensor, *, out_dtype: Optional[torch.d
         if row_index is not None:
             x = ops.gather_rows(x, row_index, ctx.status)
         return ops.gemm_tc(x, w, ctx.status, out_dtype=out_dtype, allow_partial=allow_partial, scratch=scratch)
+    if uses_split_float32(x.dtype, w) and out_dtype in (None, torch.float32):
+        return ops.gemm_f32(x, w, ctx.status, row_index=row_index)
     return ops.gemm_simt(x, w, ctx.status, out_dtype=out_dtype, row_index=row_index)
