@@ -146,7 +146,7 @@ gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float*
   __shared__ __align__(8) uint64_t sum_free;                // eight warps: the 64-k sum has been taken out
   __shared__ uint32_t tmem_base_holder;
   __shared__ volatile int abort_flag;
-  __shared__ int source[TOK];                               // rows of x, -1: none
+  __shared__ int source[TOK];                               // rows of x; -1: zeros, for an index out of range; -2: none
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int segment = blockIdx.x % segments;
@@ -186,7 +186,7 @@ gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float*
   }
   pdl_wait();
   for (int t = threadIdx.x; t < TOK; t += THREADS<TOK>) {
-    int from = -1;
+    int from = -2;
     if (t0 + t < rows) {
       from = row_index ? row_index[t0 + t] : t0 + t;
       if (from < 0 || from >= x_rows) {
@@ -274,7 +274,7 @@ gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float*
     for (int i = 0; i < BW; ++i) {
       const int r = my_row + i * ROWS_PER;
       // (columns of rows that are not there are never stored, and touch no other column)
-      if (TOK <= 64 && source[r] < 0) continue;
+      if (TOK <= 64 && source[r] == -2) continue;
       store_split(base + 3 * A_PLANE + r * ROW + (((my_k >> 3) ^ swizzle(r)) << 4) + (my_k & 4) * 2, B_PLANE, bw[i]);
     }
     __syncwarp();
