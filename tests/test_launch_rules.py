@@ -182,3 +182,13 @@ def test_weight_bytes_of_a_decode_step_in_closed_form():
         assert bench.closed_form_weight_bytes(config) == total, size
     layers = bench.closed_form_weight_bytes(bench.SIZES["8b"][1]) - 2 * 151936 * 4096
     assert abs(layers - 13.892e9) < 2e6 and 2 * 151936 * 4096 == 1_244_659_712
+
+
+def test_latent_attention_forms_keys_and_values_where_that_was_faster():
+    """Whole mixers of 16 heads, rank 512: (tokens, keys before them, whether formed heads were measured faster)."""
+    from vosti_b200 import ops
+    for new, past, formed in [([33], [0], True), ([128], [0], True), ([700], [0], True), ([2048], [0], True), ([131], [700], True),
+                              ([500] * 3, [0, 64, 0], True), ([1024] + [1] * 8, [0] + [1000] * 8, True), ([5, 17, 200], [0, 30, 1400], True),
+                              ([64, 64], [0, 0], True), ([20], [1500], False), ([8], [64], False), ([16] * 20, [100] * 20, False),
+                              ([100] + [1] * 12, [0] + [1500] * 12, False), ([1] * 16, [700] * 16, False)]:
+        assert ops.latent_forms_heads(new, [a + b for a, b in zip(new, past)], 16, 512) is formed, (new, past)

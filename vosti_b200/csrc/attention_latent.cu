@@ -36,12 +36,12 @@ constexpr float LOG2E = 1.4426950408889634f;
 
 template <typename T>
 __global__ void __launch_bounds__(256)
-latent_prep_kernel(const T* __restrict__ proj, int64_t proj_stride, T* __restrict__ qk, float* __restrict__ gate,
+latent_prep_kernel(const T* __restrict__ proj, int64_t proj_stride, T* __restrict__ qk, int qk_row, float* __restrict__ gate,
                    T* __restrict__ c_cache, T* __restrict__ r_cache, const void* __restrict__ norm_w, int norm_f32, float eps,
                    const int* __restrict__ positions, const int* __restrict__ slot_mapping, int64_t num_slots, int heads,
                    int dim, int rot, int rank, const float* __restrict__ freq, int interleaved, float magnitude,
                    unsigned* status) {
-  extern __shared__ float turn[];            // [rot]: cosines, then sines
+  extern __shared__ __align__(16) float turn[];            // [rot]: cosines, then sines
   __shared__ float scratch[32];
   pdl_wait();
   pdl_launch_dependents();
@@ -66,7 +66,7 @@ latent_prep_kernel(const T* __restrict__ proj, int64_t proj_stride, T* __restric
   const int qw = dim + rot, kw = rank + rot;
   for (int i = threadIdx.x; i < heads * rot; i += blockDim.x) {
     const int h = i / rot, j = i % rot;
-    qk[((int64_t)t * heads + h) * kw + rank + j] = from_f32<T>(turned(row + h * qw + dim, j));
+    qk[((int64_t)t * heads + h) * qk_row + qk_row - rot + j] = from_f32<T>(turned(row + h * qw + dim, j));
   }
   const T* down = row + heads * qw;
   const T* graw = down + kw;
@@ -87,6 +87,109 @@ latent_prep_kernel(const T* __restrict__ proj, int64_t proj_stride, T* __restric
   for (int i = threadIdx.x; i < rank; i += blockDim.x)
     c_cache[slot * rank + i] = from_f32<T>(to_f32(down[i]) * inv * load_flex(norm_w, norm_f32, i));
   for (int i = threadIdx.x; i < rot; i += blockDim.x) r_cache[slot * rot + i] = from_f32<T>(turned(down + rank, i));
+}
+
+__device__ __forceinline__ void put_four(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void put_four(bf16* p, float4 v) {
+  const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+  *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+}
+
+// The same for rows of whole words of four: what a token needs is asked for together, before the angles are made, where the
+// kernel above waits for its single elements one loop after the other. `rot` a multiple of 8, `rank` of 4 and at most 1,024.
+constexpr int PREP_THREADS = 128, PREP_WORDS = 2;         // threads of a token; words of the latent each of them keeps
+
+template <typename T>
+__global__ void __launch_bounds__(PREP_THREADS)
+latent_prep_words_kernel(const T* __restrict__ proj, int64_t proj_stride, T* __restrict__ qk, int qk_row, float* __restrict__ gate,
+                         T* __restrict__ c_cache, T* __restrict__ r_cache, const void* __restrict__ norm_w, int norm_f32, float eps,
+                         const int* __restrict__ positions, const int* __restrict__ slot_mapping, int64_t num_slots, int heads,
+                         int dim, int rot, int rank, const float* __restrict__ freq, int interleaved, float magnitude,
+                         unsigned* status) {
+  extern __shared__ __align__(16) float turn[];            // [rot]: cosines, then sines
+  __shared__ float scratch[32];
+  pdl_wait();
+  pdl_launch_dependents();
+  const int t = blockIdx.x, half = rot / 2, tid = threadIdx.x;
+  const T* const row = proj + (int64_t)t * proj_stride;
+  const int qw = dim + rot;
+  const T* const down = row + heads * qw;
+  const int pairs = rot / 8;                 // pairs of words of a rotated part: j and j + half, or neighbours
+  // words of pair i of a rotated part
+  auto first = [&](int i) { return interleaved ? 8 * i : 4 * i; };
+  auto second = [&](int i) { return interleaved ? 8 * i + 4 : half + 4 * i; };
+  auto source = [&](int i) { return row + i / pairs * qw + dim; };
+  float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a, latent[PREP_WORDS];
+  if (tid < heads * pairs) {
+    a = load_four(source(tid) + first(tid % pairs));
+    b = load_four(source(tid) + second(tid % pairs));
+  }
+  int64_t slot = -1;
+  if (c_cache != nullptr) {
+    slot = slot_mapping[t];
+#pragma unroll
+    for (int w = 0; w < PREP_WORDS; ++w)
+      latent[w] = (tid + w * PREP_THREADS) * 4 < rank ? load_four(down + (tid + w * PREP_THREADS) * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  const float p = (float)positions[t];
+  for (int i = tid; i < half; i += PREP_THREADS) {
+    const float angle = p * freq[i];
+    turn[i] = cosf(angle) * magnitude;
+    turn[half + i] = sinf(angle) * magnitude;
+  }
+  __syncthreads();
+  auto turned = [&](float4& a, float4& b, int i) {
+    if (interleaved) {
+      const float* const c = turn + 4 * i;
+      const float* const s = c + half;
+      a = make_float4(a.x * c[0] - a.y * s[0], a.y * c[0] + a.x * s[0], a.z * c[1] - a.w * s[1], a.w * c[1] + a.z * s[1]);
+      b = make_float4(b.x * c[2] - b.y * s[2], b.y * c[2] + b.x * s[2], b.z * c[3] - b.w * s[3], b.w * c[3] + b.z * s[3]);
+    } else {
+      const float4 c = *reinterpret_cast<const float4*>(turn + 4 * i), s = *reinterpret_cast<const float4*>(turn + half + 4 * i);
+      const float4 old = a;
+      a = make_float4(a.x * c.x - b.x * s.x, a.y * c.y - b.y * s.y, a.z * c.z - b.z * s.z, a.w * c.w - b.w * s.w);
+      b = make_float4(b.x * c.x + old.x * s.x, b.y * c.y + old.y * s.y, b.z * c.z + old.z * s.z, b.w * c.w + old.w * s.w);
+    }
+  };
+  for (int i = tid; i < heads * pairs; i += PREP_THREADS) {
+    if (i != tid) {
+      a = load_four(source(i) + first(i % pairs));
+      b = load_four(source(i) + second(i % pairs));
+    }
+    turned(a, b, i % pairs);
+    T* const to = qk + ((int64_t)t * heads + i / pairs) * qk_row + qk_row - rot;
+    put_four(to + first(i % pairs), a);
+    put_four(to + second(i % pairs), b);
+  }
+  if (gate != nullptr)
+    for (int i = tid; i < heads; i += PREP_THREADS) gate[(int64_t)t * heads + i] = 1.f / (1.f + expf(-to_f32(down[rank + rot + i])));
+  if (c_cache == nullptr) return;
+  float ss = 0.f;
+#pragma unroll
+  for (int w = 0; w < PREP_WORDS; ++w) {
+    const float4 v = latent[w];
+    ss = fmaf(v.w, v.w, fmaf(v.z, v.z, fmaf(v.y, v.y, fmaf(v.x, v.x, ss))));
+  }
+  const float inv = 1.f / sqrtf(block_sum(ss, scratch) / (float)rank + eps);
+  if (slot < 0 || slot >= num_slots) {
+    if (tid == 0) raise_fault(status, VOSTI_FAULT_SLOT_RANGE);
+    return;
+  }
+#pragma unroll
+  for (int w = 0; w < PREP_WORDS; ++w) {
+    const int c = (tid + w * PREP_THREADS) * 4;
+    if (c >= rank) break;
+    const float4 v = latent[w];
+    put_four(c_cache + slot * rank + c, make_float4(v.x * inv * load_flex(norm_w, norm_f32, c), v.y * inv * load_flex(norm_w, norm_f32, c + 1),
+                                                    v.z * inv * load_flex(norm_w, norm_f32, c + 2), v.w * inv * load_flex(norm_w, norm_f32, c + 3)));
+  }
+  for (int i = tid; i < pairs; i += PREP_THREADS) {
+    a = load_four(down + rank + first(i));
+    b = load_four(down + rank + second(i));
+    turned(a, b, i);
+    put_four(r_cache + slot * rot + first(i), a);
+    put_four(r_cache + slot * rot + second(i), b);
+  }
 }
 
 // y[t, h, o] = g[t, h] * sum_i x[t, h, i] * M[h * m_head + i * m_in + o * m_out]; a block takes 16
@@ -368,28 +471,36 @@ void launch_attend(dim3 grid, size_t smem, cudaStream_t stream, const void* qk, 
 constexpr int LATENT_MAX_RANK = 1024;
 
 // proj rows (proj_stride elements apart) start with heads * (dim + rot) query elements, then `down` (rank + rot), then a
-// gate per head; the last two are read only where c_cache and `gate` are given. qk [tokens, heads, rank + rot]
+// gate per head; the last two are read only where c_cache and `gate` are given. qk [tokens, heads, qk_row]
 // (the last rot columns of every head are written); gate float32 [tokens, heads] or null; caches
 // [pages, 1, page_size, rank | rot] or null (a run that reads another layer's cache).
-VOSTI_API int vosti_latent_prep(const void* proj, int64_t proj_stride, void* qk, float* gate, void* c_cache, void* r_cache, const void* norm_w,
+VOSTI_API int vosti_latent_prep(const void* proj, int64_t proj_stride, void* qk, int qk_row, float* gate, void* c_cache, void* r_cache, const void* norm_w,
                                 int norm_f32, float eps, const int* positions, const int* slot_mapping, int64_t num_slots,
                                 int tokens, int heads, int dim, int rot, int rank, const float* freq, int interleaved, float magnitude,
                                 int is_f32, unsigned* status, cudaStream_t stream) {
   VOSTI_REQUIRE(tokens >= 0 && heads > 0 && dim > 0 && rank > 0 && rot >= 0 && rot % 2 == 0, "latent_prep: bad sizes");
+  VOSTI_REQUIRE(qk_row >= rot, "latent_prep: rows of %d elements for a rotated part of %d", qk_row, rot);
   VOSTI_REQUIRE(rot == 0 || freq != nullptr, "latent_prep: a rotation needs frequencies");
   VOSTI_REQUIRE(c_cache == nullptr || (r_cache != nullptr && slot_mapping != nullptr && norm_w != nullptr), "latent_prep: a cache needs slots and the norm's weight");
   if (tokens == 0) return VOSTI_OK;
   VOSTI_REQUIRE(proj_stride >= (int64_t)heads * (dim + rot) + (c_cache != nullptr || gate != nullptr ? rank + rot : 0) + (gate != nullptr ? heads : 0),
                 "latent_prep: the projection's rows are too narrow");
   const size_t smem = (size_t)(rot > 0 ? rot : 1) * sizeof(float);
-  if (is_f32)
-    vosti_launch(latent_prep_kernel<float>, dim3(tokens), dim3(256), smem, stream, (const float*)proj, proj_stride, (float*)qk, gate,
-                 (float*)c_cache, (float*)r_cache, norm_w, norm_f32, eps, positions, slot_mapping, num_slots, heads, dim, rot, rank,
-                 freq, interleaved, magnitude, status);
-  else
-    vosti_launch(latent_prep_kernel<bf16>, dim3(tokens), dim3(256), smem, stream, (const bf16*)proj, proj_stride, (bf16*)qk, gate,
-                 (bf16*)c_cache, (bf16*)r_cache, norm_w, norm_f32, eps, positions, slot_mapping, num_slots, heads, dim, rot, rank,
-                 freq, interleaved, magnitude, status);
+  const uintptr_t mis = reinterpret_cast<uintptr_t>(proj) | reinterpret_cast<uintptr_t>(qk) | reinterpret_cast<uintptr_t>(c_cache) | reinterpret_cast<uintptr_t>(r_cache);
+  const bool words = rot % 8 == 0 && rot > 0 && rank % 4 == 0 && rank <= 4 * PREP_WORDS * PREP_THREADS && dim % 4 == 0 && proj_stride % 4 == 0 &&
+                     qk_row % 4 == 0 && mis % (is_f32 ? 16 : 8) == 0;
+#define VOSTI_PREP(KERNEL, T, THREADS)                                                                                        \
+  vosti_launch(KERNEL<T>, dim3(tokens), dim3(THREADS), smem, stream, (const T*)proj, proj_stride, (T*)qk, qk_row, gate,       \
+               (T*)c_cache, (T*)r_cache, norm_w, norm_f32, eps, positions, slot_mapping, num_slots, heads, dim, rot, rank,    \
+               freq, interleaved, magnitude, status)
+  if (words) {
+    if (is_f32) VOSTI_PREP(latent_prep_words_kernel, float, PREP_THREADS);
+    else VOSTI_PREP(latent_prep_words_kernel, bf16, PREP_THREADS);
+  } else {
+    if (is_f32) VOSTI_PREP(latent_prep_kernel, float, 256);
+    else VOSTI_PREP(latent_prep_kernel, bf16, 256);
+  }
+#undef VOSTI_PREP
   VOSTI_LAUNCH_CHECK();
 }
 

@@ -809,6 +809,30 @@ VOSTI_API int vosti_gemm_tc_clamped(const void* x, const void* w, void* y, int t
   VOSTI_LAUNCH_CHECK();
 }
 
+// y bf16 [tokens, features] = x w^T rounded, and for the features from `low_from` on (a multiple of 32) what the rounding left,
+// rounded again, to low bf16 [tokens, features - low_from]: hi + low keep 16 bits of the float32 sum. w row-major.
+VOSTI_API int vosti_gemm_tc_two_terms(const void* x, const void* w, void* y, void* low, int low_from, int tokens, int features, int k,
+                                      unsigned* status, cudaStream_t stream) {
+  using namespace pair_kernel;
+  VOSTI_REQUIRE(tokens >= 0 && vosti_gemm_tc_supported(features, k) && features % 32 == 0 && low_from >= 0 && low_from % 32 == 0 && low_from < features,
+                "gemm_tc_two_terms: unsupported sizes T=%d F=%d from %d K=%d", tokens, features, low_from, k);
+  VOSTI_REQUIRE((((uintptr_t)x | (uintptr_t)w | (uintptr_t)y | (uintptr_t)low) % 16) == 0, "gemm_tc_two_terms: operands must be 16-byte aligned");
+  if (tokens == 0) return VOSTI_OK;
+  CUtensorMap mw, mx;
+  VOSTI_REQUIRE(weight_map(w, features, k, BM, &mw) && make_map(&mx, x, tokens, k, BM), "gemm_tc_two_terms: cuTensorMapEncodeTiled failed");
+  constexpr size_t smem = (size_t)PAIR_STAGES * PAIR_STAGE_BYTES + 1024;
+  static const cudaError_t raised = cudaFuncSetAttribute(gemm_tc_pair_kernel<TwoTermEpilogue>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (raised != cudaSuccess) {
+    vosti_set_error("gemm_tc_two_terms: cannot configure the paired kernel: %s", cudaGetErrorString(raised));
+    return (int)raised;
+  }
+  const int tiles = ((tokens + 2 * BM - 1) / (2 * BM)) * ((features + PAIR_BN - 1) / PAIR_BN);
+  const int pairs = tiles < device_sms() / 2 ? tiles : device_sms() / 2;
+  vosti_launch_clusters(gemm_tc_pair_kernel<TwoTermEpilogue>, dim3(2 * pairs), dim3(PAIR_THREADS), 2, smem, stream, mx, mw, y, tokens,
+                        features, (k + BK - 1) / BK, features, (int)EPI_BF16, 0, TwoTermEpilogue{(bf16*)low, low_from}, status);
+  VOSTI_LAUNCH_CHECK();
+}
+
 // Sum deferred partial sums ([splits, tokens, features] float32) in split order into y
 // (bf16 or float32 [tokens, features]).
 VOSTI_API int vosti_splitk_reduce(const float* partial, void* y, int splits, int tokens, int features, int y_is_f32,

@@ -80,6 +80,10 @@ struct ClampedEpilogue {
   const float* bias;
   float limit, sigmoid_scale;
 };
+struct TwoTermEpilogue {            // what rounding leaves of the features from low_from on, rounded again, goes to low
+  bf16* low;
+  int low_from;
+};
 __device__ __forceinline__ void store_columns(const uint32_t (&r)[32], void* out, int token, int f0, int features, int ld_out,
                                               int epilogue, const PlainEpilogue&) {
   store_token_columns(r, out, token, f0, features, ld_out, epilogue);
@@ -103,6 +107,26 @@ __device__ __forceinline__ void store_columns(const uint32_t (&r)[32], void* out
   uint4* y = reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(out) + (int64_t)token * ld_out + f0 / 2);    // ld_out is a multiple of 16
   y[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
   y[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
+}
+__device__ __forceinline__ void store_columns(const uint32_t (&r)[32], void* out, int token, int f0, int features, int ld_out, int,
+                                              const TwoTermEpilogue& two) {
+  uint4* const y = reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(out) + (int64_t)token * ld_out + f0);   // features % 32 == 0
+  uint4* const z = f0 < two.low_from ? nullptr : reinterpret_cast<uint4*>(two.low + (int64_t)token * (features - two.low_from) + f0 - two.low_from);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    uint32_t hi[4], lo[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float a = __uint_as_float(r[8 * q + 2 * i]), b = __uint_as_float(r[8 * q + 2 * i + 1]);
+      const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+      const float2 back = __bfloat1622float2(h);
+      const __nv_bfloat162 l = __floats2bfloat162_rn(a - back.x, b - back.y);
+      hi[i] = *reinterpret_cast<const uint32_t*>(&h);
+      lo[i] = *reinterpret_cast<const uint32_t*>(&l);
+    }
+    y[q] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+    if (z != nullptr) z[q] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+  }
 }
 }  // namespace pair_kernel
 

@@ -1527,7 +1527,7 @@ def latent_prep(proj: torch.Tensor, qk: torch.Tensor, c_cache: Optional[torch.Te
                 rot: int, rank: int, freq: Optional[torch.Tensor], magnitude: float, interleaved: bool = False,
                 head_gate: bool = True) -> Optional[torch.Tensor]:
     """After the q | down | gate projection (csrc/attention_latent.cu): the rotated part of every
-    query head goes to the last `rot` columns of qk [tokens, heads, rank + rot]; the latent
+    query head goes to the last `rot` columns of qk [tokens, heads, rank + rot or rot]; the latent
     (root-mean-square normed with `norm_w`) and the rotated shared key part go to their cache
     slots; with `head_gate` returns sigmoid of the columns after `down`, float32 [tokens, heads]. Without
     caches (a run that reads another layer's) and head gate the projection needs query columns only;
@@ -1536,11 +1536,11 @@ def latent_prep(proj: torch.Tensor, qk: torch.Tensor, c_cache: Optional[torch.Te
     _contig(proj, qk, c_cache, r_cache, norm_w, slot_mapping, freq)
     flag = _same_dtype(proj, qk, c_cache, r_cache)
     tokens = proj.shape[0]
-    if tuple(qk.shape) != (tokens, heads, rank + rot):
+    if tuple(qk.shape) not in ((tokens, heads, rank + rot), (tokens, heads, rot)):
         raise KernelError("latent_prep: widths do not match the head sizes")
     gate = torch.empty((tokens, heads), dtype=torch.float32, device=proj.device) if head_gate else None
     num_slots = 0 if c_cache is None else c_cache.numel() // rank
-    _check(library().vosti_latent_prep(_p(proj), ctypes.c_int64(proj.shape[1]), _p(qk), _p(gate), _p(c_cache), _p(r_cache),
+    _check(library().vosti_latent_prep(_p(proj), ctypes.c_int64(proj.shape[1]), _p(qk), qk.shape[2], _p(gate), _p(c_cache), _p(r_cache),
                                        _p(norm_w), 0 if norm_w is None else _is_f32(norm_w),
                                        ctypes.c_float(eps), _p(ctx.positions), _p(slot_mapping), ctypes.c_int64(num_slots),
                                        tokens, heads, dim, rot, rank, _p(freq), int(bool(interleaved)), ctypes.c_float(magnitude), flag,
@@ -1602,6 +1602,11 @@ def latent_takes_tiles(q_lens, kv_lens, heads: int, window: int, few: bool) -> b
     many of them beside a portion are better off in the small ones. Measured at 16 heads, us, tiles of 32 and of 128 rows:
     one prompt of 64 tokens 9.9 and 11.5, of 1,024 216 and 71; a portion of 8 beside 300 single tokens at 100 keys 41 and 72,
     at 1,000 271 and 375; 300 beside 20 at 2,000 199 and 152; at 64 heads 8 beside 300 at 1,000 457 and 385."""
+    wide, small = _latent_cost(q_lens, kv_lens, heads, window, few)
+    return wide < 0.9 * small
+
+
+def _latent_cost(q_lens, kv_lens, heads: int, window: int, few: bool):
     def cost(rows, each, key, start):
         ctas = total = longest = 0.0
         for n, kv in zip(q_lens, kv_lens):
@@ -1613,7 +1618,7 @@ def latent_takes_tiles(q_lens, kv_lens, heads: int, window: int, few: bool) -> b
             total += tiles * (key * (keys if window <= 0 else min(keys, window + rows / heads)) + start)
             longest = max(longest, key * kv)
         return longest + (start if few else 0.0) + (total / 148 if ctas > 148 else 0.0)
-    return cost(128, 2, 0.071, 5.0) < 0.9 * cost(32, 1, 0.1, 1.0)
+    return cost(128, 2, 0.071, 5.0), cost(32, 1, 0.1, 1.0)
 
 
 def _latent_takes_tiles(ctx, heads: int, window: int, few: bool) -> bool:
@@ -1677,6 +1682,78 @@ def latent_attend(ctx, qk: torch.Tensor, c_cache: torch.Tensor, r_cache: torch.T
         group.block_table.shape[1], group.page_size, num_pages, None, tokens, heads, rank, rot, ctypes.c_float(scale),
         window, _p(sink), _p(scratch), LATENT_SEGMENT, segments, flag, _p(ctx.status), _stream()), "latent_attend",
         kernels=2 if segments > 1 else 1)
+    return out
+
+
+LATENT_HEADS_SCRATCH = 256 << 20     # bytes that the keys and values of a step may take at most
+LATENT_HEADS_TOKENS = 24             # tokens of the longest portion from which forming them is looked at
+LATENT_PAD = 128                     # dense key rows of a request are rounded up to this
+
+
+def latent_forms_heads(q_lens, kv_lens, heads: int, rank: int) -> bool:
+    """Whether forming keys and values of every head (csrc/attention_latent_heads.cu) is the faster way for a step of requests with
+    `q_lens` tokens and `kv_lens` keys, against the latent space (csrc/attention_latent_tc.cu and _mma.cu with their two
+    projections). Estimates in us: forming takes 9.5 ns a row of keys (16 heads, rank 512) and its attention 1.05 us a tile
+    of 64 keys in the longest CTA, besides an SM's share of them all; the latent space 9 us and 44 ns a token for the projections,
+    and its attention as in `latent_takes_tiles` or, with its keys cut, 0.1 us a CTA. Measured at 16 heads, whole mixers, latent
+    space and formed heads: a prompt of 33 tokens 49 and 43, 128 64 and 53, 700 136 and 81, 2,048 402 and 143; 64 after 1,000
+    84 and 75, 131 after 700 116 and 81, 20 after 1,500 60 and 86; 1,024 beside 8 single tokens at 1,000 250 and 199, 1,000 beside
+    12 at 1,900 307 and 306, 100 beside 12 at 1,500 154 and 273; 20 of 16 after 100 86 and 94."""
+    longest = max(q_lens, default=0)
+    if longest < LATENT_HEADS_TOKENS:
+        return False
+    size = heads / 16 * rank / 512
+    rows = sum(-(-kv // LATENT_PAD) * LATENT_PAD for kv in kv_lens)
+    tiles = sum(-(-n // 128) * max(kv - n / 2, 64.0) / 64 for n, kv in zip(q_lens, kv_lens) if n)
+    formed = 8.0 + 0.0095 * rows * size + 1.05 * max(kv_lens) / 64 + heads * tiles / 148
+    tile = 32 if longest * heads > 16 else 16
+    ctas = -(-longest * heads // tile) * len(q_lens)
+    few = ctas < LATENT_MMA_SPLIT_BELOW
+    segments = key_segments(max(kv_lens), 0, LATENT_MMA_SEGMENT, min(longest, -(-tile // heads) + 1)) if few else 1
+    attend = max(8.0, 0.1 * ctas * segments) if segments > 1 else min(_latent_cost(q_lens, kv_lens, heads, 0, few))
+    return formed < 0.75 * (9.0 + 0.044 * sum(q_lens) * size + attend)
+
+
+def _latent_forms_heads(ctx, *, heads: int, dim: int, rot: int, dv: int, rank: int, window: int, scale: float, page_size: int, q_width: int) -> bool:
+    if (window or FIXED_ORDER or scale <= 0 or len(ctx.host_q_lens) != ctx.num_requests or len(ctx.host_kv_lens) != ctx.num_requests
+            or not library().vosti_latent_heads_fits(dim, rot, dv, rank, page_size, q_width)):
+        return False
+    rows = sum(-(-kv // LATENT_PAD) * LATENT_PAD for kv in ctx.host_kv_lens)
+    if rows * (heads * (2 * dim + 4 * dv) + 2 * (rank + rot)) > LATENT_HEADS_SCRATCH:
+        return False
+    made = ctx.layout.setdefault("latent_attend.heads", {})  # once a step, not once a layer
+    if (heads, rank) not in made:
+        made[heads, rank] = latent_forms_heads(ctx.host_q_lens, ctx.host_kv_lens, heads, rank)
+    return made[heads, rank]
+
+
+def latent_attend_heads(ctx, proj: torch.Tensor, qr: torch.Tensor, kv_up: torch.Tensor, c_cache: torch.Tensor, r_cache: torch.Tensor,
+                        group, *, heads: int, dim: int, scale: float, sink: Optional[torch.Tensor] = None,
+                        gate: Optional[torch.Tensor] = None, element_gate: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """Latent attention over keys and values formed for every head (csrc/attention_latent_heads.cu): proj [tokens, width] has the
+    queries first, qr [tokens, heads, rot] their turned parts, kv_up [heads * dim + heads * dv, rank] the up projections of the
+    keys and of the values. Gates as in `head_project`. Returns the heads' outputs [tokens, heads, dv]."""
+    _contig(proj, qr, kv_up, c_cache, r_cache, sink, gate)
+    rank, rot, tokens = c_cache.shape[-1], r_cache.shape[-1], proj.shape[0]
+    dv = kv_up.shape[0] // heads - dim
+    if any(t.dtype != torch.bfloat16 for t in (proj, qr, kv_up, c_cache, r_cache)):
+        raise KernelError("latent_attend_heads takes bfloat16")
+    if element_gate is not None and (gate is not None or tuple(element_gate.shape) != (tokens, heads * dv) or element_gate.stride(1) != 1):
+        raise KernelError("latent_attend_heads: the element gate is [tokens, heads * dv] with contiguous rows, and the only gate")
+    rows = sum(-(-kv // LATENT_PAD) * LATENT_PAD for kv in ctx.host_kv_lens)
+    made = lambda *shape: torch.empty(shape, dtype=torch.bfloat16, device=proj.device)
+    c, r, kv, low, out = made(rows, rank), made(rows, rot), made(rows, heads * (dim + dv)), made(rows, heads * dv), made(tokens, heads, dv)
+    lib = library()
+    _check(lib.vosti_latent_gather(_p(c_cache), _p(r_cache), _p(ctx.kv_len), _p(group.block_table), group.block_table.shape[1],
+                                   group.page_size, c_cache.shape[0], ctx.num_requests, max(ctx.host_kv_lens), rank, rot, _p(c), _p(r),
+                                   rows, _p(ctx.status), _stream()), "latent_gather")
+    _check(lib.vosti_gemm_tc_two_terms(_p(c), _p(kv_up), _p(kv), _p(low), heads * dim, rows, heads * (dim + dv), rank, _p(ctx.status),
+                                       _stream()), "gemm_tc_two_terms")
+    _check(lib.vosti_latent_heads(_p(proj), proj.shape[1], _p(qr), _p(kv), _p(low), _p(r), rows, _p(out), _p(ctx.cu_q), _p(ctx.kv_len),
+                                  ctx.num_requests, ctx.max_q_len, tokens, heads, ctypes.c_float(scale), _p(sink), _p(gate),
+                                  _p(element_gate), 0 if element_gate is None else _is_f32(element_gate),
+                                  ctypes.c_int64(0 if element_gate is None else element_gate.stride(0)), _p(ctx.status), _stream()),
+           "latent_heads")
     return out
 
 

@@ -19,7 +19,9 @@ joins the softmax denominator once, with no key or value, unscaled. With `own_la
 has no down projection and reads the latents and rotated key parts another layer cached (the run
 order names that layer, `RunEntry.cache_from`; its kv_rank, rot_dim and rotation are this layer's).
 
-The attention runs in the latent space: the query's unrotated part is multiplied by W_uk[h]^T
+Two ways, chosen by the step's lengths (`ops.latent_forms_heads`). Where the keys are few for the tokens, k_h and v_h of all
+keys are formed for the step (csrc/attention_latent_heads.cu; k_h is rounded to the serving type, v_h is not). Otherwise
+the attention runs in the latent space: the query's unrotated part is multiplied by W_uk[h]^T
 once per token, the scores and the weighted sum are taken over the cached latents, and W_uv[h]
 is applied to the weighted latent (see csrc/attention_latent.cu). `position` names the rotation
 (kind "rope", any scaling and pairing; rotary_dim = rot_dim; the angles are formed in float32 in the kernel
@@ -66,7 +68,7 @@ class LatentAttention(Mixer):
         if self.rotation is None or not hasattr(self.rotation, "frequencies") or self.rotation.rotary_dim != self.rot:
             raise ConfigError("latent_attention: rot_dim > 0 needs a rotation over all rot_dim elements that gives frequencies")
         self.freq, self.magnitude = None, 1.0
-        self.w_in = self.w_o = self.norm = self.k_up = self.v_up = self.sink = None
+        self.w_in = self.w_o = self.norm = self.kv_up = self.k_up = self.v_up = self.sink = None
 
     def weight_specs(self) -> Dict[str, WeightSpec]:
         h, H = self.hidden_size, self.heads
@@ -92,8 +94,13 @@ class LatentAttention(Mixer):
         self.norm = tensors.get("dkv.norm")
         self.sink = tensors["sink"].float().contiguous() if self.has_sink else None
         # per head: uk as [dim, rank] (in, out), uv as [dv, rank] read with (in, out) = (rank, dv)
-        self.k_up = tensors["uk"].view(self.heads, self.dim, self.rank)
-        self.v_up = tensors["uv"].view(self.heads, self.dv, self.rank).transpose(1, 2)
+        uk, uv = tensors["uk"], tensors["uv"]
+        self.kv_up = None
+        if uk.dtype == uv.dtype == torch.bfloat16 and uk.is_cuda:      # one matrix of both, which the two views below share
+            self.kv_up = torch.cat([uk, uv], dim=0)
+            uk, uv = self.kv_up[: uk.shape[0]], self.kv_up[uk.shape[0]:]
+        self.k_up = uk.view(self.heads, self.dim, self.rank)
+        self.v_up = uv.view(self.heads, self.dv, self.rank).transpose(1, 2)
 
     def setup(self, device, dtype):
         if self.rotation is not None:
@@ -112,18 +119,25 @@ class LatentAttention(Mixer):
         group = ctx.group(cache.group)
         H, tokens = self.heads, x.shape[0]
         proj = ops.materialize(linear(ctx, x, self.w_in))
-        qk = torch.empty((tokens, H, self.rank + self.rot), dtype=proj.dtype, device=proj.device)
+        forms = (self.kv_up is not None and proj.dtype == torch.bfloat16
+                 and ops._latent_forms_heads(ctx, heads=H, dim=self.dim, rot=self.rot, dv=self.dv, rank=self.rank, window=self.window,
+                                             scale=self.scale, page_size=group.page_size, q_width=proj.shape[1]))
+        qk = torch.empty((tokens, H, self.rot if forms else self.rank + self.rot), dtype=proj.dtype, device=proj.device)
         gate = ops.latent_prep(proj, qk, cache.k if writes_cache else None, cache.v if writes_cache else None, self.norm,
                                self.eps, ctx, group.slot_mapping, heads=H, dim=self.dim, rot=self.rot, rank=self.rank,
                                freq=self.freq, magnitude=self.magnitude, interleaved=self.rotation.interleaved,
                                head_gate=self.gated)
+        element_gate = proj[:, self.gate_at: self.gate_at + H * self.dv] if self.out_gate else None
+        if forms:
+            heads_out = ops.latent_attend_heads(ctx, proj, qk, self.kv_up, cache.k, cache.v, group, heads=H, dim=self.dim,
+                                                scale=self.scale, sink=self.sink, gate=gate, element_gate=element_gate)
+            return linear(ctx, heads_out.view(tokens, H * self.dv), self.w_o, out_dtype=torch.float32, allow_partial=self.partial_out)
         # the query's unrotated part into the latent space: qk[t, h, :rank] = q[t, h, :dim] @ W_uk[h]
         q_plain = proj[:, : H * (self.dim + self.rot)].view(tokens, H, self.dim + self.rot)[:, :, : self.dim]
         ops.head_project(q_plain, self.k_up, qk[:, :, : self.rank])
         latent = ops.latent_attend(ctx, qk, cache.k, cache.v, group, scale=self.scale, window=self.window, sink=self.sink)
         heads_out = torch.empty((tokens, H, self.dv), dtype=proj.dtype, device=proj.device)
-        ops.head_project(latent, self.v_up, heads_out, gate=gate,
-                         element_gate=proj[:, self.gate_at: self.gate_at + H * self.dv] if self.out_gate else None)
+        ops.head_project(latent, self.v_up, heads_out, gate=gate, element_gate=element_gate)
         return linear(ctx, heads_out.view(tokens, H * self.dv), self.w_o, out_dtype=torch.float32, allow_partial=self.partial_out)
 
 
