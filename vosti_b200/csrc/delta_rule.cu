@@ -71,6 +71,7 @@ struct PrepArgs {
   unsigned* status;
   int decay_per_head;           // rates: heads decay columns (dt_bias [heads]) instead of heads * dk
   int gate_silu;                // the output gate is z * sigmoid(z) instead of sigmoid(z)
+  int w_words;                  // four taps, and conv_w and dt_bias on whole words
 };
 
 // One warp per unit of a token: a q head, a k head or a v head. A lane owns the channels lane,
@@ -158,9 +159,12 @@ __global__ void __launch_bounds__(256) delta_prep_kernel(PrepArgs a) {
 constexpr int WIDE_TAPS = 4;
 
 __device__ __forceinline__ void store_four(float* p, const float (&v)[4]) { *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]); }
+__device__ __forceinline__ float4 flex_four(const void* p, int is_f32, int64_t i) {       // load_flex of an aligned word
+  return is_f32 ? load_four(reinterpret_cast<const float*>(p) + i) : load_four(reinterpret_cast<const bf16*>(p) + i);
+}
 __device__ __forceinline__ void spread(float4 v, float (&to)[4]) { to[0] = v.x; to[1] = v.y; to[2] = v.z; to[3] = v.w; }
 
-template <typename T, int TOKENS_EACH>
+template <typename T, int TOKENS_EACH, int BATCHES>
 __global__ void __launch_bounds__(128) delta_prep_wide_kernel(PrepArgs a, int tokens) {
   pdl_wait();
   pdl_launch_dependents();
@@ -176,103 +180,126 @@ __global__ void __launch_bounds__(128) delta_prep_wide_kernel(PrepArgs a, int to
 #pragma unroll
   for (int k = 0; k < WIDE_TAPS; ++k)
 #pragma unroll
+    for (int u = 0; u < 4; ++u) win[k][u] = 0.f;
+  if (a.w_words) {                                         // four taps: a channel's weights are one word
+#pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const int tap = k - (WIDE_TAPS - a.taps);
-      w[k][u] = tap >= 0 ? load_flex(a.conv_w, a.w_f32, (int64_t)(c + u) * a.taps + tap) : 0.f;
-      win[k][u] = 0.f;
+      const float4 v = flex_four(a.conv_w, a.w_f32, (int64_t)(c + u) * WIDE_TAPS);
+      w[0][u] = v.x; w[1][u] = v.y; w[2][u] = v.z; w[3][u] = v.w;
     }
+  } else {
+#pragma unroll
+    for (int k = 0; k < WIDE_TAPS; ++k)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int tap = k - (WIDE_TAPS - a.taps);
+        w[k][u] = tap >= 0 ? load_flex(a.conv_w, a.w_f32, (int64_t)(c + u) * a.taps + tap) : 0.f;
+      }
+  }
   const int head = unit - 2 * a.kv_heads;                  // of a v unit
   float speed = 0.f, shift[4] = {0.f, 0.f, 0.f, 0.f};
   if (head >= 0) {
     speed = expf(load_flex(a.a_log, a.w_f32, head));
+    if (a.w_words && !a.decay_per_head) {
+      spread(flex_four(a.dt_bias, a.w_f32, head * D + lane * 4), shift);
+    } else {
 #pragma unroll
-    for (int u = 0; u < 4; ++u) shift[u] = load_flex(a.dt_bias, a.w_f32, a.decay_per_head ? head : head * D + lane * 4 + u);
+      for (int u = 0; u < 4; ++u) shift[u] = load_flex(a.dt_bias, a.w_f32, a.decay_per_head ? head : head * D + lane * 4 + u);
+    }
   }
   const int rd = a.decay_per_head ? a.heads : a.heads * D;
-  const int t_begin = blockIdx.x * TOKENS_EACH, t_end = min(tokens, t_begin + TOKENS_EACH);
-  float4 ahead[TOKENS_EACH], gates[TOKENS_EACH], rates[TOKENS_EACH];
+  // the rows before the warp's first token, asked for before its request is known (its own from the request's fourth token on)
+  const int t_first = blockIdx.x * BATCHES * TOKENS_EACH;
+  float4 before[WIDE_TAPS - 1];
 #pragma unroll
-  for (int e = 0; e < TOKENS_EACH; ++e) {
-    const int t = t_begin + e;
-    if (t >= t_end) break;
-    ahead[e] = load_four(proj + (int64_t)t * a.stride + a.off_q + c);
-    if (head >= 0) {
-      const int64_t row = (int64_t)t * (rd + cv);
-      auto rate4 = [&](int64_t at) {
-        return a.rates_f32 ? load_four(reinterpret_cast<const float*>(a.rates) + at) : load_four(reinterpret_cast<const bf16*>(a.rates) + at);
-      };
-      gates[e] = rate4(row + rd + head * D + lane * 4);
-      if (a.decay_per_head) {
-        const float r = load_flex(a.rates, a.rates_f32, row + head);
-        rates[e] = make_float4(r, r, r, r);
-      } else {
-        rates[e] = rate4(row + head * D + lane * 4);
-      }
-    }
-  }
+  for (int k = 1; k < WIDE_TAPS; ++k) before[k - 1] = load_four(proj + (int64_t)max(t_first - k, 0) * a.stride + a.off_q + c);
   int b = -1, next_first = 0;
+#pragma unroll 1
+  for (int batch = 0; batch < BATCHES; ++batch) {
+    const int t_begin = t_first + batch * TOKENS_EACH, t_end = min(tokens, t_begin + TOKENS_EACH);
+    float4 ahead[TOKENS_EACH], gates[TOKENS_EACH], rates[TOKENS_EACH];
 #pragma unroll
-  for (int e = 0; e < TOKENS_EACH; ++e) {
-    const int t = t_begin + e;
-    if (t >= t_end) break;
-    if (b < 0 || t >= next_first) {                        // a new request (or the warp's first token): fill the window anew
-      b = a.request_of[t];
-      const int first = a.cu_q[b];
-      next_first = a.cu_q[b + 1];
-      int slot = a.state_slots[b];
-      if (slot < 0 || slot >= a.num_slots) {
-        if (lane == 0 && unit == 0) raise_fault(a.status, VOSTI_FAULT_SLOT_RANGE);
-        slot = 0;
+    for (int e = 0; e < TOKENS_EACH; ++e) {
+      const int t = t_begin + e;
+      if (t >= t_end) break;
+      ahead[e] = load_four(proj + (int64_t)t * a.stride + a.off_q + c);
+      if (head >= 0) {
+        const int64_t row = (int64_t)t * (rd + cv);
+        auto rate4 = [&](int64_t at) {
+          return a.rates_f32 ? load_four(reinterpret_cast<const float*>(a.rates) + at) : load_four(reinterpret_cast<const bf16*>(a.rates) + at);
+        };
+        gates[e] = rate4(row + rd + head * D + lane * 4);
+        if (a.decay_per_head) {
+          const float r = load_flex(a.rates, a.rates_f32, row + head);
+          rates[e] = make_float4(r, r, r, r);
+        } else {
+          rates[e] = rate4(row + head * D + lane * 4);
+        }
       }
-      const float* const tail = a.state + (int64_t)slot * a.state_stride + a.conv_offset;       // [taps - 1, cc]
-      const int local = t - first;
+    }
 #pragma unroll
-      for (int k = 1; k < WIDE_TAPS; ++k) {
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (k < a.taps) v = k <= local ? load_four(proj + (int64_t)(t - k) * a.stride + a.off_q + c)
-                                       : load_four(tail + (int64_t)(a.taps - 1 + local - k) * cc + c);
-        spread(v, win[WIDE_TAPS - 1 - k]);
+    for (int e = 0; e < TOKENS_EACH; ++e) {
+      const int t = t_begin + e;
+      if (t >= t_end) break;
+      if (b < 0 || t >= next_first) {                        // a new request (or the warp's first token): fill the window anew
+        b = a.request_of[t];
+        const int first = a.cu_q[b];
+        next_first = a.cu_q[b + 1];
+        int slot = a.state_slots[b];
+        if (slot < 0 || slot >= a.num_slots) {
+          if (lane == 0 && unit == 0) raise_fault(a.status, VOSTI_FAULT_SLOT_RANGE);
+          slot = 0;
+        }
+        const float* const tail = a.state + (int64_t)slot * a.state_stride + a.conv_offset;       // [taps - 1, cc]
+        const int local = t - first;
+#pragma unroll
+        for (int k = 1; k < WIDE_TAPS; ++k) {
+          float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (k < a.taps) v = k <= local ? (t == t_first ? before[k - 1] : load_four(proj + (int64_t)(t - k) * a.stride + a.off_q + c))
+                                         : load_four(tail + (int64_t)(a.taps - 1 + local - k) * cc + c);
+          spread(v, win[WIDE_TAPS - 1 - k]);
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < WIDE_TAPS - 1; ++k)
+#pragma unroll
+          for (int u = 0; u < 4; ++u) win[k][u] = win[k + 1][u];
       }
-    } else {
+      spread(ahead[e], win[WIDE_TAPS - 1]);
+      float y[4];
 #pragma unroll
-      for (int k = 0; k < WIDE_TAPS - 1; ++k)
+      for (int u = 0; u < 4; ++u) {
+        float acc = 0.f;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) win[k][u] = win[k + 1][u];
+        for (int k = 0; k < WIDE_TAPS; ++k) if (k >= WIDE_TAPS - a.taps) acc = fmaf(w[k][u], win[k][u], acc);
+        y[u] = acc * sigmoidf_(acc);
+      }
+      if (head < 0) {
+        const float ss = warp_sum((y[0] * y[0] + y[1] * y[1]) + (y[2] * y[2] + y[3] * y[3]));
+        const bool is_q = unit < a.kv_heads;
+        const float scale = (1.f / sqrtf(ss + 1e-6f)) * (is_q ? 1.f / sqrtf((float)D) : 1.f);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) y[u] *= scale;
+        store_four((is_q ? a.q : a.k) + (int64_t)t * cq + (is_q ? unit : unit - a.kv_heads) * D + lane * 4, y);
+        continue;
+      }
+      const int64_t at = (int64_t)t * cv + head * D + lane * 4;
+      store_four(a.v + at, y);
+      float z[4], rate[4];
+      spread(gates[e], z);
+      spread(rates[e], rate);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) z[u] = a.gate_silu ? z[u] * sigmoidf_(z[u]) : sigmoidf_(z[u]);
+      store_four(a.gate + at, z);
+      if (a.decay_per_head) {
+        rate[0] = rate[1] = rate[2] = rate[3] = expf(-speed * softplusf_(rate[0] + shift[0]));
+      } else {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) rate[u] = expf(-speed * softplusf_(rate[u] + shift[u]));
+      }
+      store_four(a.decay + at, rate);
+      if (lane == 0) a.beta[(int64_t)t * a.heads + head] = sigmoidf_(to_f32(proj[(int64_t)t * a.stride + a.off_beta + head]));
     }
-    spread(ahead[e], win[WIDE_TAPS - 1]);
-    float y[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      float acc = 0.f;
-#pragma unroll
-      for (int k = 0; k < WIDE_TAPS; ++k) if (k >= WIDE_TAPS - a.taps) acc = fmaf(w[k][u], win[k][u], acc);
-      y[u] = acc * sigmoidf_(acc);
-    }
-    if (head < 0) {
-      const float ss = warp_sum((y[0] * y[0] + y[1] * y[1]) + (y[2] * y[2] + y[3] * y[3]));
-      const bool is_q = unit < a.kv_heads;
-      const float scale = (1.f / sqrtf(ss + 1e-6f)) * (is_q ? 1.f / sqrtf((float)D) : 1.f);
-#pragma unroll
-      for (int u = 0; u < 4; ++u) y[u] *= scale;
-      store_four((is_q ? a.q : a.k) + (int64_t)t * cq + (is_q ? unit : unit - a.kv_heads) * D + lane * 4, y);
-      continue;
-    }
-    const int64_t at = (int64_t)t * cv + head * D + lane * 4;
-    store_four(a.v + at, y);
-    float z[4], rate[4];
-    spread(gates[e], z);
-    spread(rates[e], rate);
-#pragma unroll
-    for (int u = 0; u < 4; ++u) z[u] = a.gate_silu ? z[u] * sigmoidf_(z[u]) : sigmoidf_(z[u]);
-    store_four(a.gate + at, z);
-    if (a.decay_per_head) {
-      rate[0] = rate[1] = rate[2] = rate[3] = expf(-speed * softplusf_(rate[0] + shift[0]));
-    } else {
-#pragma unroll
-      for (int u = 0; u < 4; ++u) rate[u] = expf(-speed * softplusf_(rate[u] + shift[u]));
-    }
-    store_four(a.decay + at, rate);
-    if (lane == 0) a.beta[(int64_t)t * a.heads + head] = sigmoidf_(to_f32(proj[(int64_t)t * a.stride + a.off_beta + head]));
   }
 }
 
@@ -752,15 +779,16 @@ VOSTI_API int vosti_delta_prep(const void* proj, int proj_f32, int stride, int o
                     ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
                       reinterpret_cast<uintptr_t>(decay) | reinterpret_cast<uintptr_t>(gate)) & 15) == 0 && (units + 3) / 4 <= 65535;
   if (wide) {
-    // one token a warp while the tokens alone do not fill the SMs' warps, four where they do
-    const int each = (int64_t)tokens * units >= 148 * 64 ? 4 : 1;
+    // one token a warp while the tokens alone do not fill the SMs' warps, twice four where they do
+    a.w_words = taps == WIDE_TAPS && ((reinterpret_cast<uintptr_t>(conv_w) | reinterpret_cast<uintptr_t>(dt_bias)) & (w_f32 ? 15 : 7)) == 0;
+    const int each = (int64_t)tokens * units >= 148 * 64 ? 8 : 1;
     const dim3 grid((tokens + each - 1) / each, (units + 3) / 4);
     if (proj_f32) {
-      if (each == 4) vosti_launch(delta_prep_wide_kernel<float, 4>, grid, dim3(128), 0, stream, a, tokens);
-      else vosti_launch(delta_prep_wide_kernel<float, 1>, grid, dim3(128), 0, stream, a, tokens);
+      if (each == 8) vosti_launch(delta_prep_wide_kernel<float, 4, 2>, grid, dim3(128), 0, stream, a, tokens);
+      else vosti_launch(delta_prep_wide_kernel<float, 1, 1>, grid, dim3(128), 0, stream, a, tokens);
     } else {
-      if (each == 4) vosti_launch(delta_prep_wide_kernel<bf16, 4>, grid, dim3(128), 0, stream, a, tokens);
-      else vosti_launch(delta_prep_wide_kernel<bf16, 1>, grid, dim3(128), 0, stream, a, tokens);
+      if (each == 8) vosti_launch(delta_prep_wide_kernel<bf16, 4, 2>, grid, dim3(128), 0, stream, a, tokens);
+      else vosti_launch(delta_prep_wide_kernel<bf16, 1, 1>, grid, dim3(128), 0, stream, a, tokens);
     }
   } else {
     vosti_launch(delta_prep_kernel, dim3(tokens, (units + 7) / 8 < 65535 ? (units + 7) / 8 : 65535), dim3(256), 0, stream, a);

@@ -22,6 +22,7 @@
 #include <cfloat>
 
 #include "common.cuh"
+#include "mma_util.cuh"
 
 namespace {
 
@@ -138,10 +139,28 @@ scan_conv4_kernel(const T* __restrict__ xz, int64_t xz_stride, const void* __res
   for (int u = 0; u < 4; ++u) {
     bias[u] = conv_b != nullptr ? load_flex(conv_b, w_f32, c + u) : 0.f;
 #pragma unroll
-    for (int k = 0; k < TAPS; ++k) { w[k][u] = load_flex(conv_w, w_f32, (int64_t)(c + u) * TAPS + k); win[k][u] = 0.f; }
+    for (int k = 0; k < TAPS; ++k) win[k][u] = 0.f;
+  }
+  if (TAPS == 4 && (reinterpret_cast<uintptr_t>(conv_w) & (w_f32 ? 15 : 7)) == 0) {        // a channel's taps are one word
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const float4 v = w_f32 ? load_four(reinterpret_cast<const float*>(conv_w) + (c + u) * 4) : load_four(reinterpret_cast<const bf16*>(conv_w) + (c + u) * 4);
+      const float taps4[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int k = 0; k < TAPS; ++k) w[k][u] = taps4[k];
+    }
+  } else {
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int k = 0; k < TAPS; ++k) w[k][u] = load_flex(conv_w, w_f32, (int64_t)(c + u) * TAPS + k);
   }
   int b = -1, next_first = 0;
   bool usable = false;
+  // the rows before the block's first token, asked for before its request is known
+  float4 before[TAPS - 1];
+#pragma unroll
+  for (int k = 1; k < TAPS; ++k) before[k - 1] = load_four(xz + (int64_t)max(t_begin - k, 0) * xz_stride + c);
   for (int t0 = t_begin; t0 < t_end; t0 += CONV_AHEAD) {
     float4 x[CONV_AHEAD];
 #pragma unroll
@@ -161,7 +180,7 @@ scan_conv4_kernel(const T* __restrict__ xz, int64_t xz_stride, const void* __res
 #pragma unroll
         for (int k = 1; k < TAPS; ++k) {               // the input k tokens back: of this portion, or from the tail
           const int back = t - first;
-          const float4 v = k <= back ? load_four(xz + (int64_t)(t - k) * xz_stride + c)
+          const float4 v = k <= back ? (t == t_begin ? before[k - 1] : load_four(xz + (int64_t)(t - k) * xz_stride + c))
                                      : load_four(tail + (int64_t)(TAPS - 1 - (k - back)) * inner + c);
           win[TAPS - 1 - k][0] = v.x; win[TAPS - 1 - k][1] = v.y; win[TAPS - 1 - k][2] = v.z; win[TAPS - 1 - k][3] = v.w;
         }
@@ -417,8 +436,8 @@ scan_line_kernel(const T* __restrict__ x, const float* __restrict__ dtp, const v
     for (int j = 0; j < 4; ++j) {
       s[j] = S[j];
       // (finite also where the rate is not: a tile's places past the last token have a step size of 0 and must change nothing)
-      const float rate = expf(load_flex(a_log, w_f32, (int64_t)(live ? c : inner - 1) * N + r * 4 + j));
-      a[j] = rate == INFINITY ? -FLT_MAX : -rate;
+      const float rate = expf(load_flex(a_log, w_f32, (int64_t)(live ? c : inner - 1) * N + r * 4 + j)) * 1.4426950408889634f;
+      a[j] = rate == INFINITY ? -FLT_MAX : -rate;               // the decay is 2^(dt a)
     }
   } else {
     fetch(0);
@@ -446,7 +465,7 @@ scan_line_kernel(const T* __restrict__ x, const float* __restrict__ dtp, const v
           g.in[u][2] = dx * B.z;
           g.in[u][3] = dx * B.w;
 #pragma unroll
-          for (int j = 0; j < 4; ++j) g.e[u][j] = expf(dt * a[j]);
+          for (int j = 0; j < 4; ++j) g.e[u][j] = fast_exp2(dt * a[j]);
         }
       };
       auto chain = [&](const Group& g, int i0) {
