@@ -154,8 +154,10 @@ __global__ void __launch_bounds__(256) delta_prep_kernel(PrepArgs a) {
 // unit and a warp takes TOKENS_EACH tokens one after the other, so that the taps' weights, the decay's constants
 // and the last inputs stay in registers and a token's inputs and results are whole words; a v head's warp also makes
 // its head's beta, decay and gate. The kernel above is bound by its scalar loads (each input read once per tap): 87 us
-// for 2,048 tokens of 16 heads (4 key heads); this one takes 61, against the 16 that the 105 MB take. What is left of that is
-// the weights: 16 single elements a lane and four constants, more loads than the data of four tokens need.
+// for 2,048 tokens of 16 heads (4 key heads); this one was bound by the rounds of loads that a warp waited for (three before its
+// first token, 148 registers and so 12 warps an SM: 58 us), so weights come as words, the rows before the first token without
+// waiting for its request, a warp takes its tokens one after the other and a thread has 72 registers (28 warps an SM): 42 us
+// past the product before it.
 constexpr int WIDE_TAPS = 4;
 
 __device__ __forceinline__ void store_four(float* p, const float (&v)[4]) { *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]); }
@@ -164,8 +166,8 @@ __device__ __forceinline__ float4 flex_four(const void* p, int is_f32, int64_t i
 }
 __device__ __forceinline__ void spread(float4 v, float (&to)[4]) { to[0] = v.x; to[1] = v.y; to[2] = v.z; to[3] = v.w; }
 
-template <typename T, int TOKENS_EACH, int BATCHES>
-__global__ void __launch_bounds__(128) delta_prep_wide_kernel(PrepArgs a, int tokens) {
+template <typename T, int TOKENS_EACH>
+__global__ void __launch_bounds__(128, 7) delta_prep_wide_kernel(PrepArgs a, int tokens) {
   pdl_wait();
   pdl_launch_dependents();
   constexpr int D = 128;
@@ -208,98 +210,88 @@ __global__ void __launch_bounds__(128) delta_prep_wide_kernel(PrepArgs a, int to
     }
   }
   const int rd = a.decay_per_head ? a.heads : a.heads * D;
+  const int t_first = blockIdx.x * TOKENS_EACH, t_end = min(tokens, t_first + TOKENS_EACH);
+  // a token's words, asked for together
+  struct Words { float4 x, gate, rate; };
+  auto ask = [&](Words& to, int t) {
+    to.x = load_four(proj + (int64_t)t * a.stride + a.off_q + c);
+    if (head < 0) return;
+    const int64_t row = (int64_t)t * (rd + cv);
+    to.gate = flex_four(a.rates, a.rates_f32, row + rd + head * D + lane * 4);
+    if (a.decay_per_head) {
+      const float r = load_flex(a.rates, a.rates_f32, row + head);
+      to.rate = make_float4(r, r, r, r);
+    } else {
+      to.rate = flex_four(a.rates, a.rates_f32, row + head * D + lane * 4);
+    }
+  };
   // the rows before the warp's first token, asked for before its request is known (its own from the request's fourth token on)
-  const int t_first = blockIdx.x * BATCHES * TOKENS_EACH;
   float4 before[WIDE_TAPS - 1];
 #pragma unroll
   for (int k = 1; k < WIDE_TAPS; ++k) before[k - 1] = load_four(proj + (int64_t)max(t_first - k, 0) * a.stride + a.off_q + c);
   int b = -1, next_first = 0;
 #pragma unroll 1
-  for (int batch = 0; batch < BATCHES; ++batch) {
-    const int t_begin = t_first + batch * TOKENS_EACH, t_end = min(tokens, t_begin + TOKENS_EACH);
-    float4 ahead[TOKENS_EACH], gates[TOKENS_EACH], rates[TOKENS_EACH];
-#pragma unroll
-    for (int e = 0; e < TOKENS_EACH; ++e) {
-      const int t = t_begin + e;
-      if (t >= t_end) break;
-      ahead[e] = load_four(proj + (int64_t)t * a.stride + a.off_q + c);
-      if (head >= 0) {
-        const int64_t row = (int64_t)t * (rd + cv);
-        auto rate4 = [&](int64_t at) {
-          return a.rates_f32 ? load_four(reinterpret_cast<const float*>(a.rates) + at) : load_four(reinterpret_cast<const bf16*>(a.rates) + at);
-        };
-        gates[e] = rate4(row + rd + head * D + lane * 4);
-        if (a.decay_per_head) {
-          const float r = load_flex(a.rates, a.rates_f32, row + head);
-          rates[e] = make_float4(r, r, r, r);
-        } else {
-          rates[e] = rate4(row + head * D + lane * 4);
-        }
+  for (int t = t_first; t < t_end; ++t) {
+    Words now = {};
+    ask(now, t);
+    if (b < 0 || t >= next_first) {                        // a new request (or the warp's first token): fill the window anew
+      b = a.request_of[t];
+      const int first = a.cu_q[b];
+      next_first = a.cu_q[b + 1];
+      int slot = a.state_slots[b];
+      if (slot < 0 || slot >= a.num_slots) {
+        if (lane == 0 && unit == 0) raise_fault(a.status, VOSTI_FAULT_SLOT_RANGE);
+        slot = 0;
       }
+      const float* const tail = a.state + (int64_t)slot * a.state_stride + a.conv_offset;       // [taps - 1, cc]
+      const int local = t - first;
+#pragma unroll
+      for (int k = 1; k < WIDE_TAPS; ++k) {
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (k < a.taps) v = k <= local ? (t == t_first ? before[k - 1] : load_four(proj + (int64_t)(t - k) * a.stride + a.off_q + c))
+                                       : load_four(tail + (int64_t)(a.taps - 1 + local - k) * cc + c);
+        spread(v, win[WIDE_TAPS - 1 - k]);
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < WIDE_TAPS - 1; ++k)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) win[k][u] = win[k + 1][u];
     }
+    spread(now.x, win[WIDE_TAPS - 1]);
+    float y[4];
 #pragma unroll
-    for (int e = 0; e < TOKENS_EACH; ++e) {
-      const int t = t_begin + e;
-      if (t >= t_end) break;
-      if (b < 0 || t >= next_first) {                        // a new request (or the warp's first token): fill the window anew
-        b = a.request_of[t];
-        const int first = a.cu_q[b];
-        next_first = a.cu_q[b + 1];
-        int slot = a.state_slots[b];
-        if (slot < 0 || slot >= a.num_slots) {
-          if (lane == 0 && unit == 0) raise_fault(a.status, VOSTI_FAULT_SLOT_RANGE);
-          slot = 0;
-        }
-        const float* const tail = a.state + (int64_t)slot * a.state_stride + a.conv_offset;       // [taps - 1, cc]
-        const int local = t - first;
+    for (int u = 0; u < 4; ++u) {
+      float acc = 0.f;
 #pragma unroll
-        for (int k = 1; k < WIDE_TAPS; ++k) {
-          float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (k < a.taps) v = k <= local ? (t == t_first ? before[k - 1] : load_four(proj + (int64_t)(t - k) * a.stride + a.off_q + c))
-                                         : load_four(tail + (int64_t)(a.taps - 1 + local - k) * cc + c);
-          spread(v, win[WIDE_TAPS - 1 - k]);
-        }
-      } else {
-#pragma unroll
-        for (int k = 0; k < WIDE_TAPS - 1; ++k)
-#pragma unroll
-          for (int u = 0; u < 4; ++u) win[k][u] = win[k + 1][u];
-      }
-      spread(ahead[e], win[WIDE_TAPS - 1]);
-      float y[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        float acc = 0.f;
-#pragma unroll
-        for (int k = 0; k < WIDE_TAPS; ++k) if (k >= WIDE_TAPS - a.taps) acc = fmaf(w[k][u], win[k][u], acc);
-        y[u] = acc * sigmoidf_(acc);
-      }
-      if (head < 0) {
-        const float ss = warp_sum((y[0] * y[0] + y[1] * y[1]) + (y[2] * y[2] + y[3] * y[3]));
-        const bool is_q = unit < a.kv_heads;
-        const float scale = (1.f / sqrtf(ss + 1e-6f)) * (is_q ? 1.f / sqrtf((float)D) : 1.f);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) y[u] *= scale;
-        store_four((is_q ? a.q : a.k) + (int64_t)t * cq + (is_q ? unit : unit - a.kv_heads) * D + lane * 4, y);
-        continue;
-      }
-      const int64_t at = (int64_t)t * cv + head * D + lane * 4;
-      store_four(a.v + at, y);
-      float z[4], rate[4];
-      spread(gates[e], z);
-      spread(rates[e], rate);
-#pragma unroll
-      for (int u = 0; u < 4; ++u) z[u] = a.gate_silu ? z[u] * sigmoidf_(z[u]) : sigmoidf_(z[u]);
-      store_four(a.gate + at, z);
-      if (a.decay_per_head) {
-        rate[0] = rate[1] = rate[2] = rate[3] = expf(-speed * softplusf_(rate[0] + shift[0]));
-      } else {
-#pragma unroll
-        for (int u = 0; u < 4; ++u) rate[u] = expf(-speed * softplusf_(rate[u] + shift[u]));
-      }
-      store_four(a.decay + at, rate);
-      if (lane == 0) a.beta[(int64_t)t * a.heads + head] = sigmoidf_(to_f32(proj[(int64_t)t * a.stride + a.off_beta + head]));
+      for (int k = 0; k < WIDE_TAPS; ++k) if (k >= WIDE_TAPS - a.taps) acc = fmaf(w[k][u], win[k][u], acc);
+      y[u] = acc * sigmoidf_(acc);
     }
+    if (head < 0) {
+      const float ss = warp_sum((y[0] * y[0] + y[1] * y[1]) + (y[2] * y[2] + y[3] * y[3]));
+      const bool is_q = unit < a.kv_heads;
+      const float scale = (1.f / sqrtf(ss + 1e-6f)) * (is_q ? 1.f / sqrtf((float)D) : 1.f);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) y[u] *= scale;
+      store_four((is_q ? a.q : a.k) + (int64_t)t * cq + (is_q ? unit : unit - a.kv_heads) * D + lane * 4, y);
+      continue;
+    }
+    const int64_t at = (int64_t)t * cv + head * D + lane * 4;
+    store_four(a.v + at, y);
+    float z[4], rate[4];
+    spread(now.gate, z);
+    spread(now.rate, rate);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) z[u] = a.gate_silu ? z[u] * sigmoidf_(z[u]) : sigmoidf_(z[u]);
+    store_four(a.gate + at, z);
+    if (a.decay_per_head) {
+      rate[0] = rate[1] = rate[2] = rate[3] = expf(-speed * softplusf_(rate[0] + shift[0]));
+    } else {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) rate[u] = expf(-speed * softplusf_(rate[u] + shift[u]));
+    }
+    store_four(a.decay + at, rate);
+    if (lane == 0) a.beta[(int64_t)t * a.heads + head] = sigmoidf_(to_f32(proj[(int64_t)t * a.stride + a.off_beta + head]));
   }
 }
 
@@ -779,16 +771,16 @@ VOSTI_API int vosti_delta_prep(const void* proj, int proj_f32, int stride, int o
                     ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
                       reinterpret_cast<uintptr_t>(decay) | reinterpret_cast<uintptr_t>(gate)) & 15) == 0 && (units + 3) / 4 <= 65535;
   if (wide) {
-    // one token a warp while the tokens alone do not fill the SMs' warps, twice four where they do
+    // one token a warp while the tokens alone do not fill the SMs' warps, eight where they do
     a.w_words = taps == WIDE_TAPS && ((reinterpret_cast<uintptr_t>(conv_w) | reinterpret_cast<uintptr_t>(dt_bias)) & (w_f32 ? 15 : 7)) == 0;
     const int each = (int64_t)tokens * units >= 148 * 64 ? 8 : 1;
     const dim3 grid((tokens + each - 1) / each, (units + 3) / 4);
     if (proj_f32) {
-      if (each == 8) vosti_launch(delta_prep_wide_kernel<float, 4, 2>, grid, dim3(128), 0, stream, a, tokens);
-      else vosti_launch(delta_prep_wide_kernel<float, 1, 1>, grid, dim3(128), 0, stream, a, tokens);
+      if (each == 8) vosti_launch(delta_prep_wide_kernel<float, 8>, grid, dim3(128), 0, stream, a, tokens);
+      else vosti_launch(delta_prep_wide_kernel<float, 1>, grid, dim3(128), 0, stream, a, tokens);
     } else {
-      if (each == 8) vosti_launch(delta_prep_wide_kernel<bf16, 4, 2>, grid, dim3(128), 0, stream, a, tokens);
-      else vosti_launch(delta_prep_wide_kernel<bf16, 1, 1>, grid, dim3(128), 0, stream, a, tokens);
+      if (each == 8) vosti_launch(delta_prep_wide_kernel<bf16, 8>, grid, dim3(128), 0, stream, a, tokens);
+      else vosti_launch(delta_prep_wide_kernel<bf16, 1>, grid, dim3(128), 0, stream, a, tokens);
     }
   } else {
     vosti_launch(delta_prep_kernel, dim3(tokens, (units + 7) / 8 < 65535 ? (units + 7) / 8 : 65535), dim3(256), 0, stream, a);

@@ -139,28 +139,10 @@ scan_conv4_kernel(const T* __restrict__ xz, int64_t xz_stride, const void* __res
   for (int u = 0; u < 4; ++u) {
     bias[u] = conv_b != nullptr ? load_flex(conv_b, w_f32, c + u) : 0.f;
 #pragma unroll
-    for (int k = 0; k < TAPS; ++k) win[k][u] = 0.f;
-  }
-  if (TAPS == 4 && (reinterpret_cast<uintptr_t>(conv_w) & (w_f32 ? 15 : 7)) == 0) {        // a channel's taps are one word
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const float4 v = w_f32 ? load_four(reinterpret_cast<const float*>(conv_w) + (c + u) * 4) : load_four(reinterpret_cast<const bf16*>(conv_w) + (c + u) * 4);
-      const float taps4[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int k = 0; k < TAPS; ++k) w[k][u] = taps4[k];
-    }
-  } else {
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-      for (int k = 0; k < TAPS; ++k) w[k][u] = load_flex(conv_w, w_f32, (int64_t)(c + u) * TAPS + k);
+    for (int k = 0; k < TAPS; ++k) { w[k][u] = load_flex(conv_w, w_f32, (int64_t)(c + u) * TAPS + k); win[k][u] = 0.f; }
   }
   int b = -1, next_first = 0;
   bool usable = false;
-  // the rows before the block's first token, asked for before its request is known
-  float4 before[TAPS - 1];
-#pragma unroll
-  for (int k = 1; k < TAPS; ++k) before[k - 1] = load_four(xz + (int64_t)max(t_begin - k, 0) * xz_stride + c);
   for (int t0 = t_begin; t0 < t_end; t0 += CONV_AHEAD) {
     float4 x[CONV_AHEAD];
 #pragma unroll
@@ -180,7 +162,7 @@ scan_conv4_kernel(const T* __restrict__ xz, int64_t xz_stride, const void* __res
 #pragma unroll
         for (int k = 1; k < TAPS; ++k) {               // the input k tokens back: of this portion, or from the tail
           const int back = t - first;
-          const float4 v = k <= back ? (t == t_begin ? before[k - 1] : load_four(xz + (int64_t)(t - k) * xz_stride + c))
+          const float4 v = k <= back ? load_four(xz + (int64_t)(t - k) * xz_stride + c)
                                      : load_four(tail + (int64_t)(TAPS - 1 - (k - back)) * inner + c);
           win[TAPS - 1 - k][0] = v.x; win[TAPS - 1 - k][1] = v.y; win[TAPS - 1 - k][2] = v.z; win[TAPS - 1 - k][3] = v.w;
         }
@@ -348,11 +330,12 @@ scan_run_kernel(const T* __restrict__ x, const float* __restrict__ dtp, const vo
 }
 
 // A long portion of 16 states a channel, tokens in order in one pass. The chain from token to token is one
-// multiply-add a state; everything else of a token (its exponentials above all) is off the chain, so 32 channels
-// a block and a token every 130 cycles (68 ns) need no chunks, whose first pass computes every exponential a second
+// multiply-add a state; everything else of a token (its exponentials above all: one ex2 of a base-2 rate, where expf took
+// eight instructions and 152 us instead of 136) is off the chain, so 32 channels
+// a block and a token every 120 cycles (62 ns) need no chunks, whose first pass computes every exponential a second
 // time. Warps 0 to 3 run the recurrence, four lanes a channel with four neighbouring states each; warps 4 to 11
 // meanwhile finish the tile before (skip, gate, store) and bring the tile after (softplus, SiLU) into the
-// other buffer. 1,499 + 549 tokens of 4,096 channels: 147 us, against 324 us of the three chunk kernels; 2,048 tokens
+// other buffer. 1,499 + 549 tokens of 4,096 channels: 131 us, against 324 us of the three chunk kernels; 2,048 tokens
 // 144 against 324, 1,024 tokens beside 30 single ones 89 against 226.
 constexpr int LINE_TOKENS = 64, LINE_STATES = 16, LINE_AHEAD = 4;          // (the dealing out of sums is written for four)
 constexpr int LINE_BRING = 256, LINE_THREADS = 128 + LINE_BRING;         // threads that bring, and all of a block
