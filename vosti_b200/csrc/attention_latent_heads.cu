@@ -293,22 +293,25 @@ latent_heads_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   } else {
     // ------------------------------------------------------------ MMA issue
     asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
-    if (lane == 0) {
-      // four issuing threads, one per warp: scores of row tile 0, of row tile 1, products of row tile 0, of row tile 1
-      const int role = warp - MMA_WARP, wg = role & 1;
-      const int my_tiles = wg ? tiles_of[1] : tiles_of[0];
-      constexpr uint32_t idesc_s = umma_instr_desc(ROWS, KT, false);
-      constexpr uint32_t idesc_o = umma_instr_desc(ROWS, D, true);
-      bool ok = true;
-      if (role < 2) {
-        const uint64_t q_desc = smem_desc_sw128(smem_u32(q_s) + wg * Q_BYTES), k_desc = smem_desc_sw128(smem_u32(kv_s));
-        if (my_tiles > 0) ok = mbar_wait(smem_u32(&q_full), 0, &abort_flag, status);
-        for (int t = 0; t < my_tiles && ok; ++t) {
-          const int stage = t % STAGES;
-          ok = mbar_wait(smem_u32(&kv_full[stage]), (t / STAGES) & 1, &abort_flag, status);
-          if (ok && t >= 1) ok = mbar_wait(smem_u32(&s_empty[wg]), (t - 1) & 1, &abort_flag, status);
-          if (!ok) break;
-          tc_fence_after();
+    // four issuing threads, one per warp: scores of row tile 0, of row tile 1, products of row tile 0, of row tile 1
+    const int role = warp - MMA_WARP, wg = role & 1;
+    const int my_tiles = wg ? tiles_of[1] : tiles_of[0];
+    constexpr uint32_t idesc_s = umma_instr_desc(ROWS, KT, false);
+    constexpr uint32_t idesc_o = umma_instr_desc(ROWS, D, true);
+    bool ok = true;
+    auto arrived = [&](uint64_t* bar, uint32_t parity) {
+      return __all_sync(0xffffffffu, mbar_wait(smem_u32(bar), parity, &abort_flag, status)) != 0;
+    };
+    if (role < 2) {
+      const uint64_t q_desc = smem_desc_sw128(smem_u32(q_s) + wg * Q_BYTES), k_desc = smem_desc_sw128(smem_u32(kv_s));
+      if (my_tiles > 0) ok = arrived(&q_full, 0);
+      for (int t = 0; t < my_tiles && ok; ++t) {
+        const int stage = t % STAGES;
+        ok = arrived(&kv_full[stage], (t / STAGES) & 1);
+        if (ok && t >= 1) ok = arrived(&s_empty[wg], (t - 1) & 1);
+        if (!ok) break;
+        tc_fence_after();
+        if (elect_one()) {
 #pragma unroll
           for (int kb = 0; kb < Q_BLOCKS; ++kb)
 #pragma unroll
@@ -317,21 +320,24 @@ latent_heads_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                         k_desc + (uint64_t)((stage * STAGE_BYTES + kb * BLOCK_BYTES + ks * 32) >> 4), idesc_s, (kb | ks) ? 1u : 0u);
           umma_commit(smem_u32(&s_full[wg]));
         }
-      } else {
-        const uint64_t v_desc = smem_desc_sw128_mn(smem_u32(kv_s) + V_AT, BLOCK_BYTES);
-        for (int t = 0; t < tiles && ok; ++t) {
-          const int stage = t % STAGES;
-          ok = mbar_wait(smem_u32(&kv_full[stage]), (t / STAGES) & 1, &abort_flag, status);
-          if (!ok) break;
-          if (t >= my_tiles) {                            // the other row tile's alone: given back as soon as it is here
-            mbar_arrive(smem_u32(&kv_empty[stage]));
-            continue;
-          }
-          ok = mbar_wait(smem_u32(&p_full[wg]), t & 1, &abort_flag, status);
-          if (!ok) break;
-          tc_fence_after();
-          const uint32_t o = tmem_base + O_COL + wg * D, p = tmem_base + P_COL + wg * KT;
-          const uint64_t hi = v_desc + (uint64_t)((stage * STAGE_BYTES) >> 4), lo = hi + (uint64_t)((LO_AT - V_AT) >> 4);
+        __syncwarp();
+      }
+    } else {
+      const uint64_t v_desc = smem_desc_sw128_mn(smem_u32(kv_s) + V_AT, BLOCK_BYTES);
+      for (int t = 0; t < tiles && ok; ++t) {
+        const int stage = t % STAGES;
+        ok = arrived(&kv_full[stage], (t / STAGES) & 1);
+        if (!ok) break;
+        if (t >= my_tiles) {                            // the other row tile's alone: given back as soon as it is here
+          if (lane == 0) mbar_arrive(smem_u32(&kv_empty[stage]));
+          continue;
+        }
+        ok = arrived(&p_full[wg], t & 1);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t o = tmem_base + O_COL + wg * D, p = tmem_base + P_COL + wg * KT;
+        const uint64_t hi = v_desc + (uint64_t)((stage * STAGE_BYTES) >> 4), lo = hi + (uint64_t)((LO_AT - V_AT) >> 4);
+        if (elect_one()) {
 #pragma unroll
           for (int ks = 0; ks < KT / 16; ++ks) {
             const uint32_t p_hi = p + (ks >> 1) * 32 + (ks & 1) * 8, p_lo = p_hi + 16;
@@ -343,6 +349,7 @@ latent_heads_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
           umma_commit(smem_u32(&p_empty[wg]));
           umma_commit(smem_u32(&kv_empty[stage]));        // (the scores of this stage were complete before its weights came)
         }
+        __syncwarp();
       }
     }
   }

@@ -376,28 +376,31 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   } else {
     // ------------------------------------------------------------ MMA issue
     asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
-    if (lane == 0) {
-      // Four issuing threads, one per warp: scores of row tile 0, scores of row tile 1, products of
-      // row tile 0, products of row tile 1. One thread alone cannot issue a tile's twelve MMAs and
-      // wait on its barriers as fast as the tensor core retires them.
-      const int role = warp - MMA_WARP, wg = role & 1;
-      const int my_tiles = wg ? tiles_of[1] : tiles_of[0];
-      constexpr uint32_t idesc_s = umma_instr_desc(ROWS, KT, false);
-      constexpr uint32_t idesc_pv = umma_instr_desc(ROWS, D, true);
-      // descriptors differ in their start address only: bits [0,14) in units of 16 bytes
-      const uint64_t q_desc = smem_desc_sw128(smem_u32(q_s) + wg * Q_BYTES), k_desc = smem_desc_sw128(smem_u32(kv_s));
-      const uint64_t v_desc = smem_desc_sw128_mn(smem_u32(kv_s) + K_BYTES, KT * 128);
-      bool ok = true;
-      if (role < 2) {
-        // S_t = Q K_t^T into the score buffer of the row tile
-        ok = mbar_wait(smem_u32(&q_full), 0, &abort_flag, status);
-        for (int t = 0; t < my_tiles && ok; ++t) {
-          const int stage = t % STAGES;
-          ok = mbar_wait(smem_u32(&kv_full[stage]), (t / STAGES) & 1, &abort_flag, status);
-          if (ok && t >= 1) ok = mbar_wait(smem_u32(&s_empty[wg]), (t - 1) & 1, &abort_flag, status);
-          if (!ok) break;
-          tc_fence_after();
-          const uint64_t kd = k_desc + (uint64_t)((stage * STAGE_BYTES) >> 4);
+    // Four issuing threads, one per warp: scores of row tile 0, scores of row tile 1, products of
+    // row tile 0, products of row tile 1. One thread alone cannot issue a tile's twelve MMAs and
+    // wait on its barriers as fast as the tensor core retires them.
+    const int role = warp - MMA_WARP, wg = role & 1;
+    const int my_tiles = wg ? tiles_of[1] : tiles_of[0];
+    constexpr uint32_t idesc_s = umma_instr_desc(ROWS, KT, false);
+    constexpr uint32_t idesc_pv = umma_instr_desc(ROWS, D, true);
+    // descriptors differ in their start address only: bits [0,14) in units of 16 bytes
+    const uint64_t q_desc = smem_desc_sw128(smem_u32(q_s) + wg * Q_BYTES), k_desc = smem_desc_sw128(smem_u32(kv_s));
+    const uint64_t v_desc = smem_desc_sw128_mn(smem_u32(kv_s) + K_BYTES, KT * 128);
+    bool ok = true;
+    auto arrived = [&](uint64_t* bar, uint32_t parity) {
+      return __all_sync(0xffffffffu, mbar_wait(smem_u32(bar), parity, &abort_flag, status)) != 0;
+    };
+    if (role < 2) {
+      // S_t = Q K_t^T into the score buffer of the row tile
+      ok = arrived(&q_full, 0);
+      for (int t = 0; t < my_tiles && ok; ++t) {
+        const int stage = t % STAGES;
+        ok = arrived(&kv_full[stage], (t / STAGES) & 1);
+        if (ok && t >= 1) ok = arrived(&s_empty[wg], (t - 1) & 1);
+        if (!ok) break;
+        tc_fence_after();
+        const uint64_t kd = k_desc + (uint64_t)((stage * STAGE_BYTES) >> 4);
+        if (elect_one()) {
 #pragma unroll
           for (int kb = 0; kb < NB; ++kb)
 #pragma unroll
@@ -406,24 +409,27 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                         kd + (uint64_t)((kb * (KT * 128) + ks * 32) >> 4), idesc_s, (kb | ks) ? 1u : 0u);
           umma_commit(smem_u32(&s_full[wg]));
         }
-      } else {
-        // (P V) of tile t, 16 keys per MMA; V rows are [key][64 features] blocks: MN-major.
-        // A stage is given back when both row tiles' products of it are complete; a row tile that
-        // ends before the other one still counts itself in for the remaining tiles, each time
-        // after the tile has arrived, so that it never runs a phase ahead.
-        for (int t = 0; t < tiles && ok; ++t) {
-          const int stage = t % STAGES;
-          ok = mbar_wait(smem_u32(&kv_full[stage]), (t / STAGES) & 1, &abort_flag, status);
-          if (!ok) break;
-          if (t >= my_tiles) {
-            mbar_arrive(smem_u32(&kv_empty[stage]));
-            continue;
-          }
-          ok = mbar_wait(smem_u32(&p_full[wg][t & 1]), (t >> 1) & 1, &abort_flag, status);
-          if (!ok) break;
-          tc_fence_after();
-          const uint64_t vd = v_desc + (uint64_t)((stage * STAGE_BYTES) >> 4);
-          const uint64_t p_desc = smem_desc_sw128(smem_u32(p_s) + (wg * 2 + (t & 1)) * P_BYTES);
+        __syncwarp();
+      }
+    } else {
+      // (P V) of tile t, 16 keys per MMA; V rows are [key][64 features] blocks: MN-major.
+      // A stage is given back when both row tiles' products of it are complete; a row tile that
+      // ends before the other one still counts itself in for the remaining tiles, each time
+      // after the tile has arrived, so that it never runs a phase ahead.
+      for (int t = 0; t < tiles && ok; ++t) {
+        const int stage = t % STAGES;
+        ok = arrived(&kv_full[stage], (t / STAGES) & 1);
+        if (!ok) break;
+        if (t >= my_tiles) {
+          if (lane == 0) mbar_arrive(smem_u32(&kv_empty[stage]));
+          continue;
+        }
+        ok = arrived(&p_full[wg][t & 1], (t >> 1) & 1);
+        if (!ok) break;
+        tc_fence_after();
+        const uint64_t vd = v_desc + (uint64_t)((stage * STAGE_BYTES) >> 4);
+        const uint64_t p_desc = smem_desc_sw128(smem_u32(p_s) + (wg * 2 + (t & 1)) * P_BYTES);
+        if (elect_one()) {
 #pragma unroll
           for (int ks = 0; ks < KT / 16; ++ks)
             umma_bf16(tmem_base + PV_COL + wg * D, p_desc + (uint64_t)((ks * 32) >> 4),
@@ -431,6 +437,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
           umma_commit(smem_u32(&p_empty[wg][t & 1]));
           umma_commit(smem_u32(&kv_empty[stage]));
         }
+        __syncwarp();
       }
     }
   }

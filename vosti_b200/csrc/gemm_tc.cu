@@ -141,19 +141,20 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = instr_desc(BN);
-      bool ok = true;
-      for (int i = 0; i < my_stages && ok; ++i) {
-        const int s = i % STAGES;
-        ok = mbar_wait(smem_u32(&full_bar[s]), (i / STAGES) & 1, &abort_flag, status);
-        if (!ok) break;
-        tc_fence_after();
-        const int held = my_blocks - i * KPS < KPS ? my_blocks - i * KPS : KPS;
+    constexpr uint32_t idesc = instr_desc(BN);
+    bool ok = true;
+    for (int i = 0; i < my_stages; ++i) {
+      const int s = i % STAGES;
+      ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&full_bar[s]), (i / STAGES) & 1, &abort_flag, status));
+      if (!ok) break;
+      tc_fence_after();
+      const int held = my_blocks - i * KPS < KPS ? my_blocks - i * KPS : KPS;
+      const uint32_t stage_addr = smem_u32(smem + s * STAGE_BYTES);
+      if (elect_one()) {
 #pragma unroll
         for (int q = 0; q < KPS; ++q) {
           if (q < held) {
-            const uint32_t a_addr = smem_u32(smem + s * STAGE_BYTES + q * BLOCK_BYTES);
+            const uint32_t a_addr = stage_addr + q * BLOCK_BYTES;
             const uint64_t da = smem_desc_sw128(a_addr), db = smem_desc_sw128(a_addr + A_BYTES);
 #pragma unroll
             for (int k = 0; k < BK / UMMA_K; ++k) {
@@ -163,8 +164,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
           }
         }
         umma_commit(smem_u32(&empty_bar[s]));     // the stage is free once these MMAs have read it
+        if (i + 1 == my_stages) umma_commit(smem_u32(&accum_bar));  // the accumulator is complete
       }
-      if (ok) umma_commit(smem_u32(&accum_bar));  // the accumulator is complete
+      __syncwarp();
     }
   } else {
     // epilogue: this warp may read the 32 accumulator lanes of its quarter only

@@ -198,36 +198,43 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
+    if (rank == 0) {
       constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(PAIR_BN >> 3) << 17) |
                                  ((uint32_t)((2 * BM) >> 4) << 24);
       uint32_t it = 0, local = 0;
       bool ok = true;
+      auto arrived = [&](uint64_t* bar, uint32_t parity) {
+        return __all_sync(0xffffffffu, mbar_wait(smem_u32(bar), parity, &abort_flag, status)) != 0;
+      };
       for (int tile = pair; tile < total_tiles && ok; tile += pairs, ++local) {
         const uint32_t as = local & 1;
-        if (local >= 2) ok = mbar_wait(smem_u32(&acc_empty[as]), ((local >> 1) - 1) & 1, &abort_flag, status);
+        if (local >= 2) ok = arrived(&acc_empty[as], ((local >> 1) - 1) & 1);
         if (!ok) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + as * PAIR_BN;
         for (int kb0 = 0; kb0 < k_blocks; kb0 += PAIR_KPS, ++it) {
           const int s = it % PAIR_STAGES;
-          ok = mbar_wait(smem_u32(&full_bar[s]), (it / PAIR_STAGES) & 1, &abort_flag, status);
+          ok = arrived(&full_bar[s], (it / PAIR_STAGES) & 1);
           if (!ok) break;
           tc_fence_after();
           const int held = k_blocks - kb0 < PAIR_KPS ? k_blocks - kb0 : PAIR_KPS;
+          const uint32_t stage_addr = smem_u32(smem + s * PAIR_STAGE_BYTES);
+          if (elect_one()) {
 #pragma unroll
-          for (int q = 0; q < PAIR_KPS; ++q) {
-            if (q < held) {
-              const uint32_t a_addr = smem_u32(smem + s * PAIR_STAGE_BYTES + q * PAIR_BLOCK_BYTES);
-              const uint64_t da = smem_desc_sw128(a_addr), db = smem_desc_sw128(a_addr + A_BYTES);
+            for (int q = 0; q < PAIR_KPS; ++q) {
+              if (q < held) {
+                const uint32_t a_addr = stage_addr + q * PAIR_BLOCK_BYTES;
+                const uint64_t da = smem_desc_sw128(a_addr), db = smem_desc_sw128(a_addr + A_BYTES);
 #pragma unroll
-              for (int k = 0; k < BK / UMMA_K; ++k)
-                umma_bf16_pair(d_tmem, da + 2 * k, db + 2 * k, idesc, (kb0 > 0 || q > 0 || k > 0) ? 1u : 0u);
+                for (int k = 0; k < BK / UMMA_K; ++k)
+                  umma_bf16_pair(d_tmem, da + 2 * k, db + 2 * k, idesc, (kb0 > 0 || q > 0 || k > 0) ? 1u : 0u);
+              }
             }
+            umma_commit_pair(smem_u32(&empty_bar[s]));
+            if (kb0 + PAIR_KPS >= k_blocks) umma_commit_pair(smem_u32(&acc_full[as]));
           }
-          umma_commit_pair(smem_u32(&empty_bar[s]));
+          __syncwarp();
         }
-        if (ok) umma_commit_pair(smem_u32(&acc_full[as]));
       }
     }
   } else {
