@@ -461,6 +461,32 @@ def test_gemm_tc_of_one_feature_tile_over_many_tokens_splits(dev, status, tokens
     assert status.item() == 0
 
 
+# one row past a tile, whole and part tiles, k-blocks that the cuts divide and don't, k inside a block, features inside a tile and odd
+@pytest.mark.parametrize("tokens,features,k", [(129, 4096, 4096), (200, 4096, 12288), (256, 256, 2056), (257, 130, 2048), (300, 1000, 4104),
+                                               (512, 2048, 4096), (653, 2048, 4096), (700, 1024, 8192), (1100, 768, 8192), (150, 6144, 4096)])
+def test_gemm_tc_of_few_tiles_over_many_tokens_splits(dev, status, tokens, features, k):
+    """Products whose tiles leave pairs of SMs idle are cut along K: a float32 sum of each part, parts added in their order."""
+    from vosti_b200 import ops
+    x = torch.randn(tokens, k, device=dev).bfloat16()
+    w = (torch.randn(features, k, device=dev) / math.sqrt(k)).bfloat16()
+    assert ops.library().vosti_gemm_tc_pair_splits(tokens, features, k) > 1
+    want = x.double() @ w.double().T
+    y = ops.gemm_tc(x, w, status, out_dtype=torch.float32)
+    assert torch.allclose(y.double(), want, atol=2e-4, rtol=2e-4)
+    assert torch.equal(y, ops.gemm_tc(x, ops.PackedWeight(w), status, out_dtype=torch.float32))
+    assert torch.equal(ops.gemm_tc(x, w, status, allow_partial=True), y.bfloat16())
+    if features % 32 == 0:
+        g, u = (want.view(tokens, -1, 2, 16)[:, :, i].reshape(tokens, -1) for i in range(2))
+        assert torch.allclose(ops.gemm_tc(x, w, status, swiglu=True).double(), g * torch.sigmoid(g) * u, atol=2e-2, rtol=2e-2)
+    ops.set_fixed_order(True)
+    try:
+        assert ops.library().vosti_gemm_tc_pair_splits(tokens, features, k) == 1
+        assert torch.allclose(ops.gemm_tc(x, w, status, out_dtype=torch.float32).double(), want, atol=2e-4, rtol=2e-4)
+    finally:
+        ops.set_fixed_order(False)
+    assert status.item() == 0
+
+
 def test_split_products_over_many_tokens_leave_the_shared_scratch_alone(dev, status):
     """A partial sum that is still to be added stays valid, and its values stay, while a split product over more
     than 128 tokens runs; such a product under way on one stream keeps its values while another stream runs one."""

@@ -163,6 +163,16 @@ def test_delta_rules_take_the_form_that_was_measured_faster():
     assert delta_step_layout([1, 48, 3]) == ({}, {"chunks": 0, "longs": 0, "shorts": 3})
 
 
+def test_products_of_few_tiles_split_where_that_is_faster(lib):
+    """The number of cuts at sizes on both sides of the line at which cutting K was measured faster and slower than one pass."""
+    for tokens, features, k, cuts in [(200, 4096, 12288, 4), (300, 4096, 12288, 2), (512, 4096, 12288, 2), (256, 6144, 4096, 3), (130, 4096, 4096, 4),
+                                      (300, 4096, 4096, 2), (653, 2048, 4096, 3), (512, 1024, 8192, 6), (1000, 1024, 8192, 4)]:
+        assert lib.vosti_gemm_tc_pair_splits(tokens, features, k) == cuts, (tokens, features, k)
+    for tokens, features, k in [(128, 4096, 12288), (653, 4096, 12288), (300, 6144, 4096), (256, 3664, 2048), (512, 2048, 2048), (130, 8192, 2048),
+                                (200, 24576, 4096), (256, 5120, 1536), (700, 1024, 512), (2048, 128, 4096)]:
+        assert lib.vosti_gemm_tc_pair_splits(tokens, features, k) == 1, (tokens, features, k)
+
+
 def test_weight_bytes_of_a_decode_step_in_closed_form():
     """What bench.py counts as the weights a decode step must read: every tensor the model
     expects except the embedding table (read by rows), two bytes each. For the 8B sizes that is

@@ -458,6 +458,47 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ partial, void* __
   }
 }
 
+// The same for rows of whole words: four neighbouring features a thread.
+__global__ void splitk_reduce4_kernel(const float* __restrict__ partial, void* __restrict__ out, int splits, int tokens, int features,
+                                      int ld_out, int epilogue) {
+  pdl_wait();
+  pdl_launch_dependents();
+  const int64_t plane = (int64_t)tokens * features, words = plane / 4;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < words; i += (int64_t)gridDim.x * blockDim.x) {
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int s = 0; s < splits; ++s) {
+      const float4 v = *reinterpret_cast<const float4*>(partial + s * plane + 4 * i);
+      acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+    }
+    const int64_t t = 4 * i / features;
+    const int f = (int)(4 * i % features);
+    if (epilogue == EPI_F32) {
+      *reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + t * ld_out + f) = acc;
+    } else {
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(acc.x, acc.y), hi = __floats2bfloat162_rn(acc.z, acc.w);
+      *reinterpret_cast<uint2*>(reinterpret_cast<bf16*>(out) + t * ld_out + f) =
+          make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+    }
+  }
+}
+
+void launch_splitk_reduce(const float* partial, void* y, int splits, int tokens, int features, int ld_out, int epilogue, cudaStream_t stream) {
+  const bool words = !is_gated(epilogue) && features % 4 == 0 && ld_out % 4 == 0 &&
+                     (reinterpret_cast<uintptr_t>(partial) % 16 | reinterpret_cast<uintptr_t>(y) % 16) == 0;
+  const int64_t n = (int64_t)tokens * features / (words ? 4 : 1);
+  const int blocks = (int)((n + 255) / 256 < 148 * 8 ? (n + 255) / 256 : 148 * 8);
+  vosti_launch(words ? splitk_reduce4_kernel : splitk_reduce_kernel, dim3(blocks), dim3(256), 0, stream, partial, y, splits, tokens, features,
+               ld_out, epilogue);
+}
+
+bool uses_pairs() {                    // VOSTI_GEMM_PAIR=0: products of many tokens on single SMs
+  static const bool on = [] {
+    const char* env = getenv("VOSTI_GEMM_PAIR");
+    return env == nullptr || env[0] != '0';
+  }();
+  return on;
+}
+
 // ------------------------------------------------------------------ host side
 // Map of a row-major [rows, k] bfloat16 matrix, box [box_rows, 64], 128-byte swizzle; what
 // lies outside the matrix reads as zero.
@@ -680,6 +721,26 @@ VOSTI_API int vosti_gemm_tc_splits(int tokens, int features, int k) {
   return splits < 1 ? 1 : splits;
 }
 
+// How many K splits a product of more than 128 tokens takes on pairs of SMs (1: none, or not a product for them). With few
+// token tiles the 256 x 256 tiles leave most of the 74 pairs without one while a tile walks all of K at 0.345 us a k-block, so K is
+// cut until the pairs are one round of units (six cuts at most; partial sums of 19 MB at most), where that is estimated to pay: a launch
+// and its first stages 4 us, the second kernel 5, the partial sums written and read 2.5 TB/s. Measured, us, one pass / split:
+// 4,096 x 12,288 of 200 tokens 69 / 33 (4 cuts), of 512 71 / 50 (2), 6,144 x 4,096 of 256 29 / 26 (3), 2,048 x 4,096 of 653 26 / 21 (3),
+// 1,024 x 8,192 of 1,000 45 / 24 (4); left whole: 3,664 x 2,048 of 256 16.9 / 16.8, 2,048 x 2,048 of 512 16.5 / 16.0, two rounds
+// of units (4,096 x 12,288 of 653: 72 / 68).
+VOSTI_API int vosti_gemm_tc_pair_splits(int tokens, int features, int k) {
+  if (tokens <= 128 || features <= BM || g_vosti_fixed_order || !uses_pairs()) return 1;
+  const int64_t tiles = (int64_t)((features + pair_kernel::PAIR_BN - 1) / pair_kernel::PAIR_BN) * ((tokens + 2 * BM - 1) / (2 * BM));
+  const int k_blocks = (k + BK - 1) / BK;
+  int splits = tiles < 74 ? (int)(74 / tiles) : 1;
+  if (splits > 6) splits = 6;
+  if (splits > k_blocks / 8) splits = k_blocks / 8;                   // at least 8 k-blocks each
+  if (splits <= 1) return 1;
+  const double partial = 4.0 * splits * tokens * features;
+  const double whole_us = 4.0 + 0.345 * k_blocks, split_us = 9.0 + 0.345 * ((k_blocks + splits - 1) / splits) + partial / 2.5e6;
+  return split_us <= 0.95 * whole_us ? splits : 1;
+}
+
 // x: [tokens, k] bf16; w: [features, k] bf16; epilogue 0: y bf16 [tokens, features];
 // 1: y float32 [tokens, features]; 2: y bf16 [tokens, features / 2] = silu(gate) * up with
 // the weight rows interleaved in blocks of 16 gate rows and their 16 up rows.
@@ -704,10 +765,7 @@ VOSTI_API int vosti_gemm_tc(const void* x, const void* w, void* y, int tokens, i
   // tensor map is that of a matrix of 64 columns
   const int w_tiles = w_packed ? (features + BM - 1) / BM : 0;
   const int w_rows = w_packed ? k_blocks * w_tiles * BM : features, w_cols = w_packed ? BK : k;
-  static const bool use_pairs = [] {                 // VOSTI_GEMM_PAIR=0: the single-CTA kernel below instead
-    const char* env = getenv("VOSTI_GEMM_PAIR");
-    return env == nullptr || env[0] != '0';
-  }();
+  const bool use_pairs = uses_pairs();
   if (tokens > 128 && splits == 1 && use_pairs) {
     // many tokens, two SMs per tile (cta_group::2)
     using namespace pair_kernel;
@@ -726,10 +784,14 @@ VOSTI_API int vosti_gemm_tc(const void* x, const void* w, void* y, int tokens, i
         return e != cudaSuccess ? (int)e : VOSTI_UNSUPPORTED;
       }
     }
-    const int tiles = ((tokens + 2 * BM - 1) / (2 * BM)) * ((features + PAIR_BN - 1) / PAIR_BN);
+    int cuts = vosti_gemm_tc_pair_splits(tokens, features, k);
+    if (workspace == nullptr || workspace_elems < (int64_t)cuts * tokens * features) cuts = 1;
+    const int tiles = ((tokens + 2 * BM - 1) / (2 * BM)) * ((features + PAIR_BN - 1) / PAIR_BN) * cuts;
     const int pairs = tiles < pair_sms / 2 ? tiles : pair_sms / 2;
-    vosti_launch_clusters(gemm_tc_pair_kernel<PlainEpilogue>, dim3(2 * pairs), dim3(PAIR_THREADS), 2, smem, stream, mx, *mw, y, tokens,
-                          features, k_blocks, ld_out, epilogue, w_tiles, PlainEpilogue{}, status);
+    vosti_launch_clusters(gemm_tc_pair_kernel<PlainEpilogue>, dim3(2 * pairs), dim3(PAIR_THREADS), 2, smem, stream, mx, *mw,
+                          cuts > 1 ? (void*)workspace : y, tokens, features, k_blocks, cuts > 1 ? features : ld_out,
+                          cuts > 1 ? (int)EPI_PARTIAL : epilogue, w_tiles, cuts, PlainEpilogue{}, status);
+    if (cuts > 1) launch_splitk_reduce(workspace, y, cuts, tokens, features, ld_out, epilogue, stream);
     VOSTI_LAUNCH_CHECK();
   }
   if (tokens > 128 && splits == 1) {
@@ -774,10 +836,7 @@ VOSTI_API int vosti_gemm_tc(const void* x, const void* w, void* y, int tokens, i
 #undef VOSTI_GEMM_ARGS
   if (rc != 0) return rc;
   if (splits > 1 && !defer_reduce) {
-    const int64_t n = (int64_t)tokens * features;
-    const int blocks = (int)((n + 255) / 256 < 148 * 8 ? (n + 255) / 256 : 148 * 8);
-    vosti_launch(splitk_reduce_kernel, dim3(blocks), dim3(256), 0, stream, (const float*)workspace, y, splits, tokens,
-                 features, ld_out, epilogue);
+    launch_splitk_reduce(workspace, y, splits, tokens, features, ld_out, epilogue, stream);
   }
   VOSTI_LAUNCH_CHECK();
 }
@@ -807,7 +866,7 @@ VOSTI_API int vosti_gemm_tc_clamped(const void* x, const void* w, void* y, int t
   const int tiles = ((tokens + 2 * BM - 1) / (2 * BM)) * ((features + PAIR_BN - 1) / PAIR_BN);
   const int pairs = tiles < device_sms() / 2 ? tiles : device_sms() / 2;
   vosti_launch_clusters(gemm_tc_pair_kernel<ClampedEpilogue>, dim3(2 * pairs), dim3(PAIR_THREADS), 2, smem, stream, mx, mw, y, tokens,
-                        features, k_blocks, features / 2, (int)EPI_SWIGLU, w_tiles, ClampedEpilogue{bias, limit, sigmoid_scale}, status);
+                        features, k_blocks, features / 2, (int)EPI_SWIGLU, w_tiles, 1, ClampedEpilogue{bias, limit, sigmoid_scale}, status);
   VOSTI_LAUNCH_CHECK();
 }
 
@@ -831,7 +890,7 @@ VOSTI_API int vosti_gemm_tc_two_terms(const void* x, const void* w, void* y, voi
   const int tiles = ((tokens + 2 * BM - 1) / (2 * BM)) * ((features + PAIR_BN - 1) / PAIR_BN);
   const int pairs = tiles < device_sms() / 2 ? tiles : device_sms() / 2;
   vosti_launch_clusters(gemm_tc_pair_kernel<TwoTermEpilogue>, dim3(2 * pairs), dim3(PAIR_THREADS), 2, smem, stream, mx, mw, y, tokens,
-                        features, (k + BK - 1) / BK, features, (int)EPI_BF16, 0, TwoTermEpilogue{(bf16*)low, low_from}, status);
+                        features, (k + BK - 1) / BK, features, (int)EPI_BF16, 0, 1, TwoTermEpilogue{(bf16*)low, low_from}, status);
   VOSTI_LAUNCH_CHECK();
 }
 
@@ -841,10 +900,7 @@ VOSTI_API int vosti_splitk_reduce(const float* partial, void* y, int splits, int
                                   cudaStream_t stream) {
   VOSTI_REQUIRE(splits >= 1 && tokens >= 0 && features >= 1, "splitk_reduce: bad sizes");
   if (tokens == 0) return VOSTI_OK;
-  const int64_t n = (int64_t)tokens * features;
-  const int blocks = (int)((n + 255) / 256 < 148 * 8 ? (n + 255) / 256 : 148 * 8);
-  vosti_launch(splitk_reduce_kernel, dim3(blocks), dim3(256), 0, stream, partial, y, splits, tokens, features, features,
-               (int)(y_is_f32 ? EPI_F32 : EPI_BF16));
+  launch_splitk_reduce(partial, y, splits, tokens, features, features, y_is_f32 ? EPI_F32 : EPI_BF16, stream);
   VOSTI_LAUNCH_CHECK();
 }
 
@@ -911,10 +967,7 @@ VOSTI_API int vosti_gemm_tc_split_static(const void* x, const void* w, void* y, 
   }
   if (rc != 0) return rc;
   if (splits > 1) {
-    const int64_t n = (int64_t)tokens * features;
-    const int blocks = (int)((n + 255) / 256 < 148 * 8 ? (n + 255) / 256 : 148 * 8);
-    vosti_launch(splitk_reduce_kernel, dim3(blocks), dim3(256), 0, stream, (const float*)scratch, y, splits, tokens,
-                 features, features, epilogue);
+    launch_splitk_reduce(scratch, y, splits, tokens, features, features, epilogue, stream);
   }
   VOSTI_LAUNCH_CHECK();
 }

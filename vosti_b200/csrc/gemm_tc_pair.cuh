@@ -2,7 +2,8 @@
 // epilogue it uses). A cluster of two CTAs computes a tile of 256 tokens x 256 features with
 // tcgen05.mma.cta_group::2: each CTA stages its 128 tokens (A) and its 128 of the 256 features (B)
 // in its own shared memory, the first CTA of the pair issues every MMA for both tensor cores,
-// and each CTA's tensor memory receives the 256 columns of its own 128 tokens. Against the
+// and each CTA's tensor memory receives the 256 columns of its own 128 tokens. A tile's K may be split over several pairs
+// (`vosti_gemm_tc_pair_splits`), whose partial sums another kernel adds in split order. Against the
 // single-CTA tile (128 x 256: 48 KB of operands per k-block and SM) an SM takes in 32 KB per
 // k-block, so a ring stage can hold two k-blocks and still be three stages deep: the lane that
 // issues the MMAs then pays one barrier wait (about 200 cycles, even when the stage landed long
@@ -134,7 +135,8 @@ template <typename EpilogueExtra>
 __global__ void __launch_bounds__(pair_kernel::PAIR_THREADS, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                     void* __restrict__ out, int tokens, int features, int k_blocks, int ld_out, int epilogue,
-                    int w_tiles, const EpilogueExtra extra, unsigned* status) {
+                    int w_tiles, int splits, const EpilogueExtra extra, unsigned* status) {
+  // splits > 1: part s of a tile's k-blocks goes, float32, to the s-th [tokens, features] slice of `out`
   using namespace pair_kernel;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -149,7 +151,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
   const uint32_t rank = cluster_rank();                       // 0: issues the MMAs
   const int pairs = gridDim.x / 2, pair = blockIdx.x / 2;
   const int m_tiles = (tokens + 2 * BM - 1) / (2 * BM), n_tiles = (features + PAIR_BN - 1) / PAIR_BN;
-  const int total_tiles = m_tiles * n_tiles;
+  const int total_tiles = m_tiles * n_tiles * splits;         // (a tile's splits one after the other)
+  auto first_block = [&](int split) { return (int)((long long)k_blocks * split / splits); };
 
   if (threadIdx.x == 0) {
     abort_flag = 0;
@@ -176,15 +179,16 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       uint32_t it = 0;
       bool ok = true;
       pdl_wait();
-      for (int tile = pair; tile < total_tiles && ok; tile += pairs) {
+      for (int unit = pair; unit < total_tiles && ok; unit += pairs) {
+        const int tile = unit / splits, kb_end = first_block(unit % splits + 1);
         const int m0 = (tile % m_tiles) * 2 * BM + (int)rank * BM, n0 = (tile / m_tiles) * PAIR_BN + (int)rank * BM;
-        for (int kb0 = 0; kb0 < k_blocks; kb0 += PAIR_KPS, ++it) {
+        for (int kb0 = first_block(unit % splits); kb0 < kb_end; kb0 += PAIR_KPS, ++it) {
           const int s = it % PAIR_STAGES;
           if (it >= PAIR_STAGES && !mbar_wait(smem_u32(&empty_bar[s]), (it / PAIR_STAGES - 1) & 1, &abort_flag, status)) {
             ok = false;
             break;
           }
-          const int held = k_blocks - kb0 < PAIR_KPS ? k_blocks - kb0 : PAIR_KPS;
+          const int held = kb_end - kb0 < PAIR_KPS ? kb_end - kb0 : PAIR_KPS;
           if (rank == 0) mbar_expect_tx(smem_u32(&full_bar[s]), (uint32_t)(2 * held * PAIR_BLOCK_BYTES));   // both CTAs' bytes
           const uint32_t bar = in_cta(smem_u32(&full_bar[s]), 0);
           for (int q = 0; q < held; ++q) {
@@ -206,18 +210,19 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       auto arrived = [&](uint64_t* bar, uint32_t parity) {
         return __all_sync(0xffffffffu, mbar_wait(smem_u32(bar), parity, &abort_flag, status)) != 0;
       };
-      for (int tile = pair; tile < total_tiles && ok; tile += pairs, ++local) {
+      for (int unit = pair; unit < total_tiles && ok; unit += pairs, ++local) {
+        const int kb_begin = first_block(unit % splits), kb_end = first_block(unit % splits + 1);
         const uint32_t as = local & 1;
         if (local >= 2) ok = arrived(&acc_empty[as], ((local >> 1) - 1) & 1);
         if (!ok) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + as * PAIR_BN;
-        for (int kb0 = 0; kb0 < k_blocks; kb0 += PAIR_KPS, ++it) {
+        for (int kb0 = kb_begin; kb0 < kb_end; kb0 += PAIR_KPS, ++it) {
           const int s = it % PAIR_STAGES;
           ok = arrived(&full_bar[s], (it / PAIR_STAGES) & 1);
           if (!ok) break;
           tc_fence_after();
-          const int held = k_blocks - kb0 < PAIR_KPS ? k_blocks - kb0 : PAIR_KPS;
+          const int held = kb_end - kb0 < PAIR_KPS ? kb_end - kb0 : PAIR_KPS;
           const uint32_t stage_addr = smem_u32(smem + s * PAIR_STAGE_BYTES);
           if (elect_one()) {
 #pragma unroll
@@ -227,11 +232,11 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                 const uint64_t da = smem_desc_sw128(a_addr), db = smem_desc_sw128(a_addr + A_BYTES);
 #pragma unroll
                 for (int k = 0; k < BK / UMMA_K; ++k)
-                  umma_bf16_pair(d_tmem, da + 2 * k, db + 2 * k, idesc, (kb0 > 0 || q > 0 || k > 0) ? 1u : 0u);
+                  umma_bf16_pair(d_tmem, da + 2 * k, db + 2 * k, idesc, (kb0 > kb_begin || q > 0 || k > 0) ? 1u : 0u);
               }
             }
             umma_commit_pair(smem_u32(&empty_bar[s]));
-            if (kb0 + PAIR_KPS >= k_blocks) umma_commit_pair(smem_u32(&acc_full[as]));
+            if (kb0 + PAIR_KPS >= kb_end) umma_commit_pair(smem_u32(&acc_full[as]));
           }
           __syncwarp();
         }
@@ -242,8 +247,10 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     uint32_t local = 0;
     bool ok = true;
     pdl_wait();
-    for (int tile = pair; tile < total_tiles && ok; tile += pairs, ++local) {
+    for (int unit = pair; unit < total_tiles && ok; unit += pairs, ++local) {
+      const int tile = unit / splits;
       const int m0 = (tile % m_tiles) * 2 * BM + (int)rank * BM, n0 = (tile / m_tiles) * PAIR_BN;
+      void* const slice = splits > 1 ? (void*)(reinterpret_cast<float*>(out) + (int64_t)(unit % splits) * tokens * features) : out;
       const uint32_t as = local & 1;
       ok = mbar_wait_warp(smem_u32(&acc_full[as]), (local >> 1) & 1, &abort_flag, status);
       if (!ok) break;
@@ -257,7 +264,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
         uint32_t r[32];
         tmem_load32(tmem_base + as * PAIR_BN + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0, r);
         if (!row_ok) continue;
-        store_columns(r, out, token, f0, features, ld_out, epilogue, extra);
+        store_columns(r, slice, token, f0, features, ld_out, epilogue, extra);
       }
       tc_fence_before();
       __syncwarp();

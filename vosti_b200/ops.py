@@ -582,9 +582,11 @@ def gemm_tc(x: torch.Tensor, w, status: torch.Tensor, *, out_dtype: Optional[tor
         epilogue, width = (EPI_F32 if out_dtype == torch.float32 else EPI_BF16), features
     lib = library()
     splits = lib.vosti_gemm_tc_splits(tokens, features, k)
+    if splits == 1:
+        splits = lib.vosti_gemm_tc_pair_splits(tokens, features, k)
     elems = splits * tokens * features if splits > 1 else 0
     # more than 128 tokens: sums of the call's own, so that products on several streams and a partial sum that is
-    # still to be added don't meet in the shared buffer (one torch.empty of at most 10 MB a call)
+    # still to be added don't meet in the shared buffer (one torch.empty of at most 20 MB a call)
     own = tokens > 128
     ws = None
     if elems:
