@@ -1,5 +1,5 @@
 """The float32 product on the tensor cores (csrc/gemm_f32.cu): against float64, bits of a row alone and among others in every
-tile width, rows picked, rows that start inside a word, operands that are not finite."""
+tile width, rows that start inside a word, operands that are not finite."""
 import pytest
 import torch
 
@@ -21,9 +21,10 @@ def draw(seed, rows, n, k):
 
 def bound(x, w):
     """Per output, over the sum of magnitudes: a rounding of the running sum per 64 k and K segment, at most four truncations (two
-    roundings' worth each) of a 64-k sum, 5 K / 16 truncations of sums 2^-8 as large, and the terms left out."""
+    roundings' worth each) of a 64-k sum, 5 K / 16 truncations of sums 2^-6 as large (two terms below 2^-7), and the terms left out: m and
+    l are below 2^-7 and 2^-15 of their operand, so m l + l m + l l is below 2^-21, eight roundings."""
     k = x.shape[1]
-    steps = -(-k // 64) + 8 + 2 * 4 + 2 * (5 * k / 16) * 2.0 ** -8 + 4
+    steps = -(-k // 64) + 8 + 2 * 4 + 2 * (5 * k / 16) * 2.0 ** -6 + 9
     return steps * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
 
 
@@ -39,8 +40,6 @@ def test_against_float64_and_rows_alone(status, rows, n, k):
     assert (y.double() - want).norm() <= (chain.double() - want).norm()
     for a, b in [(0, 1), (rows // 2, rows // 2 + 1), (0, min(rows, 40)), (max(rows - 70, 0), rows), (0, min(rows, 150)), (0, min(rows, 200))]:
         assert torch.equal(ops.gemm_f32(x[a:b].contiguous(), w, status), y[a:b])
-    index = torch.randint(0, rows, (rows // 2 + 3,), device=DEV, dtype=torch.int32)
-    assert torch.equal(ops.gemm_f32(x, w, status, row_index=index), y[index.long()]) and status.item() == 0
     # the same numbers on places that are not whole words
     xs, ws = torch.empty(rows * k + 1, device=DEV), torch.empty(n * k + 3, device=DEV)
     xs[1:], ws[3:] = x.view(-1), w.view(-1)
@@ -62,9 +61,3 @@ def test_operands_that_are_not_finite(status):
     assert torch.equal(torch.isnan(y), torch.isnan(chain)) and torch.equal(torch.isinf(y), torch.isinf(chain))
     finite = torch.isfinite(chain)
     assert torch.allclose(y[finite], chain[finite], rtol=1e-4, atol=1e-4)
-
-
-def test_a_row_index_out_of_range_is_reported(status):
-    x, w = draw(7, 5, 64, 128)
-    y = ops.gemm_f32(x, w, status, row_index=torch.tensor([0, 5, -1, 4], dtype=torch.int32, device=DEV))
-    assert status.item() != 0 and not y[1:3].any() and torch.equal(y[[0, 3]], ops.gemm_f32(x, w, status)[[0, 4]])

@@ -1,13 +1,14 @@
 // float32 matrix product on the 5th-generation tensor cores:
-//   Y[t, n] = sum_k X[row(t), k] * W[n, k]        X, W, Y float32 (W in [out, in] layout, no bias)
-// Every operand is split into three bfloat16 terms, x = h + m + l, each the rounding of what the terms before it leave
+//   Y[t, n] = sum_k X[t, k] * W[n, k]        X, W, Y float32 (W in [out, in] layout, no bias)
+// Every operand is split into three bfloat16 terms, x = h + m + l, each the upper 16 bits of what the terms before it leave
 // (8 + 8 + 8 bits: nothing of a float32 is lost), and a product is the six terms of order up to 2^-16:
-// h h + (h m + m h) + (h l + m m + l h); what is left out is below 2^-25 of |x w|. Splitting operands this way, and taking
-// the tensor core's sums out before their truncation adds up, is Ootomo and Yokota, "Recovering single
+// h h + (h m + m h) + (h l + m m + l h); what is left out is below 2^-21 of |x w| and 2^-24 in the mean. Splitting operands this way, and
+// taking the tensor core's sums out before their truncation adds up, is Ootomo and Yokota, "Recovering single
 // precision accuracy from Tensor Cores while surpassing the FP32 theoretical peak performance" (2022); here h h is summed
 // on the tensor core over 64 k only and then added, rounded to nearest, to a sum in registers, while the five small products,
-// 2^-8 of it, stay in an accumulator of their own to the end. Error against 64 bits (2-norm, normal operands): 1.1e-7
-// at K = 4,096 and 1.3e-7 at 12,288, where gemm_simt.cu's chain of multiply-adds has 1.2e-6 and 2.0e-6.
+// 2^-7 of it, stay in an accumulator of their own to the end. Error against 64 bits (2-norm, normal operands): 1.4e-7 at K = 2,048,
+// 1.7e-7 (four segments) and 2.8e-7 (one) at 4,096, 2.5e-7 at 12,288, where gemm_simt.cu's chain of multiply-adds has
+// 8.1e-7, 1.1e-6 and 2.0e-6.
 //
 // Features on M = 128, tokens on N; K in `segments` of whole 64s, one CTA of a cluster each, summed in their order
 // through distributed shared memory. The segments are chosen from (N, K) alone, the order of the products inside a
@@ -15,10 +16,11 @@
 // rows beside it (the reference chooses tiles from (N, K) only for the same reason:
 // kernels/triton_kernels/matmul.py:33-73, 95-147).
 //
-// An operand that is infinite, not a number or rounds to infinity in 16 bits makes its outputs non-finite here, and terms of
+// An operand that is infinite or not a number makes its outputs non-finite here (an infinity leaves inf - inf), and terms of
 // operands near the smallest normal number lose their low bits; outputs that are not finite, or so small that this could show
 // (below 2^-80 and not zero), are taken again as a chain of float32 multiply-adds.
 #include "tcgen05.cuh"
+#include "tensor_map.cuh"
 
 namespace {
 
@@ -28,7 +30,7 @@ constexpr int WORKERS = 256;             // threads that load, split and sum
 // Tiles of more than 128 tokens keep 96 or 128 sums a thread beside their words in flight: three warpgroups launched with
 // 168 registers a thread (64,512) share them as 232 + 232 + 40.
 template <int TOK> constexpr bool SPLITS_REGISTERS = TOK > 128;
-template <int TOK> constexpr int THREADS = SPLITS_REGISTERS<TOK> ? WORKERS + 128 : WORKERS + 32;
+template <int TOK> constexpr int THREADS = SPLITS_REGISTERS<TOK> ? WORKERS + 128 : WORKERS + 64;
 
 __device__ __forceinline__ uint32_t f32_cluster_rank() {
   uint32_t r;
@@ -45,6 +47,14 @@ __device__ __forceinline__ float4 load_cluster4(uint32_t smem_addr, uint32_t ran
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_addr), "r"(rank));
   asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(remote) : "memory");
   return v;
+}
+// A wait of a whole warp: one lane polls, the others meet it.
+__device__ __forceinline__ bool f32_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, unsigned* status) {
+  bool ok = true;
+  if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity, abort_flag, status);
+  ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+  __syncwarp();
+  return ok;
 }
 __device__ __forceinline__ void workers_sync() { asm volatile("bar.sync 1, %0;" ::"n"(WORKERS) : "memory"); }
 // Descriptor of a K-major tile of KS k a row: 128-byte swizzle for 64, 64-byte swizzle (groups of 8 rows 512 bytes apart) for 32.
@@ -91,62 +101,74 @@ __device__ __forceinline__ void add_columns(uint32_t taddr, float (&acc)[COLS]) 
   }
 }
 
-// Four neighbouring k of a row (zeros beyond k, or of a row that is not there).
-__device__ __forceinline__ float4 load_word(const float* matrix, int row, int kk, int k, bool wide) {
+// Four neighbouring k of a row from memory, element by element (zeros beyond k).
+__device__ __forceinline__ float4 load_elements(const float* row, int kk, int k) {
   float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (row < 0 || kk >= k) return v;
-  const float* p = matrix + (int64_t)row * k + kk;
-  if (wide) return *reinterpret_cast<const float4*>(p);
-  v.x = p[0];
-  if (kk + 1 < k) v.y = p[1];
-  if (kk + 2 < k) v.z = p[2];
-  if (kk + 3 < k) v.w = p[3];
+  if (kk < k) v.x = row[kk];
+  if (kk + 1 < k) v.y = row[kk + 1];
+  if (kk + 2 < k) v.z = row[kk + 2];
+  if (kk + 3 < k) v.w = row[kk + 3];
   return v;
 }
-// The three terms of four values to their places in three planes of `plane` bytes.
-__device__ __forceinline__ void store_split(uint8_t* at, int plane, float4 v) {
-  const __nv_bfloat162 h0 = __floats2bfloat162_rn(v.x, v.y), h1 = __floats2bfloat162_rn(v.z, v.w);
-  const float2 a = __bfloat1622float2(h0), b = __bfloat1622float2(h1);
-  v.x -= a.x; v.y -= a.y; v.z -= b.x; v.w -= b.y;
-  const __nv_bfloat162 m0 = __floats2bfloat162_rn(v.x, v.y), m1 = __floats2bfloat162_rn(v.z, v.w);
-  const float2 c = __bfloat1622float2(m0), d = __bfloat1622float2(m1);
-  v.x -= c.x; v.y -= c.y; v.z -= d.x; v.w -= d.y;
-  const __nv_bfloat162 l0 = __floats2bfloat162_rn(v.x, v.y), l1 = __floats2bfloat162_rn(v.z, v.w);
-  auto put = [&](uint8_t* p, const __nv_bfloat162& lo, const __nv_bfloat162& hi) {
-    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
-  };
-  put(at, h0, h1);
-  put(at + plane, m0, m1);
-  put(at + 2 * plane, l0, l1);
+// The three terms of four values, two values a word. A term is the upper half of what the terms before it leave (truncated: whole
+// words of integer and multiply-add instructions, where a rounding conversion takes its unit several cycles), the last one is exact.
+__device__ __forceinline__ void split_four(float4 v, uint32_t* h, uint32_t* m, uint32_t* l) {
+  auto upper = [](float x) { return __uint_as_float(__float_as_uint(x) & 0xffff0000u); };
+  auto both = [](float lo, float hi) { return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632); };
+  const float4 a = make_float4(v.x - upper(v.x), v.y - upper(v.y), v.z - upper(v.z), v.w - upper(v.w));
+  const float4 b = make_float4(a.x - upper(a.x), a.y - upper(a.y), a.z - upper(a.z), a.w - upper(a.w));
+  h[0] = both(v.x, v.y), h[1] = both(v.z, v.w);
+  m[0] = both(a.x, a.y), m[1] = both(a.z, a.w);
+  l[0] = both(b.x, b.y), l[1] = both(b.z, b.w);
+}
+// Eight columns of this warp's 32 lanes.
+__device__ __forceinline__ void tmem_store8(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]),
+               "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
+// D += A B with A [128 rows, 16 k] in tensor memory: a lane per row, two neighbouring k in a column.
+__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u)
+      : "memory");
 }
 
-// TOK tokens on N. Eight warps load words of both operands into registers (AHEAD stages ahead), split them into the three
-// planes of a ring stage of KS k, and between stages take the tensor core's 64-k sums out (thread: one feature, TOK / 2 tokens);
-// one lane of the ninth warp issues the MMAs. The two roles share no code from where they part (their registers differ):
-// the ninth warp ends after its last commit, the eight do the rest. The fence between the warps' stores and the MMAs that read
-// them (generic to async proxy) is the issuing lane's, after its wait: in the eight warps it would also wait for
-// the words of the next stages that are under way.
-template <int TOK, int KS, int STAGES, int AHEAD, int BLOCKS>
+// TOK tokens on N. One thread brings both operands' words of KS k into a ring of RAW stages by TMA (zeros beyond a matrix), eight
+// warps split them, the weights into three planes in tensor memory (a thread: half a feature's k), the tokens into three in
+// shared memory, and between stages take the tensor core's 64-k sums out (a thread: one feature, TOK / 2 tokens); a ninth warp
+// issues the MMAs. The bound is shared memory: with the weights' planes there too the six products read them again (10 KB for
+// each of twelve MMAs a stage of 192 tokens): us for 24,576 x 4,096, 1 / 64 / 384 rows, 152 / 283 / 570 so, 93 / 162 / 441 now,
+// gemm_simt.cu 155 / 434 / 1,689. The roles share no code from where they part (their registers differ): the warps that bring
+// and issue end after their last request, the eight do the rest.
+// WORDS: every row starts on a whole word; otherwise the eight warps read the matrices themselves, element by element.
+template <int TOK, int KS, int STAGES, int RAW, int BLOCKS, bool WORDS>
 __global__ void __launch_bounds__(THREADS<TOK>, BLOCKS)
-gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ y, const int* __restrict__ row_index,
-                int rows, int x_rows, int n, int k, int token_tiles, int segments, int wide, unsigned* status) {
+gemm_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const float* __restrict__ x,
+                const float* __restrict__ w, float* __restrict__ y, int rows, int n, int k, int token_tiles, int segments, unsigned* status) {
   static_assert(KS == 32 || KS == 64, "k of a ring stage");
   constexpr int ROW = KS * 2;                               // bytes of a row in a plane
-  constexpr int A_PLANE = FT * ROW, B_PLANE = TOK * ROW;
-  constexpr int STAGE = 3 * (A_PLANE + B_PLANE);
-  constexpr int AW = FT * KS / 4 / WORKERS, BW = TOK * KS / 4 / WORKERS;     // words a thread brings per stage
+  constexpr int B_PLANE = TOK * ROW, A_COLS = KS / 2;       // of a plane
+  constexpr int STAGE = 3 * B_PLANE, RAW_STAGE = WORDS ? (FT + TOK) * KS * 4 : 0;
+  constexpr int BW = TOK * KS / 4 / WORKERS;                // token words a thread splits per stage
   constexpr int ROWS_PER = WORKERS / (KS / 4);              // rows between a thread's words
   constexpr int COLS = TOK / 2;
-  constexpr int TMEM_COLS = 2 * TOK <= 64 ? 64 : 2 * TOK <= 128 ? 128 : 2 * TOK <= 256 ? 256 : 512;
-  static_assert(TOK * KS / 4 % WORKERS == 0 && STAGES * STAGE >= TOK * FT * 4, "tile");
+  constexpr int USED_COLS = 2 * TOK + STAGES * 3 * A_COLS;  // the sums of 64 k, the small products, the weights' planes
+  constexpr int TMEM_COLS = USED_COLS <= 256 ? 256 : 512;
+  static_assert(ROWS_PER % 8 == 0 && TOK * KS / 4 % WORKERS == 0 && USED_COLS <= 512 && TMEM_COLS * BLOCKS <= 512, "tile");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* const smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  // [RAW] stages: the weights' [KS / 32][128 features][32] with the 128-byte swizzle, the tokens' [TOK][KS]
+  uint8_t* const words = smem + STAGES * STAGE;
+  __shared__ __align__(8) uint64_t raw_full[RAW], raw_empty[RAW];
   __shared__ __align__(8) uint64_t full_bar[STAGES];        // eight warps: a stage is split and stored
   __shared__ __align__(8) uint64_t empty_bar[STAGES];       // its MMAs are complete
   __shared__ __align__(8) uint64_t sum_free;                // eight warps: the 64-k sum has been taken out
   __shared__ uint32_t tmem_base_holder;
   __shared__ volatile int abort_flag;
-  __shared__ int source[TOK];                               // rows of x; -1: zeros, for an index out of range; -2: none
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int segment = blockIdx.x % segments;
@@ -157,6 +179,10 @@ gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float*
 
   if (threadIdx.x == 0) {
     abort_flag = 0;
+    for (int s = 0; s < RAW; ++s) {
+      mbar_init(smem_u32(&raw_full[s]), 1);
+      mbar_init(smem_u32(&raw_empty[s]), WORKERS / 32);
+    }
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(smem_u32(&full_bar[s]), WORKERS / 32);
       mbar_init(smem_u32(&empty_bar[s]), 1);
@@ -165,96 +191,98 @@ gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float*
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) tmem_alloc(smem_u32(&tmem_base_holder), TMEM_COLS);
-  // the weights do not depend on the kernel before this one
-  const int my_row = threadIdx.x / (KS / 4), my_k = threadIdx.x % (KS / 4) * 4;
-  float4 a[AHEAD][AW], b[AHEAD][BW];
-  auto fetch_a = [&](float4 (&to)[AW], int stage) {
-#pragma unroll
-    for (int i = 0; i < AW; ++i) {
-      const int f = f0 + my_row + i * ROWS_PER;
-      to[i] = load_word(w, f < n ? f : -1, k_begin + stage * KS + my_k, k, wide);
-    }
-  };
-  auto fetch_b = [&](float4 (&to)[BW], int stage) {
-#pragma unroll
-    for (int i = 0; i < BW; ++i) to[i] = load_word(x, source[my_row + i * ROWS_PER], k_begin + stage * KS + my_k, k, wide);
-  };
-  if (warp < WORKERS / 32) {
-#pragma unroll
-    for (int p = 0; p < AHEAD; ++p)
-      if (p < stages) fetch_a(a[p], p);
-  }
-  pdl_wait();
-  for (int t = threadIdx.x; t < TOK; t += THREADS<TOK>) {
-    int from = -2;
-    if (t0 + t < rows) {
-      from = row_index ? row_index[t0 + t] : t0 + t;
-      if (from < 0 || from >= x_rows) {
-        raise_fault(status, VOSTI_FAULT_ROW_RANGE);
-        from = -1;
-      }
-    }
-    source[t] = from;
-  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   pdl_launch_dependents();               // (after this CTA's tensor memory is its own)
-  const uint32_t tmem_sum = tmem_base_holder, tmem_small = tmem_sum + TOK;
+  const uint32_t tmem_sum = tmem_base_holder, tmem_small = tmem_sum + TOK, tmem_a = tmem_small + TOK;
 
   if (warp >= WORKERS / 32) {
     if constexpr (SPLITS_REGISTERS<TOK>) asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
-    if (warp == WORKERS / 32 && lane == 0) {
+    if (warp == WORKERS / 32 + 1 && lane == 0 && WORDS) {
+      // the weights of the first stages do not depend on the kernel before this one
+      auto bring_w = [&](int st) {
+        const int s = st % RAW;
+        mbar_expect_tx(smem_u32(&raw_full[s]), (uint32_t)RAW_STAGE);
+        for (int p = 0; p < KS / 32; ++p)
+          tma_load_2d(smem_u32(words + s * RAW_STAGE + p * FT * 128), &map_w, k_begin + st * KS + p * 32, f0, smem_u32(&raw_full[s]));
+      };
+      auto bring_x = [&](int st) {
+        const int s = st % RAW;
+        tma_load_2d(smem_u32(words + s * RAW_STAGE + FT * KS * 4), &map_x, k_begin + st * KS, t0, smem_u32(&raw_full[s]));
+      };
+      const int first = stages < RAW ? stages : RAW;
+      for (int st = 0; st < first; ++st) bring_w(st);
+      pdl_wait();
+      for (int st = 0; st < first; ++st) bring_x(st);
+      for (int st = first; st < stages; ++st) {
+        if (!mbar_wait(smem_u32(&raw_empty[st % RAW]), (st / RAW - 1) & 1, &abort_flag, status)) break;
+        bring_w(st);
+        bring_x(st);
+      }
+    }
+    if (warp == WORKERS / 32) {
       constexpr uint32_t idesc = umma_instr_desc(FT, TOK, false);
       bool ok = true;
+      auto arrived = [&](uint64_t* bar, uint32_t parity) {
+        return __all_sync(0xffffffffu, mbar_wait(smem_u32(bar), parity, &abort_flag, status)) != 0;
+      };
       for (int st = 0; st < stages && ok; ++st) {
         const int s = st % STAGES;
-        ok = mbar_wait(smem_u32(&full_bar[s]), (st / STAGES) & 1, &abort_flag, status);
+        ok = arrived(&full_bar[s], (st / STAGES) & 1);
         if (!ok) break;
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         tc_fence_after();
-        const uint32_t base = smem_u32(smem + s * STAGE);
-        const uint64_t ah = f32_desc<KS>(base), am = f32_desc<KS>(base + A_PLANE), al = f32_desc<KS>(base + 2 * A_PLANE);
-        const uint32_t bb = base + 3 * A_PLANE;
+        const uint32_t ah = tmem_a + s * 3 * A_COLS, am = ah + A_COLS, al = am + A_COLS, bb = smem_u32(smem + s * STAGE);
         const uint64_t bh = f32_desc<KS>(bb), bm = f32_desc<KS>(bb + B_PLANE), bl = f32_desc<KS>(bb + 2 * B_PLANE);
+        if (elect_one()) {
 #pragma unroll
-        for (int q = 0; q < KS / 16; ++q) {
-          umma_bf16(tmem_small, al + 2 * q, bh + 2 * q, idesc, st > 0 || q > 0);
-          umma_bf16(tmem_small, am + 2 * q, bm + 2 * q, idesc, 1u);
-          umma_bf16(tmem_small, ah + 2 * q, bl + 2 * q, idesc, 1u);
-          umma_bf16(tmem_small, am + 2 * q, bh + 2 * q, idesc, 1u);
-          umma_bf16(tmem_small, ah + 2 * q, bm + 2 * q, idesc, 1u);
+          for (int q = 0; q < KS / 16; ++q) {
+            umma_bf16_ts(tmem_small, al + 8 * q, bh + 2 * q, idesc, st > 0 || q > 0);
+            umma_bf16_ts(tmem_small, am + 8 * q, bm + 2 * q, idesc, 1u);
+            umma_bf16_ts(tmem_small, ah + 8 * q, bl + 2 * q, idesc, 1u);
+            umma_bf16_ts(tmem_small, am + 8 * q, bh + 2 * q, idesc, 1u);
+            umma_bf16_ts(tmem_small, ah + 8 * q, bm + 2 * q, idesc, 1u);
+          }
         }
+        __syncwarp();
         const int chunk = st / (KCHUNK / KS), part = st % (KCHUNK / KS);
         if (part == 0 && chunk > 0) {
-          ok = mbar_wait(smem_u32(&sum_free), (chunk - 1) & 1, &abort_flag, status);
+          ok = arrived(&sum_free, (chunk - 1) & 1);
           if (!ok) break;
           tc_fence_after();
         }
+        if (elect_one()) {
 #pragma unroll
-        for (int q = 0; q < KS / 16; ++q) umma_bf16(tmem_sum, ah + 2 * q, bh + 2 * q, idesc, part > 0 || q > 0);
-        umma_commit(smem_u32(&empty_bar[s]));
+          for (int q = 0; q < KS / 16; ++q) umma_bf16_ts(tmem_sum, ah + 8 * q, bh + 2 * q, idesc, part > 0 || q > 0);
+          umma_commit(smem_u32(&empty_bar[s]));
+        }
+        __syncwarp();
       }
     }
     return;
   }
 
   if constexpr (SPLITS_REGISTERS<TOK>) asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
+  pdl_wait();
   float acc[COLS];
 #pragma unroll
   for (int i = 0; i < COLS; ++i) acc[i] = 0.f;
   const int quarter = warp & 3, half = warp >> 2;
   const uint32_t my_columns = ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * COLS);
-#pragma unroll
-  for (int p = 0; p < AHEAD; ++p)
-    if (p < stages) fetch_b(b[p], p);
+  // weights: half of feature `quarter * 32 + lane`'s k, whose words lie at its place in the swizzle pattern
+  const int feature = quarter * 32 + lane;
+  const uint32_t my_a = tmem_a + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * (A_COLS / 2));
+  // tokens:
+  const int my_row = threadIdx.x / (KS / 4), my_k = threadIdx.x % (KS / 4) * 4;
+  const int rows_here = rows - t0;
+  // (a thread's rows are a multiple of 8 apart: one place in the swizzle pattern for all of them)
+  const int place = my_row * ROW + (((my_k >> 3) ^ (KS == 64 ? my_row & 7 : (my_row >> 1) & 3)) << 4) + (my_k & 4) * 2;
   bool ok = true;
-  auto swizzle = [](int r) { return KS == 64 ? r & 7 : (r >> 1) & 3; };
-  auto step = [&](float4 (&aw)[AW], float4 (&bw)[BW], int st) {
+  for (int st = 0; st < stages + STAGES; ++st) {
     const int s = st % STAGES;
     if (st >= STAGES) {
       // the stage that held this slot is complete: with it, at a chunk's end, the sum over 64 k
-      ok = ok && mbar_wait_warp(smem_u32(&empty_bar[s]), (st / STAGES - 1) & 1, &abort_flag, status);
+      ok = ok && f32_wait(smem_u32(&empty_bar[s]), (st / STAGES - 1) & 1, &abort_flag, status);
       if (ok && (st - STAGES) % (KCHUNK / KS) == KCHUNK / KS - 1) {
         tc_fence_after();
         add_columns<COLS>(tmem_sum + my_columns, acc);
@@ -263,31 +291,50 @@ gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float*
         if (lane == 0) mbar_arrive(smem_u32(&sum_free));
       }
     }
-    if (!ok || st >= stages) return;
-    uint8_t* const base = smem + s * STAGE;
+    if (!ok || st >= stages) continue;
+    const uint8_t* const raw = words + st % RAW * RAW_STAGE;
+    if (WORDS) {
+      ok = f32_wait(smem_u32(&raw_full[st % RAW]), (st / RAW) & 1, &abort_flag, status);
+      if (!ok) continue;
+    }
+    if (st >= STAGES) tc_fence_after();                    // (the MMAs that read the slot's planes)
 #pragma unroll
-    for (int i = 0; i < AW; ++i) {
-      const int r = my_row + i * ROWS_PER;
-      store_split(base + r * ROW + (((my_k >> 3) ^ swizzle(r)) << 4) + (my_k & 4) * 2, A_PLANE, aw[i]);
+    for (int g = 0; g < KS / 32; ++g) {
+      uint32_t h[8], m[8], l[8];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int kk = half * (KS / 2) + g * 16 + i * 4;
+        const float4 v = WORDS ? *reinterpret_cast<const float4*>(raw + (kk / 32 * FT + feature) * 128 + (((kk % 32 >> 2) ^ (feature & 7)) << 4))
+                               : load_elements(w + (int64_t)min(f0 + feature, n - 1) * k, k_begin + st * KS + kk, k);
+        split_four(v, h + 2 * i, m + 2 * i, l + 2 * i);
+      }
+      const uint32_t at = my_a + s * 3 * A_COLS + g * 8;
+      tmem_store8(at, h);
+      tmem_store8(at + A_COLS, m);
+      tmem_store8(at + 2 * A_COLS, l);
     }
 #pragma unroll
     for (int i = 0; i < BW; ++i) {
       const int r = my_row + i * ROWS_PER;
       // (columns of rows that are not there are never stored, and touch no other column)
-      if (TOK <= 64 && source[r] == -2) continue;
-      store_split(base + 3 * A_PLANE + r * ROW + (((my_k >> 3) ^ swizzle(r)) << 4) + (my_k & 4) * 2, B_PLANE, bw[i]);
+      if (TOK <= 64 && r >= rows_here) continue;
+      const float4 v = WORDS ? *reinterpret_cast<const float4*>(raw + FT * KS * 4 + (r * KS + my_k) * 4)
+                             : load_elements(x + (int64_t)min(t0 + r, rows - 1) * k, k_begin + st * KS + my_k, k);
+      uint2 h, m, l;
+      split_four(v, &h.x, &m.x, &l.x);
+      uint8_t* const at = smem + s * STAGE + i * ROWS_PER * ROW + place;
+      *reinterpret_cast<uint2*>(at) = h;
+      *reinterpret_cast<uint2*>(at + B_PLANE) = m;
+      *reinterpret_cast<uint2*>(at + 2 * B_PLANE) = l;
     }
+    tmem_wait_stores();
+    tc_fence_before();
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncwarp();
-    if (lane == 0) mbar_arrive(smem_u32(&full_bar[s]));
-    if (st + AHEAD < stages) {
-      fetch_a(aw, st + AHEAD);
-      fetch_b(bw, st + AHEAD);
+    if (lane == 0) {
+      mbar_arrive(smem_u32(&full_bar[s]));
+      if (WORDS) mbar_arrive(smem_u32(&raw_empty[st % RAW]));
     }
-  };
-  for (int st = 0; st < stages + STAGES; st += AHEAD) {
-#pragma unroll
-    for (int p = 0; p < AHEAD; ++p)
-      if (st + p < stages + STAGES) step(a[p], b[p], st + p);
   }
   if (ok) {
     tc_fence_after();
@@ -299,9 +346,8 @@ gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float*
     if (t0 + t >= rows || f0 + f >= n) return;
     if (!(fabsf(v) <= 3.402823466e+38f) || (fabsf(v) < 8.2718061e-25f && v != 0.f)) {       // 2^-80
       v = 0.f;
-      const int from = source[t];
-      const float *xr = x + (int64_t)(from < 0 ? 0 : from) * k, *wr = w + (int64_t)(f0 + f) * k;
-      for (int kk = 0; kk < k && v == v; ++kk) v = fmaf(from < 0 ? 0.f : xr[kk], wr[kk], v);
+      const float *xr = x + (int64_t)(t0 + t) * k, *wr = w + (int64_t)(f0 + f) * k;
+      for (int kk = 0; kk < k && v == v; ++kk) v = fmaf(xr[kk], wr[kk], v);
     }
     y[(int64_t)(t0 + t) * n + f0 + f] = v;
   };
@@ -352,21 +398,36 @@ int f32_segments(int n, int k) {
   return s;
 }
 
-template <int TOK, int KS, int STAGES, int AHEAD, int BLOCKS>
-int launch_f32(const float* x, const float* w, float* y, const int* row_index, int rows, int x_rows, int n, int k, int wide,
-               unsigned* status, cudaStream_t stream) {
-  constexpr int SMEM = STAGES * 3 * (FT + TOK) * KS * 2 + 1024;
-  auto kernel = gemm_f32_kernel<TOK, KS, STAGES, AHEAD, BLOCKS>;
+// Map of a row-major [rows, k] float32 matrix (k a multiple of 4, 16-byte aligned), boxes of box_rows x box_k.
+bool f32_map(CUtensorMap* map, const float* base, int64_t rows, int k, int box_rows, int box_k, CUtensorMapSwizzle swizzle) {
+  VostiEncodeTiledFn fn = tensor_map_encoder();
+  if (!fn) return false;
+  const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)rows};
+  const cuuint64_t strides[1] = {(cuuint64_t)k * 4};
+  const cuuint32_t box[2] = {(cuuint32_t)box_k, (cuuint32_t)box_rows};
+  const cuuint32_t elem[2] = {1, 1};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int TOK, int KS, int STAGES, int RAW, int BLOCKS, bool WORDS>
+int launch_f32(const float* x, const float* w, float* y, int rows, int n, int k, unsigned* status, cudaStream_t stream) {
+  constexpr int RINGS = STAGES * 3 * TOK * KS * 2 + (WORDS ? RAW * (FT + TOK) * KS * 4 : 0);
+  constexpr int SMEM = (RINGS > TOK * FT * 4 ? RINGS : TOK * FT * 4) + 1024;       // (the rings' place holds a segment's sums at the end)
+  auto kernel = gemm_f32_kernel<TOK, KS, STAGES, RAW, BLOCKS, WORDS>;
   static const cudaError_t raised = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
   if (raised != cudaSuccess) {
     vosti_set_error("gemm_f32: %s", cudaGetErrorString(raised));
     return (int)raised;
   }
+  CUtensorMap mx = {}, mw = {};
+  VOSTI_REQUIRE(!WORDS || (f32_map(&mx, x, rows, k, TOK, KS, CU_TENSOR_MAP_SWIZZLE_NONE) && f32_map(&mw, w, n, k, FT, 32, CU_TENSOR_MAP_SWIZZLE_128B)),
+                "gemm_f32: cuTensorMapEncodeTiled failed");
   const int segments = f32_segments(n, k), token_tiles = (rows + TOK - 1) / TOK;
   const int64_t ctas = (int64_t)((n + FT - 1) / FT) * token_tiles * segments;
   VOSTI_REQUIRE(ctas <= 0x7fffffff, "gemm_f32: too many tiles for one launch");
-  const cudaError_t e = vosti_launch_clusters(kernel, dim3((unsigned)ctas), dim3(THREADS<TOK>), (unsigned)segments, SMEM, stream, x, w, y,
-                                              row_index, rows, x_rows, n, k, token_tiles, segments, wide, status);
+  const cudaError_t e = vosti_launch_clusters(kernel, dim3((unsigned)ctas), dim3(THREADS<TOK>), (unsigned)segments, SMEM, stream, mx, mw, x, w,
+                                              y, rows, n, k, token_tiles, segments, status);
   if (e != cudaSuccess) {
     vosti_set_error("gemm_f32: %s", cudaGetErrorString(e));
     return (int)e;
@@ -376,23 +437,34 @@ int launch_f32(const float* x, const float* w, float* y, const int* row_index, i
 
 }  // namespace
 
-// Whether the kernel takes a float32 [n, k] weight (a rule of the sizes only).
-VOSTI_API int vosti_gemm_f32_supported(int n, int k) { return n >= 16 && k >= 128; }
+// Whether a float32 [n, k] weight is this kernel's (a rule of the sizes only, so that a row's bits stay its own). Below, a chain of
+// multiply-adds is as fast or faster for few rows (us here / there, 1 and 384 rows: 2,048 x 512 9 / 5 and 17 / 36; 512 x 1,024 8 / 7
+// and 15 / 30, 256 x 2,048 9 / 11 and 15 / 39).
+VOSTI_API int vosti_gemm_f32_supported(int n, int k) { return n >= 16 && k >= 1024; }
 
-// x: [x_rows, k]; w: [n, k]; y: [rows, n], all float32. With row_index (int32[rows]) row t is x[row_index[t]].
-VOSTI_API int vosti_gemm_f32(const float* x, const float* w, float* y, const int* row_index, int rows, int x_rows, int n, int k,
-                             unsigned* status, cudaStream_t stream) {
-  VOSTI_REQUIRE(rows >= 0 && x_rows >= 0 && vosti_gemm_f32_supported(n, k), "gemm_f32: bad sizes rows=%d n=%d k=%d", rows, n, k);
-  VOSTI_REQUIRE(row_index != nullptr || rows == x_rows, "gemm_f32: rows != x_rows without a row index");
+// x: [rows, k]; w: [n, k]; y: [rows, n], all float32.
+VOSTI_API int vosti_gemm_f32(const float* x, const float* w, float* y, int rows, int n, int k, unsigned* status, cudaStream_t stream) {
+  VOSTI_REQUIRE(rows >= 0 && n > 0 && k > 0, "gemm_f32: bad sizes rows=%d n=%d k=%d", rows, n, k);
   if (rows == 0) return VOSTI_OK;
-  const int wide = k % 4 == 0 && (reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) % 16 == 0;
-#define VOSTI_F32(TOK, KS, STAGES, AHEAD, BLOCKS) \
-  return launch_f32<TOK, KS, STAGES, AHEAD, BLOCKS>(x, w, y, row_index, rows, x_rows, n, k, wide, status, stream)
-  const int by256 = (rows + 255) / 256 * 256, by192 = (rows + 191) / 192 * 192;
-  if (rows <= 32) VOSTI_F32(32, 32, 3, 2, 2);
-  if (rows <= 64) VOSTI_F32(64, 32, 3, 1, 2);
-  if (rows <= 128) VOSTI_F32(128, 32, 4, 1, 1);
-  if (by192 < by256) VOSTI_F32(192, 32, 3, 1, 1);
-  VOSTI_F32(256, 32, 3, 1, 1);
+  // every row starts on a whole word
+  const bool wide = k % 4 == 0 && (reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) % 16 == 0;
+#define VOSTI_F32(TOK, KS, STAGES, RAW, BLOCKS) \
+  return wide ? launch_f32<TOK, KS, STAGES, RAW, BLOCKS, true>(x, w, y, rows, n, k, status, stream) \
+              : launch_f32<TOK, KS, STAGES, RAW, BLOCKS, false>(x, w, y, rows, n, k, status, stream)
+  const int tiles = (n + FT - 1) / FT, segments = f32_segments(n, k);
+  auto ctas = [&](int tok) { return (int64_t)tiles * segments * ((rows + tok - 1) / tok); };
+  // Clusters of up to four CTAs find some 140 SMs at one CTA each. Where these take them all at once, a deeper ring of whole 64s is the
+  // fastest (us, 4,096 x 12,288, 1 row: 54, two stages 61, stages of 32 k 88; 64 rows: 74 and 111); with more CTAs, or eight a
+  // cluster, two of them an SM are (24,576 x 4,096, 1 row: 93 and 133, 64 rows: 162 and 185; 2,048 x 2,048: 11 and 17, 17 and 23).
+  const bool one_round = segments <= 4 && ctas(rows) <= 140;
+  if (rows <= 32 && one_round) VOSTI_F32(32, 64, 2, 3, 1);
+  if (rows <= 32) VOSTI_F32(32, 64, 2, 2, 1);
+  if (rows <= 64 && one_round) VOSTI_F32(64, 64, 2, 2, 1);
+  if (rows <= 64) VOSTI_F32(64, 32, 2, 3, 1);
+  // A tile of 192 tokens takes about 1.4 times as long as one of 128: the fewer rounds of CTAs decide (us, 384 rows: 24,576 x 4,096 504
+  // and 441, 6,144 x 4,096 149 and 171, 4,096 x 4,096 101 and 104).
+  const int at_once = segments > 1 ? 140 : 148;
+  if (10 * ((ctas(128) + at_once - 1) / at_once) <= 14 * ((ctas(192) + at_once - 1) / at_once)) VOSTI_F32(128, 64, 2, 2, 1);
+  VOSTI_F32(192, 32, 2, 2, 1);
 #undef VOSTI_F32
 }

@@ -246,16 +246,14 @@ def gemm_f32_supported(n: int, k: int) -> bool:
     return bool(library().vosti_gemm_f32_supported(int(n), int(k)))
 
 
-def gemm_f32(x: torch.Tensor, w: torch.Tensor, status: torch.Tensor, *, row_index: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """y = x[row_index] @ w.T of float32 matrices on the tensor cores, every operand as three bfloat16 terms
+def gemm_f32(x: torch.Tensor, w: torch.Tensor, status: torch.Tensor) -> torch.Tensor:
+    """y = x @ w.T of float32 matrices on the tensor cores, every operand as three bfloat16 terms
     (csrc/gemm_f32.cu): nearer to 64 bits than a chain of float32 multiply-adds; a row's bits do not depend on the others."""
-    _contig(x, w, row_index)
+    _contig(x, w)
     if x.dtype != torch.float32 or w.dtype != torch.float32 or x.shape[1] != w.shape[1]:
         raise KernelError("gemm_f32 takes float32 [rows, k] and [n, k]")
-    rows = x.shape[0] if row_index is None else row_index.shape[0]
-    out = torch.empty((rows, w.shape[0]), dtype=torch.float32, device=x.device)
-    _check(library().vosti_gemm_f32(_p(x), _p(w), _p(out), _p(row_index), rows, x.shape[0], w.shape[0], x.shape[1], _p(status),
-                                    _stream()), "gemm_f32")
+    out = torch.empty((x.shape[0], w.shape[0]), dtype=torch.float32, device=x.device)
+    _check(library().vosti_gemm_f32(_p(x), _p(w), _p(out), x.shape[0], w.shape[0], x.shape[1], _p(status), _stream()), "gemm_f32")
     return out
 
 

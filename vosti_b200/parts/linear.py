@@ -60,5 +60,5 @@ def linear(ctx, x: torch.Tensor, w: torch.Tensor, *, out_dtype: Optional[torch.d
             x = ops.gather_rows(x, row_index, ctx.status)
         return ops.gemm_tc(x, w, ctx.status, out_dtype=out_dtype, allow_partial=allow_partial, scratch=scratch)
     if uses_split_float32(x.dtype, w) and out_dtype in (None, torch.float32):
-        return ops.gemm_f32(x, w, ctx.status, row_index=row_index)
+        return ops.gemm_f32(x if row_index is None else ops.gather_rows(x, row_index, ctx.status), w, ctx.status)
     return ops.gemm_simt(x, w, ctx.status, out_dtype=out_dtype, row_index=row_index)
