@@ -22,7 +22,6 @@
 #include <cfloat>
 
 #include "common.cuh"
-#include "mma_util.cuh"
 
 namespace {
 
@@ -330,12 +329,11 @@ scan_run_kernel(const T* __restrict__ x, const float* __restrict__ dtp, const vo
 }
 
 // A long portion of 16 states a channel, tokens in order in one pass. The chain from token to token is one
-// multiply-add a state; everything else of a token (its exponentials above all: one ex2 of a base-2 rate, where expf took
-// eight instructions and 152 us instead of 136) is off the chain, so 32 channels
-// a block and a token every 120 cycles (62 ns) need no chunks, whose first pass computes every exponential a second
+// multiply-add a state; everything else of a token (its exponentials above all) is off the chain, so 32 channels
+// a block and a token every 130 cycles (68 ns) need no chunks, whose first pass computes every exponential a second
 // time. Warps 0 to 3 run the recurrence, four lanes a channel with four neighbouring states each; warps 4 to 11
 // meanwhile finish the tile before (skip, gate, store) and bring the tile after (softplus, SiLU) into the
-// other buffer. 1,499 + 549 tokens of 4,096 channels: 131 us, against 324 us of the three chunk kernels; 2,048 tokens
+// other buffer. 1,499 + 549 tokens of 4,096 channels: 147 us, against 324 us of the three chunk kernels; 2,048 tokens
 // 144 against 324, 1,024 tokens beside 30 single ones 89 against 226.
 constexpr int LINE_TOKENS = 64, LINE_STATES = 16, LINE_AHEAD = 4;          // (the dealing out of sums is written for four)
 constexpr int LINE_BRING = 256, LINE_THREADS = 128 + LINE_BRING;         // threads that bring, and all of a block
@@ -419,8 +417,8 @@ scan_line_kernel(const T* __restrict__ x, const float* __restrict__ dtp, const v
     for (int j = 0; j < 4; ++j) {
       s[j] = S[j];
       // (finite also where the rate is not: a tile's places past the last token have a step size of 0 and must change nothing)
-      const float rate = expf(load_flex(a_log, w_f32, (int64_t)(live ? c : inner - 1) * N + r * 4 + j)) * 1.4426950408889634f;
-      a[j] = rate == INFINITY ? -FLT_MAX : -rate;               // the decay is 2^(dt a)
+      const float rate = expf(load_flex(a_log, w_f32, (int64_t)(live ? c : inner - 1) * N + r * 4 + j));
+      a[j] = rate == INFINITY ? -FLT_MAX : -rate;
     }
   } else {
     fetch(0);
@@ -448,7 +446,7 @@ scan_line_kernel(const T* __restrict__ x, const float* __restrict__ dtp, const v
           g.in[u][2] = dx * B.z;
           g.in[u][3] = dx * B.w;
 #pragma unroll
-          for (int j = 0; j < 4; ++j) g.e[u][j] = fast_exp2(dt * a[j]);
+          for (int j = 0; j < 4; ++j) g.e[u][j] = expf(dt * a[j]);
         }
       };
       auto chain = [&](const Group& g, int i0) {
