@@ -580,7 +580,7 @@ def gemm_tc(x: torch.Tensor, w, status: torch.Tensor, *, out_dtype: Optional[tor
         epilogue, width = (EPI_F32 if out_dtype == torch.float32 else EPI_BF16), features
     lib = library()
     splits = lib.vosti_gemm_tc_splits(tokens, features, k)
-    if splits == 1:
+    if splits == 1 and INVARIANCE != "decode":          # ("decode": a prompt's portions of more than 128 tokens keep one order too)
         splits = lib.vosti_gemm_tc_pair_splits(tokens, features, k)
     elems = splits * tokens * features if splits > 1 else 0
     # more than 128 tokens: sums of the call's own, so that products on several streams and a partial sum that is
