@@ -19,28 +19,31 @@
 // Kernels:
 //   delta_chunk_prepare   one block per (chunk, head), all side by side: A, Q (B, R), then one thread per key
 //                         channel (W, O1) and per value column (U, O0)
-//   delta_chunk_run       one block per (request, head, 16 value columns): the chunks one after the other; per
-//                         chunk [W; O1] S0 and the state's update, both as 8 x 4 register tiles whose summands
-//                         are spread over 8 (4) lanes
+//   delta_chunk_run       one block per (request, head, 16 value columns): the chunks one after the other; per chunk
+//                         [W; O1] S0 and the state's update on mma.sync, every operand as three bfloat16 terms
 //
 // The scratch takes 516 floats a token and head (644 in the generalized rule); its caller bounds it and the chunks run in
 // rounds. Which steps come here and which go token by token: delta_takes_chunks in ops.py, with both sides' times.
 //
-// 2,048 tokens of one request, 16 heads of 128: 82 us and 194 us (the token-by-token kernel: 698 us); the
-// generalized rule over 1,031 + 700 + 317 tokens: 140 us and 278 us (628 us). The first is bound by shared-memory
-// latency at two blocks an SM (issue slots 43 % busy), the second by the shared-memory pipe of the 128 SMs that
-// have a block: 16-byte operand reads, the shuffles that deal the sums out, the copies of the next chunks.
+// 2,048 tokens of one request, 16 heads of 128: 79 us and 147 us (the token-by-token kernel: 698 us); the generalized rule
+// over 1,031 + 700 + 317 tokens: 138 us and 201 us (628 us). The first is bound by the shared-memory pipe at two blocks an SM.
+// The second was too (8 x 4 tiles of multiply-adds with 16-byte operand reads, shuffles, copies: 194 and 278 us); on the tensor
+// cores a chunk takes 2.3 us (generalized 3.2), of which its MMAs are 0.7 and the copies that the blocks' SMs take in
+// 0.4, the rest is two barriers and the latency between them (rows by cp.async.bulk instead: 5.6 us a chunk).
+// tcgen05 would add a commit and a read of tensor memory to each of the two products of the chain, which are
+// 64 x 16 x 128 and 128 x 16 x 32.
 //
 // The token-by-token kernel waits for a shared-memory read, a chain of multiply-adds and two shuffle reductions
 // between any two tokens; here the chain between chunks is two small products over 32 tokens.
 #include <type_traits>
 
 #include "common.cuh"
+#include "mma_util.cuh"
 
 namespace {
 
 constexpr int CHUNK = 32, HALF = 16, DK = 128, PITCH = DK + 4, COLS = 16;
-constexpr int WO = 2 * CHUNK;                    // W and O1 of a key channel, side by side
+constexpr int WO = 2 * CHUNK;                    // rows of W and of O1, one below the other
 
 struct ChunkArgs {
   const float *x, *y, *g, *b, *k, *v, *beta;     // b and k: the generalized rule's unit and write keys; beta: the gated rule's
@@ -53,11 +56,10 @@ struct ChunkArgs {
   const int *chunk_request, *chunk_first;        // per chunk: its request and its first token in the portion
   const int *long_requests, *long_chunk0;        // per long request: its number and its first chunk
   int from, count;                               // this launch's chunks; the scratch holds them, from 0 on
-  float *wo, *ends, *us, *gammas;                // [chunk, head, DK, WO], [.., (2) CHUNK, DK], [.., CHUNK, dv], [.., DK]
+  float *wo, *ends, *us, *gammas;                // [chunk, head, WO, DK], [.., (2) CHUNK, DK], [.., CHUNK, dv], [.., DK]
 };
 
 __device__ __forceinline__ float4 at4(const float* p) { return *reinterpret_cast<const float4*>(p); }
-__device__ __forceinline__ void put4(float* p, float a, float b, float c, float d) { *reinterpret_cast<float4*>(p) = make_float4(a, b, c, d); }
 __device__ __forceinline__ float dot4(float4 a, float4 b, float acc) {
   return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, acc))));
 }
@@ -260,8 +262,7 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_prepare_kernel(ChunkArgs a
   if (tid < DK) {
     const int c = tid;
     float w[CHUNK], gamma = 1.f, first_half = 1.f;
-    float* const to = a.wo + (place * DK + c) * WO;
-    float o4[4], w4[4];
+    float* const to = a.wo + place * WO * DK + c;
     each<0, CHUNK>([&](auto index) {
       constexpr int i = decltype(index)::value;
       if (i == HALF) first_half = gamma;
@@ -276,13 +277,9 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_prepare_kernel(ChunkArgs a
       }
       if (!PAIR) bg *= sbeta[i];
       w[i] = -row_sum<i>(MA + i * CHUNK, w, bg);
-      o4[i & 3] = row_sum<i + 1>(MQ + i * CHUNK, w, yg);
-      w4[i & 3] = w[i];
+      to[i * DK] = w[i];
+      to[(CHUNK + i) * DK] = row_sum<i + 1>(MQ + i * CHUNK, w, yg);
       gamma *= g;
-      if ((i & 3) == 3) {
-        put4(to + i - 3, w4[0], w4[1], w4[2], w4[3]);
-        put4(to + CHUNK + i - 3, o4[0], o4[1], o4[2], o4[3]);
-      }
     });
     a.gammas[place * DK + c] = gamma;
     // x (and k) decayed to the chunk's end
@@ -323,22 +320,74 @@ __device__ __forceinline__ void copy16(float* dst, const float* src, bool there 
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(there ? 16 : 0) : "memory");
 }
 
-constexpr int WO_PITCH = WO + 4, S_PITCH = COLS + 4, RUN_THREADS = 256;
-template <bool PAIR> constexpr int STAGE_FLOATS = DK * WO_PITCH + (PAIR ? 2 : 1) * CHUNK * (DK + S_PITCH) + DK;
+// Two neighbouring values as three words of two bfloat16 terms, each the upper half of what the terms before it leave: nothing of a
+// float32 is lost (an infinity leaves inf - inf: a state that overflows turns into NaN).
+__device__ __forceinline__ void split_two(float x, float y, uint32_t& h, uint32_t& m, uint32_t& l) {
+  auto upper = [](float v) { return __uint_as_float(__float_as_uint(v) & 0xffff0000u); };
+  auto both = [](float lo, float hi) { return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632); };
+  const float xm = x - upper(x), ym = y - upper(y);
+  h = both(x, y);
+  m = both(xm, ym);
+  l = both(xm - upper(xm), ym - upper(ym));
+}
+__device__ __forceinline__ void mma_terms(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+__device__ __forceinline__ void mma_eight(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
+  asm("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(b0));
+}
+// sum += A B (16 x 16 times 16 x 8), A and B as three terms: the product of the first terms is added rounded to nearest, those of order
+// 2^-8 to 2^-24 gather in `small` (truncated terms lean to one side: without the last two the states were up to twice as far
+// from 64 bits as a chain of multiply-adds). HALVES: the first terms in two sums of 8, which the tensor core truncates less.
+template <bool HALVES>
+__device__ __forceinline__ void mma_split(float (&sum)[4], float (&small)[4], const uint32_t (&a)[3][4], const uint32_t (&b)[3][2]) {
+  float first[4] = {0.f, 0.f, 0.f, 0.f};
+  if (HALVES) {
+    float lower[4] = {0.f, 0.f, 0.f, 0.f};
+    mma_eight(lower, a[0][0], a[0][1], b[0][0]);
+    mma_eight(first, a[0][2], a[0][3], b[0][1]);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) first[e] += lower[e];
+  } else {
+    mma_terms(first, a[0], b[0]);
+  }
+  mma_terms(small, a[2], b[1]);
+  mma_terms(small, a[1], b[2]);
+  mma_terms(small, a[2], b[0]);
+  mma_terms(small, a[1], b[1]);
+  mma_terms(small, a[0], b[2]);
+  mma_terms(small, a[1], b[0]);
+  mma_terms(small, a[0], b[1]);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) sum[e] += first[e];
+}
+
+constexpr int WO_PITCH = DK + 8, END_PITCH = DK + 4, U_PITCH = COLS + 4, RUN_THREADS = 256;
+constexpr int SP_PITCH = DK + 8, UP_PITCH = CHUNK + 8;          // bfloat16 of a value column in the state's and the updates' planes
+template <bool PAIR> constexpr int STAGE_FLOATS = WO * WO_PITCH + (PAIR ? 2 : 1) * CHUNK * (END_PITCH + U_PITCH) + DK;
 template <bool PAIR> constexpr int RUN_STAGES = PAIR ? 2 : 3;
+template <bool PAIR> constexpr int RUN_BYTES = RUN_STAGES<PAIR> * STAGE_FLOATS<PAIR> * 4 + 3 * COLS * (SP_PITCH + (PAIR ? 2 : 1) * UP_PITCH) * 2;
 
 template <bool PAIR>
 __global__ void __launch_bounds__(RUN_THREADS) delta_chunk_run_kernel(ChunkArgs a) {
   extern __shared__ __align__(16) float chunk_shared[];
   constexpr int STAGES = RUN_STAGES<PAIR>, STAGE = STAGE_FLOATS<PAIR>, ROWS = (PAIR ? 2 : 1) * CHUNK;
-  float* const S = chunk_shared + STAGES * STAGE;               // [DK][S_PITCH]
+  uint16_t* const SP = reinterpret_cast<uint16_t*>(chunk_shared + STAGES * STAGE);   // [term][value column][key channel] of the state
+  uint16_t* const UP = SP + 3 * COLS * SP_PITCH;                 // [term][value column][token] of u [and of v]
+  uint16_t* const VP = UP + 3 * COLS * UP_PITCH;
   pdl_wait();
   pdl_launch_dependents();
-  const int request = a.long_requests[blockIdx.x], h = blockIdx.y, col0 = blockIdx.z * COLS;
+  // the longest request's blocks first (three of 1,031, 700 and 317 tokens: 63 chunk times end to end, 76 if they take turns)
+  const int cols = a.dv / COLS, longs = blockIdx.x / (a.heads * cols);
+  const int request = a.long_requests[longs], h = blockIdx.x / cols % a.heads, col0 = blockIdx.x % cols * COLS;
   const int slot = a.state_slots[request];
   if (slot < 0 || slot >= a.num_slots) return;
   // the request's chunks in this launch: from chunk `begin` on, or from its first one
-  const int chunk0 = a.long_chunk0[blockIdx.x] - a.from, begin = max(0, -chunk0);
+  const int chunk0 = a.long_chunk0[longs] - a.from, begin = max(0, -chunk0);
   const int start = a.cu_q[request] + begin * CHUNK, n = min(a.cu_q[request + 1] - start, (a.count - chunk0 - begin) * CHUNK);
   if (n <= 0) return;
   const int chunks = (n + CHUNK - 1) / CHUNK;
@@ -346,132 +395,190 @@ __global__ void __launch_bounds__(RUN_THREADS) delta_chunk_run_kernel(ChunkArgs 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t row = (int64_t)a.heads * a.dv;
   float* const state = a.state + (int64_t)slot * a.state_stride + ((int64_t)h * a.dv + col0) * DK;
-  for (int i = tid; i < COLS * DK; i += RUN_THREADS) S[(i % DK) * S_PITCH + i / DK] = state[i];
 
   auto load = [&](int chunk) {
     if (chunk < chunks) {
       float* const wo = chunk_shared + chunk % STAGES * STAGE;
-      float* const ends = wo + DK * WO_PITCH;
-      float* const uv = ends + ROWS * DK;
-      float* const gam = uv + ROWS * S_PITCH;
+      float* const ends = wo + WO * WO_PITCH;
+      float* const uv = ends + ROWS * END_PITCH;
+      float* const gam = uv + ROWS * U_PITCH;
       const int64_t place = (place0 + chunk) * a.heads + h;
-      for (int i = tid; i < DK * (WO / 4); i += RUN_THREADS) {
-        const int r = i / (WO / 4), c = (i % (WO / 4)) * 4;
-        copy16(wo + r * WO_PITCH + c, a.wo + (place * DK + r) * WO + c);
+      for (int i = tid; i < WO * (DK / 4); i += RUN_THREADS) {
+        const int r = i / (DK / 4), c = (i % (DK / 4)) * 4;
+        copy16(wo + r * WO_PITCH + c, a.wo + place * WO * DK + i * 4);
       }
-      for (int i = tid; i < ROWS * (DK / 4); i += RUN_THREADS) copy16(ends + i * 4, a.ends + place * ROWS * DK + i * 4);
+      for (int i = tid; i < ROWS * (DK / 4); i += RUN_THREADS) {
+        const int r = i / (DK / 4), c = (i % (DK / 4)) * 4;
+        copy16(ends + r * END_PITCH + c, a.ends + place * ROWS * DK + i * 4);
+      }
       const int r = (tid & 127) / (COLS / 4), c = (tid % (COLS / 4)) * 4;   // 32 rows of 4 words of U, and of v
       if (tid < 128) {
-        copy16(uv + r * S_PITCH + c, a.us + (place * CHUNK + r) * a.dv + col0 + c);
+        copy16(uv + r * U_PITCH + c, a.us + (place * CHUNK + r) * a.dv + col0 + c);
       } else if (PAIR) {
         const int t = chunk * CHUNK + r;
-        copy16(uv + (CHUNK + r) * S_PITCH + c, a.v + (start + min(t, n - 1)) * row + (int64_t)h * a.dv + col0 + c, t < n);
+        copy16(uv + (CHUNK + r) * U_PITCH + c, a.v + (start + min(t, n - 1)) * row + (int64_t)h * a.dv + col0 + c, t < n);
       }
       if (tid < DK / 4) copy16(gam + tid * 4, a.gammas + place * DK + tid * 4);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
+
+  // Products are transposed: value columns on a tile's 16 rows, so that a warp splits only what it alone multiplies. A lane's results
+  // are columns g and g + 8 at two neighbouring places (2 t, 2 t + 1) of the other side.
+  const int g = lane >> 2, t = lane & 3;
+  const int tile_row = lane & 15, tile_k = (lane >> 4) * 8;      // this lane's row of an `ldmatrix` tile
+  const int rows0 = warp * 8 + 2 * t;                            // of [W; O1]: a u (the first 32), or an o, whose first part is out there
+  auto terms = [&](const uint16_t* planes, int pitch, int k0, uint32_t (&r)[3][4]) {
+#pragma unroll
+    for (int p = 0; p < 3; ++p) ldmatrix_x4(r[p], smem_addr(planes + (p * COLS + tile_row) * pitch + k0 + tile_k));
+  };
+  uint32_t wo_terms[DK / 16][3][2];
+  auto split_wo = [&](const float* wo, int ks) {
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const float2 v = *reinterpret_cast<const float2*>(wo + (warp * 8 + g) * WO_PITCH + ks * 16 + e * 8 + 2 * t);
+      split_two(v.x, v.y, wo_terms[ks][0][e], wo_terms[ks][1][e], wo_terms[ks][2][e]);
+    }
+  };
+  float S[2][4];                                                 // [8 key channels each]
+  auto publish = [&]() {
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        uint32_t term[3];
+        split_two(S[nt][2 * e], S[nt][2 * e + 1], term[0], term[1], term[2]);
+#pragma unroll
+        for (int p = 0; p < 3; ++p)
+          *reinterpret_cast<uint32_t*>(SP + (p * COLS + g + 8 * e) * SP_PITCH + warp * 16 + nt * 8 + 2 * t) = term[p];
+      }
+  };
+#pragma unroll
+  for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const float2 v = *reinterpret_cast<const float2*>(state + (g + 8 * e) * DK + warp * 16 + nt * 8 + 2 * t);
+      S[nt][2 * e] = v.x;
+      S[nt][2 * e + 1] = v.y;
+    }
+  publish();
 #pragma unroll
   for (int i = 0; i < STAGES - 1; ++i) load(i);
-  // [W; O1] S: lane = 8 summands' groups x 4 tiles of 8 rows x 4 columns
-  const int kg = lane & 7, rt = warp, ct = lane >> 3;
-  // the update: lane = 4 groups of tokens x 8 tiles of 8 key channels (4 and 4) x 4 columns
-  const int tg = lane >> 3, kt = (warp >> 2) * 8 + (lane & 7), ct2 = warp & 3;
+  const int i0 = rows0 & (CHUNK - 1);
+  float base[4] = {0.f, 0.f, 0.f, 0.f};                          // (an o's first part is asked for a chunk ahead)
+  auto ask = [&](int chunk) {
+    const float* const out = a.out + (start + chunk * CHUNK + i0) * row + (int64_t)h * a.dv + col0 + g;
+    const int left = n - chunk * CHUNK - i0;                     // this lane's tokens that there are: left of two
+#pragma unroll
+    for (int e = 0; e < 4; ++e) base[e] = (e & 1) < left ? out[(e & 1) * row + (e >> 1) * 8] : 0.f;
+  };
+  if (warp >= 4) ask(0);
+  asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+  __syncthreads();
+#pragma unroll
+  for (int ks = 0; ks < DK / 16; ++ks) split_wo(chunk_shared, ks);
 #pragma unroll 1
   for (int chunk = 0; chunk < chunks; ++chunk) {
     load(chunk + STAGES - 1);
     const float* const wo = chunk_shared + chunk % STAGES * STAGE;
-    const float* const ends = wo + DK * WO_PITCH;
-    float* const uv = const_cast<float*>(ends) + ROWS * DK;
-    const float* const gam = uv + ROWS * S_PITCH;
-    // this thread's outputs are row rt * 8 + kg: a u (the first 32 rows), or an o, whose first part is out there
-    const int i = (rt & 3) * 8 + kg;
-    float* const out = a.out + (start + chunk * CHUNK + i) * row + (int64_t)h * a.dv + col0 + ct * 4;
-    const bool reads = rt >= 4, writes = reads && chunk * CHUNK + i < n;
-    float4 base = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (writes) base = at4(out);
-    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 1) : "memory");
-    __syncthreads();
-    float acc[8][4];
+    const float* const ends = wo + WO * WO_PITCH;
+    const float* const uv = ends + ROWS * END_PITCH;
+    const float* const gam = uv + ROWS * U_PITCH;
+    if (warp < 4) {
 #pragma unroll
-    for (int r = 0; r < 8; ++r)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) acc[r][c] = 0.f;
-#pragma unroll 2
-    for (int s = 0; s < DK / 8; ++s) {
-      const int k = s * 8 + kg;
-      const float4 a0 = at4(wo + k * WO_PITCH + rt * 8), a1 = at4(wo + k * WO_PITCH + rt * 8 + 4);
-      const float4 s0 = at4(S + k * S_PITCH + ct * 4);
-      const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w}, sv[4] = {s0.x, s0.y, s0.z, s0.w};
-#pragma unroll
-      for (int r = 0; r < 8; ++r)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(av[r], sv[c], acc[r][c]);
+      for (int e = 0; e < 4; ++e) base[e] = uv[(i0 + (e & 1)) * U_PITCH + g + (e >> 1) * 8];
     }
-    // the lanes' sums meet while the rows are dealt out: half of what a lane has left goes at every step
+    if (PAIR) {
+      const int c = tid & (COLS - 1), j = (tid / COLS) * 2;
+      uint32_t term[3];
+      split_two(uv[(CHUNK + j) * U_PITCH + c], uv[(CHUNK + j + 1) * U_PITCH + c], term[0], term[1], term[2]);
 #pragma unroll
-    for (int half = 4; half >= 1; half >>= 1) {
-      const bool upper = kg & half;
-#pragma unroll
-      for (int r = 0; r < half; ++r)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const float keep = upper ? acc[r + half][c] : acc[r][c], give = upper ? acc[r][c] : acc[r + half][c];
-          acc[r][c] = keep + __shfl_xor_sync(0xffffffffu, give, half);
-        }
+      for (int p = 0; p < 3; ++p) *reinterpret_cast<uint32_t*>(VP + (p * COLS + c) * UP_PITCH + j) = term[p];
     }
-    if (reads) {
-      if (writes) put4(out, base.x + acc[0][0], base.y + acc[0][1], base.z + acc[0][2], base.w + acc[0][3]);
+    // [W; O1] S
+    uint32_t end_terms[2][ROWS / 16][3][2];
+    float sum[4] = {0.f, 0.f, 0.f, 0.f}, small[4][4];
+#pragma unroll
+    for (int e = 0; e < 16; ++e) small[e >> 2][e & 3] = 0.f;
+#pragma unroll
+    for (int ks = 0; ks < DK / 16; ++ks) {
+      uint32_t s_terms[3][4];
+      terms(SP, SP_PITCH, ks * 16, s_terms);
+      mma_split<false>(sum, small[ks & 3], s_terms, wo_terms[ks]);
+      // beside it: the update's weights, and (where three stages fit) the next chunk's [W; O1]
+#pragma unroll
+      for (int piece = ks * (ROWS / 32); piece < (ks + 1) * (ROWS / 32); ++piece) {
+        const int nt = piece & 1, e = (piece >> 1) & 1, ke = piece >> 2;
+        const float* const from = ends + (ke * 16 + e * 8 + 2 * t) * END_PITCH + warp * 16 + nt * 8 + g;
+        split_two(from[0], from[END_PITCH], end_terms[nt][ke][0][e], end_terms[nt][ke][1][e], end_terms[nt][ke][2][e]);
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) sum[e] = base[e] + (sum[e] + ((small[0][e] + small[1][e]) + (small[2][e] + small[3][e])));
+    if (warp < 4) {
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        uint32_t term[3];
+        split_two(sum[2 * e], sum[2 * e + 1], term[0], term[1], term[2]);
+#pragma unroll
+        for (int p = 0; p < 3; ++p) *reinterpret_cast<uint32_t*>(UP + (p * COLS + g + 8 * e) * UP_PITCH + i0) = term[p];
+      }
     } else {
-      float* const u = uv + i * S_PITCH + ct * 4;
-      const float4 u0 = at4(u);
-      put4(u, u0.x + acc[0][0], u0.y + acc[0][1], u0.z + acc[0][2], u0.w + acc[0][3]);
+      float* const out = a.out + (start + chunk * CHUNK + i0) * row + (int64_t)h * a.dv + col0 + g;
+      const int left = n - chunk * CHUNK - i0;
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if ((e & 1) < left) out[(e & 1) * row + (e >> 1) * 8] = sum[e];
+      ask(chunk + 1);
     }
+    if (STAGES > 2) asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");    // (the next chunk is here)
     __syncthreads();
+    // the state's decay and update
+    float add[2][4], low[2][2][4];
 #pragma unroll
-    for (int r = 0; r < 8; ++r)
+    for (int e = 0; e < 8; ++e) add[e >> 2][e & 3] = low[0][e >> 2][e & 3] = low[1][e >> 2][e & 3] = 0.f;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) acc[r][c] = 0.f;
-#pragma unroll 2
-    for (int s = 0; s < ROWS / 4; ++s) {
-      const int j = s * 4 + tg;
-      const float4 a0 = at4(ends + j * DK + kt * 4), a1 = at4(ends + j * DK + 64 + kt * 4);
-      const float4 s0 = at4(uv + j * S_PITCH + ct2 * 4);
-      const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w}, sv[4] = {s0.x, s0.y, s0.z, s0.w};
+    for (int ks = 0; ks < ROWS / 16; ++ks) {
+      uint32_t u_terms[3][4];
+      terms(ks < 2 ? UP : VP, UP_PITCH, (ks & 1) * 16, u_terms);
 #pragma unroll
-      for (int r = 0; r < 8; ++r)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(av[r], sv[c], acc[r][c]);
-    }
-#pragma unroll
-    for (int half = 4; half >= 2; half >>= 1) {
-      const bool upper = tg & (half >> 1);
-#pragma unroll
-      for (int r = 0; r < half; ++r)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const float keep = upper ? acc[r + half][c] : acc[r][c], give = upper ? acc[r][c] : acc[r + half][c];
-          acc[r][c] = keep + __shfl_xor_sync(0xffffffffu, give, half * 4);
+      for (int nt = 0; nt < 2; ++nt) {
+        mma_split<true>(add[nt], low[nt][ks & 1], u_terms, end_terms[nt][ks]);
+        if (STAGES > 2) {
+          split_wo(chunk_shared + (chunk + 1) % STAGES * STAGE, ks * 4 + nt * 2);
+          split_wo(chunk_shared + (chunk + 1) % STAGES * STAGE, ks * 4 + nt * 2 + 1);
         }
+      }
     }
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
-      const int k = (tg >> 1) * 64 + kt * 4 + (tg & 1) * 2 + r;
-      const float g = gam[k];
-      float* const s = S + k * S_PITCH + ct2 * 4;
-      const float4 s0 = at4(s);
-      put4(s, fmaf(g, s0.x, acc[r][0]), fmaf(g, s0.y, acc[r][1]), fmaf(g, s0.z, acc[r][2]), fmaf(g, s0.w, acc[r][3]));
-    }
+    for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        // what is lost in g S and in its sum with the first terms joins the small ones: one rounding of the state a chunk
+        const float decay = gam[warp * 16 + nt * 8 + 2 * t + (e & 1)], kept = decay * S[nt][e], lost = fmaf(decay, S[nt][e], -kept);
+        const float whole = kept + add[nt][e], part = whole - kept;
+        S[nt][e] = whole + (((kept - (whole - part)) + (add[nt][e] - part)) + (lost + (low[nt][0][e] + low[nt][1][e])));
+      }
+    publish();
+    if (STAGES == 2) asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
+    if (STAGES == 2) {
+#pragma unroll
+      for (int ks = 0; ks < DK / 16; ++ks) split_wo(chunk_shared + (chunk + 1) % STAGES * STAGE, ks);
+    }
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
-  for (int i = tid; i < COLS * DK; i += RUN_THREADS) state[i] = S[(i % DK) * S_PITCH + i / DK];
+#pragma unroll
+  for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+      *reinterpret_cast<float2*>(state + (g + 8 * e) * DK + warp * 16 + nt * 8 + 2 * t) = make_float2(S[nt][2 * e], S[nt][2 * e + 1]);
 }
 
 template <bool PAIR>
 int launch_chunks(ChunkArgs a, int chunks, int fit, int longs, cudaStream_t stream) {
   constexpr int prepare_bytes = prepare_floats<PAIR>() * (int)sizeof(float);
-  constexpr int run_bytes = (RUN_STAGES<PAIR> * STAGE_FLOATS<PAIR> + DK * S_PITCH) * (int)sizeof(float);
+  constexpr int run_bytes = RUN_BYTES<PAIR>;
   static bool configured = false;
   if (!configured) {
     cudaFuncSetAttribute(delta_chunk_prepare_kernel<PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, prepare_bytes);
@@ -483,7 +590,7 @@ int launch_chunks(ChunkArgs a, int chunks, int fit, int longs, cudaStream_t stre
     vosti_launch(delta_chunk_prepare_kernel<PAIR>, dim3(a.count, a.heads), dim3(256), prepare_bytes, stream, a);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) { vosti_set_error("%s", cudaGetErrorString(e)); return (int)e; }
-    vosti_launch(delta_chunk_run_kernel<PAIR>, dim3(longs, a.heads, a.dv / COLS), dim3(RUN_THREADS), run_bytes, stream, a);
+    vosti_launch(delta_chunk_run_kernel<PAIR>, dim3((unsigned)((int64_t)longs * a.heads * (a.dv / COLS))), dim3(RUN_THREADS), run_bytes, stream, a);
     e = cudaGetLastError();
     if (e != cudaSuccess) { vosti_set_error("%s", cudaGetErrorString(e)); return (int)e; }
   }
@@ -515,6 +622,7 @@ VOSTI_API int vosti_delta_chunks(const float* x, const float* y, const float* de
                 reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(scratch)) & 15) == 0, "delta_chunks: operands start on 16-byte boundaries");
   if (chunks == 0 || longs == 0) return VOSTI_OK;
   VOSTI_REQUIRE(scratch != nullptr && fit > 0, "delta_chunks: no scratch");
+  VOSTI_REQUIRE((int64_t)longs * heads * (dv / COLS) <= 0x7fffffff, "delta_chunks: too many blocks");
   if (fit > chunks) fit = chunks;
   ChunkArgs a = {};
   a.x = x; a.y = y; a.g = decay; a.b = b; a.k = k; a.v = v; a.beta = beta;
