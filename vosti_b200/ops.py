@@ -1850,7 +1850,9 @@ def delta_takes_chunks(layout: dict, heads: int, dv: int, pair: bool) -> bool:
     Where both are close, token by token stays. Measured, tokens and chunks, 16 heads: gated, one request of 64: 24 and
     29, 96: 35 and 33, 256: 89 and 47; two of 128 58 and 49; sixteen of 256 461 and 533. Generalized, one of 96: 37 and 45, 128: 49 and 49;
     two of 128 95 and 65; four of 96 99 and 85; sixteen of 64 208 and 229. 4 heads, one of 128: gated 44 and 27, generalized 45 and 37.
-    (What single tokens cost a chain beside them is put too low: a portion of 64 beside 30 stays with 59 us, chunks take 41.)"""
+    (What single tokens cost a chain beside them is put too low: a portion of 64 beside 30 stays with 59 us, chunks take 41. The
+    chunks' times are those before their products ran on the tensor cores, which take 0.65 to 0.7 of a turn: the line lies to the
+    side of token by token.)"""
     launch, chain, long, share, each = (1.4, 0.34, 0.258, 0.174, 1.04) if pair else (1.2, 0.335, 0.254, 0.089, 1.16)
     width = heads * dv / 2048
     rounds = layout["longs"] * width                     # blocks of the chunks' run, in 128
