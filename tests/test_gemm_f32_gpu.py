@@ -21,10 +21,10 @@ def draw(seed, rows, n, k):
 
 def bound(x, w):
     """Per output, over the sum of magnitudes: a rounding of the running sum per 64 k and K segment, at most four truncations (two
-    roundings' worth each) of a 64-k sum, 5 K / 16 truncations of sums 2^-6 as large (two terms below 2^-7), and the terms left out: m and
-    l are below 2^-7 and 2^-15 of their operand, so m l + l m + l l is below 2^-21, eight roundings."""
+    roundings' worth each) of a 64-k sum, 7 K / 16 truncations of sums 2^-6 as large (two terms below 2^-7), and the term left out: l is
+    below 2^-15 of its operand, so l l is below 2^-30, a fraction of one rounding."""
     k = x.shape[1]
-    steps = -(-k // 64) + 8 + 2 * 4 + 2 * (5 * k / 16) * 2.0 ** -6 + 9
+    steps = -(-k // 64) + 8 + 2 * 4 + 2 * (7 * k / 16) * 2.0 ** -6 + 1
     return steps * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
 
 
@@ -44,6 +44,24 @@ def test_against_float64_and_rows_alone(status, rows, n, k):
     xs, ws = torch.empty(rows * k + 1, device=DEV), torch.empty(n * k + 3, device=DEV)
     xs[1:], ws[3:] = x.view(-1), w.view(-1)
     assert torch.equal(ops.gemm_f32(xs[1:].view(rows, k), ws[3:].view(n, k), status), y)
+
+
+@pytest.mark.parametrize("n,k", [(200, 4096), (4096, 1024), (25000, 1024)])          # eight, four and one K segments
+@pytest.mark.parametrize("adjacent", [True, False])
+def test_rows_of_few_products_are_as_near_as_the_chain(status, n, k, adjacent):
+    """One to sixteen products a row, next to one another or anywhere. With one the result is the product rounded once, as the chain's:
+    it may differ by l l (2^-30 of the product, mean 2^-32) and a truncation of the small sum (2^-31) only, 2^-6 of a rounding."""
+    for count in (1, 2, 3, 4, 6, 8, 16):
+        gen = torch.Generator(device=DEV).manual_seed(count)
+        w, x = torch.randn(n, k, generator=gen, device=DEV), torch.zeros(70, k, device=DEV)
+        if adjacent:
+            places = torch.randint(0, k - count + 1, (70, 1), generator=gen, device=DEV) + torch.arange(count, device=DEV)
+        else:
+            places = torch.rand(70, k, generator=gen, device=DEV).argsort(1)[:, :count]
+        x.scatter_(1, places, torch.randn(70, count, generator=gen, device=DEV))
+        want = x.double() @ w.double().T
+        error = lambda y: (y.double() - want).norm().item()
+        assert error(ops.gemm_f32(x, w, status)) <= (1 + 2.0 ** -6) * error(ops.gemm_simt(x, w, status)), count
 
 
 def test_positive_sums_and_small_and_large_operands(status):

@@ -1,14 +1,16 @@
 // float32 matrix product on the 5th-generation tensor cores:
 //   Y[t, n] = sum_k X[t, k] * W[n, k]        X, W, Y float32 (W in [out, in] layout, no bias)
 // Every operand is split into three bfloat16 terms, x = h + m + l, each the upper 16 bits of what the terms before it leave
-// (8 + 8 + 8 bits: nothing of a float32 is lost), and a product is the six terms of order up to 2^-16:
-// h h + (h m + m h) + (h l + m m + l h); what is left out is below 2^-21 of |x w| and 2^-24 in the mean. Splitting operands this way, and
+// (8 + 8 + 8 bits: nothing of a float32 is lost), and a product is the eight terms of order up to 2^-24:
+// h h + (h m + m h) + (h l + m m + l h) + (m l + l m); only l l is left out, below 2^-30 of |x w| (without m l and l m a row of one
+// product was 6e-8 from 64 bits instead of the 2.5e-8 of one rounding). Splitting operands this way, and
 // taking the tensor core's sums out before their truncation adds up, is Ootomo and Yokota, "Recovering single
 // precision accuracy from Tensor Cores while surpassing the FP32 theoretical peak performance" (2022); here h h is summed
-// on the tensor core over 64 k only and then added, rounded to nearest, to a sum in registers, while the five small products,
-// 2^-7 of it, stay in an accumulator of their own to the end. Error against 64 bits (2-norm, normal operands): 1.4e-7 at K = 2,048,
-// 1.7e-7 (four segments) and 2.8e-7 (one) at 4,096, 2.5e-7 at 12,288, where gemm_simt.cu's chain of multiply-adds has
-// 8.1e-7, 1.1e-6 and 2.0e-6.
+// on the tensor core over 64 k only and then added, rounded to nearest, to a sum in registers, while the seven small products,
+// 2^-7 of it, stay in an accumulator of their own to the end (over all segments, so that a row of few products is not rounded once
+// a segment). Error against 64 bits (2-norm, normal operands): 1.1e-7 at K = 2,048,
+// 1.4e-7 (four segments) and 2.9e-7 (one) at 4,096, 2.4e-7 at 12,288, where gemm_simt.cu's chain of multiply-adds has
+// 8.1e-7, 1.1e-6 and 2.0e-6; rows of one product 2.5e-8 and of eight 2.9e-8, the chain 2.5e-8 and 5.3e-8.
 //
 // Features on M = 128, tokens on N; K in `segments` of whole 64s, one CTA of a cluster each, summed in their order
 // through distributed shared memory. The segments are chosen from (N, K) alone, the order of the products inside a
@@ -140,9 +142,9 @@ __device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, u
 // TOK tokens on N. One thread brings both operands' words of KS k into a ring of RAW stages by TMA (zeros beyond a matrix), eight
 // warps split them, the weights into three planes in tensor memory (a thread: half a feature's k), the tokens into three in
 // shared memory, and between stages take the tensor core's 64-k sums out (a thread: one feature, TOK / 2 tokens); a ninth warp
-// issues the MMAs. The bound is shared memory: with the weights' planes there too the six products read them again (10 KB for
-// each of twelve MMAs a stage of 192 tokens): us for 24,576 x 4,096, 1 / 64 / 384 rows, 152 / 283 / 570 so, 93 / 162 / 441 now,
-// gemm_simt.cu 155 / 434 / 1,689. The roles share no code from where they part (their registers differ): the warps that bring
+// issues the MMAs. The bound is shared memory: with the weights' planes there too every product reads them again (10 KB for
+// each MMA of 192 tokens; six products, us for 24,576 x 4,096, 1 / 64 / 384 rows: 152 / 283 / 570 so, 91 / 161 / 432 as it is). The
+// eight products take 93 / 162 / 472, gemm_simt.cu 154 / 435 / 1,692. The roles share no code from where they part (their registers differ): the warps that bring
 // and issue end after their last request, the eight do the rest.
 // WORDS: every row starts on a whole word; otherwise the eight warps read the matrices themselves, element by element.
 template <int TOK, int KS, int STAGES, int RAW, int BLOCKS, bool WORDS>
@@ -237,7 +239,9 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
         if (elect_one()) {
 #pragma unroll
           for (int q = 0; q < KS / 16; ++q) {
-            umma_bf16_ts(tmem_small, al + 8 * q, bh + 2 * q, idesc, st > 0 || q > 0);
+            umma_bf16_ts(tmem_small, al + 8 * q, bm + 2 * q, idesc, st > 0 || q > 0);
+            umma_bf16_ts(tmem_small, am + 8 * q, bl + 2 * q, idesc, 1u);
+            umma_bf16_ts(tmem_small, al + 8 * q, bh + 2 * q, idesc, 1u);
             umma_bf16_ts(tmem_small, am + 8 * q, bm + 2 * q, idesc, 1u);
             umma_bf16_ts(tmem_small, ah + 8 * q, bl + 2 * q, idesc, 1u);
             umma_bf16_ts(tmem_small, am + 8 * q, bh + 2 * q, idesc, 1u);
@@ -336,11 +340,8 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
       if (WORDS) mbar_arrive(smem_u32(&raw_empty[st % RAW]));
     }
   }
-  if (ok) {
-    tc_fence_after();
-    add_columns<COLS>(tmem_small + my_columns, acc);
-    tc_fence_before();
-  }
+  tc_fence_after();
+  if (ok && segments == 1) add_columns<COLS>(tmem_small + my_columns, acc);
 
   auto store = [&](int t, int f, float v) {
     if (t0 + t >= rows || f0 + f >= n) return;
@@ -355,26 +356,34 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
 #pragma unroll
     for (int i = 0; i < COLS; ++i) store(half * COLS + i, quarter * 32 + lane, acc[i]);
   } else {
-    // every MMA that read the ring is complete
+    // every MMA that read the ring is complete: its place takes the sums, then the small products
     float* const part = reinterpret_cast<float*>(smem);
+    float* const mine_at = part + half * COLS * FT + quarter * 32 + lane;
 #pragma unroll
-    for (int i = 0; i < COLS; ++i) part[(half * COLS + i) * FT + quarter * 32 + lane] = acc[i];
+    for (int i = 0; i < COLS; ++i) {
+      mine_at[i * FT] = acc[i];
+      acc[i] = 0.f;
+    }
+    if (ok) add_columns<COLS>(tmem_small + my_columns, acc);
+#pragma unroll
+    for (int i = 0; i < COLS; ++i) mine_at[(TOK + i) * FT] = acc[i];
     f32_cluster_sync();
     const int mine = (int)f32_cluster_rank();              // = segment
     const int lo = TOK * mine / segments, hi = TOK * (mine + 1) / segments;
     for (int word = threadIdx.x; word < (hi - lo) * (FT / 4); word += WORKERS) {
       const int t = lo + word / (FT / 4), f = word % (FT / 4) * 4;
       if (t0 + t >= rows) break;
-      const uint32_t at = smem_u32(&part[t * FT + f]);
-      float4 v = load_cluster4(at, 0);
+      const uint32_t at = smem_u32(&part[t * FT + f]), small_at = smem_u32(&part[(TOK + t) * FT + f]);
+      float4 v = load_cluster4(at, 0), low = load_cluster4(small_at, 0);
       for (int r = 1; r < segments; ++r) {
-        const float4 u = load_cluster4(at, r);
+        const float4 u = load_cluster4(at, r), e = load_cluster4(small_at, r);
         v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
+        low.x += e.x; low.y += e.y; low.z += e.z; low.w += e.w;
       }
-      store(t, f, v.x);
-      store(t, f + 1, v.y);
-      store(t, f + 2, v.z);
-      store(t, f + 3, v.w);
+      store(t, f, v.x + low.x);
+      store(t, f + 1, v.y + low.y);
+      store(t, f + 2, v.z + low.z);
+      store(t, f + 3, v.w + low.w);
     }
   }
   tc_fence_before();
@@ -413,7 +422,8 @@ bool f32_map(CUtensorMap* map, const float* base, int64_t rows, int k, int box_r
 template <int TOK, int KS, int STAGES, int RAW, int BLOCKS, bool WORDS>
 int launch_f32(const float* x, const float* w, float* y, int rows, int n, int k, unsigned* status, cudaStream_t stream) {
   constexpr int RINGS = STAGES * 3 * TOK * KS * 2 + (WORDS ? RAW * (FT + TOK) * KS * 4 : 0);
-  constexpr int SMEM = (RINGS > TOK * FT * 4 ? RINGS : TOK * FT * 4) + 1024;       // (the rings' place holds a segment's sums at the end)
+  constexpr int SUMS = 2 * TOK * FT * 4;                   // a segment's, in the rings' place at the end
+  constexpr int SMEM = (RINGS > SUMS ? RINGS : SUMS) + 1024;
   auto kernel = gemm_f32_kernel<TOK, KS, STAGES, RAW, BLOCKS, WORDS>;
   static const cudaError_t raised = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
   if (raised != cudaSuccess) {
