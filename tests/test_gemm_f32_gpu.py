@@ -72,6 +72,27 @@ def test_positive_sums_and_small_and_large_operands(status):
         assert rel(ops.gemm_f32(a, b, status)) <= rel(ops.gemm_simt(a, b, status))
 
 
+@pytest.mark.parametrize("rows,n,k", [(70, 200, 2048), (130, 20000, 1024), (20, 4096, 1024)])         # eight, one and four K segments
+@pytest.mark.parametrize("a,b", [(-70, -70), (-75, -68), (-105, 60), (-110, 60), (-118, 60), (-122, 70), (-130, 90), (-140, 100), (-126, 10),
+                                 (70, -122), (100, -140), (31, -112)])
+def test_operands_whose_last_bits_no_term_holds(status, rows, n, k, a, b):
+    """A third of the rows of x times 2^a, a half of w's times 2^b: the error of each of the four blocks is no larger than the chain's, a row
+    alone has the same bits, and zeros stay zeros."""
+    x, w = draw(rows + k, rows, n, k)
+    x[::3], w[::2] = (x[::3].double() * 2.0 ** a).float(), (w[::2].double() * 2.0 ** b).float()
+    x[4] = 0
+    want = x.double() @ w.double().T
+    y, chain = ops.gemm_f32(x, w, status), ops.gemm_simt(x, w, status)
+    third, odd = torch.arange(rows, device=DEV) % 3 == 0, torch.arange(n, device=DEV) % 2 == 0
+    for i in (third, ~third):
+        for j in (odd, ~odd):
+            error = lambda t: (t.double() - want)[i][:, j].norm().item()
+            assert error(y) <= error(chain), (error(y), error(chain))
+    assert not y[4].any() and status.item() == 0
+    for t in (0, 1):
+        assert torch.equal(ops.gemm_f32(x[t:t + 1], w, status)[0], y[t])
+
+
 def test_operands_that_are_not_finite(status):
     x, w = draw(6, 40, 200, 512)
     x[3, 7], x[5, 9], x[6, :], w[10, 3], x[7, 11], w[:, 11] = float("inf"), float("nan"), -3.4028234e38, float("-inf"), 3.4028e38, 0.25

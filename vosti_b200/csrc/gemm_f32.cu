@@ -18,9 +18,10 @@
 // rows beside it (the reference chooses tiles from (N, K) only for the same reason:
 // kernels/triton_kernels/matmul.py:33-73, 95-147).
 //
-// An operand that is infinite or not a number makes its outputs non-finite here (an infinity leaves inf - inf), and terms of
-// operands near the smallest normal number lose their low bits; outputs that are not finite, or so small that this could show
-// (below 2^-80 and not zero), are taken again as a chain of float32 multiply-adds.
+// Operands are split times 2^16: bfloat16 ends at 2^-133, so the last terms of what lies below 2^-110 would lose bits, whatever the size of
+// the output; scaled, the smallest float32 is 2^-133 and no operand loses any. The sums are exact powers of two apart and are scaled
+// back at the end. Outputs that are not finite then (an infinite operand leaves inf - inf, an operand from 2^112 or a sum from 2^96 on
+// overflows) go to a list that all threads work off at the end, as chains of float32 multiply-adds of the operands as they are.
 #include "tcgen05.cuh"
 #include "tensor_map.cuh"
 
@@ -112,10 +113,12 @@ __device__ __forceinline__ float4 load_elements(const float* row, int kk, int k)
   if (kk + 3 < k) v.w = row[kk + 3];
   return v;
 }
-// The three terms of four values, two values a word. A term is the upper half of what the terms before it leave (truncated: whole
+constexpr float SCALE = 65536.f, BACK = 1.f / SCALE / SCALE;
+// The three terms of four values times SCALE, two values a word. A term is the upper half of what the terms before it leave (truncated: whole
 // words of integer and multiply-add instructions, where a rounding conversion takes its unit several cycles), the last one is exact.
-__device__ __forceinline__ void split_four(float4 v, uint32_t* h, uint32_t* m, uint32_t* l) {
-  auto upper = [](float x) { return __uint_as_float(__float_as_uint(x) & 0xffff0000u); };
+__device__ __forceinline__ void split_four(float4 x, uint32_t* h, uint32_t* m, uint32_t* l) {
+  const float4 v = make_float4(x.x * SCALE, x.y * SCALE, x.z * SCALE, x.w * SCALE);
+  auto upper = [](float e) { return __uint_as_float(__float_as_uint(e) & 0xffff0000u); };
   auto both = [](float lo, float hi) { return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632); };
   const float4 a = make_float4(v.x - upper(v.x), v.y - upper(v.y), v.z - upper(v.z), v.w - upper(v.w));
   const float4 b = make_float4(a.x - upper(a.x), a.y - upper(a.y), a.z - upper(a.z), a.w - upper(a.w));
@@ -170,6 +173,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
   __shared__ __align__(8) uint64_t empty_bar[STAGES];       // its MMAs are complete
   __shared__ __align__(8) uint64_t sum_free;                // eight warps: the 64-k sum has been taken out
   __shared__ uint32_t tmem_base_holder;
+  __shared__ int again;                                     // outputs on the list
   __shared__ volatile int abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -181,6 +185,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
 
   if (threadIdx.x == 0) {
     abort_flag = 0;
+    again = 0;
     for (int s = 0; s < RAW; ++s) {
       mbar_init(smem_u32(&raw_full[s]), 1);
       mbar_init(smem_u32(&raw_empty[s]), WORKERS / 32);
@@ -343,22 +348,20 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
   tc_fence_after();
   if (ok && segments == 1) add_columns<COLS>(tmem_small + my_columns, acc);
 
+  uint16_t* const list = reinterpret_cast<uint16_t*>(segments == 1 ? smem : smem + 2 * TOK * FT * 4);     // outputs to be taken again
   auto store = [&](int t, int f, float v) {
     if (t0 + t >= rows || f0 + f >= n) return;
-    if (!(fabsf(v) <= 3.402823466e+38f) || (fabsf(v) < 8.2718061e-25f && v != 0.f)) {       // 2^-80
-      v = 0.f;
-      const float *xr = x + (int64_t)(t0 + t) * k, *wr = w + (int64_t)(f0 + f) * k;
-      for (int kk = 0; kk < k && v == v; ++kk) v = fmaf(xr[kk], wr[kk], v);
-    }
-    y[(int64_t)(t0 + t) * n + f0 + f] = v;
+    if (fabsf(v) <= 3.402823466e+38f) y[(int64_t)(t0 + t) * n + f0 + f] = v * BACK;
+    else list[atomicAdd(&again, 1)] = (uint16_t)(t * FT + f);
   };
   if (segments == 1) {
+    workers_sync();                                        // (all have split their last words: the rings' place is free)
 #pragma unroll
-    for (int i = 0; i < COLS; ++i) store(half * COLS + i, quarter * 32 + lane, acc[i]);
+    for (int i = 0; i < COLS; ++i) store(half * COLS + i, feature, acc[i]);
   } else {
     // every MMA that read the ring is complete: its place takes the sums, then the small products
     float* const part = reinterpret_cast<float*>(smem);
-    float* const mine_at = part + half * COLS * FT + quarter * 32 + lane;
+    float* const mine_at = part + half * COLS * FT + feature;
 #pragma unroll
     for (int i = 0; i < COLS; ++i) {
       mine_at[i * FT] = acc[i];
@@ -392,6 +395,15 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
     for (int i = 0; i < 64; ++i) __nanosleep(1000);
     workers_sync();
   }
+  for (int i = threadIdx.x; i < again; i += WORKERS) {
+    const int t = t0 + list[i] / FT, f = f0 + list[i] % FT;
+    if (t >= rows || f >= n) continue;                     // (the list's place after a wait that gave up)
+    const float *xr = x + (int64_t)t * k, *wr = w + (int64_t)f * k;
+    float v = 0.f;
+#pragma unroll 8
+    for (int kk = 0; kk < k; ++kk) v = fmaf(xr[kk], wr[kk], v);
+    y[(int64_t)t * n + f] = v;
+  }
   if (segments > 1) f32_cluster_sync();                     // nobody reads this CTA's sums after this
   if (warp == 0) {
     tc_fence_after();
@@ -422,7 +434,7 @@ bool f32_map(CUtensorMap* map, const float* base, int64_t rows, int k, int box_r
 template <int TOK, int KS, int STAGES, int RAW, int BLOCKS, bool WORDS>
 int launch_f32(const float* x, const float* w, float* y, int rows, int n, int k, unsigned* status, cudaStream_t stream) {
   constexpr int RINGS = STAGES * 3 * TOK * KS * 2 + (WORDS ? RAW * (FT + TOK) * KS * 4 : 0);
-  constexpr int SUMS = 2 * TOK * FT * 4;                   // a segment's, in the rings' place at the end
+  constexpr int SUMS = 2 * TOK * FT * 4 + TOK * FT;        // a segment's, and a list of its share of the outputs, in the rings' place at the end
   constexpr int SMEM = (RINGS > SUMS ? RINGS : SUMS) + 1024;
   auto kernel = gemm_f32_kernel<TOK, KS, STAGES, RAW, BLOCKS, WORDS>;
   static const cudaError_t raised = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
@@ -468,9 +480,9 @@ VOSTI_API int vosti_gemm_f32(const float* x, const float* w, float* y, int rows,
   // cluster, two of them an SM are (24,576 x 4,096, 1 row: 93 and 133, 64 rows: 162 and 185; 2,048 x 2,048: 11 and 17, 17 and 23).
   const bool one_round = segments <= 4 && ctas(rows) <= 140;
   if (rows <= 32 && one_round) VOSTI_F32(32, 64, 2, 3, 1);
-  if (rows <= 32) VOSTI_F32(32, 64, 2, 2, 1);
+  if (rows <= 32) VOSTI_F32(32, 64, 2, 2, 2);
   if (rows <= 64 && one_round) VOSTI_F32(64, 64, 2, 2, 1);
-  if (rows <= 64) VOSTI_F32(64, 32, 2, 3, 1);
+  if (rows <= 64) VOSTI_F32(64, 32, 2, 3, 2);
   // A tile of 192 tokens takes about 1.4 times as long as one of 128: the fewer rounds of CTAs decide (us, 384 rows: 24,576 x 4,096 504
   // and 441, 6,144 x 4,096 149 and 171, 4,096 x 4,096 101 and 104).
   const int at_once = segments > 1 ? 140 : 148;
