@@ -173,6 +173,12 @@ def test_products_of_few_tiles_split_where_that_is_faster(lib):
         assert lib.vosti_gemm_tc_pair_splits(tokens, features, k) == 1, (tokens, features, k)
 
 
+def test_float32_tiles_never_ask_for_more_tensor_memory_than_an_sm_has(lib):
+    """CTAs of a cluster wait for their tensor memory without a limit: shared memory keeps as many of them on an SM as it has columns for."""
+    columns = [lib.vosti_gemm_f32_columns_an_sm(tile) for tile in range(6)]
+    assert all(0 < c <= 512 for c in columns) and lib.vosti_gemm_f32_columns_an_sm(6) == -1, columns
+
+
 def test_weight_bytes_of_a_decode_step_in_closed_form():
     """What bench.py counts as the weights a decode step must read: every tensor the model
     expects except the embedding table (read by rows), two bytes each. For the 8B sizes that is

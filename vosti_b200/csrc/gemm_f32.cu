@@ -35,6 +35,21 @@ constexpr int WORKERS = 256;             // threads that load, split and sum
 template <int TOK> constexpr bool SPLITS_REGISTERS = TOK > 128;
 template <int TOK> constexpr int THREADS = SPLITS_REGISTERS<TOK> ? WORKERS + 128 : WORKERS + 64;
 
+// What a CTA of a tile takes of its SM. CTAs of a cluster wait for their tensor memory and for one another without a limit, so
+// no more of them may be on an SM than tensor memory has columns for (512), whatever registers a build happens to give
+// them: shared memory (228 KB an SM, 1 KB of it with every CTA) is padded until that many fit.
+template <int TOK, int KS, int STAGES, int RAW, bool WORDS>
+struct F32Tile {
+  static constexpr int USED_COLS = 2 * TOK + STAGES * 3 * (KS / 2);        // the sums of 64 k, the small products, the weights' planes
+  static constexpr int COLS = USED_COLS <= 256 ? 256 : 512;
+  static constexpr int RINGS = STAGES * 3 * TOK * KS * 2 + (WORDS ? RAW * (FT + TOK) * KS * 4 : 0);
+  static constexpr int SUMS = 2 * TOK * FT * 4 + TOK * FT;                 // a segment's, and a list of its share of the outputs, in the rings' place at the end
+  static constexpr int SM_BYTES = 228 * 1024, FEWEST = SM_BYTES / (512 / COLS + 1);                        // (one CTA more does not fit)
+  static constexpr int NEEDED = (RINGS > SUMS ? RINGS : SUMS) + 1024;
+  static constexpr int SMEM = NEEDED > FEWEST ? NEEDED : FEWEST;
+  static constexpr int COLS_AN_SM = SM_BYTES / (SMEM + 1024) * COLS;       // that its CTAs may ask for
+};
+
 __device__ __forceinline__ uint32_t f32_cluster_rank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -161,9 +176,9 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
   constexpr int BW = TOK * KS / 4 / WORKERS;                // token words a thread splits per stage
   constexpr int ROWS_PER = WORKERS / (KS / 4);              // rows between a thread's words
   constexpr int COLS = TOK / 2;
-  constexpr int USED_COLS = 2 * TOK + STAGES * 3 * A_COLS;  // the sums of 64 k, the small products, the weights' planes
-  constexpr int TMEM_COLS = USED_COLS <= 256 ? 256 : 512;
-  static_assert(ROWS_PER % 8 == 0 && TOK * KS / 4 % WORKERS == 0 && USED_COLS <= 512 && TMEM_COLS * BLOCKS <= 512, "tile");
+  using Tile = F32Tile<TOK, KS, STAGES, RAW, WORDS>;
+  constexpr int TMEM_COLS = Tile::COLS;
+  static_assert(ROWS_PER % 8 == 0 && TOK * KS / 4 % WORKERS == 0 && Tile::USED_COLS <= 512 && TMEM_COLS * BLOCKS <= 512 && Tile::COLS_AN_SM <= 512, "tile");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* const smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   // [RAW] stages: the weights' [KS / 32][128 features][32] with the 128-byte swizzle, the tokens' [TOK][KS]
@@ -433,9 +448,7 @@ bool f32_map(CUtensorMap* map, const float* base, int64_t rows, int k, int box_r
 
 template <int TOK, int KS, int STAGES, int RAW, int BLOCKS, bool WORDS>
 int launch_f32(const float* x, const float* w, float* y, int rows, int n, int k, unsigned* status, cudaStream_t stream) {
-  constexpr int RINGS = STAGES * 3 * TOK * KS * 2 + (WORDS ? RAW * (FT + TOK) * KS * 4 : 0);
-  constexpr int SUMS = 2 * TOK * FT * 4 + TOK * FT;        // a segment's, and a list of its share of the outputs, in the rings' place at the end
-  constexpr int SMEM = (RINGS > SUMS ? RINGS : SUMS) + 1024;
+  constexpr int SMEM = F32Tile<TOK, KS, STAGES, RAW, WORDS>::SMEM;
   auto kernel = gemm_f32_kernel<TOK, KS, STAGES, RAW, BLOCKS, WORDS>;
   static const cudaError_t raised = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
   if (raised != cudaSuccess) {
@@ -457,7 +470,20 @@ int launch_f32(const float* x, const float* w, float* y, int rows, int n, int k,
   return VOSTI_OK;
 }
 
+template <int TOK, int KS, int STAGES, int RAW>
+constexpr int f32_cols_an_sm() {
+  const int words = F32Tile<TOK, KS, STAGES, RAW, true>::COLS_AN_SM, elements = F32Tile<TOK, KS, STAGES, RAW, false>::COLS_AN_SM;
+  return words > elements ? words : elements;
+}
+
 }  // namespace
+
+// Tensor memory columns that the CTAs of a tile (0 .. 5, -1 beyond) may ask for on one SM.
+VOSTI_API int vosti_gemm_f32_columns_an_sm(int tile) {
+  constexpr int of[] = {f32_cols_an_sm<32, 64, 2, 3>(), f32_cols_an_sm<32, 64, 2, 2>(), f32_cols_an_sm<64, 64, 2, 2>(),
+                        f32_cols_an_sm<64, 32, 2, 3>(), f32_cols_an_sm<128, 64, 2, 2>(), f32_cols_an_sm<192, 32, 2, 2>()};
+  return tile >= 0 && tile < (int)(sizeof(of) / sizeof(of[0])) ? of[tile] : -1;
+}
 
 // Whether a float32 [n, k] weight is this kernel's (a rule of the sizes only, so that a row's bits stay its own). Below, a chain of
 // multiply-adds is as fast or faster for few rows (us here / there, 1 and 384 rows: 2,048 x 512 9 / 5 and 17 / 36; 512 x 1,024 8 / 7
