@@ -173,6 +173,15 @@ def test_products_of_few_tiles_split_where_that_is_faster(lib):
         assert lib.vosti_gemm_tc_pair_splits(tokens, features, k) == 1, (tokens, features, k)
 
 
+def test_float32_weights_go_to_the_product_whose_single_row_was_faster(lib):
+    """Weights on both sides of the line between the tensor cores and the chain of multiply-adds; rows that do not start on whole words stay."""
+    for n, k in [(16, 2048), (2048, 2048), (2048, 2304), (160, 4096), (4096, 1024), (4096, 1536), (8192, 1024), (4096, 4096), (24576, 4096), (4096, 12288)]:
+        assert lib.vosti_gemm_f32_supported(n, k), (n, k)
+    for n, k in [(512, 1024), (1024, 1024), (3072, 1024), (1024, 1536), (2048, 1920), (3072, 1920), (4096, 512), (8, 4096), (4096, 4098), (2048, 2049),
+                 (512, 1026)]:
+        assert not lib.vosti_gemm_f32_supported(n, k), (n, k)
+
+
 def test_float32_tiles_never_ask_for_more_tensor_memory_than_an_sm_has(lib):
     """CTAs of a cluster wait for their tensor memory without a limit: shared memory keeps as many of them on an SM as it has columns for."""
     columns = [lib.vosti_gemm_f32_columns_an_sm(tile) for tile in range(6)]

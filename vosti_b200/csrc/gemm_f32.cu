@@ -161,8 +161,8 @@ __device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, u
 // warps split them, the weights into three planes in tensor memory (a thread: half a feature's k), the tokens into three in
 // shared memory, and between stages take the tensor core's 64-k sums out (a thread: one feature, TOK / 2 tokens); a ninth warp
 // issues the MMAs. The bound is shared memory: with the weights' planes there too every product reads them again (10 KB for
-// each MMA of 192 tokens; six products, us for 24,576 x 4,096, 1 / 64 / 384 rows: 152 / 283 / 570 so, 91 / 161 / 432 as it is). The
-// eight products take 93 / 162 / 472, gemm_simt.cu 154 / 435 / 1,692. The roles share no code from where they part (their registers differ): the warps that bring
+// each MMA of 192 tokens; at first, six products, us for 24,576 x 4,096, 1 / 64 / 384 rows: 152 / 283 / 570 so, 91 / 161 / 432 as it is). The
+// eight products of scaled operands take 99 / 169 / 494, gemm_simt.cu 155 / 435 / 1,699. The roles share no code from where they part (their registers differ): the warps that bring
 // and issue end after their last request, the eight do the rest.
 // WORDS: every row starts on a whole word; otherwise the eight warps read the matrices themselves, element by element.
 template <int TOK, int KS, int STAGES, int RAW, int BLOCKS, bool WORDS>
@@ -485,10 +485,12 @@ VOSTI_API int vosti_gemm_f32_columns_an_sm(int tile) {
   return tile >= 0 && tile < (int)(sizeof(of) / sizeof(of[0])) ? of[tile] : -1;
 }
 
-// Whether a float32 [n, k] weight is this kernel's (a rule of the sizes only, so that a row's bits stay its own). Below, a chain of
-// multiply-adds is as fast or faster for few rows (us here / there, 1 and 384 rows: 2,048 x 512 9 / 5 and 17 / 36; 512 x 1,024 8 / 7
-// and 15 / 30, 256 x 2,048 9 / 11 and 15 / 39).
-VOSTI_API int vosti_gemm_f32_supported(int n, int k) { return n >= 16 && k >= 1024; }
+// Whether a float32 [n, k] weight is this kernel's (a rule of the sizes only, so that a row's bits stay its own): where one row is no slower
+// than gemm_simt.cu's chain of multiply-adds; with more rows it is faster from 8 to 16 on everywhere. us, here / there, one row: 1,024 x 1,024
+// 7.7 / 6.6, 3,072 x 1,024 9.2 / 7.4, 4,096 x 1,024 9.9 / 9.8, 8,192 x 1,024 13.6 / 13.9, 2,048 x 1,920 12.0 / 11.2, 4,096 x 1,536 12.0 / 13.2,
+// 16 x 2,048 7.6 / 10.2, 2,048 x 2,048 10.5 / 11.3, 2,048 x 2,304 11.8 / 12.2. Rows that do not start on whole words are read element
+// by element: 4,096 x 4,098 60 / 39.
+VOSTI_API int vosti_gemm_f32_supported(int n, int k) { return n >= 16 && k % 4 == 0 && (k >= 2048 || (k >= 1024 && n >= 4096)); }
 
 // x: [rows, k]; w: [n, k]; y: [rows, n], all float32.
 VOSTI_API int vosti_gemm_f32(const float* x, const float* w, float* y, int rows, int n, int k, unsigned* status, cudaStream_t stream) {
@@ -502,15 +504,15 @@ VOSTI_API int vosti_gemm_f32(const float* x, const float* w, float* y, int rows,
   const int tiles = (n + FT - 1) / FT, segments = f32_segments(n, k);
   auto ctas = [&](int tok) { return (int64_t)tiles * segments * ((rows + tok - 1) / tok); };
   // Clusters of up to four CTAs find some 140 SMs at one CTA each. Where these take them all at once, a deeper ring of whole 64s is the
-  // fastest (us, 4,096 x 12,288, 1 row: 54, two stages 61, stages of 32 k 88; 64 rows: 74 and 111); with more CTAs, or eight a
-  // cluster, two of them an SM are (24,576 x 4,096, 1 row: 93 and 133, 64 rows: 162 and 185; 2,048 x 2,048: 11 and 17, 17 and 23).
+  // fastest (us, 4,096 x 12,288, 1 row: 54, two stages 73, stages of 32 k 108; 64 rows: 77 and 128); with more CTAs, or eight a
+  // cluster, two of them an SM are (24,576 x 4,096, 1 row: 101 and 136, 64 rows: 176 and 194; 2,048 x 2,048: 11 and 17, 19 and 27).
   const bool one_round = segments <= 4 && ctas(rows) <= 140;
   if (rows <= 32 && one_round) VOSTI_F32(32, 64, 2, 3, 1);
   if (rows <= 32) VOSTI_F32(32, 64, 2, 2, 2);
   if (rows <= 64 && one_round) VOSTI_F32(64, 64, 2, 2, 1);
   if (rows <= 64) VOSTI_F32(64, 32, 2, 3, 2);
-  // A tile of 192 tokens takes about 1.4 times as long as one of 128: the fewer rounds of CTAs decide (us, 384 rows: 24,576 x 4,096 504
-  // and 441, 6,144 x 4,096 149 and 171, 4,096 x 4,096 101 and 104).
+  // A tile of 192 tokens takes about 1.4 times as long as one of 128: the fewer rounds of CTAs decide (us, 384 rows: 24,576 x 4,096 546
+  // and 486, 6,144 x 4,096 164 and 186, 4,096 x 4,096 109 and 113).
   const int at_once = segments > 1 ? 140 : 148;
   if (10 * ((ctas(128) + at_once - 1) / at_once) <= 14 * ((ctas(192) + at_once - 1) / at_once)) VOSTI_F32(128, 64, 2, 2, 1);
   VOSTI_F32(192, 32, 2, 2, 1);

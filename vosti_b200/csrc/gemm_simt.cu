@@ -1,6 +1,6 @@
 // Plain matrix product on the CUDA cores with true float32 arithmetic:
 //   Y[t, n] = sum_k X[row(t), k] * W[n, k]        (W in [out, in] layout, no bias)
-// It is the float32 product of weights of K < 1,024 (gemm_f32.cu has the others) and the fallback of the bfloat16 path for
+// It is the float32 product of weights that gemm_f32.cu does not take (`vosti_gemm_f32_supported`) and the fallback of the bfloat16 path for
 // operand types or sizes the tensor-core kernel refuses. Each output is one thread's
 // sequential fused multiply-add chain over k = 0..K-1, so a row's value never depends
 // on the other rows of the launch (the reference's matmul has the same property by

@@ -4,7 +4,7 @@ bfloat16 x bfloat16 goes to the tensor-core kernel when it takes the sizes, floa
 tensor-core kernel that splits every operand into three bfloat16 terms (float32 results, no reduced precision);
 every other combination (a 32-bit weight under bfloat16 serving, sizes those kernels refuse) goes to the
 CUDA-core kernel with float32 arithmetic.
-The choice depends on types and on (N, K) only, never on the number of rows.
+The choice depends on the weight only (its type, (N, K) and, in float32, where it starts), never on the number of rows.
 """
 from __future__ import annotations
 
@@ -25,7 +25,7 @@ def uses_tensor_cores(x_dtype: torch.dtype, w) -> bool:
 
 
 def uses_split_float32(x_dtype: torch.dtype, w) -> bool:
-    return (x_dtype == torch.float32 and w.dtype == torch.float32 and w.is_cuda
+    return (x_dtype == torch.float32 and w.dtype == torch.float32 and w.is_cuda and w.data_ptr() % 16 == 0
             and ops.gemm_f32_supported(w.shape[0], w.shape[1]))
 
 
