@@ -190,7 +190,7 @@ def near(got, want):
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("taps,per_head,silu", [(1, False, False), (2, True, True), (4, False, True), (4, True, False)])
-@pytest.mark.parametrize("kv,heads,lengths", [(1, 2, (1, 2, 3)), (2, 4, (5, 1, 7, 1200))])
+@pytest.mark.parametrize("kv,heads,lengths", [(1, 2, (1, 2, 3)), (2, 4, (5, 1, 7, 1200)), (2, 4, (5, 1, 7, 5100))])
 def test_preparation_of_wide_heads(dtype, taps, per_head, silu, kv, heads, lengths):
     """Heads of 128 (whole words, one or four tokens a warp), portions shorter than the taps and starts from a tail."""
     gen = torch.Generator().manual_seed(taps + heads)

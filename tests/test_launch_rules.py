@@ -173,6 +173,14 @@ def test_products_of_few_tiles_split_where_that_is_faster(lib):
         assert lib.vosti_gemm_tc_pair_splits(tokens, features, k) == 1, (tokens, features, k)
 
 
+def test_delta_preparation_takes_the_tokens_a_warp_that_were_measured_faster(lib):
+    """(tokens, heads of q, k and v) on both sides of the line between one and four tokens a warp; the times are beside the rule."""
+    for tokens, units in [(1, 24), (395, 24), (600, 24), (1200, 24), (1500, 24), (200, 48), (350, 48), (700, 48), (1200, 8), (3000, 8)]:
+        assert lib.vosti_delta_prep_tokens(tokens, units) == 1, (tokens, units)
+    for tokens, units in [(2048, 24), (3000, 24), (1000, 48), (1500, 48), (2048, 48), (1 << 20, 8192)]:
+        assert lib.vosti_delta_prep_tokens(tokens, units) == 4, (tokens, units)
+
+
 def test_float32_weights_go_to_the_product_whose_single_row_was_faster(lib):
     """Weights on both sides of the line between the tensor cores and the chain of multiply-adds; rows that do not start on whole words stay."""
     for n, k in [(16, 2048), (2048, 2048), (2048, 2304), (160, 4096), (4096, 1024), (4096, 1536), (8192, 1024), (4096, 4096), (24576, 4096), (4096, 12288)]:

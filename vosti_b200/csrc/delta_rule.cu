@@ -156,8 +156,7 @@ __global__ void __launch_bounds__(256) delta_prep_kernel(PrepArgs a) {
 // its head's beta, decay and gate. The kernel above is bound by its scalar loads (each input read once per tap): 87 us
 // for 2,048 tokens of 16 heads (4 key heads); this one was bound by the rounds of loads that a warp waited for (three before its
 // first token, 148 registers and so 12 warps an SM: 58 us), so weights come as words, the rows before the first token without
-// waiting for its request, a warp takes its tokens one after the other and a thread has 72 registers (28 warps an SM): 42 us
-// past the product before it.
+// waiting for its request, and a thread has 72 registers (28 warps an SM; with several tokens a warp 40 to 64 bytes of them lie in local memory): 40 us past the product before it.
 constexpr int WIDE_TAPS = 4;
 
 __device__ __forceinline__ void store_four(float* p, const float (&v)[4]) { *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]); }
@@ -740,6 +739,13 @@ general_scan_kernel(const float* __restrict__ r, const float* __restrict__ k, co
 
 }  // namespace
 
+// Tokens that a warp of the preparation of wide heads takes one after the other (units: heads of q, k and v). A warp waits for each token's
+// loads in turn, so one each while the SMs (28 warps of them at a time) run through at most some ten rounds; then four, which
+// share the weights and the earlier rows. us, one / four / eight tokens a warp: 24 units, 395 tokens 12.8 / 15.4 / 25.1, 1,000 25.7 /
+// 25.5 / 31.1, 1,500 36.0 / 38.2 / 42.8, 2,048 49.0 / 44.0 / 46.6, 3,000 70.6 / 64.6 / 74.0; 48 units, 260 tokens 16.8 / 17.5 / 27.4, 700 34.5 /
+// 37.3 / 41.3, 1,000 47.6 / 43.5 / 46.3, 2,048 93.9 / 83.8 / 81.7; 8 units, 2,048 tokens 17.1 / 18.2 / 28.5.
+VOSTI_API int vosti_delta_prep_tokens(int tokens, int units) { return (int64_t)tokens * units >= 148 * 270 ? 4 : 1; }
+
 VOSTI_API int vosti_delta_prep(const void* proj, int proj_f32, int stride, int off_q, int off_k, int off_v, int off_beta,
                                const void* rates, int rates_f32, int kv_heads, int heads, int dk, int dv, int taps,
                                const void* conv_w, const void* a_log, const void* dt_bias, int w_f32, float* state,
@@ -771,15 +777,14 @@ VOSTI_API int vosti_delta_prep(const void* proj, int proj_f32, int stride, int o
                     ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
                       reinterpret_cast<uintptr_t>(decay) | reinterpret_cast<uintptr_t>(gate)) & 15) == 0 && (units + 3) / 4 <= 65535;
   if (wide) {
-    // one token a warp while the tokens alone do not fill the SMs' warps, eight where they do
     a.w_words = taps == WIDE_TAPS && ((reinterpret_cast<uintptr_t>(conv_w) | reinterpret_cast<uintptr_t>(dt_bias)) & (w_f32 ? 15 : 7)) == 0;
-    const int each = (int64_t)tokens * units >= 148 * 64 ? 8 : 1;
+    const int each = vosti_delta_prep_tokens(tokens, units);
     const dim3 grid((tokens + each - 1) / each, (units + 3) / 4);
     if (proj_f32) {
-      if (each == 8) vosti_launch(delta_prep_wide_kernel<float, 8>, grid, dim3(128), 0, stream, a, tokens);
+      if (each == 4) vosti_launch(delta_prep_wide_kernel<float, 4>, grid, dim3(128), 0, stream, a, tokens);
       else vosti_launch(delta_prep_wide_kernel<float, 1>, grid, dim3(128), 0, stream, a, tokens);
     } else {
-      if (each == 8) vosti_launch(delta_prep_wide_kernel<bf16, 8>, grid, dim3(128), 0, stream, a, tokens);
+      if (each == 4) vosti_launch(delta_prep_wide_kernel<bf16, 4>, grid, dim3(128), 0, stream, a, tokens);
       else vosti_launch(delta_prep_wide_kernel<bf16, 1>, grid, dim3(128), 0, stream, a, tokens);
     }
   } else {
