@@ -190,6 +190,20 @@ def test_float32_weights_go_to_the_product_whose_single_row_was_faster(lib):
         assert not lib.vosti_gemm_f32_supported(n, k), (n, k)
 
 
+def test_a_product_that_is_cut_needs_its_workspace(lib):
+    """One that is missing or too small is refused before anything else happens, in the narrow and in the paired product alike."""
+    def call(tokens, features, k, elems):
+        code = lib.vosti_gemm_tc(None, None, None, tokens, features, k, 0, ctypes.c_void_p(16 if elems else 0), ctypes.c_int64(elems), 0, 0, 0,
+                                 None, None)
+        return code, lib.vosti_last_error().decode()
+
+    lib.vosti_last_error.restype = ctypes.c_char_p
+    for tokens, features, k, parts in [(8, 4096, 4096, lib.vosti_gemm_tc_splits(8, 4096, 4096)), (200, 4096, 12288, 4)]:
+        for elems in (0, parts * tokens * features - 1):
+            code, message = call(tokens, features, k, elems)
+            assert code != 0 and f"workspace too small for {parts} splits" in message, (tokens, elems, message)
+
+
 def test_float32_tiles_never_ask_for_more_tensor_memory_than_an_sm_has(lib):
     """CTAs of a cluster wait for their tensor memory without a limit: shared memory keeps as many of them on an SM as it has columns for."""
     columns = [lib.vosti_gemm_f32_columns_an_sm(tile) for tile in range(6)]

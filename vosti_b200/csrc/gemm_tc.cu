@@ -746,8 +746,9 @@ VOSTI_API int vosti_gemm_tc_pair_splits(int tokens, int features, int k) {
 // the weight rows interleaved in blocks of 16 gate rows and their 16 up rows.
 // With `defer_reduce` and more than one split the partial sums stay in the workspace
 // ([splits, tokens, features] float32) for a consumer that sums them itself; y is not written.
+// `whole_pairs`: products on pairs of SMs keep their K whole (otherwise vosti_gemm_tc_pair_splits cuts it, which also needs the workspace).
 VOSTI_API int vosti_gemm_tc(const void* x, const void* w, void* y, int tokens, int features, int k, int epilogue,
-                            float* workspace, int64_t workspace_elems, int defer_reduce, int w_packed, unsigned* status,
+                            float* workspace, int64_t workspace_elems, int defer_reduce, int whole_pairs, int w_packed, unsigned* status,
                             cudaStream_t stream) {
   VOSTI_REQUIRE(tokens >= 0 && vosti_gemm_tc_supported(features, k), "gemm_tc: unsupported sizes F=%d K=%d", features, k);
   VOSTI_REQUIRE((epilogue >= EPI_BF16 && epilogue <= EPI_SWIGLU) || is_gated(epilogue), "gemm_tc: unknown epilogue %d", epilogue);
@@ -757,8 +758,10 @@ VOSTI_API int vosti_gemm_tc(const void* x, const void* w, void* y, int tokens, i
   const int ld_out = is_gated(epilogue) ? features / 2 : features;
   const int k_blocks = (k + BK - 1) / BK;
   const int splits = vosti_gemm_tc_splits(tokens, features, k);
-  VOSTI_REQUIRE(splits == 1 || (workspace != nullptr && workspace_elems >= (int64_t)splits * tokens * features),
-                "gemm_tc: workspace too small for %d splits", splits);
+  const int cuts = splits > 1 || whole_pairs ? 1 : vosti_gemm_tc_pair_splits(tokens, features, k);
+  const int parts = splits > 1 ? splits : cuts;
+  VOSTI_REQUIRE(parts == 1 || (workspace != nullptr && workspace_elems >= (int64_t)parts * tokens * features),
+                "gemm_tc: workspace too small for %d splits", parts);
   CUtensorMap mw_storage, mx;
   const CUtensorMap* mw = &mw_storage;
   // a packed weight is [k blocks][feature tiles][128][64], zero-padded to whole tiles: its
@@ -784,8 +787,6 @@ VOSTI_API int vosti_gemm_tc(const void* x, const void* w, void* y, int tokens, i
         return e != cudaSuccess ? (int)e : VOSTI_UNSUPPORTED;
       }
     }
-    int cuts = vosti_gemm_tc_pair_splits(tokens, features, k);
-    if (workspace == nullptr || workspace_elems < (int64_t)cuts * tokens * features) cuts = 1;
     const int tiles = ((tokens + 2 * BM - 1) / (2 * BM)) * ((features + PAIR_BN - 1) / PAIR_BN) * cuts;
     const int pairs = tiles < pair_sms / 2 ? tiles : pair_sms / 2;
     vosti_launch_clusters(gemm_tc_pair_kernel<PlainEpilogue>, dim3(2 * pairs), dim3(PAIR_THREADS), 2, smem, stream, mx, *mw,

@@ -580,7 +580,8 @@ def gemm_tc(x: torch.Tensor, w, status: torch.Tensor, *, out_dtype: Optional[tor
         epilogue, width = (EPI_F32 if out_dtype == torch.float32 else EPI_BF16), features
     lib = library()
     splits = lib.vosti_gemm_tc_splits(tokens, features, k)
-    if splits == 1 and INVARIANCE != "decode":          # ("decode": a prompt's portions of more than 128 tokens keep one order too)
+    whole = INVARIANCE == "decode"                      # (a prompt's portions of more than 128 tokens keep one order too)
+    if splits == 1 and not whole:
         splits = lib.vosti_gemm_tc_pair_splits(tokens, features, k)
     elems = splits * tokens * features if splits > 1 else 0
     # more than 128 tokens: sums of the call's own, so that products on several streams and a partial sum that is
@@ -594,7 +595,7 @@ def gemm_tc(x: torch.Tensor, w, status: torch.Tensor, *, out_dtype: Optional[tor
     if splits > 1 and not own:
         _SPLIT_GENERATION[scratch] = _SPLIT_GENERATION.get(scratch, 0) + 1
     _check(lib.vosti_gemm_tc(_p(x), _p(w_data), _p(out), tokens, features, k, epilogue, _p(ws),
-                             ctypes.c_int64(ws.numel() if ws is not None else 0), int(defer), int(packed), _p(status),
+                             ctypes.c_int64(ws.numel() if ws is not None else 0), int(defer), int(whole), int(packed), _p(status),
                              _stream()),
            "gemm_tc", kernels=2 if splits > 1 and not defer else 1)
     if defer:
