@@ -239,3 +239,19 @@ def test_latent_attention_forms_keys_and_values_where_that_was_faster():
                               ([64, 64], [0, 0], True), ([20], [1500], False), ([8], [64], False), ([16] * 20, [100] * 20, False),
                               ([100] + [1] * 12, [0] + [1500] * 12, False), ([1] * 16, [700] * 16, False)]:
         assert ops.latent_forms_heads(new, [a + b for a, b in zip(new, past)], 16, 512) is formed, (new, past)
+
+
+def test_latent_attention_forms_no_heads_where_a_batch_must_not_change_a_prompt(lib, monkeypatch):
+    from types import SimpleNamespace
+    from vosti_b200 import ops
+
+    def forms(q, kv):
+        ctx = SimpleNamespace(num_requests=len(q), host_q_lens=q, host_kv_lens=kv, layout={})
+        return ops._latent_forms_heads(ctx, heads=16, dim=128, rot=64, dv=128, rank=512, window=0, scale=0.07, page_size=16, q_width=3664)
+
+    alone, beside = ([100], [100]), ([100] + [1] * 12, [100] + [1500] * 12)
+    assert forms(*alone) and not forms(*beside)              # the same prompt in two forms
+    for name, value in (("INVARIANCE", "decode"), ("FIXED_ORDER", True)):
+        with monkeypatch.context() as m:
+            m.setattr(ops, name, value)
+            assert not forms(*alone) and not forms(*beside)

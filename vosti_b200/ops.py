@@ -1716,7 +1716,8 @@ def latent_forms_heads(q_lens, kv_lens, heads: int, rank: int) -> bool:
 
 
 def _latent_forms_heads(ctx, *, heads: int, dim: int, rot: int, dv: int, rank: int, window: int, scale: float, page_size: int, q_width: int) -> bool:
-    if (window or FIXED_ORDER or scale <= 0 or len(ctx.host_q_lens) != ctx.num_requests or len(ctx.host_kv_lens) != ctx.num_requests
+    # ("decode": as its products, a prompt's attention keeps one order of arithmetic alone and beside others; the two forms round keys differently)
+    if (window or FIXED_ORDER or INVARIANCE == "decode" or scale <= 0 or len(ctx.host_q_lens) != ctx.num_requests or len(ctx.host_kv_lens) != ctx.num_requests
             or not library().vosti_latent_heads_fits(dim, rot, dv, rank, page_size, q_width)):
         return False
     rows = sum(-(-kv // LATENT_PAD) * LATENT_PAD for kv in ctx.host_kv_lens)
