@@ -137,22 +137,23 @@ def test_cuda_core_attention_takes_the_way_that_was_measured_faster():
     assert simt_way([128] + [0] + [9], [128, 50, 9], 32, 8, window=40) == 1
 
 
-def test_delta_rules_take_the_form_that_was_measured_faster():
+def test_delta_rules_take_the_form_that_was_measured_faster(lib):
     """Steps (heads, values a head, tokens of the requests) on both sides of the line between chunks and token by token, for
-    both rules; chunks are taken nowhere that they were measured slower."""
+    both rules. Of 3,279 measured steps the rule takes chunks in 20 where they were more than 3 % slower, none of them here."""
     from vosti_b200.ops import delta_step_layout, delta_takes_chunks
     takes = lambda pair, heads, dv, q: delta_takes_chunks(delta_step_layout(q)[1], heads, dv, pair)
     gated = {True: [(16, 128, [96]), (16, 128, [256]), (16, 128, [2048]), (16, 128, [128] * 2), (16, 128, [256] * 4), (16, 128, [1031, 700, 317]),
-                    (16, 128, [300] + [1] * 30), (4, 128, [96]), (4, 128, [128]), (4, 128, [256] * 8), (2, 128, [128] * 2), (8, 128, [128] * 4),
-                    (32, 128, [256]), (32, 128, [700]), (16, 64, [128] * 2), (8, 256, [128]), (64, 128, [256])],
-             False: [(16, 128, [49]), (16, 128, [64]), (16, 128, [64] * 4), (16, 128, [256] * 8), (16, 128, [256] * 16), (16, 128, [64] * 16),
-                     (8, 256, [96]), (8, 256, [96] * 4), (32, 128, [96] * 4), (16, 64, [256] * 8), (64, 128, [128] * 4), (64, 128, [64] + [1] * 30),
-                     (4, 128, [49])]}
-    general = {True: [(16, 128, [256]), (16, 128, [2048]), (16, 128, [128] * 2), (16, 128, [96] * 4), (16, 128, [128] * 4), (16, 128, [256] * 16),
-                      (16, 128, [1031, 700, 317]), (4, 128, [128]), (4, 128, [256]), (8, 128, [128] * 4), (32, 128, [128]), (32, 128, [256] * 8),
-                      (4, 128, [300] + [1] * 30), (64, 128, [128])],
-               False: [(16, 128, [49]), (16, 128, [96]), (4, 128, [64]), (4, 128, [96] * 4), (16, 128, [64] * 16), (32, 128, [64] * 16),
-                       (32, 128, [128] * 16), (64, 128, [96] * 8), (64, 128, [64] * 4), (4, 128, [64] + [1] * 30), (4, 128, [100] + [48] * 8)]}
+                    (16, 128, [300] + [1] * 30), (16, 128, [80]), (16, 128, [64] + [1] * 30), (16, 128, [256] * 8), (16, 128, [256] * 16),
+                    (4, 128, [64]), (4, 128, [96]), (4, 128, [128]), (4, 128, [256] * 8), (2, 128, [128] * 2), (8, 128, [128] * 4),
+                    (32, 128, [256]), (32, 128, [700]), (32, 128, [96] * 4), (16, 64, [128] * 2), (8, 256, [96]), (8, 256, [96] * 4),
+                    (8, 256, [128]), (64, 128, [256]), (64, 128, [64] + [1] * 30)],
+             False: [(16, 128, [49]), (16, 128, [64] * 4), (16, 128, [64] * 16), (64, 128, [64]), (64, 128, [80]), (4, 128, [49])]}
+    general = {True: [(16, 128, [128]), (16, 128, [256]), (16, 128, [2048]), (16, 128, [128] * 2), (16, 128, [64] * 4), (16, 128, [96] * 4),
+                      (16, 128, [128] * 4), (16, 128, [64] * 16), (16, 128, [256] * 16), (16, 128, [1031, 700, 317]), (16, 128, [96] + [1] * 30),
+                      (4, 128, [96]), (4, 128, [128]), (4, 128, [256]), (8, 128, [128] * 4), (32, 128, [128]), (32, 128, [128] * 16),
+                      (32, 128, [256] * 8), (4, 128, [300] + [1] * 30), (64, 128, [128]), (64, 128, [64] * 4), (64, 128, [96] * 8)],
+               False: [(16, 128, [49]), (16, 128, [80]), (16, 128, [96]), (16, 128, [112]), (16, 128, [49] * 16), (2, 128, [64]), (4, 128, [64]),
+                       (4, 128, [96] * 4), (64, 128, [49] * 4)]}
     for pair, table in ((False, gated), (True, general)):
         for want, steps in table.items():
             for step in steps:

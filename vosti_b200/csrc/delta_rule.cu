@@ -810,6 +810,23 @@ static int scan_rows(int dk) {
   return dk <= 32 ? 8 : 16;
 }
 
+static int scan_lanes(int dk) {          // of a value column
+  int ks = 1;
+  while (ks * scan_rows(dk) < dk) ks *= 2;
+  return ks;
+}
+
+// Value columns of a block of either rule's token-by-token kernel: 8 or more, fewer while the grid would leave SMs idle.
+VOSTI_API int vosti_delta_scan_columns(int requests, int heads, int dk, int dv) {
+  const int ks = scan_lanes(dk);
+  int threads = SCAN_THREADS;
+  while (threads > 64 && threads / 2 >= 8 * ks &&
+         (int64_t)requests * heads * ((dv + threads / ks - 1) / (threads / ks)) < 296)
+    threads /= 2;
+  if (threads < 8 * ks) threads = 8 * ks;
+  return threads / ks;
+}
+
 // `most` > 0: requests that bring more tokens than that are left alone (the chunked kernels take them).
 VOSTI_API int vosti_delta_scan(const float* q, const float* k, const float* v, const float* beta, const float* decay,
                                float* out, float* state, int64_t state_stride, const int* cu_q, const int* state_slots,
@@ -819,16 +836,7 @@ VOSTI_API int vosti_delta_scan(const float* q, const float* k, const float* v, c
   VOSTI_REQUIRE(heads <= 65535, "delta_scan: too many heads");
   VOSTI_REQUIRE(state_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(state) & 15) == 0, "delta_scan: state slots must be 16-byte aligned");
   if (requests == 0) return VOSTI_OK;
-  const int rows = scan_rows(dk);
-  int ks = 1;
-  while (ks * rows < dk) ks *= 2;
-  // blocks of 8 columns or more; smaller blocks while the grid would leave SMs idle
-  int threads = SCAN_THREADS;
-  while (threads > 64 && threads / 2 >= 8 * ks &&
-         (int64_t)requests * heads * ((dv + threads / ks - 1) / (threads / ks)) < 296)
-    threads /= 2;
-  if (threads < 8 * ks) threads = 8 * ks;
-  const int cols = threads / ks;
+  const int rows = scan_rows(dk), ks = scan_lanes(dk), cols = vosti_delta_scan_columns(requests, heads, dk, dv), threads = cols * ks;
   VOSTI_REQUIRE((dv + cols - 1) / cols <= 65535, "delta_scan: too many value channels");
   const dim3 grid(requests, heads, (dv + cols - 1) / cols);
   const size_t smem = 2 * (size_t)(TOKENS * (3 * ks * rows + cols) + TOKENS) * sizeof(float);
@@ -904,15 +912,7 @@ VOSTI_API int vosti_general_delta_scan(const float* r, const float* k, const flo
   VOSTI_REQUIRE(heads <= 65535, "general_delta_scan: too many heads");
   VOSTI_REQUIRE(state_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(state) & 15) == 0, "general_delta_scan: state slots must be 16-byte aligned");
   if (requests == 0) return VOSTI_OK;
-  const int rows = scan_rows(dk);
-  int ks = 1;
-  while (ks * rows < dk) ks *= 2;
-  int threads = SCAN_THREADS;
-  while (threads > 64 && threads / 2 >= 8 * ks &&
-         (int64_t)requests * heads * ((dv + threads / ks - 1) / (threads / ks)) < 296)
-    threads /= 2;
-  if (threads < 8 * ks) threads = 8 * ks;
-  const int cols = threads / ks;
+  const int rows = scan_rows(dk), ks = scan_lanes(dk), cols = vosti_delta_scan_columns(requests, heads, dk, dv), threads = cols * ks;
   VOSTI_REQUIRE((dv + cols - 1) / cols <= 65535, "general_delta_scan: too many value channels");
   const dim3 grid(requests, heads, (dv + cols - 1) / cols);
   const size_t smem = 2 * (size_t)(TOKENS * (5 * ks * rows + cols)) * sizeof(float);

@@ -1839,37 +1839,47 @@ def delta_prep(proj: torch.Tensor, rates: torch.Tensor, offsets: dict, *, kv_hea
 
 
 DELTA_CHUNK = 32     # tokens of a chunk (csrc/delta_chunks.cu)
+DELTA_KEYS = 128     # key channels of the heads that it takes
 DELTA_SHORT = 48     # requests that bring at most this many tokens are always served token by token
 DELTA_SCRATCH = 1 << 26      # floats (256 MB) of scratch at most: about 8,000 tokens of 16 heads of 128; more chunks run in rounds
 
 
+# us of a step token by token: the launch, a request's start, and by the columns of a block (8, 16 or 32: more requests, larger blocks) the longest
+# request's chain a token (0: its share is always more), its share of a busier SM, and a block's a token and SM. Of the chunks: both
+# launches, a turn of the chain, a chunk's and a request's share of the 128 blocks, the preparation of 296 chunks and heads, what the
+# launches no longer overlap, a third launch for the short requests. (gated, generalized)
+_DELTA_TOKENS = {False: (1.07, 1.14, {8: (0.346, 0.275, 0.043), 16: (0.0, 0.429, 0.052), 32: (0.0, 0.532, 0.204)}),
+                 True: (1.0, 1.38, {8: (0.361, 0.017, 0.2), 16: (0.485, 0.294, 0.2), 32: (0.784, 0.456, 0.365)})}
+_DELTA_CHUNKS = {False: (14.0, 2.22, 2.23, 0.88, 17.4, 1.08, 2.2), True: (21.6, 2.96, 2.89, 1.07, 29.5, 0.87, 4.5)}
+
+
 def delta_takes_chunks(layout: dict, heads: int, dv: int, pair: bool) -> bool:
     """Whether the chunked kernels are the faster way for a step laid out by `delta_step_layout` (`pair`: the generalized rule).
-    Both sides in us, fitted to sweeps of 2 to 64 heads of 128 (values of 64, 128 and 256), 1 to 16 long requests of 49 to
-    2,048 tokens and shorter ones beside them. Token by token a step takes its longest portion's chain or, with
-    more blocks than the GPU holds, a share of the GPU a token. Chunks take two launches, the longest portion's chunks
-    in turn or a share of the GPU a chunk, the preparation of all of them, and one more launch for the short requests.
-    Where both are close, token by token stays. Measured, tokens and chunks, 16 heads: gated, one request of 64: 24 and
-    29, 96: 35 and 33, 256: 89 and 47; two of 128 58 and 49; sixteen of 256 461 and 533. Generalized, one of 96: 37 and 45, 128: 49 and 49;
-    two of 128 95 and 65; four of 96 99 and 85; sixteen of 64 208 and 229. 4 heads, one of 128: gated 44 and 27, generalized 45 and 37.
-    (What single tokens cost a chain beside them is put too low: a portion of 64 beside 30 stays with 59 us, chunks take 41. The
-    chunks' times are those before their products ran on the tensor cores, which take 0.65 to 0.7 of a turn: the line lies to the
-    side of token by token.)"""
-    launch, chain, long, share, each = (1.4, 0.34, 0.258, 0.174, 1.04) if pair else (1.2, 0.335, 0.254, 0.089, 1.16)
-    width = heads * dv / 2048
-    rounds = layout["longs"] * width                     # blocks of the chunks' run, in 128
+    Both sides in us, fitted to 3,279 steps: 2 to 64 heads of 128 (values of 64, 128 and 256), 1 to 16 long requests of 49 to
+    2,048 tokens, 0 to 30 shorter ones beside them (nine in ten estimates of either side are within 10 %). Token by token a step takes its
+    longest request's chain, or its share of an SM and the blocks' on it; chunks take two launches, the longest portion's chunks
+    in turn or a share of the GPU a chunk, the preparation of all of them, and one more launch for the short requests. Where both are
+    close, token by token stays: over those steps the choice takes 0.3 % more than the faster way. Measured, tokens and chunks, 16 heads:
+    gated, one request of 49: 20 and 25, 64: 25 and 25, 96: 35 and 28, 256: 90 and 41; two of 128 59 and 42; four of 64 43 and 44; sixteen of
+    64 122 and 134, of 256 463 and 425; 64 beside 30 single tokens 55 and 40. Generalized, one of 96: 38 and 41, 128: 49 and 45; two of 128
+    96 and 60; four of 64 68 and 62; sixteen of 49 163 and 187, of 64 208 and 189; 96 beside 30 single tokens 93 and 64."""
+    launch, each, by_columns = _DELTA_TOKENS[pair]
+    columns = library().vosti_delta_scan_columns(layout["longs"] + layout["shorts"], heads, DELTA_KEYS, dv)
+    chain, share, block = by_columns[min(max(columns, 8), 32)]
+    blocks = heads * -(-dv // columns) / 148             # of a request, an SM
 
     def one_by_one(longest, tokens, requests):
-        return launch + max(chain * longest, long * longest + width * (share * tokens + each * requests)) if requests else 0.0
-    launch2, turn, part, prepare, full, third, start = (22.3, 3.27, 3.78, 20.1, 3.2, 5.8, 1.96) if pair else (14.9, 2.79, 3.09, 12.2, 3.2, 0.0, 1.52)
+        return launch + max(chain * longest, share * longest + blocks * (block * tokens + each * requests)) if requests else 0.0
+    both, turn, part, start, prepare, apart, third = _DELTA_CHUNKS[pair]
     chunks, longs, shorts = layout["chunks"], layout["longs"], layout["shorts"]
-    cost = launch2 + max(turn * -(-layout["longest"] // DELTA_CHUNK), part * width * chunks + start * rounds) + prepare * heads * chunks / 296
-    cost += 5.0 * ((dv - 1) // 128)                      # (the preparation takes 128 value columns at a time)
-    cost += full * min(1.0, max(0.0, (128 * rounds + heads * chunks - 96) / 64))          # (beyond that the two launches don't overlap)
+    width = heads * dv / 2048
+    rounds = longs * width                               # blocks of the chunks' run, in 128
+    cost = both + max(turn * -(-layout["longest"] // DELTA_CHUNK), part * width * chunks + start * rounds) + prepare * heads * chunks / 296
+    cost += 4.3 * ((dv - 1) // 128)                      # (the preparation takes 128 value columns at a time)
+    cost += apart * min(1.0, max(0.0, (128 * rounds + heads * chunks - 96) / 64))
     if shorts:
         cost += third + one_by_one(layout["short_longest"], layout["short_tokens"], shorts)
-    tokens = one_by_one(layout["longest"], layout["tokens"] + layout["short_tokens"], longs + shorts)
-    return cost < (0.88 if rounds > 24 else 0.95 if pair else 0.97) * tokens
+    return cost < 0.94 * one_by_one(layout["longest"], layout["tokens"] + layout["short_tokens"], longs + shorts)
 
 
 def delta_step_layout(q_lens):
