@@ -120,6 +120,32 @@ def test_a_token_that_is_not_finite_reaches_no_earlier_one(monkeypatch, rule):
         assert torch.equal(out[:45], outs[0][:45]) and not torch.isfinite(out[45:]).any()
 
 
+@pytest.mark.parametrize("rule", ["gated", "general"])
+def test_a_start_state_that_is_not_finite_stays_in_its_value_column(monkeypatch, rule):
+    """An infinite entry of a start state (NaN from the first chunk on: its lower terms are inf - inf) spoils that value column's read-outs and
+    state, and not a bit of another's."""
+    monkeypatch.setattr(ops, "delta_takes_chunks", lambda *a: True)
+    gen = torch.Generator().manual_seed(4)
+    ins = inputs(rule, 80, 2, 2, 128, "mixed", gen)
+    start = torch.randn(2, 128, DK, generator=gen)           # [head, value, key]
+    got = []
+    for value in (None, float("inf"), float("-inf"), float("nan")):
+        case = start.clone()
+        if value is not None:
+            case[1, 5, 3] = value
+        harness = Harness([None], [StateSpec((2 * DK * 128,), torch.float32)], torch.float32)
+        ctx = harness.context([StepEntry("r", [0] * 80)])
+        state = harness.cache.layer_caches[0].state
+        state[ctx.host_state_slots[0]] = case.reshape(-1).to(DEV)
+        out = scan(rule, ins, harness, ctx, 2, 2, 128).view(80, 2, 128)
+        got.append((out.cpu(), state[ctx.host_state_slots[0]].view(2, 128, DK).cpu()))
+    others = torch.ones(2, 128, dtype=torch.bool)
+    others[1, 5] = False
+    for out, state in got[1:]:
+        assert torch.equal(out[:, others], got[0][0][:, others]) and torch.equal(state[others], got[0][1][others])
+        assert not torch.isfinite(out[:, 1, 5]).any() and not torch.isfinite(state[1, 5]).any()
+
+
 @pytest.mark.parametrize("rule,lengths,chunks", [("gated", (49, 3), False), ("gated", (300, 1), True), ("general", (64,), False),
                                                  ("general", (700, 20), True), ("gated", (1000,), True)])
 def test_the_rule_itself_chooses(monkeypatch, rule, lengths, chunks):
