@@ -152,7 +152,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
   const int pairs = gridDim.x / 2, pair = blockIdx.x / 2;
   const int m_tiles = (tokens + 2 * BM - 1) / (2 * BM), n_tiles = (features + PAIR_BN - 1) / PAIR_BN;
   const int total_tiles = m_tiles * n_tiles * splits;         // (a tile's splits one after the other)
-  auto first_block = [&](int split) { return (int)((long long)k_blocks * split / splits); };
+  auto first_block = [&](int split) { return splits == 1 ? k_blocks * split : k_blocks * split / splits; };
 
   if (threadIdx.x == 0) {
     abort_flag = 0;
