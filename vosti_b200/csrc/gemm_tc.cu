@@ -66,11 +66,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   // hold only reaches output columns that are not stored.
   // w_tiles > 0: the weight is stored tile by tile ([k block][feature tile][128][64], w_tiles
   // feature tiles) and map_w sees it as a matrix of 64 columns; 0: row-major [features, k]
-  // KPS: k-blocks per stage of the ring. The lane that issues the MMAs pays about 200 cycles for
-  // the barrier wait that follows its own commit (even when the stage landed long before), 85
-  // for the commit and 95 for the loop, beside 56 per MMA: with one k-block per stage that is
-  // 610 cycles per k-block, with two 416. Launches with so few CTAs that each has an SM (and its
-  // shared memory) to itself, whose time is k-blocks x that cost, take two k-blocks per stage.
+  // KPS: k-blocks per stage of the ring. Each stage costs the warp that issues the MMAs a barrier wait after its own commit (even
+  // when the stage landed long before), the commit and the loop. One CTA an SM, ns a k-block of K = 2,048 to 8,192 with one and with two
+  // of them a stage: 8 tokens 253 and 193, 64 tokens 261 and 194, 128 tokens 280 and 221 (one tile); 267 and 203, 326 and 207, 291 and 274
+  // (64 tiles). Launches with so few CTAs that each has an SM (and its shared memory) to itself, whose time is k-blocks x that
+  // cost, take two k-blocks per stage.
   constexpr int B_BYTES = BN * BK * 2;
   constexpr int BLOCK_BYTES = A_BYTES + B_BYTES;
   constexpr int STAGE_BYTES = KPS * BLOCK_BYTES;

@@ -5,10 +5,8 @@
 // and each CTA's tensor memory receives the 256 columns of its own 128 tokens. A tile's K may be split over several pairs
 // (`vosti_gemm_tc_pair_splits`), whose partial sums another kernel adds in split order. Against the
 // single-CTA tile (128 x 256: 48 KB of operands per k-block and SM) an SM takes in 32 KB per
-// k-block, so a ring stage can hold two k-blocks and still be three stages deep: the lane that
-// issues the MMAs then pays one barrier wait (about 200 cycles, even when the stage landed long
-// before) and one commit per eight MMAs, 830 cycles for the 1,024 the tensor cores need, where the
-// single-CTA kernel with one k-block per stage pays 610 for 512.
+// k-block, so a ring stage can hold two k-blocks and still be three stages deep: one barrier wait and one commit for eight
+// MMAs. A pair alone takes 278 ns a k-block, where its tensor cores need 512 cycles (262 ns at 1,950 MHz); 70 of them side by side 455.
 //
 // Barriers. full[s] lives in the first CTA and counts the bytes of both CTAs' copies (the copies of
 // the second CTA name it through the shared::cluster window); empty[s] and acc_full[a] exist in
