@@ -89,12 +89,6 @@ latent_prep_kernel(const T* __restrict__ proj, int64_t proj_stride, T* __restric
   for (int i = threadIdx.x; i < rot; i += blockDim.x) r_cache[slot * rot + i] = from_f32<T>(turned(down + rank, i));
 }
 
-__device__ __forceinline__ void put_four(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
-__device__ __forceinline__ void put_four(bf16* p, float4 v) {
-  const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
-  *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
-}
-
 // The same for rows of whole words of four: what a token needs is asked for together, before the angles are made, where the
 // kernel above waits for its single elements one loop after the other. `rot` a multiple of 8, `rank` of 4 and at most 1,024.
 constexpr int PREP_THREADS = 128, PREP_WORDS = 2;         // threads of a token; words of the latent each of them keeps
@@ -158,8 +152,8 @@ latent_prep_words_kernel(const T* __restrict__ proj, int64_t proj_stride, T* __r
     }
     turned(a, b, i % pairs);
     T* const to = qk + ((int64_t)t * heads + i / pairs) * qk_row + qk_row - rot;
-    put_four(to + first(i % pairs), a);
-    put_four(to + second(i % pairs), b);
+    store_four(to + first(i % pairs), a);
+    store_four(to + second(i % pairs), b);
   }
   if (gate != nullptr)
     for (int i = tid; i < heads; i += PREP_THREADS) gate[(int64_t)t * heads + i] = 1.f / (1.f + expf(-to_f32(down[rank + rot + i])));
@@ -180,15 +174,15 @@ latent_prep_words_kernel(const T* __restrict__ proj, int64_t proj_stride, T* __r
     const int c = (tid + w * PREP_THREADS) * 4;
     if (c >= rank) break;
     const float4 v = latent[w];
-    put_four(c_cache + slot * rank + c, make_float4(v.x * inv * load_flex(norm_w, norm_f32, c), v.y * inv * load_flex(norm_w, norm_f32, c + 1),
+    store_four(c_cache + slot * rank + c, make_float4(v.x * inv * load_flex(norm_w, norm_f32, c), v.y * inv * load_flex(norm_w, norm_f32, c + 1),
                                                     v.z * inv * load_flex(norm_w, norm_f32, c + 2), v.w * inv * load_flex(norm_w, norm_f32, c + 3)));
   }
   for (int i = tid; i < pairs; i += PREP_THREADS) {
     a = load_four(down + rank + first(i));
     b = load_four(down + rank + second(i));
     turned(a, b, i);
-    put_four(r_cache + slot * rot + first(i), a);
-    put_four(r_cache + slot * rot + second(i), b);
+    store_four(r_cache + slot * rot + first(i), a);
+    store_four(r_cache + slot * rot + second(i), b);
   }
 }
 

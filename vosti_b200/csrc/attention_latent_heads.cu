@@ -42,16 +42,6 @@ __device__ __forceinline__ int dense_start(const int* kv_len, int b) {
   return sum;
 }
 
-// D += A B with A [128 rows, 16 k] in tensor memory: a lane per row, two neighbouring k in a column.
-__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u)
-      : "memory");
-}
-
 // 16 dense rows a block: grid (rows / 16 of the longest request, requests).
 __global__ void __launch_bounds__(128)
 latent_gather_kernel(const bf16* __restrict__ c_cache, const bf16* __restrict__ r_cache, const int* __restrict__ kv_len,

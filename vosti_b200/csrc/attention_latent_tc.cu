@@ -34,16 +34,6 @@ constexpr uint32_t TMEM_COLS = 512, S_COL = 0, P_COL = 2 * KT, O_COL = 4 * KT;
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr size_t SMEM_BYTES = 1024 + Q_BYTES + (size_t)STAGES * STAGE_BYTES;
 
-// D += A B with A [128 rows, 16 k] in tensor memory: a lane per row, two neighbouring k in a column.
-__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u)
-      : "memory");
-}
-
 __global__ void __launch_bounds__(THREADS, 1)
 latent_attend_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_c,
                         const __grid_constant__ CUtensorMap map_r, float* __restrict__ out, const int* __restrict__ positions,

@@ -50,15 +50,6 @@ struct F32Tile {
   static constexpr int COLS_AN_SM = SM_BYTES / (SMEM + 1024) * COLS;       // that its CTAs may ask for
 };
 
-__device__ __forceinline__ uint32_t f32_cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void f32_cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ float4 load_cluster4(uint32_t smem_addr, uint32_t rank) {
   uint32_t remote;
   float4 v;
@@ -147,16 +138,6 @@ __device__ __forceinline__ void tmem_store8(uint32_t taddr, const uint32_t (&r)[
                "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
                : "memory");
 }
-// D += A B with A [128 rows, 16 k] in tensor memory: a lane per row, two neighbouring k in a column.
-__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u)
-      : "memory");
-}
-
 // TOK tokens on N. One thread brings both operands' words of KS k into a ring of RAW stages by TMA (zeros beyond a matrix), eight
 // warps split them, the weights into three planes in tensor memory (a thread: half a feature's k), the tokens into three in
 // shared memory, and between stages take the tensor core's 64-k sums out (a thread: one feature, TOK / 2 tokens); a ninth warp
@@ -385,8 +366,8 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
     if (ok) add_columns<COLS>(tmem_small + my_columns, acc);
 #pragma unroll
     for (int i = 0; i < COLS; ++i) mine_at[(TOK + i) * FT] = acc[i];
-    f32_cluster_sync();
-    const int mine = (int)f32_cluster_rank();              // = segment
+    cluster_sync_all();
+    const int mine = (int)cluster_rank();              // = segment
     const int lo = TOK * mine / segments, hi = TOK * (mine + 1) / segments;
     for (int word = threadIdx.x; word < (hi - lo) * (FT / 4); word += WORKERS) {
       const int t = lo + word / (FT / 4), f = word % (FT / 4) * 4;
@@ -419,7 +400,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
     for (int kk = 0; kk < k; ++kk) v = fmaf(xr[kk], wr[kk], v);
     y[(int64_t)t * n + f] = v;
   }
-  if (segments > 1) f32_cluster_sync();                     // nobody reads this CTA's sums after this
+  if (segments > 1) cluster_sync_all();                     // nobody reads this CTA's sums after this
   if (warp == 0) {
     tc_fence_after();
     tmem_dealloc(tmem_sum, TMEM_COLS);

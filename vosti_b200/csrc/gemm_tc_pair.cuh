@@ -24,15 +24,6 @@ constexpr int PAIR_BLOCK_BYTES = 2 * A_BYTES;      // one k-block: 128 tokens x 
 constexpr int PAIR_STAGE_BYTES = PAIR_KPS * PAIR_BLOCK_BYTES;
 constexpr int PAIR_THREADS = 192;
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 // The address of the same shared-memory location in CTA `rank` of the cluster.
 __device__ __forceinline__ uint32_t in_cta(uint32_t smem_addr, uint32_t rank) {
   uint32_t remote;

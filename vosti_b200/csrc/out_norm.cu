@@ -25,13 +25,6 @@ __device__ __forceinline__ float4 flex4(const void* p, int is_f32, int64_t i) {
   const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
   return make_float4(lo.x, lo.y, hi.x, hi.y);
 }
-__device__ __forceinline__ void put4(bf16* p, float4 v) {
-  const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
-  uint2 raw;
-  raw.x = *reinterpret_cast<const unsigned*>(&lo);
-  raw.y = *reinterpret_cast<const unsigned*>(&hi);
-  *reinterpret_cast<uint2*>(p) = raw;
-}
 __device__ __forceinline__ float dot4(float4 v) { return (v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w); }
 
 constexpr int MAX_TERMS = 2;
@@ -192,7 +185,7 @@ out_norm_stream_kernel(const OutNorm a, TO* __restrict__ out, unsigned* status) 
       x.z = fmaf(s.z, y.z * inv * (a.offset + w.z), x.z);
       x.w = fmaf(s.w, y.w * inv * (a.offset + w.w), x.w);
       *reinterpret_cast<float4*>(a.stream_out + base + i) = x;
-      if (out != nullptr) put4(out + base + i, x);
+      if (out != nullptr) store_four(out + base + i, x);
     } else {
       const float s = a.scale != nullptr ? load_flex(a.scale, a.scale_f32, i) : 1.f;
       const float x = fmaf(s, rows_smem[i] * inv * (a.offset + load_flex(a.w, a.w_f32, i)), a.stream[base + i]);
