@@ -233,13 +233,20 @@ def test_weight_bytes_of_a_decode_step_in_closed_form():
 
 
 def test_latent_attention_forms_keys_and_values_where_that_was_faster():
-    """Whole mixers of 16 heads, rank 512: (tokens, keys before them, whether formed heads were measured faster)."""
+    """Whole mixers of 16 heads and rank 512, then of others: (tokens, keys before them, whether formed heads were measured faster)."""
     from vosti_b200 import ops
     for new, past, formed in [([33], [0], True), ([128], [0], True), ([700], [0], True), ([2048], [0], True), ([131], [700], True),
                               ([500] * 3, [0, 64, 0], True), ([1024] + [1] * 8, [0] + [1000] * 8, True), ([5, 17, 200], [0, 30, 1400], True),
                               ([64, 64], [0, 0], True), ([20], [1500], False), ([8], [64], False), ([16] * 20, [100] * 20, False),
                               ([100] + [1] * 12, [0] + [1500] * 12, False), ([1] * 16, [700] * 16, False)]:
         assert ops.latent_forms_heads(new, [a + b for a, b in zip(new, past)], 16, 512) is formed, (new, past)
+    for heads, rank, new, past, formed in [
+            (8, 512, [33], [0], True), (8, 512, [300], [1500], True), (8, 512, [64], [1000], False), (8, 512, [300] + [1] * 30, [0] + [500] * 30, False),
+            (32, 512, [64], [1000], True), (32, 512, [1024] + [1] * 8, [0] + [1000] * 8, True), (32, 512, [30], [1000], False),
+            (64, 512, [64], [0], True), (64, 512, [131], [700], True), (128, 512, [64], [0], True), (128, 512, [40] * 8, [0] * 8, True),
+            (16, 256, [64], [0], True), (16, 256, [131], [700], True), (16, 256, [64], [1000], False), (16, 256, [100] + [1] * 12, [0] + [1500] * 12, False),
+            (64, 256, [64], [1000], True), (64, 256, [24], [200], False), (64, 256, [30], [1000], False)]:
+        assert ops.latent_forms_heads(new, [a + b for a, b in zip(new, past)], heads, rank) is formed, (heads, rank, new, past)
 
 
 def test_latent_attention_forms_no_heads_where_a_batch_must_not_change_a_prompt(lib, monkeypatch):

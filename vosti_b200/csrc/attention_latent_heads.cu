@@ -14,7 +14,9 @@
 //
 // A CTA's two row tiles are the request's i-th and i-th last, so that all CTAs walk the same number of keys, or it has one
 // where that still leaves no more CTAs than SMs. A tile of 64 keys costs the tensor core 1,152 cycles a row tile (384
-// scores, 768 sums) and its softmax thread some 1,000; the keys' 56 KB a tile are what two row tiles share.
+// scores, 768 sums) and its softmax thread some 1,000; the keys' 56 KB a tile are what two row tiles share. 2,048 tokens of 16 heads: 64 us
+// (in the latent space 265 and two projections), tensor cores 43 % and issue slots 29 % busy on the 128 SMs that have a block.
+// (The softmax's 200 registers are moved to it at run time; 8 bytes of the 128 that the launch starts with lie in local memory.)
 #include "common.cuh"
 #include "latent.cuh"
 #include "mma_util.cuh"

@@ -25,12 +25,13 @@
 // The scratch takes 516 floats a token and head (644 in the generalized rule); its caller bounds it and the chunks run in
 // rounds. Which steps come here and which go token by token: delta_takes_chunks in ops.py, with both sides' times.
 //
-// 2,048 tokens of one request, 16 heads of 128: 80 us and 136 us (the token-by-token kernel: 698 us); the generalized rule
-// over 1,031 + 700 + 317 tokens: 140 us and 172 us (628 us). The first is bound by the shared-memory pipe at two blocks an SM.
-// The second was too (8 x 4 tiles of multiply-adds with 16-byte operand reads, shuffles, copies: 194 and 278 us); on the tensor
-// cores a chunk takes 2.1 us (generalized 2.7), of which its MMAs are 0.7 and the copies that the blocks' SMs take in
-// 0.4, the rest is two barriers and the latency between them (a copy a row by
-// cp.async.bulk instead: 5.6 us a chunk; four whole ones from a padded scratch: 2.1).
+// 2,048 tokens of one request, 16 heads of 128, each launch alone: 79 us and 159 us, 224 for both after one another, whose launches
+// overlap (the token-by-token kernel: 695 us); the generalized rule over 1,031 + 700 + 317 tokens: 138 us and 215 us, 330 for
+// both (648 us). The first is bound by the shared-memory pipe at two blocks an SM.
+// The second was too (8 x 4 tiles of multiply-adds with 16-byte operand reads, shuffles, copies: 194 and 281 us); on the tensor
+// cores a chunk takes 2.5 us (generalized 3.4), of which its MMAs are 0.7 and the copies that the blocks' SMs take in
+// 0.4, the rest is two barriers and the latency between them: tensor cores 37 % and issue slots 43 % busy, shared memory 43 %. (A copy a row by
+// cp.async.bulk instead took 2.7 times as long a chunk; four whole ones from a padded scratch as long as it is.)
 // tcgen05 would add a commit and a read of tensor memory to each of the two products of the chain, which are
 // 64 x 16 x 128 and 128 x 16 x 32.
 //

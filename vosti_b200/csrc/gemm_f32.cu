@@ -138,13 +138,15 @@ __device__ __forceinline__ void tmem_store8(uint32_t taddr, const uint32_t (&r)[
                "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
                : "memory");
 }
+
 // TOK tokens on N. One thread brings both operands' words of KS k into a ring of RAW stages by TMA (zeros beyond a matrix), eight
 // warps split them, the weights into three planes in tensor memory (a thread: half a feature's k), the tokens into three in
 // shared memory, and between stages take the tensor core's 64-k sums out (a thread: one feature, TOK / 2 tokens); a ninth warp
-// issues the MMAs. The bound is shared memory: with the weights' planes there too every product reads them again (10 KB for
-// each MMA of 192 tokens; at first, six products, us for 24,576 x 4,096, 1 / 64 / 384 rows: 152 / 283 / 570 so, 91 / 161 / 432 as it is). The
-// eight products of scaled operands take 99 / 169 / 494, gemm_simt.cu 155 / 435 / 1,699. The roles share no code from where they part (their registers differ): the warps that bring
-// and issue end after their last request, the eight do the rest.
+// issues the MMAs. With the weights' planes in shared memory too, every product read them again (10 KB for each MMA of 192 tokens):
+// six products, us for 24,576 x 4,096, 1 / 64 / 384 rows, 152 / 283 / 570 so and 91 / 161 / 432 as it is; the eight products of
+// scaled operands take 99 / 169 / 494, gemm_simt.cu 155 / 435 / 1,699. At 384 rows the tensor cores are 64 % busy, issue slots 47 %,
+// shared memory 37 %. The roles share no code from where they part (their registers differ): the warps that bring and issue end after
+// their last request, the eight do the rest.
 // WORDS: every row starts on a whole word; otherwise the eight warps read the matrices themselves, element by element.
 template <int TOK, int KS, int STAGES, int RAW, int BLOCKS, bool WORDS>
 __global__ void __launch_bounds__(THREADS<TOK>, BLOCKS)
