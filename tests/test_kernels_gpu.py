@@ -42,6 +42,11 @@ def test_embedding(dev, status, dtype, hidden, vocab):
     bad[3] = vocab
     out = ops.embedding(bad, table, status)
     assert status.item() == 1 and out[3].abs().max() == 0        # reported, not read
+    # rows that do not start on whole words (a table inside another tensor)
+    held = torch.empty(vocab * hidden + 1, device=dev, dtype=dtype)
+    held[1:] = table.view(-1)
+    assert torch.equal(ops.embedding(ids, held[1:].view(vocab, hidden), status), table[ids.long()])
+    assert torch.equal(ops.embedding(ids, held[1:].view(vocab, hidden), status, out_dtype=torch.float32), table[ids.long()].float())
 
 
 @pytest.mark.parametrize("dtype", DTYPES)

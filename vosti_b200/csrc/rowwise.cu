@@ -29,7 +29,8 @@ __global__ void embedding_kernel(const int* __restrict__ ids, const int* __restr
   TO* dst = out + (int64_t)t * hidden;
   if (resolved != nullptr && threadIdx.x == 0) resolved[t] = id;
   const int bytes = hidden * (int)sizeof(T);
-  if (sizeof(TO) == 4 && sizeof(T) == 2 && hidden % 8 == 0) {
+  const bool words = ((reinterpret_cast<uintptr_t>(table) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(rounded)) & 15) == 0;
+  if (sizeof(TO) == 4 && sizeof(T) == 2 && hidden % 8 == 0 && words) {
     // a float32 stream from a bfloat16 table: 16-byte words in, two out, and the row's rounding beside it if asked for
     const uint4* s8 = reinterpret_cast<const uint4*>(src);
     for (int i = threadIdx.x; i < hidden / 8; i += blockDim.x) {
@@ -59,7 +60,7 @@ __global__ void embedding_kernel(const int* __restrict__ ids, const int* __restr
       dst[i] = from_f32<TO>(v);
       if (rounded != nullptr) rounded[(int64_t)t * hidden + i] = __float2bfloat16_rn(v);
     }
-  } else if (bytes % 16 == 0) {
+  } else if (bytes % 16 == 0 && words) {
     const int4* s4 = reinterpret_cast<const int4*>(src);
     int4* d4 = reinterpret_cast<int4*>(dst);
     for (int i = threadIdx.x; i < bytes / 16; i += blockDim.x) d4[i] = bad ? make_int4(0, 0, 0, 0) : s4[i];
