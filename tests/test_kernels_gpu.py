@@ -78,6 +78,24 @@ def test_silu_mul(dev, dtype):
     assert torch.allclose(out.float(), (g * torch.sigmoid(g) * u).to(dtype).float(), **tol(dtype))
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_rows_that_are_not_there_are_reported_as_rows(dev, status, dtype):
+    """By the gather and by the float32 products that take their rows by index, on the tensor cores and on the CUDA cores: zeros, and the
+    bit of a row index (not of a token)."""
+    from types import SimpleNamespace
+    from vosti_b200 import ops
+    from vosti_b200.parts.linear import linear, uses_split_float32
+    x, index = torch.randn(9, 2048, device=dev).to(dtype), torch.tensor([3, 9, -1, 0], dtype=torch.int32, device=dev)
+    rows = ops.gather_rows(x, index, status)
+    assert torch.equal(rows[[0, 3]], x[[3, 0]]) and not rows[1:3].any() and status.item() == 1 << 5
+    for k in (2048, 80):
+        w = torch.randn(48, k, device=dev).to(dtype)
+        assert uses_split_float32(dtype, w) == (dtype == torch.float32 and k == 2048)
+        status.zero_()
+        y = linear(SimpleNamespace(status=status), x[:, :k].contiguous(), w, row_index=index, out_dtype=torch.float32)
+        assert not y[1:3].any() and y[0].any() and status.item() == 1 << 5
+
+
 @pytest.mark.parametrize("xdt,wdt,ydt", [(torch.float32, torch.float32, torch.float32),
                                          (torch.bfloat16, torch.bfloat16, torch.bfloat16),
                                          (torch.bfloat16, torch.bfloat16, torch.float32),

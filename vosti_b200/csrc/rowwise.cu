@@ -9,12 +9,12 @@
 // With `source`, row t takes its id from values[source[t]] where source[t] >= 0: a token the
 // sampler of the step before left on the device, which the host has not read yet.
 // `scale` multiplies the row in float32 (1: a plain copy), for architectures that scale
-// their embeddings. `resolved` (or null) receives the id every row was taken for.
+// their embeddings. `resolved` (or null) receives the id every row was taken for. An id that names no row is reported as `fault`.
 template <typename T, typename TO = T>
 __global__ void embedding_kernel(const int* __restrict__ ids, const int* __restrict__ source,
                                  const int* __restrict__ values, const T* __restrict__ table,
                                  TO* __restrict__ out, int hidden, int vocab, float scale, unsigned* status,
-                                 bf16* __restrict__ rounded, int* __restrict__ resolved) {
+                                 bf16* __restrict__ rounded, int* __restrict__ resolved, unsigned fault) {
   pdl_wait();
   pdl_launch_dependents();
   const int t = blockIdx.x;
@@ -22,7 +22,7 @@ __global__ void embedding_kernel(const int* __restrict__ ids, const int* __restr
   if (source != nullptr && source[t] >= 0) id = values[source[t]];
   const bool bad = id < 0 || id >= vocab;
   if (bad) {
-    if (threadIdx.x == 0) raise_fault(status, VOSTI_FAULT_TOKEN_RANGE);
+    if (threadIdx.x == 0) raise_fault(status, fault);
     id = 0;
   }
   const T* src = table + (int64_t)id * hidden;
@@ -76,9 +76,22 @@ VOSTI_API int vosti_embedding(const int* ids, const int* source, const int* valu
                 tokens, hidden, vocab);
   if (tokens == 0) return VOSTI_OK;
   if (is_f32)
-    vosti_launch(embedding_kernel<float>, dim3(tokens), dim3(128), 0, stream, ids, source, values, (const float*)table, (float*)out, hidden, vocab, scale, status, (bf16*)nullptr, resolved);
+    vosti_launch(embedding_kernel<float>, dim3(tokens), dim3(128), 0, stream, ids, source, values, (const float*)table, (float*)out, hidden, vocab, scale, status, (bf16*)nullptr, resolved, (unsigned)VOSTI_FAULT_TOKEN_RANGE);
   else
-    vosti_launch(embedding_kernel<bf16>, dim3(tokens), dim3(128), 0, stream, ids, source, values, (const bf16*)table, (bf16*)out, hidden, vocab, scale, status, (bf16*)nullptr, resolved);
+    vosti_launch(embedding_kernel<bf16>, dim3(tokens), dim3(128), 0, stream, ids, source, values, (const bf16*)table, (bf16*)out, hidden, vocab, scale, status, (bf16*)nullptr, resolved, (unsigned)VOSTI_FAULT_TOKEN_RANGE);
+  VOSTI_LAUNCH_CHECK();
+}
+
+// out [count, width] = the rows of x [x_rows, width] that `rows` names.
+VOSTI_API int vosti_gather_rows(const int* rows, const void* x, void* out, int count, int width, int x_rows, int is_f32, unsigned* status,
+                                cudaStream_t stream) {
+  VOSTI_REQUIRE(count >= 0 && width > 0 && x_rows >= 0, "gather_rows: bad sizes %d of %d rows of %d", count, x_rows, width);
+  if (count == 0) return VOSTI_OK;
+  const int* const none = nullptr;
+  if (is_f32)
+    vosti_launch(embedding_kernel<float>, dim3(count), dim3(128), 0, stream, rows, none, none, (const float*)x, (float*)out, width, x_rows, 1.f, status, (bf16*)nullptr, (int*)nullptr, (unsigned)VOSTI_FAULT_ROW_RANGE);
+  else
+    vosti_launch(embedding_kernel<bf16>, dim3(count), dim3(128), 0, stream, rows, none, none, (const bf16*)x, (bf16*)out, width, x_rows, 1.f, status, (bf16*)nullptr, (int*)nullptr, (unsigned)VOSTI_FAULT_ROW_RANGE);
   VOSTI_LAUNCH_CHECK();
 }
 
@@ -91,9 +104,9 @@ VOSTI_API int vosti_embedding_stream(const int* ids, const int* source, const in
   VOSTI_REQUIRE(tokens >= 0 && hidden > 0 && vocab > 0, "embedding: bad sizes T=%d H=%d V=%d", tokens, hidden, vocab);
   if (tokens == 0) return VOSTI_OK;
   if (is_f32)
-    vosti_launch(embedding_kernel<float, float>, dim3(tokens), dim3(128), 0, stream, ids, source, values, (const float*)table, out, hidden, vocab, scale, status, (bf16*)rounded, resolved);
+    vosti_launch(embedding_kernel<float, float>, dim3(tokens), dim3(128), 0, stream, ids, source, values, (const float*)table, out, hidden, vocab, scale, status, (bf16*)rounded, resolved, (unsigned)VOSTI_FAULT_TOKEN_RANGE);
   else
-    vosti_launch(embedding_kernel<bf16, float>, dim3(tokens), dim3(128), 0, stream, ids, source, values, (const bf16*)table, out, hidden, vocab, scale, status, (bf16*)rounded, resolved);
+    vosti_launch(embedding_kernel<bf16, float>, dim3(tokens), dim3(128), 0, stream, ids, source, values, (const bf16*)table, out, hidden, vocab, scale, status, (bf16*)rounded, resolved, (unsigned)VOSTI_FAULT_TOKEN_RANGE);
   VOSTI_LAUNCH_CHECK();
 }
 

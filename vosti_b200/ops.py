@@ -633,7 +633,11 @@ def hint_prefetch(w, limit: Optional[int] = None) -> bool:
 
 def gather_rows(x: torch.Tensor, rows: torch.Tensor, status: torch.Tensor) -> torch.Tensor:
     """x[rows] for int32 row indices (the embedding kernel over an activation matrix)."""
-    return embedding(rows, x, status)
+    _contig(rows, x)
+    out = torch.empty((rows.shape[0], x.shape[1]), dtype=x.dtype, device=x.device)
+    _check(library().vosti_gather_rows(_p(rows), _p(x), _p(out), rows.shape[0], x.shape[1], x.shape[0], _is_f32(x), _p(status), _stream()),
+           "gather_rows")
+    return out
 
 
 FIXED_ORDER = False              # set_fixed_order: one order of arithmetic however the work is cut
