@@ -10,11 +10,12 @@
 // sampler of the step before left on the device, which the host has not read yet.
 // `scale` multiplies the row in float32 (1: a plain copy), for architectures that scale
 // their embeddings. `resolved` (or null) receives the id every row was taken for. An id that names no row is reported as `fault`.
+// `words`: every operand starts on a 16-byte boundary.
 template <typename T, typename TO = T>
 __global__ void embedding_kernel(const int* __restrict__ ids, const int* __restrict__ source,
                                  const int* __restrict__ values, const T* __restrict__ table,
                                  TO* __restrict__ out, int hidden, int vocab, float scale, unsigned* status,
-                                 bf16* __restrict__ rounded, int* __restrict__ resolved, unsigned fault) {
+                                 bf16* __restrict__ rounded, int* __restrict__ resolved, int words, unsigned fault) {
   pdl_wait();
   pdl_launch_dependents();
   const int t = blockIdx.x;
@@ -29,7 +30,6 @@ __global__ void embedding_kernel(const int* __restrict__ ids, const int* __restr
   TO* dst = out + (int64_t)t * hidden;
   if (resolved != nullptr && threadIdx.x == 0) resolved[t] = id;
   const int bytes = hidden * (int)sizeof(T);
-  const bool words = ((reinterpret_cast<uintptr_t>(table) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(rounded)) & 15) == 0;
   if (sizeof(TO) == 4 && sizeof(T) == 2 && hidden % 8 == 0 && words) {
     // a float32 stream from a bfloat16 table: 16-byte words in, two out, and the row's rounding beside it if asked for
     const uint4* s8 = reinterpret_cast<const uint4*>(src);
@@ -69,6 +69,10 @@ __global__ void embedding_kernel(const int* __restrict__ ids, const int* __restr
   }
 }
 
+static int on_words(const void* a, const void* b, const void* c) {
+  return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15) == 0;
+}
+
 VOSTI_API int vosti_embedding(const int* ids, const int* source, const int* values, const void* table, void* out,
                               int tokens, int hidden, int vocab, int is_f32, float scale, int* resolved, unsigned* status,
                               cudaStream_t stream) {
@@ -76,9 +80,9 @@ VOSTI_API int vosti_embedding(const int* ids, const int* source, const int* valu
                 tokens, hidden, vocab);
   if (tokens == 0) return VOSTI_OK;
   if (is_f32)
-    vosti_launch(embedding_kernel<float>, dim3(tokens), dim3(128), 0, stream, ids, source, values, (const float*)table, (float*)out, hidden, vocab, scale, status, (bf16*)nullptr, resolved, (unsigned)VOSTI_FAULT_TOKEN_RANGE);
+    vosti_launch(embedding_kernel<float>, dim3(tokens), dim3(128), 0, stream, ids, source, values, (const float*)table, (float*)out, hidden, vocab, scale, status, (bf16*)nullptr, resolved, on_words(table, out, nullptr), (unsigned)VOSTI_FAULT_TOKEN_RANGE);
   else
-    vosti_launch(embedding_kernel<bf16>, dim3(tokens), dim3(128), 0, stream, ids, source, values, (const bf16*)table, (bf16*)out, hidden, vocab, scale, status, (bf16*)nullptr, resolved, (unsigned)VOSTI_FAULT_TOKEN_RANGE);
+    vosti_launch(embedding_kernel<bf16>, dim3(tokens), dim3(128), 0, stream, ids, source, values, (const bf16*)table, (bf16*)out, hidden, vocab, scale, status, (bf16*)nullptr, resolved, on_words(table, out, nullptr), (unsigned)VOSTI_FAULT_TOKEN_RANGE);
   VOSTI_LAUNCH_CHECK();
 }
 
@@ -89,9 +93,9 @@ VOSTI_API int vosti_gather_rows(const int* rows, const void* x, void* out, int c
   if (count == 0) return VOSTI_OK;
   const int* const none = nullptr;
   if (is_f32)
-    vosti_launch(embedding_kernel<float>, dim3(count), dim3(128), 0, stream, rows, none, none, (const float*)x, (float*)out, width, x_rows, 1.f, status, (bf16*)nullptr, (int*)nullptr, (unsigned)VOSTI_FAULT_ROW_RANGE);
+    vosti_launch(embedding_kernel<float>, dim3(count), dim3(128), 0, stream, rows, none, none, (const float*)x, (float*)out, width, x_rows, 1.f, status, (bf16*)nullptr, (int*)nullptr, on_words(x, out, nullptr), (unsigned)VOSTI_FAULT_ROW_RANGE);
   else
-    vosti_launch(embedding_kernel<bf16>, dim3(count), dim3(128), 0, stream, rows, none, none, (const bf16*)x, (bf16*)out, width, x_rows, 1.f, status, (bf16*)nullptr, (int*)nullptr, (unsigned)VOSTI_FAULT_ROW_RANGE);
+    vosti_launch(embedding_kernel<bf16>, dim3(count), dim3(128), 0, stream, rows, none, none, (const bf16*)x, (bf16*)out, width, x_rows, 1.f, status, (bf16*)nullptr, (int*)nullptr, on_words(x, out, nullptr), (unsigned)VOSTI_FAULT_ROW_RANGE);
   VOSTI_LAUNCH_CHECK();
 }
 
@@ -104,9 +108,9 @@ VOSTI_API int vosti_embedding_stream(const int* ids, const int* source, const in
   VOSTI_REQUIRE(tokens >= 0 && hidden > 0 && vocab > 0, "embedding: bad sizes T=%d H=%d V=%d", tokens, hidden, vocab);
   if (tokens == 0) return VOSTI_OK;
   if (is_f32)
-    vosti_launch(embedding_kernel<float, float>, dim3(tokens), dim3(128), 0, stream, ids, source, values, (const float*)table, out, hidden, vocab, scale, status, (bf16*)rounded, resolved, (unsigned)VOSTI_FAULT_TOKEN_RANGE);
+    vosti_launch(embedding_kernel<float, float>, dim3(tokens), dim3(128), 0, stream, ids, source, values, (const float*)table, out, hidden, vocab, scale, status, (bf16*)rounded, resolved, on_words(table, out, rounded), (unsigned)VOSTI_FAULT_TOKEN_RANGE);
   else
-    vosti_launch(embedding_kernel<bf16, float>, dim3(tokens), dim3(128), 0, stream, ids, source, values, (const bf16*)table, out, hidden, vocab, scale, status, (bf16*)rounded, resolved, (unsigned)VOSTI_FAULT_TOKEN_RANGE);
+    vosti_launch(embedding_kernel<bf16, float>, dim3(tokens), dim3(128), 0, stream, ids, source, values, (const bf16*)table, out, hidden, vocab, scale, status, (bf16*)rounded, resolved, on_words(table, out, rounded), (unsigned)VOSTI_FAULT_TOKEN_RANGE);
   VOSTI_LAUNCH_CHECK();
 }
 
